@@ -94,6 +94,11 @@ int32_t nyb200_set_fusion(nyb200_engine *e, int32_t on);
  * smaller than the terms it is made of -- the batch is evaluated again with binary64 contractions before
  * results are returned, so the returned bounds stay within the parity tolerance of the reference's
  * binary64 CPU path.  Default 5e-5; 0 disables the re-run (bounds remain sound, only looser).
+ * One thing no precision settles: where no slopes are given, an unstable neuron takes the lower line of slope 1 if u > -l
+ * and of slope 0 otherwise, and at a tie (l + u within the rounding of the interval pass) another arithmetic may take the
+ * other line.  Both are sound; single bounds of such a domain then differ by up to a percent, and it is not flagged.  The
+ * choices of batches of 64 domains and more are those of the interval pass in TF32 pairs, whatever form the backward
+ * pass takes, and those of smaller batches the binary64 ones.
  * nyb200_batch_refined reports how many domains of the last run were evaluated with binary64 contractions because of
  * it (0 = fast path only; a batch of a few domains is evaluated that way as a whole, where that is the faster path). */
 int32_t nyb200_set_refine_tolerance(nyb200_engine *e, float tol);

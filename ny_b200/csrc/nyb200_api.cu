@@ -49,7 +49,7 @@ void free_net(Net &net) {
     for (auto *v : {&net.umma, &net.umma_fwd, &net.umma_adj})
         for (auto &u : *v) { cudaFree(u.wh); cudaFree(u.wl); cudaFree(u.f16); }
     for (float *p : net.wt) cudaFree(p);
-    for (auto *v : {&net.win_bwd, &net.win_fwd, &net.win_pm}) { for (WinOp &o : *v) if (o.block) cudaFree(o.block); v->clear(); }
+    for (auto *v : {&net.win_bwd, &net.win_fwd}) { for (WinOp &o : *v) if (o.block) cudaFree(o.block); v->clear(); }
     if (net.frag_block) cudaFree(net.frag_block);
     net.frag_block = nullptr;
     net.owned.clear(); net.umma.clear(); net.umma_fwd.clear(); net.umma_adj.clear(); net.wt.clear(); net.frag.clear();
@@ -247,7 +247,6 @@ int create_net(nyb200_engine *e, int32_t n_layers, const nyb200_layer_desc *ld, 
             l1 = sum > l1 ? sum : l1;
         }
         net.wmax.push_back(wmin < wmax * 7.450580596923828e-09f ? -wmax : wmax);
-        net.wl1.push_back((float)(l1 * 1.0001));
         // sum over a chunk of 64 of 2^-50 max|a| q_j <= eps |a| * 64 * 2^-50 / eps * (row sum of |W|) max|z|, eps >= 7.1e-7
         net.v.qfl[k] = !conv && net.wmax[k] > 0.f ? (float)(64.0 * kWinFloor / 7.1e-7 * l1 * 1.0001) : 0.f;
         float *dw = nullptr;
@@ -618,7 +617,17 @@ int find_net(nyb200_engine *e, int net_id, Net **out) {
     return NYB200_OK;
 }
 
+// Scratch of one slice of an interval convolution.  Slices that fit in L2 are no faster: their launches fill the SMs less well
+// (residual network, 256 domains: 50.1 ms in whole layers, 52.6 in slices of 192 MB, 53.3 of 64).
+constexpr size_t kConvColsMost = (size_t)4 << 30;
+
 // Interval forward pass for the resident batch.  fwd_mode: 0 clamp-only, 1 constrained, 2 plain IBP.
+// The slope of an unstable neuron's lower line is a step function of its interval (relax_neuron: u > -l), so a bound jumps
+// where a rounding of this pass decides a tie: its products are TF32 pairs, and fp16 pairs, as exact and faster, are for the
+// backward pass alone, where a rounding moves a bound by no more than itself.  (With fp16 pairs here 4096 domains of
+// 784 -> 8x256 -> 10 took 1.19 ms instead of 1.21, 1024 of a convolutional classifier 2.38 instead of 3.09 and 256 of a
+// residual network 41.8 instead of 49.9, and up to three choices of such a batch, 2345 of a small residual network's, were
+// others: single bounds moved by 0.8 %.)
 int run_forward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int fwd_mode) {
     const NetView &nv = net.v;
     int D = b.D;
@@ -633,17 +642,13 @@ int run_forward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int fw
         if (net.umma_fwd.empty()) {
             net.umma_fwd.resize(nv.L);
             for (int k = 1; k < nv.L; ++k) {
-                if (!net.is_conv(k)) NYB_TRY(umma_prepare_forward_layer(e, nv.W[k], nv.dims[k], nv.dims[k + 1], net.wmax[k], &net.umma_fwd[k]));
-                else {
-                    net.win_pm.resize(nv.L);
-                    NYB_TRY(win_prepare(e, nv.W[k], net.wmax[k], net.geom[k], 2, &net.win_pm[k]));
-                    if (!net.win_pm[k].ok) NYB_TRY(prepare_conv_forward_operand(e, nv.W[k], net.geom[k], true, &net.umma_fwd[k]));
-                }
+                if (!net.is_conv(k)) NYB_TRY(umma_prepare_forward_layer(e, nv.W[k], nv.dims[k], nv.dims[k + 1], &net.umma_fwd[k]));
+                else NYB_TRY(prepare_conv_forward_operand(e, nv.W[k], net.geom[k], true, &net.umma_fwd[k]));
             }
         }
         int mo = 0;
         for (int k = 1; k < nv.L; ++k)
-            if (!net.is_conv(k) || net.win_pm[k].ok) mo = nv.dims[k + 1] > mo ? nv.dims[k + 1] : mo;
+            if (!net.is_conv(k)) mo = nv.dims[k + 1] > mo ? nv.dims[k + 1] : mo;
         if (mo == 0) mo = 8;
         ldf = (2 * mo + 7) & ~7;
         Fl = (float *)ws_get(e, "fwd", (size_t)2 * D * ldf * 4);
@@ -651,7 +656,7 @@ int run_forward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int fw
         if (!Fl || !derr) return NYB200_ERR_OOM;
     }
     size_t np = nv.nps;
-    unsigned *zmax_rows = nullptr;   // largest input magnitude of every (layer, domain), reported by the products
+    unsigned *zmax_rows = nullptr;   // largest input magnitude of every (layer, domain), for the charges of fp16 contractions
     if (tensor) {
         zmax_rows = (unsigned *)ws_get(e, "fwd_zmax", (size_t)nv.L * D * 4);
         if (!zmax_rows) return NYB200_ERR_OOM;
@@ -681,37 +686,41 @@ int run_forward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int fw
         if (k == 0) { zl = p.in_lo; zu = p.in_hi; in_ds = b.box_stride; Deff = b.box_stride ? D : 1; }
         else { zl = p.zl + nv.pre_off[k - 1]; zu = p.zu + nv.pre_off[k - 1]; in_ds = (long)np; Deff = D; }
         const bool tk = tensor && k >= 1 && !net.is_conv(k) && net.skip_of(k) < 0;
-        const bool twin = tensor && k >= 1 && net.is_conv(k) && net.win_pm[k].ok;
-        const bool tconv = tensor && k >= 1 && net.is_conv(k) && !twin;
-        unsigned *zmax = nullptr;
-        if (twin) NYB_TRY(conv_win(e, net.win_pm[k], 2 * D, zl, (long)np, Fl, ldf, nullptr, nullptr, 1, &zmax, derr));
-        else if (tk && net.umma_fwd[k].f16) {   // zl rows, then zu rows
-            zmax = zmax_rows + (size_t)k * D;
-            NYB_TRY(launch_umma_f16(e, net.umma_fwd[k], 2 * D, zl, (int)np, Fl, ldf, derr, nullptr, zmax, D));
-        } else if (tk) NYB_TRY(launch_umma(e, net.umma_fwd[k], 2 * D, zl, (int)np, Fl, ldf, derr));
+        const bool tconv = tensor && k >= 1 && net.is_conv(k);
+        // does a contraction through layer i take fp16 pairs, and the products in front of it know nothing of its inputs' size?
+        auto wants_zmax = [&](int i) { return tensor && i >= 1 && i < nv.L && !net.is_conv(i) && net.skip_of(i) < 0 && nv.qfl[i] > 0.f; };
+        if (tk) NYB_TRY(launch_umma(e, net.umma_fwd[k], 2 * D, zl, (int)np, Fl, ldf, derr));   // zl rows, then zu rows
         else if (tconv) {
-            // per-pixel products of the lower-end rows, then the upper-end rows, with [W+ | W-]; then the gather
+            // per-pixel products of the lower-end rows, then the upper-end rows, with [W+ | W-]; then the gather.  Slices of
+            // domains bound the product space, which grows with the batch.
             const ConvGeom &g = net.geom[k];
             const int plane = g.ih * g.iw, N = 2 * g.oc * g.kh * g.kw;
-            if ((long)2 * D * plane > 0x7fffffffL) return set_err(e, NYB200_ERR_UNSUPPORTED, "batch too large for the convolution's product space");
-            float *cols = (float *)ws_get(e, "conv_cols", (size_t)2 * D * plane * N * 4);
+            const size_t per = (size_t)2 * plane * N * 4;
+            const int most = (int)std::min<size_t>({(size_t)D, std::max<size_t>(1, kConvColsMost / per), 0x7fffffffUL / (2UL * plane)});
+            float *cols = (float *)ws_get(e, "conv_cols", (size_t)most * per);
             if (!cols) return NYB200_ERR_OOM;
-            NYB_TRY(launch_umma(e, net.umma_fwd[k], 2 * D * plane, zl, (int)np, cols, N, derr, plane));
-            launch_ibp_conv_gather(e, nv, g, k, D, cols, umma_eps(g.ic, 1) * 1.000001, p.raw_lo, p.raw_hi, p.q, (long)np);
+            for (int d0 = 0; d0 < D; d0 += most) {
+                const int n = std::min(most, D - d0);
+                const size_t at = (size_t)d0 * np;
+                if (n == D) NYB_TRY(launch_umma(e, net.umma_fwd[k], 2 * D * plane, zl, (int)np, cols, N, derr, plane));
+                else {
+                    NYB_TRY(launch_umma(e, net.umma_fwd[k], n * plane, zl + at, (int)np, cols, N, derr, plane));
+                    NYB_TRY(launch_umma(e, net.umma_fwd[k], n * plane, zu + at, (int)np, cols + (size_t)n * plane * N, N, derr, plane));
+                }
+                launch_ibp_conv_gather(e, nv, g, k, n, cols, umma_eps(g.ic, 1) * 1.000001, p.raw_lo + at, p.raw_hi + at, p.q + at, (long)np);
+            }
         }
         else if (net.is_conv(k)) launch_ibp_conv(e, nv, net.geom[k], k, Deff, zl, zu, in_ds, p.raw_lo, p.raw_hi, p.q, (long)np);
         else launch_ibp_linear(e, nv, k, Deff, zl, zu, in_ds, p.raw_lo, p.raw_hi, p.q, (long)np);
         long raw_ds = (Deff == 1 && D > 1) ? 0 : (long)np;
-        if (net.skip_of(k) >= 0 && !twin)  // pre_k = W z + b + relu(pre_j): interval sum, outward
+        if (net.skip_of(k) >= 0)  // pre_k = W z + b + relu(pre_j): interval sum, outward
             launch_skip_interval(e, D, nv.dims[k + 1], (long)np, p.raw_lo, p.raw_hi, nv.pre_off[k], p.zl, p.zu,
                                  nv.pre_off[net.skip_of(k)]);
         launch_ibp_finish(e, nv, k, D, fwd_mode, p.raw_lo, p.raw_hi, raw_ds, fwd_mode >= 2 ? nullptr : p.inh_lo,
                           fwd_mode >= 2 ? nullptr : p.inh_hi, (long)b.inh_stride, p.code, p.sbeta, b.has_alpha ? p.alpha : nullptr, p.pre_lo,
-                          p.pre_hi, p.zl, p.zu, p.tab, p.zabs, p.flags, tk || twin ? Fl : nullptr, ldf,
-                          twin ? win_eps(net.win_pm[k]) : tk ? layer_eps(net.umma_fwd[k], nv.dims[k]) * 1.000001 : 0.0, p.q, tk ? fwd_tol : 0.f, cj,
-                          cj ? chain_cj_eps(net, nv.L, k) : 0.f, chain_kappa(), twin ? zmax + D : zmax,
-                          zmax ? 2.0 * kWinFloor * (double)net.wl1[k] : 0.0,
-                          twin && net.skip_of(k) >= 0 ? nv.pre_off[net.skip_of(k)] : -1);
+                          p.pre_hi, p.zl, p.zu, p.tab, p.zabs, p.flags, tk ? Fl : nullptr, ldf,
+                          tk ? umma_eps(nv.dims[k], 1) * 1.000001 : 0.0, p.q, tk ? fwd_tol : 0.f, cj, cj ? chain_cj_eps(net, nv.L, k) : 0.f, chain_kappa(),
+                          wants_zmax(k) ? zmax_rows + (size_t)k * D : nullptr, wants_zmax(k + 1) ? zmax_rows + (size_t)(k + 1) * D : nullptr);
     }
     NYB_CUDA(e, cudaGetLastError());
     return NYB200_OK;
@@ -849,7 +858,7 @@ int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float
             NYB_WS(qsum, float *, e, "win_qsum", (size_t)D * 4);
             const bool one = q_ds(k) == 0;
             NYB_TRY(launch_sum_weights(e, one ? 1 : D, K, p.q + nv.pre_off[k], np, qsum));
-            NYB_TRY(conv_win(e, net.win_bwd[k], M, cur, p.lda, dst, ldd, p.rpen, qsum, one ? M : R, nullptr, derr));
+            NYB_TRY(conv_win(e, net.win_bwd[k], M, cur, p.lda, dst, ldd, p.rpen, qsum, one ? M : R, derr));
         } else if (net.is_conv(k) && tensor) {
             // reshape (implicit: channel-strided operand) + GEMM with W_col on the tensor cores + col2im gather
             const ConvGeom &g = net.geom[k];

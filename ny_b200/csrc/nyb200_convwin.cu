@@ -1,5 +1,5 @@
 // Convolutions on the tensor cores as windows over an image (implicit GEMM): the transposed convolution of coefficient
-// rows (CROWN backward), the interval convolution's products, the attack's forward and gradient convolutions.  For every
+// rows (CROWN backward), the attack's and the optimisation's forward and gradient convolutions.  For every
 // output pixel, out[n] = sum over taps and channels of in[pixel shifted by the tap][c] * W[tap][c][n].
 //
 // What it replaces wrote the products of every pixel with every tap to memory and gathered them again (a residual layer
@@ -370,9 +370,8 @@ k_split_image(int C, int plane, int Cp, const float *__restrict__ A, long lda, c
 }
 
 // Weights of a window operand: [part][tap][n_blocks * Nb][Cp] fp16, high parts then low parts, zero padded.  sel: how a
-// (tap, channel c, column n) maps to W_col [oc x ic*kh*kw]: 0 transposed (c = oc, n = input channel and stride parity), 1 forward (c = ic, n = oc),
-// 2 forward with the positive parts in columns [0, oc) and the negative ones in [oc, 2 oc).  tap_index: tap -> ky*kw+kx; for sel 0 per
-// parity (py, px), -1 where the tap does not reach it.
+// (tap, channel c, column n) maps to W_col [oc x ic*kh*kw]: 0 transposed (c = oc, n = input channel and stride parity), 1 forward (c = ic, n = oc).
+// tap_index: tap -> ky*kw+kx; for sel 0 per parity (py, px), -1 where the tap does not reach it.
 __global__ void k_win_weights(const float *__restrict__ W, int oc, int ic, int kk, int taps, const int *__restrict__ tap_index, int sel, int st, int NN,
                               int Cp, float scale, __half *__restrict__ out) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x, n_el = (long)taps * NN * Cp;
@@ -384,11 +383,7 @@ __global__ void k_win_weights(const float *__restrict__ W, int oc, int ic, int k
         const int px = n % st, ci = (n / st) % ic, py = n / (st * ic);
         const int kt = py < st ? tap_index[(py * st + px) * taps + tap] : -1;
         if (c < oc && kt >= 0) w = W[((long)c * ic + ci) * kk + kt];
-    } else if (sel == 1) { if (c < ic && n < oc) w = W[((long)n * ic + c) * kk + k]; }
-    else if (c < ic && n < 2 * oc) {
-        w = W[((long)(n % oc) * ic + c) * kk + k];
-        w = n < oc ? fmaxf(w, 0.f) : fminf(w, 0.f);
-    }
+    } else if (c < ic && n < oc) w = W[((long)n * ic + c) * kk + k];
     w *= scale;
     const __half h = __float2half_rn(w);
     out[t] = h;
@@ -445,7 +440,7 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
     const int s = g.sh;
     if (g.sh != g.sw || s > 4 || !(wmax > 0.f) || !std::isfinite(wmax)) return NYB200_OK;
     const int Cin = kind == 0 ? g.oc : g.ic;
-    P.N = kind == 0 ? g.ic : kind == 1 ? g.oc : 2 * g.oc;
+    P.N = kind == 0 ? g.ic : g.oc;
     P.Cp = Cin <= 16 ? 16 : Cin <= 32 ? 32 : (Cin + 63) / 64 * 64;
     P.sw = std::min(P.Cp, 64) * 2;
     P.swa = P.Cp <= 32 ? P.Cp * 4 : 128;   // high and low parts side by side, or one of them
@@ -591,8 +586,7 @@ int launch_win(nyb200_engine *e, const WinOp &op, int rows, const void *hi, cons
 
 // A whole convolution of fp32 rows A [rows x lda] (channel planes) into out [rows x ldo]: row magnitudes, split, window
 // products.  rpen / q_sum / R: see k_split_image (null where nothing is certified).
-int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long lda, float *out, long ldo, double *rpen, const float *q_sum, int R,
-             unsigned **row_max_out, int *err) {
+int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long lda, float *out, long ldo, double *rpen, const float *q_sum, int R, int *err) {
     const Params &P = *(const Params *)op.params;
     const int plane = op.in_h * op.in_w;
     const size_t n = (size_t)rows * plane * P.Cp;
@@ -606,7 +600,6 @@ int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long l
     NYB_CUDA(e, launch_pdl(k_split_image, dim3((unsigned)rows, (unsigned)((plane + 31) / 32)), dim3(256), (size_t)64 * (P.Cp / 2 + 1) * 4, e, op.in_c, plane,
                            P.Cp, A, lda, (const unsigned *)words, hi, lo, row_inv, rpen, q_sum, R));
     e->launches += 2;
-    if (row_max_out) *row_max_out = words;
     return launch_win(e, op, rows, hi, lo, row_inv, out, ldo, nullptr, err);
 }
 

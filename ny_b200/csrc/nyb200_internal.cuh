@@ -93,8 +93,7 @@ struct Net {
     std::vector<float *> wt;          // W_k^T, row-major [dims[k] x dims[k+1]] (adjoint pass; built on first use)
     std::vector<UmmaLayer> umma_adj;  // tcgen05 operands of the adjoint pass (from wt)
     std::vector<float> wmax;          // per layer: largest |weight|; negative when some weight is too small beside it for fp16 pairs
-    std::vector<float> wl1;           // per layer: largest row sum of |weight| (one output's weights)
-    std::vector<WinOp> win_bwd, win_fwd, win_pm;   // window forms of the convolution layers (built on first use)
+    std::vector<WinOp> win_bwd, win_fwd;   // window forms of the convolution layers (built on first use)
     void *frag_block = nullptr;
     std::vector<float *> frag;        // into frag_block: weights in binary64-fragment order (nyb200_direct.cu; built on first use)
 };
@@ -260,7 +259,7 @@ void launch_ibp_finish(nyb200_engine *e, const NetView &nv, int k, int D, int mo
                        float *zl, float *zu, float4 *tab, float *zabs, int *flags, const float *F = nullptr, int ldf = 0,
                        double eps = 0.0, float *q = nullptr, float fwd_tol = 0.f,
                        float *cj = nullptr, float cj_eps = 0.f, float cj_kappa = 0.f,
-                       const unsigned *zmax = nullptr, double floor_rate = 0.0, int skip_off = -1);
+                       const unsigned *zmax = nullptr, unsigned *zmax_next = nullptr);
 void launch_seed(nyb200_engine *e, const float *spec, int S, int nL, int D, int lda, float *A);
 // A [D*2n x lda] = per domain the n x n identity for the lower rows, then again for the upper rows.
 void launch_seed_identity(nyb200_engine *e, int n, int D, int lda, float *A);
@@ -414,8 +413,7 @@ void launch_conv_plain(nyb200_engine *e, const ConvGeom &g, int rows, const floa
 constexpr double kWinFloor = 8.8817841970012523e-16;   // 2^-50: error of a vanishing element, of its row's largest magnitude
 double win_eps(const WinOp &op);
 int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g, int kind, WinOp *out);
-int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long lda, float *out, long ldo, double *rpen, const float *q_sum, int R,
-             unsigned **row_max_out, int *err);
+int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long lda, float *out, long ldo, double *rpen, const float *q_sum, int R, int *err);
 int launch_sum_weights(nyb200_engine *e, int D, int n, const float *q, long stride, float *q_sum);
 
 // ---- tcgen05 contraction (nyb200_umma.cu) ----
@@ -424,10 +422,9 @@ int umma_prepare_layer(nyb200_engine *e, const float *W, int K, int N, UmmaLayer
 // k at A[m * lda + k * a_plane + p], result column n at C[(m * N + n) * a_plane + p] (ldc unused).
 int launch_umma(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err,
                 int a_plane = 0, const ConcFuse *cf = nullptr);
-// The same on fp16 operand pairs (nyb200_umma16.cu).  row_max (optional): largest magnitude of the rows from row_from on.
+// The same on fp16 operand pairs (nyb200_umma16.cu).
 int umma_prepare_f16(nyb200_engine *e, const float *W, int K, int N, float wmax, UmmaLayer *out);
-int launch_umma_f16(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err, const ConcFuse *cf = nullptr,
-                    unsigned *row_max = nullptr, int row_from = 0);
+int launch_umma_f16(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err, const ConcFuse *cf = nullptr);
 double f16_eps(int K);
 int f16_segments(int K);   // K segments that even the largest batch is cut into
 void launch_concretize_fused(nyb200_engine *e, int M, int R, int S, int slots, const double *part, const int *bad,
@@ -436,6 +433,6 @@ void launch_concretize_fused(nyb200_engine *e, int M, int R, int S, int slots, c
 double umma_eps(int K, int chain = 0);
 inline double layer_eps(const UmmaLayer &L, int K) { return L.f16 ? f16_eps(K) : umma_eps(K, L.chain); }
 // Builds the forward-pass operand of Linear_k: the [n_in x 2 n_out] matrix (W+^T | W-^T).
-int umma_prepare_forward_layer(nyb200_engine *e, const float *W, int n_in, int n_out, float wmax, UmmaLayer *out);
+int umma_prepare_forward_layer(nyb200_engine *e, const float *W, int n_in, int n_out, UmmaLayer *out);
 
 }  // namespace nyb

@@ -221,12 +221,13 @@ __global__ void k_ibp_finish(NetView nv, int k, int D, int mode, int last, const
                              float *__restrict__ zu, float4 *__restrict__ tab, float *__restrict__ zabs,
                              int *__restrict__ flags, const float *__restrict__ F, int ldf, double eps,
                              float *__restrict__ q, float fwd_tol, float *__restrict__ cj, float cj_eps, float cj_kappa,
-                             const unsigned *__restrict__ zmax, double floor_rate, int skip_off, double inv_rel) {
+                             const unsigned *__restrict__ zmax, unsigned *__restrict__ zmax_next, double inv_rel) {
     pdl_trigger();
     pdl_wait();
     int n = nv.dims[k + 1], off = nv.pre_off[k];
     long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long total = (long)D * n;
+    const unsigned here = __ballot_sync(0xffffffffu, t < total);
     if (t >= total) return;
     const int d = total <= 0xffffffffL ? (int)((unsigned)t / (unsigned)n) : (int)(t / n), j = (int)(t - (long)d * n);
     long o = (long)d * nv.nps + off + j;
@@ -241,16 +242,10 @@ __global__ void k_ibp_finish(NetView nv, int k, int D, int mode, int last, const
         double b = nv.b[k] ? (double)nv.b[k][j] : 0.0;
         double qq = (fabs(pu) + fabs(nu)) * inv_rel;
         double slack = eps * qq + 2.3e-16 * (qq + fabs(b));
-        // window products: what the smallest intervals of the row lose to fp16's exponent range (zmax: its largest end)
-        if (zmax) slack += floor_rate * (double)__uint_as_float(zmax[d]) + 1e-37;
         l = __double2float_rd(pl + nu + b - slack);
         u = __double2float_ru(pu + nl + b + slack);
-        if (skip_off >= 0) {   // pre_k = W z + b + relu(pre_j): interval sum, outward
-            l = __fadd_rd(l, zl[(long)d * nv.nps + skip_off + j]);
-            u = __fadd_ru(u, zu[(long)d * nv.nps + skip_off + j]);
-        }
         if (isnan(l) || isnan(u)) { l = -INFINITY; u = INFINITY; }
-        // (qfl: what the contraction through this layer loses to the exponent range)
+        // (qfl: what the contraction through this layer loses to fp16's exponent range; zmax: its input's largest magnitude)
         q[o] = __double2float_ru(qq + (zmax ? (double)nv.qfl[k] * (double)__uint_as_float(zmax[d]) : 0.0));
         // The slack widens the interval; where that is visible against the width of an unstable neuron the
         // relaxation built from it (and everything downstream) is visibly looser than the binary64 pass's:
@@ -282,6 +277,13 @@ __global__ void k_ibp_finish(NetView nv, int k, int D, int mode, int last, const
     zabs[o] = za;
     if (cj) cj[o] = __fmaf_ru(1.9073487e-7f /* 1.6 * 2^-23 */ + cj_kappa * 1.001f, za, cw);
     zl[o] = pl; zu[o] = pu;
+    if (zmax_next) {   // the domain's largest post-activation end: one atomic per warp where its neurons are one domain's
+        const unsigned m = __float_as_uint(fmaxf(fabsf(pl), fabsf(pu)));
+        if (__all_sync(here, d == __shfl_sync(here, d, 0))) {
+            const unsigned w = __reduce_max_sync(here, m);
+            if ((threadIdx.x & 31) == 0) atomicMax(&zmax_next[d], w);
+        } else atomicMax(&zmax_next[d], m);
+    }
 }
 
 // ---------------------------------------------------------------- seed
@@ -907,12 +909,12 @@ void launch_ibp_finish(nyb200_engine *e, const NetView &nv, int k, int D, int mo
                        const float *raw_hi, long raw_dstride, const float *inh_lo, const float *inh_hi, long inh_dstride,
                        const signed char *code, const float *sbeta, const float *alpha, float *pre_lo, float *pre_hi,
                        float *zl, float *zu, float4 *tab, float *zabs, int *flags, const float *F, int ldf, double eps,
-                       float *q, float fwd_tol, float *cj, float cj_eps, float cj_kappa, const unsigned *zmax, double floor_rate, int skip_off) {
+                       float *q, float fwd_tol, float *cj, float cj_eps, float cj_kappa, const unsigned *zmax, unsigned *zmax_next) {
     long total = (long)D * nv.dims[k + 1];
     int last = (k == nv.L - 1);
     launch_pdl(k_ibp_finish, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, e, nv, k, D, mode, last, raw_lo, raw_hi,
                raw_dstride, inh_lo, inh_hi, inh_dstride, code, sbeta, alpha, pre_lo, pre_hi, zl, zu, tab, zabs, flags, F, ldf, eps, q, fwd_tol, cj,
-               cj_eps, cj_kappa, zmax, floor_rate, skip_off, 1.0 / (1.0 - 2.0 * eps) * (1.0 + 1e-15));
+               cj_eps, cj_kappa, zmax, zmax_next, 1.0 / (1.0 - 2.0 * eps) * (1.0 + 1e-15));
     NYB_COUNT(e);
 }
 

@@ -307,7 +307,7 @@ int prepare_transposed(nyb200_engine *e, Net &net, bool tensor) {
 
 // out[rows x oc*oh*ow] = convolution k of the rows of Z (no bias), on the tensor path: per-pixel products, gather.
 int conv_forward_tensor(nyb200_engine *e, Net &net, int k, int rows, const float *Z, int ldz, float *out, int ldo, int *derr) {
-    if (net.win_fwd[k].ok) return conv_win(e, net.win_fwd[k], rows, Z, ldz, out, ldo, nullptr, nullptr, 1, nullptr, derr);
+    if (net.win_fwd[k].ok) return conv_win(e, net.win_fwd[k], rows, Z, ldz, out, ldo, nullptr, nullptr, 1, derr);
     const ConvGeom &g = net.geom[k];
     const int plane = g.ih * g.iw, N = g.oc * g.kh * g.kw;
     if ((long)rows * plane > 0x7fffffffL) return set_err(e, NYB200_ERR_UNSUPPORTED, "batch too large for the convolution's product space");

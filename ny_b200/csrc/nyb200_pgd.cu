@@ -200,7 +200,7 @@ static int pgd_backward(nyb200_engine *e, Net &net, bool tensor, int K, float *G
             open_grad.push_back({gstash, net.skip_of(k)});
         }
         if (net.is_conv(k) && tensor && net.win_bwd[k].ok) {
-            NYB_TRY(conv_win(e, net.win_bwd[k], K, g, ld, gn, ld, nullptr, nullptr, 1, nullptr, derr));
+            NYB_TRY(conv_win(e, net.win_bwd[k], K, g, ld, gn, ld, nullptr, nullptr, 1, derr));
         } else if (net.is_conv(k) && tensor) {
             const ConvGeom &cg = net.geom[k];
             const int plane = cg.oh * cg.ow, taps = cg.ic * cg.kh * cg.kw;

@@ -528,13 +528,13 @@ __global__ void k_build_wpm(const float *__restrict__ W, int n_in, int n_out, fl
     out[t] = (n < n_out) ? fmaxf(w, 0.f) : fminf(w, 0.f);
 }
 
-int umma_prepare_forward_layer(nyb200_engine *e, const float *W, int n_in, int n_out, float wmax, UmmaLayer *out) {
+int umma_prepare_forward_layer(nyb200_engine *e, const float *W, int n_in, int n_out, UmmaLayer *out) {
     float *tmp = nullptr;
     size_t n = (size_t)n_in * 2 * n_out;
     if (cudaMalloc(&tmp, n * 4) != cudaSuccess) return NYB200_ERR_OOM;
     k_build_wpm<<<(unsigned)((n + 255) / 256), 256, 0, e->stream>>>(W, n_in, n_out, tmp);
     e->launches++;
-    int st = wmax > 0.f ? umma_prepare_f16(e, tmp, n_in, 2 * n_out, wmax, out) : umma_prepare_layer(e, tmp, n_in, 2 * n_out, out);
+    int st = umma_prepare_layer(e, tmp, n_in, 2 * n_out, out);
     // interval products keep one stage per chain: their slack is compared against every unstable neuron's width
     // and compounds through the layers, where the coefficient products' charge is only compared against the bound
     out->chain = 1;

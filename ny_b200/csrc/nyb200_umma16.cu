@@ -60,8 +60,6 @@ struct Params {
     int M, N, K, chunks, segs, per_seg;
     int a_tma, c_tma;             // A and C by TMA, or directly
     float w_inv;
-    unsigned *row_max;            // largest magnitude of rows >= row_from (float bits, cleared by the caller), or null
-    int row_from;
     int *err;
 };
 
@@ -398,7 +396,6 @@ k_umma_f16(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
         for (int t = t_first; t < tiles && !dead; t += t_step) {
             int c0;
             const int nc = chunks_of(t, c0), row_base = row_of(t);
-            const bool report = P.row_max && (t / P.segs) % n_tiles == 0;
             for (int c = 0; c < nc; ++c) {
                 const bool ok = __all_sync(0xffffffffu, P.a_tma ? mbar_wait(smem_u32(&b_raw[s]), ph) : mbar_wait(smem_u32(&b_empty[s]), ph ^ 1));
                 if (!ok) { if (lane == 0) { atomicExch(P.err, 35); *abort_flag = 1; } dead = true; break; }
@@ -438,11 +435,7 @@ k_umma_f16(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                         // infinite m stays infinite, a zero one zero)
                         const unsigned f = (unsigned)min(268 - (int)(__float_as_uint(m) >> 23), 253);
                         const float sc = __uint_as_float(f << 23);
-                        if (l8 == 0) {
-                            sc_row[h * 8 + g * 2] = __uint_as_float((254 - f) << 23);
-                            const int row = row_base + r0 + h * 8 + g * 2;
-                            if (report && row >= P.row_from && row < P.M) atomicMax(P.row_max + row - P.row_from, __float_as_uint(m));
-                        }
+                        if (l8 == 0) sc_row[h * 8 + g * 2] = __uint_as_float((254 - f) << 23);
 #pragma unroll
                         for (int p = 0; p < 2; ++p) {
                             const float4 x = p ? x1 : x0;
@@ -570,14 +563,13 @@ static void pick_tile(int M, int N, int chunks, int sms, bool fixed, int &bn, in
     }
 }
 
-int launch_umma_f16(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err, const ConcFuse *cf,
-                    unsigned *row_max, int row_from) {
+int launch_umma_f16(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err, const ConcFuse *cf) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
     if (e->reserve_sms > 0 && sms > e->reserve_sms + 1) sms -= e->reserve_sms;   // left to a concurrent collective
     f16::Params P;
     P.A = A; P.lda = lda; P.M = M; P.N = L.N; P.K = L.K; P.chunks = (L.K + BK - 1) / BK;
-    P.w_inv = L.w_inv; P.row_max = row_max; P.row_from = row_from; P.err = err;
+    P.w_inv = L.w_inv; P.err = err;
     int bn, segs;
     pick_tile(M, L.N, P.chunks, sms, cf != nullptr, bn, segs);
     if (cf && segs > 1) return set_err(e, NYB200_ERR_INTERNAL, "fused concretisation of a segmented contraction");
