@@ -18,13 +18,17 @@
 //               (no kernel writes weights);
 //   warp 1      the pair's first CTA: issues the products, the whole warp with one elected lane; per chunk Al*Wh + Ah*Wl first,
 //               then Ah*Wh with the accumulator scaled by 2^-11 at its first step (scale-input-d): the cross terms round at
-//               their own magnitude and join exactly.  The second CTA: reports its weight tiles to the first;
+//               their own magnitude and join exactly.  The second CTA: reports its operands, weights and split rows, to the first;
 //   warp 2      owns the tensor memory (two accumulators of BN columns);
 //   warps 4-11  epilogue: thread = one row, BN / 2 columns in registers; results leave by TMA through 4 KB per warp (row
 //               per thread, direct stores took 32 lines per instruction and 10 of a tile's 25 thousand cycles);
 //   warps 12-19 split the fp32 tile in place: eight lanes hold 64 values of a row, whose largest magnitude is three
 //               shuffles, and the parts of a row's 256 bytes lie in the same 256 bytes, so a warp synchronises with itself
 //               alone.  Operands a tensor map cannot describe are loaded directly.
+// Across a pair: split rows and weights are reported to the first CTA by one thread (arrive_first; its memory barrier is on the
+// way of every chunk: the optimisation of 2048 cells takes 45.1 ms with it, 43.4 with an arrival that orders nothing beyond its
+// CTA), drained accumulators by every epilogue warp (arrive_first_relaxed; one thread with a barrier there too: 45.9 ms).
+// The scales an epilogue warp has read go back to its own CTA's splitting warps by a barrier of theirs.
 // A long contraction with few tiles is cut into K segments, each an output of its own, added in a fixed order by
 // k_sum_segments.
 //
@@ -68,13 +72,44 @@ struct Params {
 using namespace umma;
 using namespace f16;
 
-// An arrival at a barrier of the pair's first CTA.  (Scope of the CTA: what the other CTA's products read is ordered by the
-// proxy fence before it; a release to the cluster is a full memory barrier, a thousand cycles per chunk here.)
+// An arrival at a barrier of the pair's first CTA: a release to the cluster, so that what this thread has written or has seen
+// written by its own CTA's warps is ordered before what the first CTA does after the barrier's phase.  It is a full memory
+// barrier; one thread per chunk does it for all warps, which report to a barrier of their own CTA.
 __device__ __forceinline__ void arrive_first(unsigned bar) {
     asm volatile(
         "{\n\t.reg .b32 r;\n\t"
         "mapa.shared::cluster.u32 r, %0, 0;\n\t"
-        "mbarrier.arrive.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar) : "memory");
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar) : "memory");
+}
+// The same for tensor memory alone, which has an order of its own: what was loaded before tcgen05.fence::before_thread_sync and
+// this arrival is out of the accumulator before the products that follow the wait and tcgen05.fence::after_thread_sync.
+__device__ __forceinline__ void arrive_first_relaxed(unsigned bar) {
+    asm volatile(
+        "{\n\t.reg .b32 r;\n\t"
+        "mapa.shared::cluster.u32 r, %0, 0;\n\t"
+        "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar) : "memory");
+}
+// The waits that go with them.
+template <bool ACQUIRE>
+__device__ __forceinline__ bool wait_second(unsigned bar, unsigned parity) {
+    const long long t0 = clock64();
+    for (;;) {
+        unsigned ok;
+        if constexpr (ACQUIRE)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        else
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+        if (clock64() - t0 > WAIT_LIMIT_CYCLES) return false;
+    }
 }
 template <int CG>
 __device__ __forceinline__ void mma_elect(unsigned d, unsigned long long a, unsigned long long b, unsigned idesc, unsigned accumulate) {
@@ -154,18 +189,19 @@ k_umma_f16(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
     float *scales = (float *)(out_base + 8 * OUT_BYTES);
     unsigned long long *bars = (unsigned long long *)(scales + SCALES * BM);
     unsigned long long *b_a = bars, *b_raw = b_a + STAGES, *b_w = b_raw + STAGES, *b_w2 = b_w + STAGES, *b_empty = b_w2 + STAGES,
-                       *b_full = b_empty + STAGES, *b_drained = b_full + 2;
-    unsigned *tmem_slot = (unsigned *)(b_drained + 2);
+                       *b_full = b_empty + STAGES, *b_drained = b_full + 2, *b_scales = b_drained + 2;
+    unsigned *tmem_slot = (unsigned *)(b_scales + SCALES);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = CG == 1 ? 0 : (int)(blockIdx.x & 1);
     pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            mbar_init(smem_u32(&b_a[s]), 8 * CG); mbar_init(smem_u32(&b_raw[s]), 1); mbar_init(smem_u32(&b_w[s]), 1);
+            mbar_init(smem_u32(&b_a[s]), 8); mbar_init(smem_u32(&b_raw[s]), 1); mbar_init(smem_u32(&b_w[s]), 1);
             mbar_init(smem_u32(&b_w2[s]), 1); mbar_init(smem_u32(&b_empty[s]), 1);
         }
         for (int b = 0; b < 2; ++b) { mbar_init(smem_u32(&b_full[b]), 1); mbar_init(smem_u32(&b_drained[b]), 8 * CG); }
+        for (int s = 0; s < SCALES; ++s) mbar_init(smem_u32(&b_scales[s]), 8);
         *abort_flag = 0;
         if (smem_u32(smem) & 1023u) atomicExch(P.err, 38);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -244,9 +280,10 @@ k_umma_f16(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                 const int nc = chunks_of(t, c0);
                 const unsigned idesc = make_idesc_f16(BM * CG, width_of(t));
                 for (int c = 0; c < nc; ++c) {
-                    ok = __all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_drained[buf]), bph));
+                    ok = CG == 1 ? mbar_wait_soon(smem_u32(&b_drained[buf]), bph) : wait_second<false>(smem_u32(&b_drained[buf]), bph);
+                    ok = __all_sync(0xffffffffu, ok);
                     if (!ok) { if (lane == 0) { atomicExch(P.err, 32); *abort_flag = 1; } break; }
-                    ok = mbar_wait_soon(smem_u32(&b_w[s]), ph) && (CG == 1 || mbar_wait_soon(smem_u32(&b_w2[s]), ph)) && mbar_wait_soon(smem_u32(&b_a[s]), ph);
+                    ok = mbar_wait_soon(smem_u32(&b_w[s]), ph) && mbar_wait_soon(smem_u32(&b_a[s]), ph) && (CG == 1 || wait_second<true>(smem_u32(&b_w2[s]), ph));
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) { if (lane == 0) { atomicExch(P.err, 33); *abort_flag = 1; } break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -266,13 +303,13 @@ k_umma_f16(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                 }
             }
         } else if (CG == 2 && warp == 1 && lane == 0) {
-            // ------------------------------------------------------------ the second CTA's weights have arrived
+            // ------------------------------------------------------------ the second CTA's operands are ready
             unsigned s = 0, ph = 0;
             bool ok = true;
             for (int t = t_first; t < tiles && ok && !*abort_flag; t += t_step) {
                 int c0;
                 for (int c = 0, nc = chunks_of(t, c0); c < nc; ++c) {
-                    ok = mbar_wait_soon(smem_u32(&b_w[s]), ph);
+                    ok = mbar_wait_soon(smem_u32(&b_w[s]), ph) && mbar_wait_soon(smem_u32(&b_a[s]), ph);
                     if (!ok) { atomicExch(P.err, 37); *abort_flag = 1; break; }
                     arrive_first(smem_u32(&b_w2[s]));
                     if (++s == STAGES) { s = 0; ph ^= 1; }
@@ -313,7 +350,10 @@ k_umma_f16(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) { if constexpr (CG == 1) mbar_arrive(smem_u32(&b_drained[buf])); else arrive_first(smem_u32(&b_drained[buf])); }
+                if (lane == 0) {
+                    if constexpr (CG == 1) mbar_arrive(smem_u32(&b_drained[buf]));
+                    else { arrive_first_relaxed(smem_u32(&b_drained[buf])); mbar_arrive(smem_u32(&b_scales[slot])); }
+                }
                 if (++slot == SCALES) slot = 0;
                 if ((buf ^= 1) == 0) bph ^= 1;
             }
@@ -391,13 +431,14 @@ k_umma_f16(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
         const int r0 = w * 16 + (rsub & 1) * 4 + (rsub >> 1);
         // byte offsets in the tile: the fp32 values read, the parts written; group g: ^ 32 g, + 256 g; the parts' second box: ^ 64
         const unsigned off_r = r0 * 128 + ((l8 ^ (r0 & 7)) << 4), off_w = r0 * 128 + (((l8 >> 1) ^ (r0 & 7)) << 4) + (l8 & 1) * 8;
-        unsigned s = 0, ph = 0, slot = 0;
+        unsigned s = 0, ph = 0, slot = 0, sph = 1;
         bool dead = false;
         for (int t = t_first; t < tiles && !dead; t += t_step) {
             int c0;
             const int nc = chunks_of(t, c0), row_base = row_of(t);
             for (int c = 0; c < nc; ++c) {
-                const bool ok = __all_sync(0xffffffffu, P.a_tma ? mbar_wait(smem_u32(&b_raw[s]), ph) : mbar_wait(smem_u32(&b_empty[s]), ph ^ 1));
+                const bool ok = __all_sync(0xffffffffu, (P.a_tma ? mbar_wait(smem_u32(&b_raw[s]), ph) : mbar_wait(smem_u32(&b_empty[s]), ph ^ 1)) &&
+                                                            (CG == 1 || mbar_wait(smem_u32(&b_scales[slot]), sph)));
                 if (!ok) { if (lane == 0) { atomicExch(P.err, 35); *abort_flag = 1; } dead = true; break; }
                 unsigned char *ah = smem + s * STAGE;
                 float *sc_row = scales + slot * BM + r0;
@@ -453,9 +494,9 @@ k_umma_f16(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) { if constexpr (CG == 1) mbar_arrive(smem_u32(&b_a[s])); else arrive_first(smem_u32(&b_a[s])); }
+                if (lane == 0) mbar_arrive(smem_u32(&b_a[s]));
                 if (++s == STAGES) { s = 0; ph ^= 1; }
-                if (++slot == SCALES) slot = 0;
+                if (++slot == SCALES) { slot = 0; sph ^= 1; }
             }
         }
     }

@@ -156,3 +156,16 @@ def test_kfsb_reduce_operators_and_fallback():
     assert a == [(0, 3), (0, 4), (0, 1)][bab.kfsb_fallback_index(0, 3)]
     with pytest.raises(ValueError):
         bab.select_fsb(eng, 0, Net, prop, None, None, take, [0], k=3, reduce="median")
+
+
+def test_arrivals_at_another_ctas_barrier_state_their_scope():
+    """An mbarrier arrival orders its thread's writes for its own CTA unless it says otherwise; at the barrier of another CTA of
+    the cluster it has to say `.release.cluster` (or `.relaxed.cluster`, where tensor memory alone is ordered)."""
+    csrc = os.path.join(ROOT, "ny_b200", "csrc")
+    seen = 0
+    for f in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, f)) as h:
+            for m in re.finditer(r"mbarrier\.arrive[.\w]*shared::cluster[.\w]*", h.read()):
+                seen += 1
+                assert re.match(r"mbarrier\.arrive\.(release|relaxed)\.cluster\.", m.group(0)), (f, m.group(0))
+    assert seen
