@@ -42,17 +42,11 @@ void *ws_get(nyb200_engine *e, const char *name, size_t bytes) {
     return p;
 }
 
-// Releases every device allocation a registered network owns (weights, biases, the operands built for the
-// tensor-core passes, the transposed weights of the adjoint pass).
+// Releases every device allocation a registered network owns.
 void free_net(Net &net) {
-    for (float *p : net.owned) cudaFree(p);
-    for (auto *v : {&net.umma, &net.umma_fwd, &net.umma_adj})
-        for (auto &u : *v) { cudaFree(u.wh); cudaFree(u.wl); cudaFree(u.f16); }
-    for (float *p : net.wt) cudaFree(p);
-    for (auto *v : {&net.win_bwd, &net.win_fwd}) { for (WinOp &o : *v) if (o.block) cudaFree(o.block); v->clear(); }
-    if (net.frag_block) cudaFree(net.frag_block);
-    net.frag_block = nullptr;
-    net.owned.clear(); net.umma.clear(); net.umma_fwd.clear(); net.umma_adj.clear(); net.wt.clear(); net.frag.clear();
+    for (void *p : net.owned) cudaFree(p);
+    net.owned.clear(); net.umma.clear(); net.umma_chain.clear(); net.umma_fwd.clear(); net.umma_adj.clear(); net.wt.clear(); net.frag.clear();
+    net.win_bwd.clear(); net.win_fwd.clear(); net.umma_whole = false;
 }
 
 }  // namespace nyb
@@ -174,6 +168,43 @@ static void expand_bias(const float *b, int oc, int plane, std::vector<float> &o
 
 namespace nyb {
 
+// What create_net asks about a layer's weights: largest magnitude and smallest non-zero one (as bits, the latter as its
+// distance from infinity, so that zeroed words are the start of both), largest sum of magnitudes of a row (binary64 bits).
+struct LayerStats { unsigned long long l1_bits; unsigned max_bits, inv_min_bits; };
+struct LayerRows { const float *W[kMaxLinear]; int n[kMaxLinear], len[kMaxLinear]; };
+
+static float bits_float(unsigned b) { float f; memcpy(&f, &b, 4); return f; }
+
+// One block per row (grid x) of every layer (grid y).  A walk over all weights in one dependent binary64 sum on the host took
+// two milliseconds for a network of 0.7 million.
+__global__ void __launch_bounds__(256) k_layer_stats(LayerRows rows, LayerStats *__restrict__ out) {
+    const int k = blockIdx.y;
+    if ((int)blockIdx.x >= rows.n[k]) return;
+    const float *w = rows.W[k] + (long)blockIdx.x * rows.len[k];
+    unsigned mx = 0, inv = 0;
+    double sum = 0.0;
+    for (int i = threadIdx.x; i < rows.len[k]; i += 256) {
+        const unsigned b = __float_as_uint(w[i]) & 0x7fffffffu;   // ordered as the magnitudes are, NaN above infinity
+        mx = max(mx, b);
+        if (b > 0 && b < 0x7f800000u) inv = max(inv, 0x7f800000u - b);
+        sum += (double)__uint_as_float(b);
+    }
+    __shared__ double part[8];
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    inv = __reduce_max_sync(0xffffffffu, inv);
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((threadIdx.x & 31) == 0) {
+        part[threadIdx.x >> 5] = sum;
+        atomicMax(&out[k].max_bits, mx);
+        atomicMax(&out[k].inv_min_bits, inv);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 8; ++i) sum += part[i];
+        if (mx < 0x7f800000u) atomicMax(&out[k].l1_bits, (unsigned long long)__double_as_longlong(sum));   // (not of a row with a NaN in it)
+    }
+}
+
 int create_net(nyb200_engine *e, int32_t n_layers, const nyb200_layer_desc *ld, const float *wflat,
                const float *bflat, int32_t *net_id) {
     if (n_layers < 1 || n_layers > kMaxLinear) return set_err(e, NYB200_ERR_UNSUPPORTED, "layer count out of range");
@@ -221,54 +252,74 @@ int create_net(nyb200_engine *e, int32_t n_layers, const nyb200_layer_desc *ld, 
     net.v.pre_off[n_layers] = off;
     net.v.n_pre = off;
     net.v.nps = (off + 3) & ~3;
-    // a failed upload releases what the earlier layers allocated
+    // Weights, biases and the layers' statistics in one block; a failed upload releases it
     struct Guard { Net &n; bool armed = true; ~Guard() { if (armed) free_net(n); } } guard{net};
-    size_t wo = 0, bo = 0;
-    std::vector<float> expanded;
-    for (int k = 0; k < n_layers; ++k) {
+    Carve c;
+    float *bias[kMaxLinear] = {};
+    LayerStats *stats = nullptr;
+    LayerRows rows;
+    auto weights_of = [&](int k) {
         const nyb200_layer_desc &l = ld[k];
-        const bool conv = l.kind == NYB200_LAYER_CONV2D;
-        size_t nw = conv ? (size_t)l.out_channels * l.in_channels * l.kernel_h * l.kernel_w
-                         : (size_t)l.in_features * l.out_features;
-        // largest weight, smallest non-zero one and largest row sum (a fp16 pair holds a weight's 22 bits unless it is more
-        // than 2^27 times smaller than the largest: such a layer keeps its TF32 operands)
-        const size_t row_len = conv ? nw / (size_t)l.out_channels : (size_t)l.in_features;
-        float wmax = 0.f, wmin = INFINITY;
-        double l1 = 0.0;
-        for (size_t r = 0; r < nw; r += row_len) {
-            double sum = 0.0;
-            for (size_t i = r; i < r + row_len; ++i) {
-                const float a = std::fabs(wflat[wo + i]);
-                if (!std::isfinite(a)) return set_err(e, NYB200_ERR_NUMERICAL, "non-finite weight");
-                wmax = a > wmax ? a : wmax;
-                if (a > 0.f && a < wmin) wmin = a;
-                sum += a;
-            }
-            l1 = sum > l1 ? sum : l1;
+        return net.kind[k] == NYB200_LAYER_CONV2D ? (size_t)l.out_channels * l.in_channels * l.kernel_h * l.kernel_w : (size_t)l.in_features * l.out_features;
+    };
+    for (int pass = 0; pass < 2; ++pass) {
+        c.used = 0;
+        int most_rows = 0;
+        for (int k = 0; k < n_layers; ++k) {
+            const size_t nw = weights_of(k);
+            net.v.W[k] = (const float *)c.take(nw * 4);
+            bias[k] = ld[k].has_bias ? (float *)c.take((size_t)ld[k].out_features * 4) : nullptr;
+            net.v.b[k] = bias[k];
+            rows.W[k] = net.v.W[k];
+            rows.n[k] = net.kind[k] == NYB200_LAYER_CONV2D ? ld[k].out_channels : ld[k].out_features;   // one output's weights each
+            rows.len[k] = (int)(nw / (size_t)rows.n[k]);
+            most_rows = std::max(most_rows, rows.n[k]);
         }
-        net.wmax.push_back(wmin < wmax * 7.450580596923828e-09f ? -wmax : wmax);
-        // sum over a chunk of 64 of 2^-50 max|a| q_j <= eps |a| * 64 * 2^-50 / eps * (row sum of |W|) max|z|, eps >= 7.1e-7
-        net.v.qfl[k] = !conv && net.wmax[k] > 0.f ? (float)(64.0 * kWinFloor / 7.1e-7 * l1 * 1.0001) : 0.f;
-        float *dw = nullptr;
-        NYB_CUDA(e, cudaMalloc(&dw, nw * sizeof(float)));
-        net.owned.push_back(dw);
-        NYB_CUDA(e, cudaMemcpy(dw, wflat + wo, nw * sizeof(float), cudaMemcpyHostToDevice));
-        net.v.W[k] = dw;
-        wo += nw;
-        if (l.has_bias) {
+        stats = (LayerStats *)c.take((size_t)n_layers * sizeof(LayerStats));
+        if (pass == 0) {
+            void *block = nullptr;
+            NYB_CUDA(e, cudaMalloc(&block, c.used));
+            net.owned.push_back(block);
+            c.block = (char *)block;
+            continue;
+        }
+        size_t wo = 0, bo = 0;
+        std::vector<float> expanded;
+        for (int k = 0; k < n_layers; ++k) {
+            const nyb200_layer_desc &l = ld[k];
+            const bool conv = l.kind == NYB200_LAYER_CONV2D;
+            const size_t nw = weights_of(k);
+            NYB_CUDA(e, cudaMemcpyAsync(const_cast<float *>(net.v.W[k]), wflat + wo, nw * 4, cudaMemcpyHostToDevice, e->stream));
+            wo += nw;
+            if (!l.has_bias) continue;
             if (!bflat) return set_err(e, NYB200_ERR_INVALID, "has_bias set but bflat is null");
-            size_t nb = conv ? (size_t)l.out_channels : (size_t)l.out_features;
+            const size_t nb = conv ? (size_t)l.out_channels : (size_t)l.out_features;
             for (size_t i = 0; i < nb; ++i)
                 if (!std::isfinite(bflat[bo + i])) return set_err(e, NYB200_ERR_NUMERICAL, "non-finite bias");
             const float *src = bflat + bo;
             if (conv) { expand_bias(bflat + bo, l.out_channels, l.out_h * l.out_w, expanded); src = expanded.data(); }
-            float *db = nullptr;
-            NYB_CUDA(e, cudaMalloc(&db, (size_t)l.out_features * sizeof(float)));
-            net.owned.push_back(db);
-            NYB_CUDA(e, cudaMemcpy(db, src, (size_t)l.out_features * sizeof(float), cudaMemcpyHostToDevice));
-            net.v.b[k] = db;
+            NYB_CUDA(e, cudaMemcpyAsync(bias[k], src, (size_t)l.out_features * 4, cudaMemcpyHostToDevice, e->stream));
+            if (conv) NYB_CUDA(e, cudaStreamSynchronize(e->stream));   // the next layer's bias is expanded in the same place
             bo += nb;
         }
+        NYB_CUDA(e, cudaMemsetAsync(stats, 0, (size_t)n_layers * sizeof(LayerStats), e->stream));
+        k_layer_stats<<<dim3((unsigned)most_rows, (unsigned)n_layers), 256, 0, e->stream>>>(rows, stats);
+        e->launches++;
+        NYB_CUDA(e, cudaGetLastError());
+    }
+    std::vector<LayerStats> ls((size_t)n_layers);
+    NYB_CUDA(e, cudaMemcpyAsync(ls.data(), stats, ls.size() * sizeof(LayerStats), cudaMemcpyDeviceToHost, e->stream));
+    NYB_CUDA(e, cudaStreamSynchronize(e->stream));   // (the caller's arrays may go away, too)
+    for (int k = 0; k < n_layers; ++k) {
+        // a fp16 pair holds a weight's 22 bits unless it is more than 2^27 times smaller than the largest: such a layer keeps
+        // its TF32 operands
+        const float wmax = bits_float(ls[k].max_bits), wmin = bits_float(0x7f800000u - ls[k].inv_min_bits);
+        if (!std::isfinite(wmax)) return set_err(e, NYB200_ERR_NUMERICAL, "non-finite weight");
+        net.wmax.push_back(wmin < wmax * 7.450580596923828e-09f ? -wmax : wmax);
+        // sum over a chunk of 64 of 2^-50 max|a| q_j <= eps |a| * 64 * 2^-50 / eps * (row sum of |W|) max|z|, eps >= 7.1e-7
+        double l1;
+        memcpy(&l1, &ls[k].l1_bits, 8);
+        net.v.qfl[k] = net.kind[k] == NYB200_LAYER_LINEAR && net.wmax[k] > 0.f ? (float)(64.0 * kWinFloor / 7.1e-7 * l1 * 1.0001) : 0.f;
     }
     int id = e->next_net++;
     e->nets[id] = net;
@@ -341,14 +392,17 @@ static int32_t gemm_f32_impl(nyb200_engine *e, int32_t m, int32_t k, int32_t n, 
         NYB_WS(derr, int *, e, "umma_err", 256);
         NYB_CUDA(e, cudaMemsetAsync(derr, 0, 4, e->stream));
         UmmaLayer ul;
-        NYB_TRY(umma_prepare_layer(e, db, k, n, &ul));
+        Carve c;
+        NYB_TRY(umma_prepare_layer(e, WeightSource{db}, k, n, &ul, c));
+        NYB_WS(op, char *, e, "gemm_operand", c.used);
+        c.block = op; c.used = 0;
+        NYB_TRY(umma_prepare_layer(e, WeightSource{db}, k, n, &ul, c));
         int st = launch_umma(e, ul, m, da, k, dc, n, derr);
         int herr = 0;
         cudaError_t cs = cudaGetLastError();
         if (cs == cudaSuccess) cs = cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, e->stream);
         if (cs == cudaSuccess) cs = cudaMemcpyAsync(c_out, dc, (size_t)m * n * 4, cudaMemcpyDeviceToHost, e->stream);
         if (cs == cudaSuccess) cs = cudaStreamSynchronize(e->stream);
-        cudaFree(ul.wh); cudaFree(ul.wl);
         NYB_TRY(st);
         NYB_CUDA(e, cs);
         if (herr) return set_err(e, NYB200_ERR_INTERNAL, "tcgen05 pipeline wait expired (code " + std::to_string(herr) + ")");
@@ -640,11 +694,16 @@ int run_forward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int fw
     int *derr = nullptr;
     if (tensor) {
         if (net.umma_fwd.empty()) {
-            net.umma_fwd.resize(nv.L);
-            for (int k = 1; k < nv.L; ++k) {
-                if (!net.is_conv(k)) NYB_TRY(umma_prepare_forward_layer(e, nv.W[k], nv.dims[k], nv.dims[k + 1], &net.umma_fwd[k]));
-                else NYB_TRY(prepare_conv_forward_operand(e, nv.W[k], net.geom[k], true, &net.umma_fwd[k]));
-            }
+            std::vector<UmmaLayer> fwd((size_t)nv.L);
+            NYB_TRY(build_operands(e, net, [&](Carve &c) -> int {
+                for (int k = 1; k < nv.L; ++k) {
+                    const ConvGeom &g = net.geom[k];
+                    if (!net.is_conv(k)) NYB_TRY(umma_prepare_signed(e, nv.W[k], 1, nv.dims[k], nv.dims[k + 1], &fwd[k], c));
+                    else NYB_TRY(umma_prepare_signed(e, nv.W[k], g.kh * g.kw, g.ic, g.oc, &fwd[k], c));
+                }
+                return NYB200_OK;
+            }));
+            net.umma_fwd = std::move(fwd);
         }
         int mo = 0;
         for (int k = 1; k < nv.L; ++k)
@@ -726,24 +785,35 @@ int run_forward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int fw
     return NYB200_OK;
 }
 
-// tcgen05 operands of the backward products A * W_k (Linear) and of the im2col-space product of a
-// transposed convolution (W_col [oc x ic*kh*kw] is its [K x N] operand).
-int prepare_backward_operands(nyb200_engine *e, Net &net) {
+// Operands of the backward products A * W_k.  chain: what the fused chain and the contraction behind it read (every hidden
+// layer that a chain can start at or pass, as TF32 pairs, and the first layer's own form); otherwise the own form of every
+// layer, a convolution's being its window or the im2col-space operand W_col [oc x ic*kh*kw].
+int prepare_backward_operands(nyb200_engine *e, Net &net, bool chain) {
     const NetView &nv = net.v;
-    if (!net.umma.empty()) return NYB200_OK;
-    net.umma.resize(nv.L);
-    for (int k = 0; k < nv.L; ++k) {
-        if (!net.is_conv(k)) {
-            if (net.wmax[k] > 0.f) NYB_TRY(umma_prepare_f16(e, nv.W[k], nv.dims[k + 1], nv.dims[k], net.wmax[k], &net.umma[k]));
-            if (!(net.wmax[k] > 0.f) || (k > 0 && chain_eligible(net, k + 1)))
-                NYB_TRY(umma_prepare_layer(e, nv.W[k], nv.dims[k + 1], nv.dims[k], &net.umma[k]));
-        } else {
+    if (chain ? !net.umma_chain.empty() : net.umma_whole) return NYB200_OK;
+    std::vector<UmmaLayer> own = net.umma, hidden((size_t)nv.L);
+    std::vector<WinOp> win = net.win_bwd;
+    own.resize(nv.L);
+    win.resize(nv.L);
+    NYB_TRY(build_operands(e, net, [&](Carve &c) -> int {
+        for (int k = 0; k < nv.L; ++k) {
+            const int K = nv.dims[k + 1], N = nv.dims[k];
+            if (chain && k > 0) {
+                if (chain_eligible(net, k + 1)) NYB_TRY(umma_prepare_layer(e, WeightSource{nv.W[k]}, K, N, &hidden[k], c));
+                continue;
+            }
+            if (!net.umma.empty() && net.umma[k].ready()) continue;   // the first layer's, of an earlier set
+            if (!net.is_conv(k)) { NYB_TRY(umma_prepare_own(e, WeightSource{nv.W[k]}, K, N, net.wmax[k], &own[k], c)); continue; }
             const ConvGeom &g = net.geom[k];
-            net.win_bwd.resize(nv.L);
-            NYB_TRY(win_prepare(e, nv.W[k], net.wmax[k], g, 0, &net.win_bwd[k]));
-            if (!net.win_bwd[k].ok) NYB_TRY(umma_prepare_layer(e, nv.W[k], g.oc, g.ic * g.kh * g.kw, &net.umma[k]));
+            NYB_TRY(win_prepare(e, nv.W[k], net.wmax[k], g, 0, &win[k], c));
+            if (!win[k].ok) NYB_TRY(umma_prepare_layer(e, WeightSource{nv.W[k]}, g.oc, g.ic * g.kh * g.kw, &own[k], c));
         }
-    }
+        return NYB200_OK;
+    }));
+    net.umma = std::move(own);
+    net.win_bwd = std::move(win);
+    if (chain) net.umma_chain = std::move(hidden);
+    else net.umma_whole = true;
     return NYB200_OK;
 }
 
@@ -755,16 +825,19 @@ int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float
         NYB_CUDA(e, cudaMemcpyAsync(p.min_lower, clear, sizeof(clear), cudaMemcpyHostToDevice, e->stream));
         return run_backward_direct(e, net, b, p, nullptr, b.D);
     }
-    int *derr = nullptr;
-    if (tensor) {
-        NYB_TRY(prepare_backward_operands(e, net));
-        derr = (int *)ws_get(e, "umma_err", 256);
-        if (!derr) return NYB200_ERR_OOM;
-    }
     // top < 0: the whole network, seeded with the spec rows.  top >= 0: the pass starts at Linear_top's output
     // with one identity row per neuron (b.S = dims[top + 1]): the partial pass of the CROWN-IBP collection.
     const bool partial = top >= 0;
     int D = b.D, S = b.S, R = b.R, L = partial ? top + 1 : nv.L;
+    // Fused chain: seed, identity pass and the contractions L-1 .. 1 with their relaxations run as one kernel that
+    // keeps the rows on the SM; what is left for the loop below is Linear_0's (wide) contraction.
+    const bool fused = tensor && e->fuse_chain && !ckpt && chain_eligible(net, L) && (nv.nps % 4 == 0) && (p.lda % 4 == 0);
+    int *derr = nullptr;
+    if (tensor) {
+        NYB_TRY(prepare_backward_operands(e, net, fused));
+        derr = (int *)ws_get(e, "umma_err", 256);
+        if (!derr) return NYB200_ERR_OOM;
+    }
     int M = D * R;
     long np = nv.nps;
     bool shared_box = (b.box_stride == 0 && D > 1);
@@ -789,9 +862,6 @@ int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float
         const std::string name = slot == 0 ? std::string("skip_coeff") : "skip_coeff_" + std::to_string(slot);
         return (float *)ws_get(e, name.c_str(), (size_t)M * p.lda * 4);
     };
-    // Fused chain: seed, identity pass and the contractions L-1 .. 1 with their relaxations run as one kernel that
-    // keeps the rows on the SM; what is left for the loop below is Linear_0's (wide) contraction.
-    const bool fused = tensor && e->fuse_chain && !ckpt && chain_eligible(net, L) && (nv.nps % 4 == 0) && (p.lda % 4 == 0);
     if (!fused) {
         if (partial) launch_seed_identity(e, S, D, p.lda, cur);
         else launch_seed(e, p.spec, S, nv.dims[L], D, p.lda, cur);

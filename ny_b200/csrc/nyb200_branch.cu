@@ -134,7 +134,7 @@ int babsr_select(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int *
     float *backup = score + (size_t)D * np;
     int *derr = nullptr;
     if (tensor) {
-        NYB_TRY(prepare_backward_operands(e, net));
+        NYB_TRY(prepare_backward_operands(e, net, false));
         derr = (int *)ws_get(e, "umma_err", 256);
         if (!derr) return NYB200_ERR_OOM;
         NYB_CUDA(e, cudaMemsetAsync(derr, 0, 4, e->stream));

@@ -558,8 +558,8 @@ int launch_chain(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int L
     for (int l = 0; l < L - 1; ++l) {
         const int k = L - 1 - l;  // contraction with W_k: K = dims[k + 1], N = dims[k]; then ReLU k-1 and the charges of lin k-1
         Layer &Ly = P.layer[l];
-        memcpy(&Ly.tm_hi, net.umma[k].tm_hi, sizeof(CUtensorMap));
-        memcpy(&Ly.tm_lo, net.umma[k].tm_lo, sizeof(CUtensorMap));
+        memcpy(&Ly.tm_hi, net.umma_chain[k].tm_hi, sizeof(CUtensorMap));
+        memcpy(&Ly.tm_lo, net.umma_chain[k].tm_lo, sizeof(CUtensorMap));
         Ly.K = nv.dims[k + 1]; Ly.N = nv.dims[k];
         Ly.relu_off = nv.pre_off[k - 1];
         Ly.q_ds = (k - 1 == 0 && shared_box) ? 0 : nv.nps;

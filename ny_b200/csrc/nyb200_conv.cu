@@ -333,19 +333,6 @@ k_conv_plain(ConvGeom g, int rows, const float *__restrict__ Z, int ldz, const f
 // (channel-strided operand, tap-major result); only the gather differs.  Any stride is covered (a stride s uses
 // one tap in s*s per pixel; the unused products are wasted tensor work, not traffic that matters here).
 
-// Wf[ci][(co, ky, kx)] = W_col[co][(ci, ky, kx)]; with `split`: [max(W, 0) | min(W, 0)], 2*oc*kk columns.
-__global__ void k_build_conv_fwd(const float *__restrict__ W, int oc, int ic, int kk, int split, float *__restrict__ out) {
-    const int N = (split ? 2 : 1) * oc * kk;
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)ic * N) return;
-    int ci = (int)(t / N), n = (int)(t % N);
-    int neg = n >= oc * kk;
-    int r = n - (neg ? oc * kk : 0);
-    int co = r / kk, tap = r % kk;
-    float w = W[((long)co * ic + ci) * kk + tap];
-    out[t] = split ? (neg ? fminf(w, 0.f) : fmaxf(w, 0.f)) : w;
-}
-
 // Interval convolution from the products of the lower-end rows (m = d) and upper-end rows (m = D + d) of a
 // non-negative input interval with [W+ | W-]: lo = W+ zl + W- zu + b, hi = W+ zu + W- zl + b, q = |W| zu.
 // The taps of an output are summed in binary64; every product carries a rounding of at most eps times the sum of
@@ -410,20 +397,6 @@ k_conv_fwd_gather(ConvGeom g, const float *__restrict__ cols, float *__restrict_
 }
 
 }  // namespace
-
-int prepare_conv_forward_operand(nyb200_engine *e, const float *W, const ConvGeom &g, bool split, UmmaLayer *out) {
-    const int kk = g.kh * g.kw, N = (split ? 2 : 1) * g.oc * kk;
-    float *tmp = nullptr;
-    size_t n = (size_t)g.ic * N;
-    if (cudaMalloc(&tmp, n * 4) != cudaSuccess) return NYB200_ERR_OOM;
-    k_build_conv_fwd<<<(unsigned)((n + 255) / 256), 256, 0, e->stream>>>(W, g.oc, g.ic, kk, split ? 1 : 0, tmp);
-    e->launches++;
-    int st = umma_prepare_layer(e, tmp, g.ic, N, out);
-    if (split) out->chain = 1;  // interval products: see umma_prepare_forward_layer
-    cudaStreamSynchronize(e->stream);
-    cudaFree(tmp);
-    return st;
-}
 
 void launch_ibp_conv_gather(nyb200_engine *e, const NetView &nv, const ConvGeom &g, int k, int D, const float *cols, double eps,
                             float *raw_lo, float *raw_hi, float *q, long out_dstride) {

@@ -432,7 +432,7 @@ double win_eps(const WinOp &op) {
 
 // Window form of a convolution layer (kind: the `sel` of k_win_weights).  Leaves out->ok false where it does not apply:
 // strides over 4, weights that do not fit in shared memory next to three halo tiles.
-int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g, int kind, WinOp *out) {
+int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g, int kind, WinOp *out, Carve &c) {
     out->ok = false;
     static_assert(sizeof(Params) <= sizeof(out->params), "parameter storage");
     Params P;
@@ -521,16 +521,14 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
     P.w_inv = 1.f / scale;
     const int NN = P.n_blocks * P.Nb;
     const size_t n_el = (size_t)P.taps * NN * P.Cp;
-    char *block = nullptr;
-    const size_t wb = (2 * n_el * 2 + 255) / 256 * 256;
-    if (cudaMalloc(&block, wb + tap_index.size() * 4) != cudaSuccess) return set_err(e, NYB200_ERR_OOM, "device allocation failed for a convolution operand");
-    out->block = block;
-    NYB_CUDA(e, cudaMemcpyAsync(block + wb, tap_index.data(), tap_index.size() * 4, cudaMemcpyHostToDevice, e->stream));
-    k_win_weights<<<(unsigned)((n_el + 255) / 256), 256, 0, e->stream>>>(W, g.oc, g.ic, g.kh * g.kw, P.taps, (const int *)(block + wb), kind, s, NN,
-                                                                        P.Cp, scale, (__half *)block);
+    out->ok = true;
+    void *block = c.take(2 * n_el * 2);
+    int *taps_dev = (int *)c.take(tap_index.size() * 4);
+    if (!c.block) return NYB200_OK;
+    NYB_CUDA(e, cudaMemcpyAsync(taps_dev, tap_index.data(), tap_index.size() * 4, cudaMemcpyHostToDevice, e->stream));   // pageable: staged on return
+    k_win_weights<<<(unsigned)((n_el + 255) / 256), 256, 0, e->stream>>>(W, g.oc, g.ic, g.kh * g.kw, P.taps, taps_dev, kind, s, NN, P.Cp, scale,
+                                                                        (__half *)block);
     e->launches++;
-    NYB_CUDA(e, cudaGetLastError());
-    NYB_CUDA(e, cudaStreamSynchronize(e->stream));   // tap_index is a local
     EncodeFn enc = encoder();
     if (!enc) return set_err(e, NYB200_ERR_INTERNAL, "cuTensorMapEncodeTiled unavailable");
     cuuint64_t dims[2] = {(cuuint64_t)P.Cp, (cuuint64_t)2 * P.taps * NN}, strides[1] = {(cuuint64_t)P.Cp * 2};
@@ -540,7 +538,6 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
         return set_err(e, NYB200_ERR_INTERNAL, "cuTensorMapEncodeTiled failed for a convolution operand");
     out->in_h = kind == 0 ? g.oh : g.ih; out->in_w = kind == 0 ? g.ow : g.iw; out->in_c = Cin;
     memcpy(out->params, &P, sizeof(P));
-    out->ok = true;
     return NYB200_OK;
 }
 

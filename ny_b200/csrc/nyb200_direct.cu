@@ -829,23 +829,19 @@ k_pass_table(NetView nv, int boxes, const int *__restrict__ idx, const float4 *_
 int prepare_fragments(nyb200_engine *e, Net &net) {
     const NetView &nv = net.v;
     if (!net.frag.empty()) return NYB200_OK;
-    // one allocation for the network: a device allocation costs more than packing its weights
-    size_t total = 0, at[kMaxLinear];
-    for (int k = 0; k < nv.L; ++k) {
-        at[k] = total;
-        total += (size_t)((nv.dims[k + 1] + 15) / 16) * ((nv.dims[k] + 7) / 8) * 512;
-    }
-    char *p = nullptr;
-    if (cudaMalloc(&p, total) != cudaSuccess) return set_err(e, NYB200_ERR_OOM, "device allocation failed for the fragment-ordered weights");
-    net.frag_block = p;
-    for (int k = 0; k < nv.L; ++k) {
-        const int K = nv.dims[k + 1], N = nv.dims[k], kg = (K + 15) / 16, nt = (N + 7) / 8;
-        const long n = (long)nt * kg * 32;
-        k_pack_fragments<<<(unsigned)((n + 255) / 256), 256, 0, e->stream>>>(nv.W[k], K, N, kg, nt, (float4 *)(p + at[k]));
-        e->launches++;
-        net.frag.push_back((float *)(p + at[k]));
-    }
-    NYB_CUDA(e, cudaStreamSynchronize(e->stream));   // once per network: passes fetch weights ahead of the kernels in front of them
+    std::vector<float *> frag((size_t)nv.L);
+    NYB_TRY(build_operands(e, net, [&](Carve &c) {
+        for (int k = 0; k < nv.L; ++k) {
+            const int K = nv.dims[k + 1], N = nv.dims[k], kg = (K + 15) / 16, nt = (N + 7) / 8;
+            const long n = (long)nt * kg * 32;
+            frag[k] = (float *)c.take((size_t)n * 16);
+            if (!c.block) continue;
+            k_pack_fragments<<<(unsigned)((n + 255) / 256), 256, 0, e->stream>>>(nv.W[k], K, N, kg, nt, (float4 *)frag[k]);
+            e->launches++;
+        }
+        return (int)NYB200_OK;
+    }));
+    net.frag = std::move(frag);
     return NYB200_OK;
 }
 

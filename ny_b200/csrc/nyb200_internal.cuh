@@ -58,8 +58,9 @@ struct ConcFuse {
 };
 
 struct UmmaLayer {
-    float *wh = nullptr, *wl = nullptr;
-    int K = 0, N = 0, kpad = 0;
+    float *wh = nullptr, *wl = nullptr;   // (in a block of the network's, or of the caller's)
+    int K = 0, N = 0;
+    bool ready() const { return wh || f16; }
     int chain = 0;  // K stages per tensor-memory accumulation chain for this operand; 0 = the kernel's default
     alignas(64) unsigned char tm_hi[128];
     alignas(64) unsigned char tm_lo[128];
@@ -72,15 +73,34 @@ struct UmmaLayer {
 // A convolution in window form (nyb200_convwin.cu): its fp16 weights, their tensor map and the kernel's parameters.
 struct WinOp {
     bool ok = false;
-    void *block = nullptr;
     int in_h = 0, in_w = 0, in_c = 0;
     alignas(64) unsigned char tm_w[128];
     alignas(8) unsigned char params[1280];
 };
 
+// One device block cut into pieces.  Operand sets are built by a function that runs twice: with no block it adds up what it
+// will take, with one it fills it (build_operands).
+struct Carve {
+    char *block = nullptr;
+    size_t used = 0;
+    void *take(size_t bytes) {
+        void *p = block ? block + used : nullptr;
+        used += (bytes + 255) & ~(size_t)255;
+        return p;
+    }
+};
+
+// Where the element (k, n) of a [K x N] operand comes from: taps 0: row-major W [K x N].  Otherwise W [outputs x K x taps]
+// (taps 1: the transpose of a layer's weights; more: a convolution's products of one pixel), n = output * taps + tap; with
+// `split` the positive parts of that in the first half of the columns, the negative ones in the second.
+struct WeightSource {
+    const float *W;
+    int taps = 0, split = 0;
+};
+
 struct Net {
     NetView v;
-    std::vector<float *> owned;
+    std::vector<void *> owned;    // device blocks: weights and biases, then one for every operand set built since
     int max_dim = 0;
     std::vector<int> kind;        // per layer: NYB200_LAYER_LINEAR or NYB200_LAYER_CONV2D
     std::vector<ConvGeom> geom;   // per layer; meaningful for conv layers
@@ -88,14 +108,16 @@ struct Net {
     bool is_conv(int k) const { return !kind.empty() && kind[k] == NYB200_LAYER_CONV2D; }
     int skip_of(int k) const { return skip.empty() ? -1 : skip[k]; }
     bool has_skip() const { for (int j : skip) if (j >= 0) return true; return false; }
-    std::vector<UmmaLayer> umma;  // filled on first use of the tcgen05 path
-    std::vector<UmmaLayer> umma_fwd;  // interval forward operands [W+ | W-] per layer (entry 0 unused)
-    std::vector<float *> wt;          // W_k^T, row-major [dims[k] x dims[k+1]] (adjoint pass; built on first use)
-    std::vector<UmmaLayer> umma_adj;  // tcgen05 operands of the adjoint pass (from wt)
+    // operand sets, each built by the first call that reads it
+    std::vector<UmmaLayer> umma;        // backward products: a layer's own form (the fused chain builds and reads entry 0 alone)
+    std::vector<UmmaLayer> umma_chain;  // hidden layers as the fused chain reads them (entry 0 unused)
+    std::vector<UmmaLayer> umma_fwd;    // interval forward operands [W+ | W-] per layer (entry 0 unused)
+    std::vector<float *> wt;            // W_k^T, row-major [dims[k] x dims[k+1]] (binary64 forward products)
+    std::vector<UmmaLayer> umma_adj;    // forward products of the adjoint pass and the attack
+    bool umma_whole = false;            // every entry of umma / win_bwd is there
     std::vector<float> wmax;          // per layer: largest |weight|; negative when some weight is too small beside it for fp16 pairs
-    std::vector<WinOp> win_bwd, win_fwd;   // window forms of the convolution layers (built on first use)
-    void *frag_block = nullptr;
-    std::vector<float *> frag;        // into frag_block: weights in binary64-fragment order (nyb200_direct.cu; built on first use)
+    std::vector<WinOp> win_bwd, win_fwd;   // window forms of the convolution layers, with umma and umma_adj
+    std::vector<float *> frag;        // weights in binary64-fragment order (nyb200_direct.cu)
 };
 
 struct DevBuf {
@@ -331,7 +353,7 @@ int create_net(nyb200_engine *e, int32_t n_layers, const nyb200_layer_desc *ld, 
 int finish_batch_public(nyb200_engine *e);
 int run_batch_public(nyb200_engine *e);
 void launch_dgemm(nyb200_engine *e, int m, int n, int k, const double *a, const double *b, double *c);
-int prepare_backward_operands(nyb200_engine *e, Net &net);
+int prepare_backward_operands(nyb200_engine *e, Net &net, bool chain);
 // ---- fused backward chain (nyb200_chain.cu) ----
 bool chain_eligible(const Net &net, int L);
 double chain_eps(int K);
@@ -400,9 +422,8 @@ void launch_conv_transpose(nyb200_engine *e, const ConvGeom &g, int M, const flo
 // Sums the tap-major im2col-space products cols[(m * taps + tap) * plane + (oy, ox)] into C[m, (ci, y, x)]
 // (binary64 sums of the fp32 entries, one cast: charged through the layer's rounding rate).
 void launch_col2im(nyb200_engine *e, const ConvGeom &g, int M, const float *cols, float *C, int ldc);
-// Forward convolutions on the tensor path: operand Wf [ic x oc*kh*kw] (or [W+ | W-] with `split`), the per-pixel
-// products through launch_umma(a_plane = ih*iw), then one of the gathers.
-int prepare_conv_forward_operand(nyb200_engine *e, const float *W, const ConvGeom &g, bool split, UmmaLayer *out);
+// Forward convolutions on the tensor path: per-pixel products with the operand [ic x oc*kh*kw] (or [W+ | W-]) through
+// launch_umma(a_plane = ih*iw), then one of the gathers.
 void launch_ibp_conv_gather(nyb200_engine *e, const NetView &nv, const ConvGeom &g, int k, int D, const float *cols, double eps,
                             float *raw_lo, float *raw_hi, float *q, long out_dstride);
 void launch_conv_fwd_gather(nyb200_engine *e, const ConvGeom &g, int rows, const float *cols, float *out, int ldo);
@@ -412,18 +433,18 @@ void launch_conv_plain(nyb200_engine *e, const ConvGeom &g, int rows, const floa
 // ---- convolutions as windows over an image (nyb200_convwin.cu) ----
 constexpr double kWinFloor = 8.8817841970012523e-16;   // 2^-50: error of a vanishing element, of its row's largest magnitude
 double win_eps(const WinOp &op);
-int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g, int kind, WinOp *out);
+int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g, int kind, WinOp *out, Carve &c);
 int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long lda, float *out, long ldo, double *rpen, const float *q_sum, int R, int *err);
 int launch_sum_weights(nyb200_engine *e, int D, int n, const float *q, long stride, float *q_sum);
 
 // ---- tcgen05 contraction (nyb200_umma.cu) ----
-int umma_prepare_layer(nyb200_engine *e, const float *W, int K, int N, UmmaLayer *out);
+int umma_prepare_layer(nyb200_engine *e, const WeightSource &src, int K, int N, UmmaLayer *out, Carve &c);
 // a_plane > 0 selects the transposed-convolution form: GEMM row r = (m, p) with p < a_plane, operand element
 // k at A[m * lda + k * a_plane + p], result column n at C[(m * N + n) * a_plane + p] (ldc unused).
 int launch_umma(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err,
                 int a_plane = 0, const ConcFuse *cf = nullptr);
 // The same on fp16 operand pairs (nyb200_umma16.cu).
-int umma_prepare_f16(nyb200_engine *e, const float *W, int K, int N, float wmax, UmmaLayer *out);
+int umma_prepare_f16(nyb200_engine *e, const WeightSource &src, int K, int N, float wmax, UmmaLayer *out, Carve &c);
 int launch_umma_f16(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err, const ConcFuse *cf = nullptr);
 double f16_eps(int K);
 int f16_segments(int K);   // K segments that even the largest batch is cut into
@@ -432,7 +453,41 @@ void launch_concretize_fused(nyb200_engine *e, int M, int R, int S, int slots, c
                              float *out_hi, float *min_lower, float loose_tol);
 double umma_eps(int K, int chain = 0);
 inline double layer_eps(const UmmaLayer &L, int K) { return L.f16 ? f16_eps(K) : umma_eps(K, L.chain); }
-// Builds the forward-pass operand of Linear_k: the [n_in x 2 n_out] matrix (W+^T | W-^T).
-int umma_prepare_forward_layer(nyb200_engine *e, const float *W, int n_in, int n_out, UmmaLayer *out);
+// The operand of an interval product: (W+^T | W-^T) of a fully connected layer (taps 1), or of a convolution's pixels.
+int umma_prepare_signed(nyb200_engine *e, const float *W, int taps, int K, int n_out, UmmaLayer *out, Carve &c);
+// A fully connected layer's own form: fp16 pairs, or TF32 ones where its weights span too much (wmax < 0) or are all zero.
+inline int umma_prepare_own(nyb200_engine *e, const WeightSource &src, int K, int N, float wmax, UmmaLayer *out, Carve &c) {
+    return wmax > 0.f ? umma_prepare_f16(e, src, K, N, wmax, out, c) : umma_prepare_layer(e, src, K, N, out, c);
+}
+
+// Builds an operand set in one allocation (several small ones cost a network's first calls milliseconds), owned by the network;
+// build(Carve &) runs twice, see Carve, and the caller publishes the set when this has succeeded.  Returns when the set is
+// complete: contractions load weights ahead of the kernels in front of them.
+template <class F>
+int build_operands(nyb200_engine *e, Net &net, F &&build) {
+    Carve c;
+    NYB_TRY(build(c));
+    if (!c.used) return NYB200_OK;
+    void *block = nullptr;
+    NYB_CUDA(e, cudaMalloc(&block, c.used));
+    c.block = (char *)block;
+    c.used = 0;
+    int st = build(c);
+    if (st == NYB200_OK) st = check_cuda(e, cudaGetLastError(), "operand set");
+    if (st == NYB200_OK) st = check_cuda(e, cudaStreamSynchronize(e->stream), "operand set");
+    if (st != NYB200_OK) { cudaFree(block); return st; }
+    net.owned.push_back(block);
+    return NYB200_OK;
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ float weight_at(const WeightSource &s, int k, int n, int K, int N) {
+    if (s.taps == 0) return s.W[(long)k * N + n];
+    const int half = s.split ? N / 2 : N;
+    const bool neg = n >= half;
+    const int r = neg ? n - half : n;
+    const float w = s.W[((long)(r / s.taps) * K + k) * s.taps + r % s.taps];
+    return !s.split ? w : neg ? fminf(w, 0.f) : fmaxf(w, 0.f);
+}
+#endif
 
 }  // namespace nyb

@@ -275,32 +275,40 @@ __global__ void k_gather_params(NetView nv, int D, int max_splits, const float4 
 
 }  // namespace
 
-// W_k^T (row-major [dims[k] x dims[k+1]]) for every Linear layer, and its tcgen05 operands: what a forward
-// product Z * W_k^T needs (the parameter adjoint and the concrete forward pass of the attack).
+// What a forward product Z * W_k^T needs (the parameter adjoint and the concrete forward pass of the attack): on the tensor
+// path the operands, otherwise W_k^T itself (row-major [dims[k] x dims[k+1]]).
 int prepare_transposed(nyb200_engine *e, Net &net, bool tensor) {
     const NetView &nv = net.v;
     const int L = nv.L;
-    if (net.wt.empty()) {
-        net.wt.resize(L, nullptr);
-        for (int k = 0; k < L; ++k) {
-            if (net.is_conv(k)) continue;  // a convolution's forward product runs the convolution itself
-            NYB_CUDA(e, cudaMalloc(&net.wt[k], (size_t)nv.dims[k] * nv.dims[k + 1] * 4));
-            dim3 grid((nv.dims[k] + 31) / 32, (nv.dims[k + 1] + 31) / 32), blk(32, 8);
-            k_transpose<<<grid, blk, 0, e->stream>>>(nv.W[k], nv.dims[k + 1], nv.dims[k], net.wt[k]);
-            e->launches++;
-        }
+    if (!tensor && net.wt.empty()) {
+        std::vector<float *> wt((size_t)L, nullptr);
+        NYB_TRY(build_operands(e, net, [&](Carve &c) {
+            for (int k = 0; k < L; ++k) {
+                if (net.is_conv(k)) continue;  // a convolution's forward product runs the convolution itself
+                wt[k] = (float *)c.take((size_t)nv.dims[k] * nv.dims[k + 1] * 4);
+                if (!c.block) continue;
+                dim3 grid((nv.dims[k] + 31) / 32, (nv.dims[k + 1] + 31) / 32), blk(32, 8);
+                k_transpose<<<grid, blk, 0, e->stream>>>(nv.W[k], nv.dims[k + 1], nv.dims[k], wt[k]);
+                e->launches++;
+            }
+            return (int)NYB200_OK;
+        }));
+        net.wt = std::move(wt);
     }
     if (tensor && net.umma_adj.empty()) {
-        net.umma_adj.resize(L);
-        for (int k = 0; k < L; ++k) {
-            if (!net.is_conv(k) && net.wmax[k] > 0.f) NYB_TRY(umma_prepare_f16(e, net.wt[k], nv.dims[k], nv.dims[k + 1], net.wmax[k], &net.umma_adj[k]));
-            else if (!net.is_conv(k)) NYB_TRY(umma_prepare_layer(e, net.wt[k], nv.dims[k], nv.dims[k + 1], &net.umma_adj[k]));
-            else {
-                net.win_fwd.resize(L);
-                NYB_TRY(win_prepare(e, nv.W[k], net.wmax[k], net.geom[k], 1, &net.win_fwd[k]));
-                if (!net.win_fwd[k].ok) NYB_TRY(prepare_conv_forward_operand(e, nv.W[k], net.geom[k], false, &net.umma_adj[k]));
+        std::vector<UmmaLayer> adj((size_t)L);
+        std::vector<WinOp> win((size_t)L);
+        NYB_TRY(build_operands(e, net, [&](Carve &c) -> int {
+            for (int k = 0; k < L; ++k) {
+                if (!net.is_conv(k)) { NYB_TRY(umma_prepare_own(e, WeightSource{nv.W[k], 1, 0}, nv.dims[k], nv.dims[k + 1], net.wmax[k], &adj[k], c)); continue; }
+                const ConvGeom &g = net.geom[k];
+                NYB_TRY(win_prepare(e, nv.W[k], net.wmax[k], g, 1, &win[k], c));
+                if (!win[k].ok) NYB_TRY(umma_prepare_layer(e, WeightSource{nv.W[k], g.kh * g.kw, 0}, g.ic, g.oc * g.kh * g.kw, &adj[k], c));
             }
-        }
+            return NYB200_OK;
+        }));
+        net.umma_adj = std::move(adj);
+        net.win_fwd = std::move(win);
     }
     return NYB200_OK;
 }

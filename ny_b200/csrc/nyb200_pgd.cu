@@ -239,7 +239,7 @@ int pgd_attack(nyb200_engine *e, int net_id, const float *spec, int S, const flo
     e->batch = Batch();  // workspace names are shared with the resident batch
 
     NYB_TRY(prepare_transposed(e, *net, tensor));
-    if (tensor) NYB_TRY(prepare_backward_operands(e, *net));
+    if (tensor) NYB_TRY(prepare_backward_operands(e, *net, false));
     NYB_WS(dspec, float *, e, "spec", (size_t)S * nL * 4);
     NYB_WS(dlo, float *, e, "in_lo", (size_t)n0 * 4);
     NYB_WS(dhi, float *, e, "in_hi", (size_t)n0 * 4);
@@ -330,7 +330,7 @@ int point_vjp(nyb200_engine *e, int net_id, int K, const float *x, const float *
     const int ld = (net->max_dim + 7) & ~7;
     e->batch = Batch();  // workspace names are shared with the resident batch
     NYB_TRY(prepare_transposed(e, *net, tensor));
-    if (tensor) NYB_TRY(prepare_backward_operands(e, *net));
+    if (tensor) NYB_TRY(prepare_backward_operands(e, *net, false));
     NYB_WS(X, float *, e, "pgd_x", (size_t)K * ld * 4);
     NYB_WS(acts, float *, e, "pgd_act", (size_t)L * K * ld * 4);
     NYB_WS(G0, float *, e, "pgd_g0", (size_t)K * ld * 4);

@@ -75,14 +75,14 @@ static int chunk_stages_cfg(int K) { return (K + BK - 1) / BK >= 8 ? 2 : 1; }
 
 using namespace umma;
 
-// Splits W [K x N] (row-major) into TF32 high/low parts stored transposed and K-padded:
+// Splits an operand [K x N] into TF32 high/low parts stored transposed and K-padded:
 // Wh_T, Wl_T are [N x Kpad] row-major with zeros for k >= K.
-__global__ void k_split_weights(const float *__restrict__ W, int K, int N, int Kpad, float *__restrict__ Wh,
+__global__ void k_split_weights(WeightSource src, int K, int N, int Kpad, float *__restrict__ Wh,
                                 float *__restrict__ Wl) {
     long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long)N * Kpad) return;
     int n = (int)(t / Kpad), k = (int)(t % Kpad);
-    float w = (k < K) ? W[(long)k * N + n] : 0.f;
+    float w = (k < K) ? weight_at(src, k, n, K, N) : 0.f;
     float h = rn_tf32(w);
     float l = rn_tf32(w - h);
     Wh[t] = h;
@@ -465,15 +465,14 @@ static int make_tmap(CUtensorMap *tm, const float *base, int rows, int kpad, int
     return r == CUDA_SUCCESS ? 0 : 2;
 }
 
-int umma_prepare_layer(nyb200_engine *e, const float *W, int K, int N, UmmaLayer *out) {
+int umma_prepare_layer(nyb200_engine *e, const WeightSource &src, int K, int N, UmmaLayer *out, Carve &c) {
     int kpad = (K + BK - 1) / BK * BK;
     size_t n = (size_t)N * kpad;
-    float *wh = nullptr, *wl = nullptr;
-    if (cudaMalloc(&wh, n * 4) != cudaSuccess) return NYB200_ERR_OOM;
-    if (cudaMalloc(&wl, n * 4) != cudaSuccess) { cudaFree(wh); return NYB200_ERR_OOM; }
-    k_split_weights<<<(unsigned)((n + 255) / 256), 256, 0, e->stream>>>(W, K, N, kpad, wh, wl);
+    float *wh = (float *)c.take(n * 4), *wl = (float *)c.take(n * 4);
+    if (!c.block) return NYB200_OK;
+    k_split_weights<<<(unsigned)((n + 255) / 256), 256, 0, e->stream>>>(src, K, N, kpad, wh, wl);
     e->launches++;
-    out->wh = wh; out->wl = wl; out->K = K; out->N = N; out->kpad = kpad;
+    out->wh = wh; out->wl = wl; out->K = K; out->N = N;
     static_assert(sizeof(CUtensorMap) == sizeof(out->tm_hi), "tensor map storage size");
     if (make_tmap((CUtensorMap *)out->tm_hi, wh, N, kpad) || make_tmap((CUtensorMap *)out->tm_lo, wl, N, kpad))
         return set_err(e, NYB200_ERR_INTERNAL, "cuTensorMapEncodeTiled failed");
@@ -519,28 +518,11 @@ int launch_umma(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int
     return NYB200_OK;
 }
 
-// (W+^T | W-^T) as a row-major [n_in x 2 n_out] matrix from W [n_out x n_in].
-__global__ void k_build_wpm(const float *__restrict__ W, int n_in, int n_out, float *__restrict__ out) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)n_in * 2 * n_out) return;
-    int k = (int)(t / (2 * n_out)), n = (int)(t % (2 * n_out));
-    float w = W[(long)(n % n_out) * n_in + k];
-    out[t] = (n < n_out) ? fmaxf(w, 0.f) : fminf(w, 0.f);
-}
-
-int umma_prepare_forward_layer(nyb200_engine *e, const float *W, int n_in, int n_out, UmmaLayer *out) {
-    float *tmp = nullptr;
-    size_t n = (size_t)n_in * 2 * n_out;
-    if (cudaMalloc(&tmp, n * 4) != cudaSuccess) return NYB200_ERR_OOM;
-    k_build_wpm<<<(unsigned)((n + 255) / 256), 256, 0, e->stream>>>(W, n_in, n_out, tmp);
-    e->launches++;
-    int st = umma_prepare_layer(e, tmp, n_in, 2 * n_out, out);
+int umma_prepare_signed(nyb200_engine *e, const float *W, int taps, int K, int n_out, UmmaLayer *out, Carve &c) {
     // interval products keep one stage per chain: their slack is compared against every unstable neuron's width
     // and compounds through the layers, where the coefficient products' charge is only compared against the bound
     out->chain = 1;
-    cudaStreamSynchronize(e->stream);
-    cudaFree(tmp);
-    return st;
+    return umma_prepare_layer(e, WeightSource{W, taps, 1}, K, 2 * n_out * taps, out, c);
 }
 
 // Worst-case relative rounding of this kernel's product against S = |A||W| (see the model above).

@@ -519,12 +519,12 @@ k_sum_segments(long total, int N, int segs, const float *__restrict__ part, floa
     C[t / N * ldc + t % N] = s;
 }
 
-// W [K x N] (row-major) scaled by 2^e into fp16 high and low parts, transposed and K-padded: [2][N][kpad].
-__global__ void k_split_weights_f16(const float *__restrict__ W, int K, int N, int kpad, float scale, __half *__restrict__ out) {
+// An operand [K x N] scaled by 2^e into fp16 high and low parts, transposed and K-padded: [2][N][kpad].
+__global__ void k_split_weights_f16(WeightSource src, int K, int N, int kpad, float scale, __half *__restrict__ out) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x, n_el = (long)N * kpad;
     if (t >= n_el) return;
     const int n = (int)(t / kpad), k = (int)(t % kpad);
-    const float w = k < K ? W[(long)k * N + n] * scale : 0.f;
+    const float w = k < K ? weight_at(src, k, n, K, N) * scale : 0.f;
     const __half h = __float2half_rn(w);
     out[t] = h;
     out[n_el + t] = __float2half_rn((w - __half2float(h)) * 2048.f);
@@ -563,22 +563,20 @@ static bool make_map(void *out, CUtensorMapDataType type, int size, const void *
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The fp16 operand of W [K x N] (device); wmax: its largest magnitude (net.wmax, positive: the layer qualifies).
-int umma_prepare_f16(nyb200_engine *e, const float *W, int K, int N, float wmax, UmmaLayer *out) {
+// The fp16 operand [K x N] of `src`; wmax: its largest magnitude (net.wmax, positive: the layer qualifies).
+int umma_prepare_f16(nyb200_engine *e, const WeightSource &src, int K, int N, float wmax, UmmaLayer *out, Carve &c) {
     const int kpad = (K + BK - 1) / BK * BK;
     const size_t n_el = (size_t)N * kpad;
-    __half *block = nullptr;
-    if (cudaMalloc(&block, 2 * n_el * 2) != cudaSuccess) return set_err(e, NYB200_ERR_OOM, "device allocation failed for a contraction operand");
+    __half *block = (__half *)c.take(2 * n_el * 2);
+    if (!c.block) return NYB200_OK;
     out->f16 = block;
     out->K = K; out->N = N;
     int ex;
     frexpf(wmax, &ex);                       // wmax in [2^(ex-1), 2^ex)
     const float scale = ldexpf(1.f, std::max(-126, std::min(15 - ex, 126)));
     out->w_inv = 1.f / scale;
-    k_split_weights_f16<<<(unsigned)((n_el + 255) / 256), 256, 0, e->stream>>>(W, K, N, kpad, scale, block);
+    k_split_weights_f16<<<(unsigned)((n_el + 255) / 256), 256, 0, e->stream>>>(src, K, N, kpad, scale, block);
     e->launches++;
-    NYB_CUDA(e, cudaGetLastError());
-    NYB_CUDA(e, cudaStreamSynchronize(e->stream));   // the contraction loads weights without waiting for earlier kernels
     for (int i = 0; i < 2; ++i)
         if (!make_map(i ? out->tm16_lo : out->tm16_hi, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, block + i * n_el, kpad, N, kpad, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B))
             return set_err(e, NYB200_ERR_INTERNAL, "cuTensorMapEncodeTiled failed for a contraction operand");
