@@ -258,7 +258,7 @@ def run_ours(args, rank, world, local_rank):
     eng = B200Engine(local_rank, stream.cuda_stream)
     from ny_b200 import engine as E
 
-    eng.set_path(E.PATH_TF32X3 if args.path == "tf32x3" else E.PATH_F64)
+    eng.set_path(E.PATH_AUTO if args.path == "tf32x3" else E.PATH_F64)
     eng.set_fusion(bool(args.fusion))
     reserve = args.reserve_sms if args.reserve_sms >= 0 else (2 if world > 1 else 0)   # room for the min-reduce beside the kernels
     eng.set_reserved_sms(reserve)
@@ -358,7 +358,7 @@ def run_ours(args, rank, world, local_rank):
     for i in range(1, B):
         st_i = torch.cuda.Stream(device=local_rank)
         e_i = B200Engine(local_rank, st_i.cuda_stream)
-        e_i.set_path(E.PATH_TF32X3 if args.path == "tf32x3" else E.PATH_F64)
+        e_i.set_path(E.PATH_AUTO if args.path == "tf32x3" else E.PATH_F64)
         e_i.set_fusion(bool(args.fusion))
         e_i.set_reserved_sms(reserve)
         e_i.set_launch_overlap(False)
@@ -459,7 +459,7 @@ def run_ours(args, rank, world, local_rank):
         from ny_b200.pool import EnginePool
 
         def configure(e):
-            e.set_path(E.PATH_TF32X3 if args.path == "tf32x3" else E.PATH_F64)
+            e.set_path(E.PATH_AUTO if args.path == "tf32x3" else E.PATH_F64)
             e.set_fusion(bool(args.fusion))
 
         pool = EnginePool(local_rank, B, configure)
@@ -605,7 +605,7 @@ def run_alpha_crown(args, rank, world, local_rank):
     torch.cuda.set_device(local_rank)
     stream = torch.cuda.current_stream()
     eng = B200Engine(local_rank, stream.cuda_stream)
-    eng.set_path(E.PATH_TF32X3 if args.path == "tf32x3" else E.PATH_F64)
+    eng.set_path(E.PATH_AUTO if args.path == "tf32x3" else E.PATH_F64)
     wl = W.config_alpha_crown()
     nid = eng.register_network(wl.net)
     pl, pu = eng.ibp_forward_gpu(nid, wl.in_lo, wl.in_hi)
@@ -691,7 +691,7 @@ def run_cnn(args, local_rank, kind="cnn"):
     torch.cuda.set_device(local_rank)
     stream = torch.cuda.current_stream()
     eng = B200Engine(local_rank, stream.cuda_stream)
-    eng.set_path(E.PATH_TF32X3 if args.path == "tf32x3" else E.PATH_F64)
+    eng.set_path(E.PATH_AUTO if args.path == "tf32x3" else E.PATH_F64)
     wl = W.config_cnn() if kind == "cnn" else W.config_resnet()
     nid = eng.register_network(wl.net)
     pl, pu = eng.ibp_forward_gpu(nid, wl.in_lo, wl.in_hi)
@@ -806,7 +806,7 @@ def run_search(args, rank, world, local_rank):
         dist = dist_mod
         dist.init_process_group("nccl", device_id=torch.device("cuda", local_rank))
     eng = B200Engine(local_rank, torch.cuda.current_stream().cuda_stream)
-    eng.set_path(E.PATH_TF32X3 if args.path == "tf32x3" else E.PATH_F64)
+    eng.set_path(E.PATH_AUTO if args.path == "tf32x3" else E.PATH_F64)
     wl = W.config_mlp_bab(seed=7, hidden=256, depth=4, n_in=64, n_out=10, eps=0.05, n_fix=0)
     nid = eng.register_network(wl.net)
     root, _, _, _ = eng.crown_bounds(nid, wl.spec, wl.in_lo, wl.in_hi)
@@ -822,7 +822,7 @@ def run_search(args, rank, world, local_rank):
     if resident and dist is None and args.search_engines > 1:
         from ny_b200.pool import EnginePool
 
-        pool = EnginePool(local_rank, args.search_engines, lambda e: e.set_path(E.PATH_TF32X3 if args.path == "tf32x3" else E.PATH_F64))
+        pool = EnginePool(local_rank, args.search_engines, lambda e: e.set_path(E.PATH_AUTO if args.path == "tf32x3" else E.PATH_F64))
         handle = pool.register_network(wl.net)
 
     def search():
@@ -940,7 +940,7 @@ def run_pgd(args, local_rank, kind="cnn"):
 
     torch.cuda.set_device(local_rank)
     eng = B200Engine(local_rank, torch.cuda.current_stream().cuda_stream)
-    eng.set_path(E.PATH_TF32X3 if args.path == "tf32x3" else E.PATH_F64)
+    eng.set_path(E.PATH_AUTO if args.path == "tf32x3" else E.PATH_F64)
     wl = W.config_cnn() if kind == "cnn" else W.config_resnet()
     nid = eng.register_network(wl.net)
     K, steps = 1024, 100

@@ -45,9 +45,11 @@ typedef struct {
     float beta;
 } nyb200_split;
 
-/* Arithmetic used for the A*W contraction of the backward pass. */
-#define NYB200_PATH_F64 0   /* binary64 FMA accumulation of exact fp32 products */
-#define NYB200_PATH_TF32X3 1 /* tcgen05 3xTF32 split products, chunked TMEM accumulators */
+/* Arithmetic of the contractions. */
+#define NYB200_PATH_F64 0    /* binary64 accumulation of exact fp32 products */
+#define NYB200_PATH_TF32X3 1 /* tcgen05: three products of split operands (pairs of TF32 or of fp16 parts, 22 bits either way) */
+#define NYB200_PATH_AUTO 2   /* NYB200_PATH_TF32X3, except where binary64 is the faster form: plain CROWN of fully connected
+                                networks and their batches of a few domains */
 
 /* ---- lifecycle ---------------------------------------------------------------------------
  * Engine construction/provenance: GemmEngine::backend_provenance (crates/ny-core/src/gemm.rs:313)
@@ -76,19 +78,20 @@ int32_t nyb200_set_reserved_sms(nyb200_engine *e, int32_t n);
  * could have run there does not (three batches in flight: 0.957 ms per step without against 0.973 ms with).
  * ny_b200/pool.py switches it off for pools of more than one engine. */
 int32_t nyb200_set_launch_overlap(nyb200_engine *e, int32_t on);
-/* Select the contraction arithmetic (NYB200_PATH_*).  Default NYB200_PATH_TF32X3; NYB200_PATH_F64 is the
- * slower binary64 reference arithmetic on the same device. */
+/* Select the contraction arithmetic (NYB200_PATH_*) of all calls that follow.  Default NYB200_PATH_AUTO; NYB200_PATH_F64 is the
+ * slower binary64 reference arithmetic on the same device, NYB200_PATH_TF32X3 the tensor cores whatever the size. */
 int32_t nyb200_set_path(nyb200_engine *e, int32_t path);
-/* Layer fusion of the NYB200_PATH_TF32X3 backward pass.  On (default): where the network allows it (Linear layers
+/* Layer fusion.  On (default): in binary64 a fully connected network's interval pass and its backward pass are one kernel each
+ * (nyb200_direct.cu).  In the backward pass on the tensor cores, where the network allows it (Linear layers
  * without skips, hidden widths <= 256 and multiples of 4) the contractions of all hidden layers and their ReLU
  * relaxations run as one kernel that keeps a tile of coefficient rows on the SM from the specification rows down to
  * the first layer's input; only the first layer's (wide) contraction and the concretisation follow as separate
- * launches.  Off: one contraction launch and one relaxation launch per layer.  Both compute the same quantities
- * with the same per-coefficient arithmetic; they differ in the accumulation order of the tensor-core sums (and its
+ * launches.  Off: one contraction launch and one relaxation launch per layer, on either path.  Both compute the same quantities
+ * with the same per-coefficient arithmetic; they differ in the accumulation order of the sums (and its
  * certified rounding charge), i.e. by a few ulps of the coefficients.  No counterpart in the reference, whose
  * engines launch per layer (crates/ny-cuda/src/sound_crown.rs:348-376). */
 int32_t nyb200_set_fusion(nyb200_engine *e, int32_t on);
-/* Adaptive precision of the NYB200_PATH_TF32X3 path.  Every rounding of that path is charged to the
+/* Adaptive precision of the tensor path.  Every rounding of that path is charged to the
  * bounds as a penalty; when, for some domain of a batch, that penalty exceeds `tol` times
  * max(|bound|, 1% of the domain's largest bound) -- which happens for narrow boxes, where a bound is much
  * smaller than the terms it is made of -- the batch is evaluated again with binary64 contractions before

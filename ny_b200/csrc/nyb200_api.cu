@@ -131,9 +131,10 @@ int32_t nyb200_use_own_stream(nyb200_engine *e) {
 
 int32_t nyb200_set_path(nyb200_engine *e, int32_t path) {
     if (!e) return NYB200_ERR_INVALID;
-    if (path != NYB200_PATH_F64 && path != NYB200_PATH_TF32X3) return set_err(e, NYB200_ERR_INVALID, "unknown path");
+    if (path != NYB200_PATH_F64 && path != NYB200_PATH_TF32X3 && path != NYB200_PATH_AUTO) return set_err(e, NYB200_ERR_INVALID, "unknown path");
     std::lock_guard<std::mutex> g(e->mu);
-    e->path = path;
+    e->path = path == NYB200_PATH_F64 ? NYB200_PATH_F64 : NYB200_PATH_TF32X3;
+    e->small_direct = path == NYB200_PATH_AUTO;
     return NYB200_OK;
 }
 
@@ -685,7 +686,7 @@ constexpr size_t kConvColsMost = (size_t)4 << 30;
 int run_forward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int fwd_mode) {
     const NetView &nv = net.v;
     int D = b.D;
-    if (e->path == NYB200_PATH_F64 && fwd_mode < 2 && p.inh_lo && direct_eligible(net)) return run_forward_direct(e, net, b, p, fwd_mode, nullptr, D);
+    if (e->path == NYB200_PATH_F64 && e->fuse_chain && fwd_mode < 2 && p.inh_lo && direct_eligible(net)) return run_forward_direct(e, net, b, p, fwd_mode, nullptr, D);
     // The tcgen05 path covers every layer whose input is a post-ReLU interval (lower end >= 0) of a
     // per-domain batch; the first layer (arbitrary-sign box, usually shared) stays on the binary64 kernel.
     const bool tensor = (e->path == NYB200_PATH_TF32X3) && D >= 64 && nv.L > 1;
@@ -820,7 +821,7 @@ int prepare_backward_operands(nyb200_engine *e, Net &net, bool chain) {
 int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float *const *ckpt, int ld_ckpt, int top) {
     const NetView &nv = net.v;
     const bool tensor = (e->path == NYB200_PATH_TF32X3);
-    if (!tensor && !ckpt && top < 0 && direct_eligible(net)) {
+    if (!tensor && e->fuse_chain && !ckpt && top < 0 && direct_eligible(net)) {
         const float clear[8] = {INFINITY, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         NYB_CUDA(e, cudaMemcpyAsync(p.min_lower, clear, sizeof(clear), cudaMemcpyHostToDevice, e->stream));
         return run_backward_direct(e, net, b, p, nullptr, b.D);
@@ -1058,7 +1059,7 @@ int run_batch(nyb200_engine *e) {
     NYB_TRY(batch_ptrs(e, *net, e->batch, p));
     Timing &t = e->timing;
     fold_timing(t);  // the previous run's events are about to be reused
-    const bool direct = !e->batch.external_tables && direct_eligible(*net) && (e->path == NYB200_PATH_F64 || direct_pays(*net, e->batch.S, e->batch.D));
+    const bool direct = !e->batch.external_tables && ((e->path == NYB200_PATH_F64 && e->fuse_chain && direct_eligible(*net)) || direct_pays(e, *net, e->batch.S, e->batch.D));
     const bool tensor = e->path == NYB200_PATH_TF32X3 && !direct;
     if (tensor) {
         int *derr = (int *)ws_get(e, "umma_err", 256);

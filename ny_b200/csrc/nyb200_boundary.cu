@@ -296,7 +296,7 @@ int32_t nyb200_crown_resnet_beta_batched(nyb200_engine *e, const nyb200_domain_r
         NYB_CUDA(e, cudaMemsetAsync(derr, 0, 4, e->stream));
     }
     const int saved_path = e->path;
-    if (direct_pays(*net, num_specs, D)) e->path = NYB200_PATH_F64;   // a few domains: directly in binary64, as the split-list call does
+    if (direct_pays(e, *net, num_specs, D)) e->path = NYB200_PATH_F64;   // a few domains: directly in binary64, as the split-list call does
     const int rc = run_backward(e, *net, e->batch, p, nullptr, 0);
     e->path = saved_path;
     NYB_TRY(rc);

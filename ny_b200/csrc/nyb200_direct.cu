@@ -921,6 +921,7 @@ bool direct_eligible(const Net &net) {
 
 bool crown_direct_eligible(const nyb200_engine *e, const Net &net, int S, int D) {
     const NetView &nv = net.v;
+    if (!e->fuse_chain || (e->path == NYB200_PATH_TF32X3 && !e->small_direct)) return false;   // the caller asks for the per-layer or the tensor form
     if (e->error_channel == NYB200_ERRCH_REFERENCE || nv.L < 2 || !direct_eligible(net)) return false;
     double down = 0.0, macs = 0.0;
     for (int k = 0; k < nv.L; ++k) {
@@ -1017,8 +1018,8 @@ static double direct_macs(const NetView &nv, int S) {
 // Below this size a batch is evaluated directly instead of on the 3xTF32 path (which its caller then need not check for
 // visible rounding charges), if it is a batch of a few domains at all.  The tensor path costs about 40 us plus 20 us per layer whatever the batch; the direct one
 // runs at about 8e12 multiply-adds a second once it fills the GPU.
-bool direct_pays(const Net &net, int S, int D) {
-    return D <= 64 && direct_eligible(net) && direct_macs(net.v, S) * D <= 8e12 * (40e-6 + 20e-6 * net.v.L);
+bool direct_pays(const nyb200_engine *e, const Net &net, int S, int D) {
+    return e->path == NYB200_PATH_TF32X3 && e->small_direct && e->fuse_chain && D <= 64 && direct_eligible(net) && direct_macs(net.v, S) * D <= 8e12 * (40e-6 + 20e-6 * net.v.L);
 }
 
 // Interval pass of the n domains idx (null: all b.D) of the resident batch, modes 0 and 1.

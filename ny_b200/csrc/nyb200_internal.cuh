@@ -174,7 +174,8 @@ struct nyb200_engine {
     int reserve_sms = 0;                          // see nyb200_set_reserved_sms
     bool launch_overlap = true;                   // see nyb200_set_launch_overlap
     cudaStream_t own_stream = nullptr;            // created by nyb200_use_own_stream, destroyed with the engine
-    int path = NYB200_PATH_TF32X3;
+    int path = NYB200_PATH_TF32X3;                // _F64 or _TF32X3
+    bool small_direct = true;                     // NYB200_PATH_AUTO: what binary64 does faster goes there
     float refine_tol = 5e-5f;  // see nyb200_set_refine_tolerance
     int error_channel = NYB200_ERRCH_IMMEDIATE;  // see nyb200_set_error_channel
     bool fuse_chain = true;                       // see nyb200_set_fusion
@@ -379,7 +380,7 @@ struct CrownSplits {
 };
 // The same for fully connected networks, binary64, one kernel per partial pass (nyb200_direct.cu)
 bool direct_eligible(const Net &net);
-bool direct_pays(const Net &net, int S, int D);
+bool direct_pays(const nyb200_engine *e, const Net &net, int S, int D);
 int run_forward_direct(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int mode, const int *idx, int n);
 int run_backward_direct(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, const int *idx, int n, float *ckpt = nullptr);
 int flagged_domains(nyb200_engine *e, int D, const int *flags, int n, int **idx);

@@ -422,7 +422,7 @@ int optimize_batch(nyb200_engine *e, const nyb200_opt_config &cfg, float *grad_h
     cudaEventRecord(tm.ev[0], e->stream);
     // a batch of a few domains is evaluated directly (direct_pays), as the plain bound of the same batch is; the adjoint's
     // products, which only propose parameters, stay on the tensor path
-    const bool direct = tensor && direct_pays(*net, S, D);
+    const bool direct = direct_pays(e, *net, S, D);
     static const float clear_words[8] = {INFINITY, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     bool clear = b.external_tables;
     if (!b.external_tables && direct) NYB_TRY(run_forward_direct(e, *net, b, p, b.mode, nullptr, D));

@@ -28,7 +28,7 @@ _NAMES = {
     UNSUPPORTED: "UnsupportedOp", SHAPE: "ShapeMismatch", INVALID: "InvalidSpec", NUMERICAL: "NumericalInstability",
     DEADLINE: "DeadlineExceeded", OOM: "MemoryExceeded", INTERNAL: "InternalError",
 }
-PATH_F64, PATH_TF32X3 = 0, 1
+PATH_F64, PATH_TF32X3, PATH_AUTO = 0, 1, 2
 ERRCH_IMMEDIATE, ERRCH_REFERENCE = 0, 1
 
 EXPORTS = [
@@ -421,6 +421,7 @@ class B200Engine:
         self._check(self._L.nyb200_set_launch_overlap(self._h, 1 if on else 0))
 
     def set_path(self, path: int):
+        """PATH_AUTO (default), PATH_TF32X3 (the tensor cores, whatever the size) or PATH_F64."""
         self._check(self._L.nyb200_set_path(self._h, path))
 
     def set_error_channel(self, mode: int):

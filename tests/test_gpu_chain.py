@@ -14,9 +14,10 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def eng():
-    from ny_b200 import B200Engine
+    from ny_b200 import B200Engine, engine
 
     e = B200Engine(0)
+    e.set_path(engine.PATH_TF32X3)   # plain CROWN too: by default it is evaluated in binary64 whether the chain is on or off
     yield e
     e.close()
 

@@ -77,3 +77,42 @@ def test_direct_bound_of_a_few_domains_matches_the_oracle(eng, oracle, dims, D):
     lo2, hi2, _ = eng.bab_bound_batch(nid, wl.spec, np.repeat(wl.in_lo[None], D, 0), np.repeat(wl.in_hi[None], D, 0), rl, ru, splits, ns)
     assert np.all(np.abs(lo2[f] - lo[f]) <= 1e-6 * scale) and np.all(np.abs(hi2[f] - hi[f]) <= 1e-6 * scale)
     eng.release_network(nid)
+
+
+@pytest.mark.parametrize("dims,D", [([20, 33, 64, 5], 12), ([96, 64, 64, 64, 10], 40)])
+def test_path_and_fusion_select_the_form(dims, D):
+    """The default takes a few domains, and plain CROWN, directly in binary64; PATH_TF32X3 keeps both on the tensor cores and
+    PATH_F64 with fusion off takes one launch per layer.  All agree to the roundings they charge."""
+    from ny_b200 import B200Engine, engine
+
+    net = W.make_mlp(dims, 600 + D)
+    g = np.random.Generator(np.random.PCG64(D))
+    x0 = g.uniform(0, 1, dims[0]).astype(np.float32)
+    lo, hi, wide = x0 - np.float32(0.02), x0 + np.float32(0.02), np.full(net.n_pre, 1e30, np.float32)
+    spec = W.margin_spec(dims[-1], 0)
+    e = B200Engine(0)
+    e.set_refine_tolerance(0.0)
+    nid = e.register_network(net)
+
+    def both(path, fusion):
+        e.set_path(path)
+        e.set_fusion(fusion)
+        for _ in range(2):     # the second time without preparing operands
+            n0 = e.launch_count()
+            b = e.bab_bound_batch(nid, spec, lo, hi, -wide, wide, np.zeros((D, 0), SPLIT_DTYPE), np.zeros(D, np.int32))
+            n1 = e.launch_count()
+            c = e.crown_bounds(nid, spec, lo, hi)
+        return np.concatenate(b[:2], 1), np.concatenate(c[:2], 1), n1 - n0, e.launch_count() - n1
+
+    auto = both(engine.PATH_AUTO, True)
+    tensor = both(engine.PATH_TF32X3, True)
+    layers = both(engine.PATH_F64, False)
+    direct = both(engine.PATH_F64, True)
+    assert auto[2] == direct[2] < min(tensor[2], layers[2]) and auto[3] == direct[3] < min(tensor[3], layers[3])
+    assert np.array_equal(auto[0], direct[0]) and np.array_equal(auto[1], direct[1])
+    assert not np.array_equal(auto[0], tensor[0]) and not np.array_equal(auto[1], tensor[1])
+    for got in (auto, tensor, layers):
+        for i in range(2):
+            scale = np.abs(direct[i]).max()
+            assert np.all(np.abs(got[i] - direct[i]) <= (5e-4 if got is tensor else 1e-5) * scale)
+    e.close()
