@@ -15,7 +15,7 @@
 // scaled by powers of two so that their largest magnitude lies in [2^14, 2^15).  Ah*Wh goes into a MAIN accumulator that is
 // drained into fp32 registers every few steps, Al*Wh + Ah*Wl into a CROSS accumulator added once at the end.
 // Rounding (win_eps): operand split 0.75 * 2^-20 as for a TF32 pair; each MMA step at most one fp32 ulp of the
-// accumulated magnitude (the model of k_umma_tf32x3, tests/test_gpu_convwin.py); one fp32 addition per chain.  An element
+// accumulated magnitude (the model of k_umma_tf32x3; element by element in tests/test_gpu_rates.py); one fp32 addition per chain.  An element
 // more than 2^29 times smaller than its row's largest loses its low bits to fp16's exponent range: an absolute error of
 // at most 2^-50 of that largest magnitude, which k_split_image charges to the row separately; weights that small
 // make a layer ineligible (win_prepare gets a negative wmax).

@@ -36,6 +36,7 @@
 // MMA step, eight of size 2^-10 S and four of size S per chunk; one fp32 rounding per chunk and segment.  An element more
 // than 2^29 times smaller than its chunk's largest loses low bits to the exponent range, an absolute error of at most
 // 2^-50 of that largest: q carries it (NetView::qfl).  A layer whose weights span more than that keeps its TF32 form.
+// tests/test_gpu_rates.py holds every element of a product against that rate.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
