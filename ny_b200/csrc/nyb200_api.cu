@@ -71,6 +71,7 @@ int32_t nyb200_create(int32_t device_ordinal, nyb200_engine **out) {
     if (prop.major != 10) return NYB200_ERR_UNSUPPORTED;  // kernels are built for sm_100a only
     nyb200_engine *e = new nyb200_engine();
     e->device = device_ordinal;
+    e->sms = prop.multiProcessorCount;
     for (int i = 0; i < 3; ++i) cudaEventCreate(&e->timing.ev[i]);
     *out = e;
     return NYB200_OK;

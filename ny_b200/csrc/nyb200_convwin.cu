@@ -561,9 +561,7 @@ int launch_win(nyb200_engine *e, const WinOp &op, int rows, const void *hi, cons
         if (enc(&tm[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(i && !packed ? lo : hi), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 swizzle_of(P.swa), CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return set_err(e, NYB200_ERR_INTERNAL, "cuTensorMapEncodeTiled failed for an image operand");
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
-    if (e->reserve_sms > 0 && sms > e->reserve_sms) sms -= e->reserve_sms;
+    const int sms = usable_sms(e);
     const long tiles = (long)rows * P.tiles_y * P.tiles_x;
     if (tiles > 0x7fffffffL - 65536) return set_err(e, NYB200_ERR_UNSUPPORTED, "batch too large for one convolution");
     const int per_block = (int)std::min<long>(tiles, std::max(1, sms / P.n_blocks));

@@ -871,11 +871,12 @@ int launch_pass(nyb200_engine *e, const PackedNet &pn, int top, int n_rows, int 
     const int groups = (int)(((long)D * 2 * n_rows + 7) / 8), tiles = (wide + 7) / 8;
     // Warps per group of rows: enough that a warp's columns fit its accumulators, and while the launch is small (fewer
     // than eight warps per SM) more of them, down to one tile each: a group's products are a serial chain.
+    const int sms = usable_sms(e);
     int NW = 1;
-    while (NW < 8 && (tiles > NW * 8 || ((long)groups * NW < 148 * 8 && tiles > NW))) NW *= 2;
+    while (NW < 8 && (tiles > NW * 8 || ((long)groups * NW < (long)sms * 8 && tiles > NW))) NW *= 2;
     // a launch that leaves SMs idle all the same: clusters of two to eight CTAs of eight warps each
     int C = 1;
-    while (NW >= 8 && C < 8 && groups * C * 2 <= 148 && tiles >= NW * 2) { C *= 2; NW *= 2; }
+    while (NW >= 8 && C < 8 && groups * C * 2 <= sms && tiles >= NW * 2) { C *= 2; NW *= 2; }
     const int per = (tiles + NW - 1) / NW;
     int MT = 8 / (NW / C);
     const int bufs = C > 1 || (written + 7) / 8 > NW * 8 ? 2 : 1;   // one sweep per layer: the rows are replaced in place
@@ -969,7 +970,7 @@ int crown_direct(nyb200_engine *e, int net_id, const float *spec, int S, const f
     const signed char *code = split ? p.code : nullptr;
     const PackedNet pn = packed(*net);
     // few boxes: a wide CTA shortens the serial chain over the layers; many: smaller ones share an SM
-    const dim3 per_box((unsigned)D), box_threads(D < 148 ? 512 : 256);
+    const dim3 per_box((unsigned)D), box_threads(D < usable_sms(e) ? 512 : 256);
     int zdim = 0;
     for (int k = 0; k < L; ++k) zdim = nv.dims[k] > zdim ? nv.dims[k] : zdim;
     zdim = (zdim + 1) & ~1;
@@ -1033,9 +1034,10 @@ int run_forward_direct(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p,
     zdim = (zdim + 1) & ~1;
     // Few domains: a cluster of CTAs per domain spreads its outputs over the idle SMs, and wide CTAs shorten the serial
     // chain over the layers; many: one small CTA per domain, several to an SM.
+    const int sms = usable_sms(e);
     int C = 1;
-    while (C < 8 && n * C * 2 <= 128) C *= 2;   // (clusters live inside a GPC: not every SM can be used)
-    const int threads = n * C <= 148 ? 512 : 256;
+    while (C < 8 && n * C * 2 <= sms * 7 / 8) C *= 2;   // (clusters live inside a GPC: not every SM can be used)
+    const int threads = n * C <= sms ? 512 : 256;
     const size_t smem = (size_t)zdim * (32 + 12) + (size_t)nv.nps * 5;
     NYB_TRY(allow_smem(e, (const void *)k_direct_forward, smem));
     NYB_CUDA(e, launch_pdl_cluster(k_direct_forward, dim3((unsigned)(n * C)), dim3(threads), C, smem, e, nv, mode, zdim, idx,

@@ -171,6 +171,7 @@ using nyb::ResidentFrontier;
 struct nyb200_engine {
     int device = 0;
     cudaStream_t stream = nullptr;
+    int sms = 1;                                  // of the device
     int reserve_sms = 0;                          // see nyb200_set_reserved_sms
     bool launch_overlap = true;                   // see nyb200_set_launch_overlap
     cudaStream_t own_stream = nullptr;            // created by nyb200_use_own_stream, destroyed with the engine
@@ -267,6 +268,9 @@ namespace nyb {
 // Returns a device buffer of at least `bytes` under `name` (grow-only); nullptr on failure.
 void *ws_get(nyb200_engine *e, const char *name, size_t bytes);
 int set_err(nyb200_engine *e, int code, const std::string &msg);
+// SMs that a launch may count on: the device's without those left to a concurrent collective
+// (at least two stay: a pair of CTAs has to fit).
+inline int usable_sms(const nyb200_engine *e) { return e->reserve_sms > 0 && e->sms > e->reserve_sms + 1 ? e->sms - e->reserve_sms : e->sms; }
 int check_cuda(nyb200_engine *e, cudaError_t st, const char *what);
 
 // ---- kernel launchers (nyb200_kernels.cu) ----

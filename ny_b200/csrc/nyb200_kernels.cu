@@ -970,7 +970,7 @@ void launch_relax(nyb200_engine *e, const NetView &nv, int r, int lin_k, int M, 
         // 16 warps fit an SM: a slab's rows are shared by two warps while one each would be fewer than three rounds of them
         // (1000 domains, 256 columns: 20 -> 16 us; fewer registers for 24 warps spilled and was slower)
         const long slab_warps = (long)D * ((n + 127) / 128);
-        const int parts = slab_warps < 148 * 16 * 3 ? 2 : 1;
+        const int parts = slab_warps < (long)usable_sms(e) * 16 * 3 ? 2 : 1;
         const long dwarps = slab_warps * parts;
         const unsigned dgrid = (unsigned)((dwarps * 32 + 255) / 256);
 #define NYB_RELAX_DOM(RELAX, BIAS) \

@@ -494,9 +494,7 @@ int launch_umma(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int
             attr_set[dev] = true;
         }
     }
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
-    if (e->reserve_sms > 0 && sms > e->reserve_sms) sms -= e->reserve_sms;   // left to a concurrent collective
+    const int sms = usable_sms(e);
     int tiles = ((M + BM - 1) / BM) * ((L.N + BN - 1) / BN);
     int grid = tiles < sms ? tiles : sms;
     // The fp32 operand goes through TMA when a tensor map can describe it: rows of K contiguous values, base and row

@@ -604,9 +604,7 @@ static void pick_tile(int M, int N, int chunks, int sms, bool fixed, int &bn, in
 }
 
 int launch_umma_f16(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err, const ConcFuse *cf) {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
-    if (e->reserve_sms > 0 && sms > e->reserve_sms + 1) sms -= e->reserve_sms;   // left to a concurrent collective
+    const int sms = usable_sms(e);
     f16::Params P;
     P.A = A; P.lda = lda; P.M = M; P.N = L.N; P.K = L.K; P.chunks = (L.K + BK - 1) / BK;
     P.w_inv = L.w_inv; P.err = err;

@@ -169,3 +169,12 @@ def test_arrivals_at_another_ctas_barrier_state_their_scope():
                 seen += 1
                 assert re.match(r"mbarrier\.arrive\.(release|relaxed)\.cluster\.", m.group(0)), (f, m.group(0))
     assert seen
+
+
+def test_launches_ask_for_the_number_of_sms():
+    """Launches are sized by usable_sms (the device's SMs without the reserved ones): no SM count is written into the code."""
+    csrc = os.path.join(ROOT, "ny_b200", "csrc")
+    for f in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, f)) as h:
+            for i, line in enumerate(h, 1):
+                assert not re.search(r"(?<![\w.])148(?![\w.])", line.split("//")[0]), (f, i, line.strip())
