@@ -52,7 +52,6 @@ struct Params {
     float w_inv;
     float *out;
     long ldo;
-    unsigned *row_max;                           // [rows] largest |output| as float bits, or null
     int *err;
 };
 
@@ -262,29 +261,17 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
             const int y = (ty * TY + (pr >> 3)) * P.s, x = (tx * TX + (pr & 7)) * P.s;
             const float scale = (P.row_inv ? P.row_inv[row] : 1.f) * P.w_inv;
             float *o = P.out + (long)row * P.ldo + y * P.out_w + x;
-            float mx = 0.f;
             if (y < P.out_h && x < P.out_w) {
                 if (P.pair) {
 #pragma unroll
                     for (int j = 0; j < 16; j += 2)
-                        if (j < n_here) {
-                            const float2 v = make_float2(sum[j] * scale, sum[j + 1] * scale);
-                            *(float2 *)(o + col_off[col0 + j]) = v;
-                            mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
-                        }
+                        if (j < n_here) *(float2 *)(o + col_off[col0 + j]) = make_float2(sum[j] * scale, sum[j + 1] * scale);
                 } else {
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        if (j < n_here && (P.exact || (y + (col_off[NB + col0 + j] >> 4) < P.out_h && x + (col_off[NB + col0 + j] & 15) < P.out_w))) {
-                            const float v = sum[j] * scale;
-                            o[col_off[col0 + j]] = v;
-                            mx = fmaxf(mx, fabsf(v));   // (a NaN is caught by the concretisation, not by the scale)
-                        }
+                        if (j < n_here && (P.exact || (y + (col_off[NB + col0 + j] >> 4) < P.out_h && x + (col_off[NB + col0 + j] & 15) < P.out_w)))
+                            o[col_off[col0 + j]] = sum[j] * scale;
                 }
-            }
-            if (P.row_max) {
-                for (int s = 16; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
-                if (lane == 0 && mx > 0.f) atomicMax(P.row_max + row, __float_as_uint(mx));
             }
         }
     }
@@ -541,14 +528,11 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
     return NYB200_OK;
 }
 
-size_t win_operand_elems(const WinOp &op) { return (size_t)op.in_h * op.in_w * ((const Params *)op.params)->Cp; }
-
 // The window products of `rows` split images hi / lo (scales row_inv) into out [rows x ldo] (channel planes).
-int launch_win(nyb200_engine *e, const WinOp &op, int rows, const void *hi, const void *lo, const float *row_inv, float *out, long ldo,
-               unsigned *row_max, int *err) {
+int launch_win(nyb200_engine *e, const WinOp &op, int rows, const void *hi, const void *lo, const float *row_inv, float *out, long ldo, int *err) {
     Params P;
     memcpy(&P, op.params, sizeof(P));
-    P.rows = rows; P.row_inv = row_inv; P.out = out; P.ldo = ldo; P.row_max = row_max; P.err = err;
+    P.rows = rows; P.row_inv = row_inv; P.out = out; P.ldo = ldo; P.err = err;
     EncodeFn enc = encoder();
     alignas(64) CUtensorMap tm[2];
     const bool packed = P.Cp <= 32;
@@ -595,7 +579,7 @@ int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long l
     NYB_CUDA(e, launch_pdl(k_split_image, dim3((unsigned)rows, (unsigned)((plane + 31) / 32)), dim3(256), (size_t)64 * (P.Cp / 2 + 1) * 4, e, op.in_c, plane,
                            P.Cp, A, lda, (const unsigned *)words, hi, lo, row_inv, rpen, q_sum, R));
     e->launches += 2;
-    return launch_win(e, op, rows, hi, lo, row_inv, out, ldo, nullptr, err);
+    return launch_win(e, op, rows, hi, lo, row_inv, out, ldo, err);
 }
 
 int launch_sum_weights(nyb200_engine *e, int D, int n, const float *q, long stride, float *q_sum) {

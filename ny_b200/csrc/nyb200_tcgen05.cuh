@@ -134,16 +134,7 @@ __device__ __forceinline__ unsigned long long make_desc_sw(unsigned smem_addr, i
 __device__ __forceinline__ unsigned make_idesc_f16(int m, int n) {
     return (1u << 4) | ((unsigned)(n >> 3) << 17) | ((unsigned)(m >> 4) << 24);
 }
-__device__ __forceinline__ void mma_f16(unsigned d_tmem, unsigned long long adesc, unsigned long long bdesc, unsigned idesc,
-                                        unsigned accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// The same issued by a whole converged warp, one elected lane doing it: with every lane in the loop the descriptors are
+// A product of fp16 operands, issued by a whole converged warp with one elected lane doing it: with every lane in the loop the descriptors are
 // warp-uniform values and stay in uniform registers, where the instruction wants them; from a single-lane branch every
 // product costs some ninety cycles of moving them there, which is what a product of few columns takes.
 __device__ __forceinline__ void mma_f16_elect(unsigned d_tmem, unsigned long long adesc, unsigned long long bdesc, unsigned idesc,
