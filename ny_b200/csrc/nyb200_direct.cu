@@ -1009,18 +1009,28 @@ int crown_direct(nyb200_engine *e, int net_id, const float *spec, int S, const f
     return NYB200_OK;
 }
 
-// The cost of a domain's direct evaluation in binary64 multiply-adds (backward rows; the interval pass is a fifth of it).
-static double direct_macs(const NetView &nv, int S) {
-    double macs = 0.0;
-    for (int k = 0; k < nv.L; ++k) macs += (double)nv.dims[k] * nv.dims[k + 1];
-    return 2.0 * S * macs;
-}
-
-// Below this size a batch is evaluated directly instead of on the 3xTF32 path (which its caller then need not check for
-// visible rounding charges), if it is a batch of a few domains at all.  The tensor path costs about 40 us plus 20 us per layer whatever the batch; the direct one
-// runs at about 8e12 multiply-adds a second once it fills the GPU.
+// Is a batch evaluated directly instead of on the tensor path (whose rounding charges its caller would then have to check)?
+//
+// Fewer than 64 domains: the interval pass of so few is binary64 on either path, so the slopes are the same ones; from 64 on
+// they are those of TF32 products, and a batch must not take other lower lines because another form is faster for it (784 ->
+// 8x256 -> 10, 9 rows: 390 us directly and 399 on the tensor path at 128 domains, 592 and 415 at 256).
+// Below that, time per call directly / on the tensor path in us, 9 rows unless said otherwise, nothing flagged:
+//   784->8x256->10     16 domains 240/302   37 246/332   63 252/353       64->9x256->10 63 242/397   784->9x128->10 63 199/280
+//   784->9x400->10      4 253/369   16 348/408   37 620/464              784->9x301->10 16 313/425   37 517/469   63 523/521
+//   784->9x512->10      4 276/387   16 481/432   37 725/509              1 row: 63 domains 376/600
+// So up to 256 columns (a warp's tiles stay in its ring of weights) it is the work of all layers that decides, and the line
+// lies where 8e12 multiply-adds a second would take the tensor path's 40 us and 20 more per layer, 147 domains of the first
+// network if there were no other limit; wider layers are slower, and their line is the work of the widest one: 5e7 products.
 bool direct_pays(const nyb200_engine *e, const Net &net, int S, int D) {
-    return e->path == NYB200_PATH_TF32X3 && e->small_direct && e->fuse_chain && D <= 64 && direct_eligible(net) && direct_macs(net.v, S) * D <= 8e12 * (40e-6 + 20e-6 * net.v.L);
+    if (e->path != NYB200_PATH_TF32X3 || !e->small_direct || !e->fuse_chain || D >= 64 || !direct_eligible(net)) return false;
+    const NetView &nv = net.v;
+    double macs = 0.0, wide = 0.0;
+    for (int k = 0; k < nv.L; ++k) {
+        macs += (double)nv.dims[k] * nv.dims[k + 1];
+        if (k > 0) wide = nv.dims[k] > wide ? (double)nv.dims[k] : wide;
+    }
+    const double rows = 2.0 * S * D;
+    return rows * macs <= 8e12 * (40e-6 + 20e-6 * nv.L) && (wide <= 256.0 || rows * wide * wide <= 5e7);
 }
 
 // Interval pass of the n domains idx (null: all b.D) of the resident batch, modes 0 and 1.

@@ -49,10 +49,10 @@ def test_direct_crown_matches_the_oracle(eng, oracle, dims, boxes):
     eng.release_network(nid)
 
 
-@pytest.mark.parametrize("dims,D", [([5, 9, 3], 1), ([17, 33, 15, 4], 3), ([96, 64, 64, 64, 10], 64), ([784, 256, 256, 256, 10], 7),
+@pytest.mark.parametrize("dims,D", [([5, 9, 3], 1), ([17, 33, 15, 4], 3), ([96, 64, 64, 64, 10], 63), ([784, 256, 256, 256, 10], 7),
                                     ([40, 520, 130, 6], 2), ([30, 100, 301, 100, 10], 33)])
 def test_direct_bound_of_a_few_domains_matches_the_oracle(eng, oracle, dims, D):
-    """Batches of at most 64 domains: interval pass and backward pass in one kernel each (clusters of CTAs per domain and
+    """Batches of fewer than 64 domains: interval pass and backward pass in one kernel each (clusters of CTAs per domain and
     per group of rows), at ragged widths and row counts, split multipliers included."""
     net = W.make_mlp(dims, 500 + sum(dims) + D)
     g = np.random.Generator(np.random.PCG64(D))
@@ -115,4 +115,29 @@ def test_path_and_fusion_select_the_form(dims, D):
         for i in range(2):
             scale = np.abs(direct[i]).max()
             assert np.all(np.abs(got[i] - direct[i]) <= (5e-4 if got is tensor else 1e-5) * scale)
+    e.close()
+
+
+@pytest.mark.parametrize("dims,rows,D,direct", [
+    ([30, 40, 40, 5], 4, 63, True), ([30, 40, 40, 5], 4, 64, False),                   # 64 domains and more: TF32 intervals
+    ([784] + [256] * 8 + [10], 9, 63, True), ([20, 256, 256, 10], 9, 1, True),
+    ([20, 400, 400, 5], 4, 39, True), ([20, 400, 400, 5], 4, 40, False),               # 5e7 products of the widest layer
+    ([20, 257, 40, 5], 4, 63, True), ([20, 64, 512, 10], 9, 10, True), ([20, 64, 512, 10], 9, 11, False),
+])
+def test_which_batches_go_direct(dims, rows, D, direct):
+    from ny_b200 import B200Engine, engine
+
+    net = W.make_mlp(dims, 3)
+    x0 = np.full(dims[0], 0.4, np.float32)
+    wide = np.full(net.n_pre, 1e30, np.float32)
+    e = B200Engine(0)
+    e.set_refine_tolerance(0.0)
+    nid = e.register_network(net)
+    args = (W.margin_spec(dims[-1], 0)[:rows], x0 - np.float32(0.02), x0 + np.float32(0.02), -wide, wide, np.zeros((D, 0), SPLIT_DTYPE), np.zeros(D, np.int32))
+    got = {}
+    for path in (engine.PATH_AUTO, engine.PATH_F64, engine.PATH_TF32X3):
+        e.set_path(path)
+        got[path] = e.bab_bound_batch(nid, *args)
+    same = [p for p in (engine.PATH_F64, engine.PATH_TF32X3) if np.array_equal(got[engine.PATH_AUTO][0], got[p][0])]
+    assert same == [engine.PATH_F64 if direct else engine.PATH_TF32X3]
     e.close()
