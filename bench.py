@@ -522,7 +522,7 @@ def run_ours(args, rank, world, local_rank):
             kernel, k_ms = "k_chain", chain_ms
             k_flops = 2.0 * S2 * (dims[-1] * dims[-2] + sum(dims[k] * dims[k + 1] for k in range(1, len(dims) - 2))) * D
         else:
-            kernel, k_ms, k_flops = "k_umma_tf32x3", gemm_ms, FLOPS_PER_DOMAIN * D
+            kernel, k_ms, k_flops = "k_umma_f16", gemm_ms, FLOPS_PER_DOMAIN * D
         achieved = k_flops / (k_ms / 1e3) / 1e12 if k_ms > 0 else None
         if tf32_peak:
             peak_tf, peak_src = tf32_peak, "measured tf32 (torch.matmul with TF32 allowed, 8192^3, best of 10, this run)"
@@ -553,7 +553,7 @@ def run_ours(args, rank, world, local_rank):
             "ms_per_step_spread": {"blocks": int(blocks), "min": float(per_step.min()), "p10": float(np.percentile(per_step, 10)),
                                    "median": ms_per_step, "p90": float(np.percentile(per_step, 90)), "max": float(per_step.max())},
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f64" if eng_path_name(eng) == "f64" else "tf32x3", "data": "synthetic",
+            "dtype": dtype_of(eng_path_name(eng)), "data": "synthetic",
             "config": {"workload": "beta-CROWN bound of BaB domains, ReLU MLP 784->8x256->10, 9 spec rows (both bound "
                                    "directions), 8 splits/domain, constrained forward re-propagation",
                        "domains_per_gpu": D, "global_batch": D * world, "parallelism": f"domain-sharded x{world}",
@@ -649,7 +649,7 @@ def run_alpha_crown(args, rank, world, local_rank):
     line = {
         "metric": "alpha-CROWN domains optimised/sec (20 projected-Adam iterations)", "value": D / (ms / 1e3), "unit": UNIT,
         "n_gpus": 1, "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": ms, "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": args.path, "data": "synthetic",
+        "scaling": "weak", "vs_baseline": None, "dtype": dtype_of(args.path), "data": "synthetic",
         "config": {"workload": "alpha-CROWN optimisation, ReLU MLP 784->9x512->10, box x0+-0.015, 9 spec rows, 20 "
                                "projected-Adam iterations (lr 0.1) on per-neuron alpha, 2048 input-split cells",
                    "domains_per_gpu": D, "iterations": iters,
@@ -745,7 +745,7 @@ def run_cnn(args, local_rank, kind="cnn"):
     line = {
         "metric": METRIC, "value": D / (ms / 1e3), "unit": UNIT, "n_gpus": 1, "steps": args.steps,
         "warmup": max(args.warmup, 3), "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f64 convolutions, " + args.path + " fully connected", "data": "synthetic",
+        "dtype": dtype_of(args.path), "data": "synthetic",
         "config": {"workload": ("beta-CROWN bound of BaB domains, CNN 3x32x32 conv(16,k4,s2,p1)-conv(32,k4,s2,p1)-FC100-FC10, "
                                 "box x0+-2/255, 9 spec rows (both directions), 8 splits/domain, transposed-convolution backward")
                                if kind == "cnn" else
@@ -877,7 +877,7 @@ def run_search(args, rank, world, local_rank):
         _emit({
             "metric": "BaB domains bounded/sec (beta-CROWN), whole search loop", "value": value, "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": dt * 1e3 / args.steps, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": args.path, "data": "synthetic",
+            "scaling": "weak", "vs_baseline": None, "dtype": dtype_of(args.path), "data": "synthetic",
             "config": {"workload": f"branch and bound on a ReLU MLP 64->4x256->10, box x0+-0.05, one property row, {rounds} rounds "
                                    f"of up to {batch} domains per GPU, intercept branching, "
                                    + (f"{opt_it} optimisation iterations per domain with warm start" if opt_it > 1 else "one bound per domain")
@@ -963,7 +963,7 @@ def run_pgd(args, local_rank, kind="cnn"):
     line = {
         "metric": "PGD restart-steps/sec", "value": K * steps / (ms / 1e3), "unit": "restart-steps/s", "n_gpus": 1,
         "steps": n, "warmup": 2, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": args.path, "data": "synthetic",
+        "dtype": dtype_of(args.path), "data": "synthetic",
         "config": {"workload": ("PGD attack, 1024 restarts x 100 steps, step 0.25*eps, margin loss, CNN 3x32x32 "
                                 "conv(16,k4,s2,p1)-conv(32,k4,s2,p1)-FC100-FC10, box x0+-2/255") if kind == "cnn" else
                                ("PGD attack, 1024 restarts x 100 steps, step 0.25*eps, margin loss, residual CNN 3x32x32 "
@@ -988,6 +988,12 @@ def run_pgd(args, local_rank, kind="cnn"):
 
 def eng_path_name(eng):
     return getattr(eng, "_path_name", "tf32x3")
+
+
+def dtype_of(path):
+    """Operands as pairs of TF32 parts (interval pass, fused chain) or of fp16 parts (other contractions, convolutions), 22 bits
+    either way, fp32 sums; or binary64."""
+    return "f64" if path == "f64" else "tf32x3/fp16x3 (22-bit operands as pairs, fp32 accumulation)"
 
 
 def main():
