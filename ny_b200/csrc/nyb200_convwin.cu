@@ -418,7 +418,17 @@ double win_eps(const WinOp &op) {
 }
 
 // Window form of a convolution layer (kind: the `sel` of k_win_weights).  Leaves out->ok false where it does not apply:
-// strides over 4, weights that do not fit in shared memory next to three halo tiles.
+// strides over 4, weights that do not fit in shared memory next to three halo tiles, and transposed convolutions whose
+// im2col-space product is the faster form.  A tile costs its products whatever part of it lies inside the image, the product
+// space what is written there: the line lies at 650 elements of the space per product step of a tile.  Backward pass, 1024
+// domains of a classifier of two strided 4x4 convolutions, 8 rows each, us in all; the second one as windows / as products:
+//   16 -> 16 channels, side 32 (1820 elements a step) 1460 / 1612   28 (1394) 1446 / 1654   16 (455) 727 / 686
+//   32 -> 16           side 32 ( 910)                 2017 / 2080   28 ( 697) 2081 / 2176   16 (228) 916 / 796
+//   32 ->  8           side 32 ( 455)                 1873 / 1818   28 ( 348) 1981 / 1929   16 (114) 871 / 706
+//   16 ->  8           side 32 ( 910)                 1334 / 1367   28 ( 697) 1363 / 1375   16 (228) 696 / 597
+// and the first one (3 input channels): side 32 (683) 1612 / 1687, 28 (523) 1651 / 1609, 16 (341) 686 / 627.  Residual blocks
+// lie far on the window's side (64 channels, side 8: 1024 a step, 878 / 1654), a stem of 64 channels on 3 x 32 x 32 on the
+// other (192; 256 domains 49.7 / 48.8 ms).  The forward form has no such cases.
 int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g, int kind, WinOp *out, Carve &c) {
     out->ok = false;
     static_assert(sizeof(Params) <= sizeof(out->params), "parameter storage");
@@ -484,6 +494,8 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
     if (P.taps > MAXT || P.bx * P.in_step > 256 || P.by * P.in_step > 256) return NYB200_OK;
     for (int t = 0; t < P.taps; ++t) P.tap_off[t] = (unsigned short)(((tap_at[t].first * P.bx + tap_at[t].second) * P.swa) >> 4);
     const int ksteps = P.sw / 32;
+    const long space = (long)g.oh * g.ow * g.ic * g.kh * g.kw, steps = (long)P.taps * P.nchunk * ksteps;
+    if (kind == 0 && space < 650 * steps * P.tiles_y * P.tiles_x) return NYB200_OK;
     P.pair = P.s == 2 && P.exact && P.out_w % 2 == 0;
     P.slot_bytes = (P.bx * P.by * P.swa + 1023) / 1024 * 1024;
     // columns per CTA: as many as leave room for the weights and three halo buffers

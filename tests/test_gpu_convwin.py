@@ -17,6 +17,13 @@ NETS = [
     ((16, 9, 10), ((64, 3, 1, 1), (65, 3, 2, 1))),
     ((7, 13, 20), ((66, 4, 4, 0), (130, 3, 1, 1))),
     ((5, 12, 12), ((8, 1, 2, 0), (20, 7, 1, 3))),
+    # the backward pass takes windows where an im2col product space is large beside a tile's products (the others above it does
+    # not): the same edges with more input channels
+    ((40, 17, 9), ((16, 3, 1, 1),)),
+    ((130, 10, 9), ((65, 3, 1, 1),)),
+    ((9, 31, 17), ((16, 5, 3, 2),)),
+    ((20, 12, 12), ((20, 7, 1, 3),)),
+    ((64, 16, 16), ((64, 3, 1, 1), (64, 3, 2, 1))),
 ]
 
 

@@ -1,6 +1,6 @@
 """The rounding rates that every bound of the tensor path is charged with, element by element: |computed - exact| against
 rate * sum |a||b| plus the share of fp16's exponent range, for the contraction on fp16 pairs (nyb200_umma16.cu) and for the
-convolution windows (nyb200_convwin.cu).  Products are taken through point_vjp_batched on networks of one layer: the
+convolutions (nyb200_convwin.cu; transposed ones whose im2col products are the faster form: nyb200_umma.cu).  Products are taken through point_vjp_batched on networks of one layer: the
 gradients of K rows are rows * W (a transposed convolution), the values with unit rows are the forward product.  Operands:
 normal with rows of very different size, one sign (the largest accumulators), alternating (the most cancellation), and rows
 of a few huge values among tiny ones (the exponent range)."""
@@ -76,8 +76,11 @@ def test_contraction_on_fp16_pairs(eng, m, k, n, kind):
 
 
 # in (c, h, w), (channels, kernel, stride, padding): planes around the 8 x 16 tile, every tap parity, 16 / 32 / 64-channel pixels
-CONVS = [((1, 5, 5), (1, 1, 1, 0)), ((3, 32, 32), (16, 4, 2, 1)), ((16, 17, 9), (33, 3, 1, 1)), ((15, 16, 8), (17, 3, 2, 1)),
-         ((4, 15, 31), (31, 5, 3, 2)), ((64, 9, 10), (65, 3, 1, 1)), ((66, 12, 20), (130, 3, 2, 1)), ((5, 12, 12), (20, 7, 1, 3))]
+CONVS = [((1, 5, 5), (1, 1, 1, 0)), ((16, 17, 9), (33, 3, 1, 1)), ((15, 16, 8), (17, 3, 2, 1)),
+         ((4, 15, 31), (31, 5, 3, 2)), ((64, 9, 10), (65, 3, 1, 1)), ((66, 12, 20), (130, 3, 2, 1)), ((5, 12, 12), (20, 7, 1, 3)),
+         # ... and where the transposed form takes windows too
+         ((3, 32, 32), (16, 4, 2, 1)), ((7, 16, 8), (16, 3, 1, 1)), ((24, 17, 9), (15, 3, 1, 1)), ((56, 17, 9), (31, 3, 1, 0)), ((130, 10, 9), (65, 3, 1, 1)),
+         ((5, 30, 30), (15, 3, 2, 1)), ((9, 31, 17), (16, 5, 3, 2)), ((20, 12, 12), (20, 7, 1, 3)), ((64, 16, 16), (64, 3, 2, 1))]
 
 
 def _window(ic, oc, kh, kw, s, pad, kind):
@@ -106,6 +109,17 @@ def _win_rate(*geom):
     return (SPLIT + chain * U23 + 2 * steps * U23 * 2.0 ** -10 + (chains + 1) * U24) * 1.000001
 
 
+def _transposed_rate(ic, oc, k, s, p, oh, ow, h, w):
+    tiles = -(-(-(-h // s)) // 16) * -(-(-(-w // s)) // 8)
+    steps = _window(ic, oc, k, k, s, p, "transposed")[1]
+    if oh * ow * ic * k * k >= 650 * steps * tiles:
+        return _win_rate(ic, oc, k, k, s, p, "transposed"), True
+    stages = (oc + 31) // 32                  # im2col products on TF32 pairs: K = oc, and the cast of the sum over the taps
+    cs = 2 if stages >= 8 else 1
+    cross = 8 * U23 * (cs - 1 + 2.0 ** -10)
+    return (SPLIT + min(cs, stages) * 4 * U23 + cross + -(-stages // cs) * U24 + 5.97e-8) * 1.000001, False
+
+
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("chw,conv", CONVS)
 def test_convolution_windows(eng, chw, conv, kind):
@@ -127,7 +141,9 @@ def test_convolution_windows(eng, chw, conv, kind):
     got = eng.point_vjp_batched(nid, a, masks=zero.repeat(m, 0)).astype(np.float64)
     a64 = a.astype(np.float64)
     rest = transposed(np.ones((1, n1)), t.abs())
-    bound = _win_rate(c, oc, k, k, s, p, "transposed") * transposed(np.abs(a64), t.abs()) + (2.0 ** -48 * np.abs(a64).max(axis=1, keepdims=True) + 1e-37) * rest
+    rate, window = _transposed_rate(c, oc, k, s, p, layer.oh, layer.ow, h, w)
+    assert window == (CONVS.index((chw, conv)) >= 7)
+    bound = rate * transposed(np.abs(a64), t.abs()) + (2.0 ** -48 * np.abs(a64).max(axis=1, keepdims=True) + 1e-37) * rest
     err = np.abs(got - transposed(a64, t))
     assert np.all(err <= bound), float((err / np.maximum(bound, 1e-300)).max())
 
