@@ -429,7 +429,9 @@ __device__ __forceinline__ void relax_dom_rows(int r0, int r1, long m0, int j, f
     // Rows are taken RB at a time: all their loads are issued before the first is used, so a lane has RB
     // independent 16-byte requests in flight (a warp that walks one row after the other is latency bound), and their sums
     // are reduced together: each step halves the rows a lane holds, six shuffles for up to four rows instead of twenty.
-    constexpr int RB = 3;
+    // (Three at a time are as fast for nine rows and lose where four would be one batch: 4096 domains, 512 columns, 4 rows
+    // 1380 -> 1333 us a call, 7 rows 1840 -> 1779; the residual network's 100 domains, 4 rows, 13.8 -> 13.4 ms.)
+    constexpr int RB = 4;
     for (int rbase = r0; rbase < r1; rbase += RB) {
         float4 a[RB];
 #pragma unroll
@@ -967,10 +969,12 @@ void launch_relax(nyb200_engine *e, const NetView &nv, int r, int lin_k, int M, 
 #define NYB_RELAX_LAUNCH(RELAX, BIAS) \
     k_relax_v4<RELAX, BIAS><<<grid, 256, 0, e->stream>>>(n, off, M, R, S, (long)nv.nps, A, lda, Asrc, lds, tab, zabs, q, q_dstride, bk, aup, epsf, rb, rabs, rpen)
         const int D = M / R;
-        // 16 warps fit an SM: a slab's rows are shared by two warps while one each would be fewer than three rounds of them
-        // (1000 domains, 256 columns: 20 -> 16 us; fewer registers for 24 warps spilled and was slower)
+        // 16 warps fit an SM: a slab's rows are shared by two warps while one each would leave some of those places empty (1000
+        // domains, 256 columns: 20 -> 16 us; fewer registers for 24 warps spilled and was slower).  Not beyond: both load the
+        // slab's tables (1564 domains, 400 columns, 4 rows, two warps 686 us a call, one 650; eight such batches through
+        // three engines 3.64 and 3.38 ms)
         const long slab_warps = (long)D * ((n + 127) / 128);
-        const int parts = slab_warps < (long)usable_sms(e) * 16 * 3 ? 2 : 1;
+        const int parts = slab_warps < (long)usable_sms(e) * 16 ? 2 : 1;
         const long dwarps = slab_warps * parts;
         const unsigned dgrid = (unsigned)((dwarps * 32 + 255) / 256);
 #define NYB_RELAX_DOM(RELAX, BIAS) \
