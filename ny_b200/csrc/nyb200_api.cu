@@ -757,7 +757,7 @@ int run_forward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int fw
             const ConvGeom &g = net.geom[k];
             const int plane = g.ih * g.iw, N = 2 * g.oc * g.kh * g.kw;
             const size_t per = (size_t)2 * plane * N * 4;
-            const int most = (int)std::min<size_t>({(size_t)D, std::max<size_t>(1, kConvColsMost / per), 0x7fffffffUL / (2UL * plane)});
+            const int most = (int)std::min<size_t>({(size_t)D, std::max<size_t>(1, kConvColsMost / per), 0x7fffffffUL / (2UL * plane), 65535UL});   // (the gather's grid)
             float *cols = (float *)ws_get(e, "conv_cols", (size_t)most * per);
             if (!cols) return NYB200_ERR_OOM;
             for (int d0 = 0; d0 < D; d0 += most) {

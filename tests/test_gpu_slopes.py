@@ -110,3 +110,25 @@ def test_interval_convolution_in_slices_is_that_of_smaller_batches():
     for i in range(2):
         assert np.array_equal(whole[i][:200], first[i]) and np.array_equal(whole[i][200:], last[i])
     eng.close()
+
+
+def test_interval_convolution_of_more_domains_than_a_grid_has_rows():
+    from ny_b200 import B200Engine
+
+    net = W.make_cnn(47, (1, 4, 4), ((2, 3, 1, 1), (3, 3, 1, 1)), (2,))
+    g = np.random.Generator(np.random.PCG64(2))
+    D = 65600
+    lo = g.random((D, 16), dtype=np.float32)
+    hi = lo + np.float32(0.05)
+    wide = np.full(net.n_pre, 1e30, np.float32)
+    eng = B200Engine(0)
+    eng.set_refine_tolerance(0.0)
+    nid = eng.register_network(net)
+
+    def bounds(a, b):
+        return eng.bab_bound_batch(nid, W.margin_spec(2, 0), lo[a:b], hi[a:b], -wide, wide, np.zeros((b - a, 0), SPLIT_DTYPE), np.zeros(b - a, np.int32))
+
+    whole, last = bounds(0, D), bounds(D - 200, D)
+    for i in range(2):
+        assert np.all(np.isfinite(whole[i])) and np.allclose(whole[i][-200:], last[i], rtol=1e-5, atol=1e-5)
+    eng.close()
