@@ -37,7 +37,7 @@ constexpr int EPI_GROUPS = 4;             // epilogue groups of four warps, sixt
 constexpr int THREADS = 128 + EPI_GROUPS * 128;
 constexpr int SMEM_MOST = 226 * 1024;
 
-struct Source { int dy, dx, ntaps, tap0; };   // first halo row / column relative to the tile; its taps
+struct Source { int dy, dx, ntaps, tap0, tw; };   // first halo row / column relative to the tile; its taps, tw in a row
 
 struct Params {
     int rows, Cp, sw, swa, nchunk, Nb, N, n_blocks;   // channels padded, bytes of a weight row and of a pixel row in shared memory,
@@ -47,7 +47,6 @@ struct Params {
     int bx, by, tiles_y, tiles_x;                // halo box, tiles of a row
     int slot_bytes, slots, w_tile_bytes;
     Source src[MAXS];
-    unsigned short tap_off[MAXT];                // halo offset of a tap, in 16-byte units
     const float *row_inv;                        // [rows] scale of the row, undone; null: 1
     float w_inv;
     float *out;
@@ -60,22 +59,28 @@ struct Params {
 using namespace umma;
 using namespace win;
 
-// Roles: warp 0 loads halo tiles, warp 1 issues the products, warp 2 owns the tensor memory, the other sixteen warps are
+// Roles: warp 0 loads halo tiles, warps 1 and 3 issue the products, warp 2 owns the tensor memory, the other sixteen warps are
 // four epilogue groups of sixteen columns each: a tile of 64 columns is drained by all four at once (one tensor-memory
 // round trip per chain; a group that walked all columns took eight, and 10 of the 14 thousand cycles of a tile), narrower
 // tiles go to them in turn (a small layer's tile is a few dozen products; its way through the barriers and tensor memory
 // is longer than they take).
-// Per tile: Al*Wh over all taps into the tile's CROSS columns, then Ah*[Wh | Wl] as one product of twice the columns, in
-// chains: its first half is MAIN, the second joins CROSS.  Up to 32 channels the high and low parts share a pixel's row
-// (one load); from 64 on they are two tiles, and the low one is free for the next loads after the first pass.
+// Per tile: warp 3 adds Al*Wh and Ah*Wl over all taps into the tile's CROSS columns, warp 1 Ah*Wh in chains, each into MAIN
+// columns of its own.  Up to 32 channels the high and low parts share a pixel's row (one load); from 64 on they are two tiles,
+// and the low one is free for the next loads after its pass.
+// What bounds it: the issue of products and the drain.  A 128 x 64 x 16 product of operands in shared memory takes 48 cycles
+// of the tensor core (their bytes), so a tile of 64 columns, 9 taps and 64 channels 5.2 thousand.  From one warp, whose loop
+// the compiler took for divergent, with [Wh | Wl] as one product of 128 columns (4.0 thousand) it was 12.2 thousand; with
+// converged loops (mbar_wait_warp) 9.7; with two warps and 64-column products, which halve what the epilogue drains and
+// double its buffers, 8.5, of which 3.7 are the epilogue's stores.  1024 domains of a classifier of two strided 4x4
+// convolutions 3.08 -> 2.76 ms a call, 256 domains of a residual network 48.8 -> 45.3, its attack 50.3 -> 47.5.
 template <int KS, int NB>
 __global__ void __launch_bounds__(win::THREADS, 1)
 k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo, const __grid_constant__ CUtensorMap tm_w,
            const __grid_constant__ Params P) {
     constexpr bool PACK = KS < 4;
     constexpr int CS = NB / 16, TG = EPI_GROUPS / CS;                       // column groups, tile groups
-    constexpr int MAIN_BUFS = NB == 64 ? 3 : NB == 32 ? 5 : 8, CROSS_BUFS = NB == 64 ? 2 : NB == 32 ? 6 : 8;
-    static_assert(MAIN_BUFS * 2 * NB + CROSS_BUFS * NB <= 512, "tensor memory columns");
+    constexpr int MAIN_BUFS = NB == 64 ? 6 : NB == 32 ? 10 : 16, CROSS_BUFS = NB == 64 ? 2 : NB == 32 ? 6 : 8;
+    static_assert((MAIN_BUFS + CROSS_BUFS) * NB <= 512, "tensor memory columns");
     static_assert(CROSS_BUFS % TG == 0, "a cross buffer and its tile-start barrier belong to one group");
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -91,9 +96,9 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
     const int n_block = blockIdx.x % P.n_blocks;
     pdl_trigger();
     if (threadIdx.x == 0) {
-        for (int s = 0; s < P.slots; ++s) { mbar_init(smem_u32(&b_full[s]), 1); mbar_init(smem_u32(&b_empty[s]), 1); }
-        for (int b = 0; b < MAIN_BUFS; ++b) { mbar_init(smem_u32(&b_mf[b]), 1); mbar_init(smem_u32(&b_me[b]), 128 * CS); }
-        for (int b = 0; b < CROSS_BUFS; ++b) { mbar_init(smem_u32(&b_cf[b]), 1); mbar_init(smem_u32(&b_ce[b]), 128 * CS); mbar_init(smem_u32(&b_ts[b]), 1); }
+        for (int s = 0; s < P.slots; ++s) { mbar_init(smem_u32(&b_full[s]), 1); mbar_init(smem_u32(&b_empty[s]), 2); }
+        for (int b = 0; b < MAIN_BUFS; ++b) { mbar_init(smem_u32(&b_mf[b]), 1); mbar_init(smem_u32(&b_me[b]), 4 * CS); }
+        for (int b = 0; b < CROSS_BUFS; ++b) { mbar_init(smem_u32(&b_cf[b]), 1); mbar_init(smem_u32(&b_ce[b]), 4 * CS); mbar_init(smem_u32(&b_ts[b]), 1); }
         mbar_init(smem_u32(b_w), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -139,74 +144,96 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                 }
             }
         done_load:;
-        } else if (warp == 1) {
-            // ------------------------------------------------------------ products
-            const unsigned idesc1 = make_idesc_f16(128, NB), idesc2 = make_idesc_f16(128, 2 * NB);
+        } else if (warp == 1 || warp == 3) {
+            // ------------------------------------------------------------ products: warp 3 the cross terms, warp 1 the chains
+            const bool cross = warp == 3;
+            const unsigned idesc = make_idesc_f16(128, NB);
             // a descriptor is its constant upper word and the start address in 16-byte units plus the fixed bit 16
             const unsigned a_hi = (unsigned)(make_desc_sw(0, P.swa, (unsigned)(P.bx * P.swa)) >> 32), w_hi = (unsigned)(make_desc_sw(0, P.sw, (unsigned)(8 * P.sw)) >> 32);
-            const unsigned w_lo0 = ((smem_u32(wbase) & 0x3FFFF) >> 4) | (1u << 16), w_tap = (unsigned)(P.nchunk * 2 * P.w_tile_bytes) >> 4,
-                           w_chunk = (unsigned)(2 * P.w_tile_bytes) >> 4;
+            const unsigned w_lo0 = ((smem_u32(wbase) & 0x3FFFF) >> 4) | (1u << 16), w_part = (unsigned)P.w_tile_bytes >> 4, w_chunk = 2 * w_part,
+                           w_tap = (unsigned)P.nchunk * w_chunk;
             auto desc = [](unsigned hi, unsigned lo) { return ((unsigned long long)hi << 32) | lo; };
-            bool ok = mbar_wait_soon(smem_u32(b_w), 0);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) { atomicExch(P.err, 22); *abort_flag = 1; }
+            const unsigned px = (unsigned)P.swa >> 4;   // from a tap's pixels to the next one's
+            auto fail = [&](int code) { if (lane == 0) { atomicExch(P.err, code); *abort_flag = 1; } };
+            bool ok = mbar_wait_warp(smem_u32(b_w), 0);
+            if (!ok) fail(22);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             int sl = 0, mbuf = 0, cb = 0;
             unsigned ph = 0, mph = 1, cph = 1;
-            for (int t = t0; t < tiles && ok && !*abort_flag; t += tstep) {
-                if (!__all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_ce[cb]), cph))) { atomicExch(P.err, 23); *abort_flag = 1; break; }
+            auto next_slot = [&]() { if (++sl == P.slots) { sl = 0; ph ^= 1; } };
+            for (int t = t0; t < tiles && ok && !flag_warp(abort_flag); t += tstep) {
+                if (!mbar_wait_warp(smem_u32(&b_ce[cb]), cph)) { fail(23); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned d_cross = tmem_base + (unsigned)(MAIN_BUFS * 2 * NB + cb * NB);
-                unsigned cross_on = 0;
+                const unsigned d_cross = tmem_base + (unsigned)((MAIN_BUFS + cb) * NB);
+                unsigned on = 0;
                 bool begun = false;
                 for (int s = 0; s < P.n_src && ok; ++s) {
-                    const int nt = P.src[s].ntaps, tap0 = P.src[s].tap0;
-                    for (int ch = 0; ch < P.nchunk && ok; ++ch) {
-                        if (!__all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_full[sl]), ph))) { atomicExch(P.err, 24); *abort_flag = 1; ok = false; break; }
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        unsigned a_lo = ((smem_u32(ring + (size_t)sl * P.slot_bytes) & 0x3FFFF) >> 4) | (1u << 16);
-                        unsigned w_lo = w_lo0 + tap0 * w_tap + ch * w_chunk;
-                        for (int tap = 0; tap < nt; ++tap, w_lo += w_tap) {
-                            const unsigned a = a_lo + P.tap_off[tap0 + tap] + (PACK ? 2 * KS : 0);
+                    const int nt = P.src[s].ntaps, tap0 = P.src[s].tap0, tw = P.src[s].tw;
+                    const unsigned row_step = (unsigned)(P.bx - tw) * px;   // further, to the next row's first tap
+                    for (int ch = 0; ch < P.nchunk; ++ch) {
+                        const unsigned w0 = w_lo0 + tap0 * w_tap + ch * w_chunk;
+                        // the pixels' parts in the slot (a) times the weights' part (w), tap by tap, into the cross accumulator
+                        auto cross_pass = [&](unsigned a, unsigned w) {
+                            for (int tap = 0, tx = 0; tap < nt; ++tap) {
 #pragma unroll
-                            for (int k = 0; k < KS; ++k) {
-                                mma_f16_elect(d_cross, desc(a_hi, a + 2 * k), desc(w_hi, w_lo + 2 * k), idesc1, cross_on);
-                                cross_on = 1;
+                                for (int k = 0; k < KS; ++k) {
+                                    mma_f16_elect(d_cross, desc(a_hi, a + 2 * k), desc(w_hi, w + 2 * k), idesc, on);
+                                    on = 1;
+                                }
+                                w += w_tap;
+                                a += px;
+                                if (++tx == tw) { tx = 0; a += row_step; }
                             }
-                        }
+                        };
+                        auto start_of_slot = [&]() { return (((smem_u32(ring) + (unsigned)(sl * P.slot_bytes)) & 0x3FFFF) >> 4) | (1u << 16); };
                         if (!PACK) {
-                            mma_commit_elect(smem_u32(&b_empty[sl]));
-                            if (++sl == P.slots) { sl = 0; ph ^= 1; }
-                            if (!__all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_full[sl]), ph))) { atomicExch(P.err, 25); *abort_flag = 1; ok = false; break; }
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            a_lo = ((smem_u32(ring + (size_t)sl * P.slot_bytes) & 0x3FFFF) >> 4) | (1u << 16);
-                        }
-                        w_lo = w_lo0 + tap0 * w_tap + ch * w_chunk;
-                        for (int first = 0; first < nt && ok; first += P.tpc) {
-                            if (!__all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_me[mbuf]), mph))) { atomicExch(P.err, 26); *abort_flag = 1; ok = false; break; }
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            // The tile's groups may look at its first buffer now: the buffer's previous use, perhaps other
-                            // groups', is over.  (A barrier's parity only tells one use from the next; a group that
-                            // waited two uses ahead would take the use before the last for its own.  The other buffers'
-                            // previous uses end before this chain does: products complete in order.)  One barrier per cross buffer:
-                            // the next tile that uses it waits for this one's groups.
-                            if (!begun) { if (lane == 0) mbar_arrive(smem_u32(&b_ts[cb])); begun = true; }
-                            const unsigned d_main = tmem_base + (unsigned)(mbuf * 2 * NB);
-                            const int end = min(nt, first + P.tpc);
-                            for (int tap = first; tap < end; ++tap, w_lo += w_tap) {
-                                const unsigned a = a_lo + P.tap_off[tap0 + tap];
-#pragma unroll
-                                for (int k = 0; k < KS; ++k)
-                                    mma_f16_elect(d_main, desc(a_hi, a + 2 * k), desc(w_hi, w_lo + 2 * k), idesc2, (tap > first || k > 0) ? 1u : 0u);
+                            if (cross) {   // the low parts' tile is this warp's alone
+                                if (!mbar_wait_warp(smem_u32(&b_full[sl]), ph)) { fail(24); ok = false; break; }
+                                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                                cross_pass(start_of_slot(), w0);
+                                mma_commit_elect(smem_u32(&b_empty[sl]));
+                                mma_commit_elect(smem_u32(&b_empty[sl]));
                             }
-                            mma_commit_elect(smem_u32(&b_mf[mbuf]));
-                            if (++mbuf == MAIN_BUFS) { mbuf = 0; mph ^= 1; }
+                            next_slot();
                         }
+                        if (!mbar_wait_warp(smem_u32(&b_full[sl]), ph)) { fail(25); ok = false; break; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        unsigned a = start_of_slot(), w = w0;
+                        if (cross) {
+                            if (PACK) cross_pass(a + 2 * KS, w0);
+                            cross_pass(a, w0 + w_part);
+                        } else
+                            for (int tap = 0, tx = 0; tap < nt;) {
+                                if (!mbar_wait_warp(smem_u32(&b_me[mbuf]), mph)) { fail(26); ok = false; break; }
+                                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                                // The tile's groups may look at its first buffer now: the buffer's previous use, perhaps other
+                                // groups', is over.  (A barrier's parity only tells one use from the next; a group that
+                                // waited two uses ahead would take the use before the last for its own.  The other buffers'
+                                // previous uses end before this chain does: the chains complete in order.)  One barrier per cross
+                                // buffer: the next tile that uses it waits for this one's groups.
+                                if (!begun) { if (lane == 0) mbar_arrive(smem_u32(&b_ts[cb])); __syncwarp(); begun = true; }
+                                const unsigned d_main = tmem_base + (unsigned)(mbuf * NB);
+                                const int end = min(nt, tap + P.tpc);
+                                on = 0;
+                                for (; tap < end; ++tap) {
+#pragma unroll
+                                    for (int k = 0; k < KS; ++k) {
+                                        mma_f16_elect(d_main, desc(a_hi, a + 2 * k), desc(w_hi, w + 2 * k), idesc, on);
+                                        on = 1;
+                                    }
+                                    w += w_tap;
+                                    a += px;
+                                    if (++tx == tw) { tx = 0; a += row_step; }
+                                }
+                                mma_commit_elect(smem_u32(&b_mf[mbuf]));
+                                if (++mbuf == MAIN_BUFS) { mbuf = 0; mph ^= 1; }
+                            }
+                        if (!ok) break;
                         mma_commit_elect(smem_u32(&b_empty[sl]));
-                        if (++sl == P.slots) { sl = 0; ph ^= 1; }
+                        next_slot();
                     }
                 }
-                if (ok) mma_commit_elect(smem_u32(&b_cf[cb]));
+                if (cross && ok) mma_commit_elect(smem_u32(&b_cf[cb]));
                 if (++cb == CROSS_BUFS) { cb = 0; cph ^= 1; }
             }
         }
@@ -219,24 +246,38 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
         int cb = tgroup % CROSS_BUFS;
         unsigned cph = 0;
         for (int t = t0 + tgroup * tstep; t < tiles; t += TG * tstep) {
-            float sum[16], cs[16];
+            float sum[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) sum[j] = cs[j] = 0.f;
+            for (int j = 0; j < 16; ++j) sum[j] = 0.f;
             bool ok = __all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_ts[cb]), cph));
             if (!ok) { if (lane == 0) { atomicExch(P.err, 29); *abort_flag = 1; } break; }
-            for (int i = 0; i < P.chains && ok; ++i) {
-                ok = __all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_mf[mbuf]), mph));
+            // two chains at a time: their loads out of tensor memory overlap
+            for (int i = 0; i < P.chains && ok; i += 2) {
+                const unsigned m0 = mbuf, ph0 = mph;
+                if (++mbuf == MAIN_BUFS) { mbuf = 0; mph ^= 1; }
+                const unsigned m1 = mbuf, ph1 = mph;
+                const bool two = i + 1 < P.chains;
+                if (two && ++mbuf == MAIN_BUFS) { mbuf = 0; mph ^= 1; }
+                ok = __all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_mf[m0]), ph0));
                 if (!ok) { if (lane == 0) { atomicExch(P.err, 27); *abort_flag = 1; } break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                unsigned r[16], c[16];
-                tmem_ld16(lane_base + mbuf * 2 * NB + col0, r);
-                tmem_ld16(lane_base + mbuf * 2 * NB + NB + col0, c);
+                unsigned r[16], r1[16];
+                tmem_ld16(lane_base + m0 * NB + col0, r);
+                if (two) {
+                    ok = __all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_mf[m1]), ph1));
+                    if (!ok) { if (lane == 0) { atomicExch(P.err, 27); *abort_flag = 1; } break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    tmem_ld16(lane_base + m1 * NB + col0, r1);
+                }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(smem_u32(&b_me[mbuf]));
+                __syncwarp();
+                if (lane == 0) { mbar_arrive(smem_u32(&b_me[m0])); if (two) mbar_arrive(smem_u32(&b_me[m1])); }
 #pragma unroll
-                for (int u = 0; u < 16; ++u) { sum[u] += __uint_as_float(r[u]); cs[u] += __uint_as_float(c[u]); }
-                if (++mbuf == MAIN_BUFS) { mbuf = 0; mph ^= 1; }
+                for (int u = 0; u < 16; ++u) sum[u] += __uint_as_float(r[u]);
+                if (two)
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) sum[u] += __uint_as_float(r1[u]);
             }
             if (!ok) break;
             ok = __all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_cf[cb]), cph));
@@ -244,12 +285,13 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             {
                 unsigned c[16];
-                tmem_ld16(lane_base + MAIN_BUFS * 2 * NB + cb * NB + col0, c);
+                tmem_ld16(lane_base + (MAIN_BUFS + cb) * NB + col0, c);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(smem_u32(&b_ce[cb]));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&b_ce[cb]));
 #pragma unroll
-                for (int u = 0; u < 16; ++u) sum[u] = fmaf(__uint_as_float(c[u]) + cs[u], 4.8828125e-4f /* 2^-11 */, sum[u]);
+                for (int u = 0; u < 16; ++u) sum[u] = fmaf(__uint_as_float(c[u]), 4.8828125e-4f /* 2^-11 */, sum[u]);
             }
             // the chains and the cross buffers of the other groups' tiles lie in between
             const unsigned skip = (unsigned)((TG - 1) * P.chains) + mbuf;
@@ -469,7 +511,7 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
         span(g.kh, g.ph, ylo, yhi); span(g.kw, g.pw, xlo, xhi);
         TH = yhi - ylo + 1; TW = xhi - xlo + 1;
         P.n_src = 1;
-        P.src[0].dy = ylo; P.src[0].dx = xlo; P.src[0].ntaps = TH * TW; P.src[0].tap0 = 0;
+        P.src[0].dy = ylo; P.src[0].dx = xlo; P.src[0].ntaps = TH * TW; P.src[0].tap0 = 0; P.src[0].tw = TW;
         for (int h = 0; h < TH; ++h)
             for (int w = 0; w < TW; ++w) tap_at.push_back({h, w});
         for (int py = 0; py < s; ++py)
@@ -483,7 +525,7 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
             for (int rx = 0; rx < s && rx < g.kw; ++rx) {
                 const int th = (g.kh - ry + s - 1) / s, tw = (g.kw - rx + s - 1) / s;
                 Source &so = P.src[P.n_src++];
-                so.dy = ry - g.ph; so.dx = rx - g.pw; so.ntaps = th * tw; so.tap0 = (int)tap_at.size();
+                so.dy = ry - g.ph; so.dx = rx - g.pw; so.ntaps = th * tw; so.tap0 = (int)tap_at.size(); so.tw = tw;
                 for (int h = 0; h < th; ++h)
                     for (int w = 0; w < tw; ++w) { tap_at.push_back({h, w}); tap_index.push_back((ry + s * h) * g.kw + rx + s * w); }
                 TH = std::max(TH, th); TW = std::max(TW, tw);
@@ -492,7 +534,6 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
     P.taps = (int)tap_at.size();
     P.bx = TX + TW - 1; P.by = TY + TH - 1;
     if (P.taps > MAXT || P.bx * P.in_step > 256 || P.by * P.in_step > 256) return NYB200_OK;
-    for (int t = 0; t < P.taps; ++t) P.tap_off[t] = (unsigned short)(((tap_at[t].first * P.bx + tap_at[t].second) * P.swa) >> 4);
     const int ksteps = P.sw / 32;
     const long space = (long)g.oh * g.ow * g.ic * g.kh * g.kw, steps = (long)P.taps * P.nchunk * ksteps;
     if (kind == 0 && space < 650 * steps * P.tiles_y * P.tiles_x) return NYB200_OK;

@@ -65,6 +65,31 @@ __device__ __forceinline__ bool mbar_wait_soon(unsigned bar, unsigned parity) {
     }
 }
 
+// The wait of a converged warp that issues products.  Every exit is a vote, so the warp stays converged in the compiler's eyes
+// too and its loops' descriptors live in uniform registers, where tcgen05.mma wants them.  After a wait, or a look at a flag in
+// shared memory, that lets lanes leave one by one, they are vector values that each product first moves over: 130 SM cycles a
+// product where the tensor core takes 48 (128 x 64 x 16, operands in shared memory) to 64 (128 columns); from a single-lane
+// branch 95 to 105, and 169 instead of 128 for 256 columns.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned bar, unsigned parity) {
+    long long t0 = 0;
+    for (;;) {
+        unsigned ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (__all_sync(0xffffffffu, ok)) return true;
+        const long long now = clock64();
+        if (t0 == 0) t0 = now;
+        if (__any_sync(0xffffffffu, now - t0 > WAIT_LIMIT_CYCLES)) return false;
+    }
+}
+// A flag in shared memory, read by a converged warp.
+__device__ __forceinline__ bool flag_warp(const volatile int *flag) { return __any_sync(0xffffffffu, *flag); }
+
 __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap *tm, int x, int y, unsigned bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
