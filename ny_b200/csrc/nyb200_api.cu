@@ -737,8 +737,14 @@ int run_forward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int fw
     NYB_CUDA(e, cudaMemsetAsync(p.flags, 0, (size_t)D * 4, e->stream));
     NYB_CUDA(e, cudaMemsetAsync(p.code, 0, (size_t)D * np, e->stream));
     NYB_CUDA(e, cudaMemsetAsync(p.sbeta, 0, (size_t)D * np * 4, e->stream));
+    p.beta_max = nullptr;
+    if (e->path == NYB200_PATH_TF32X3 && fwd_mode < 2 && net.has_conv()) {   // what k_relax_image bounds its rows with
+        p.beta_max = (float *)ws_get(e, "beta_max", (size_t)nv.L * D * 4);
+        if (!p.beta_max) return NYB200_ERR_OOM;
+        NYB_CUDA(e, cudaMemsetAsync(p.beta_max, 0, (size_t)nv.L * D * 4, e->stream));
+    }
     if (fwd_mode != 2 && b.max_splits > 0)
-        launch_scatter_splits(e, nv, p.splits, p.nsplits, b.max_splits, D, p.code, p.sbeta, p.flags);
+        launch_scatter_splits(e, nv, p.splits, p.nsplits, b.max_splits, D, p.code, p.sbeta, p.flags, p.beta_max);
     for (int k = 0; k < nv.L; ++k) {
         NYB_DEADLINE(e, "interval pass");
         const float *zl, *zu;
@@ -858,11 +864,49 @@ int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float
     float *cur = p.A0, *nxt = p.A1;
     // Open identity branches (blocks may nest or overlap, several may start at the same variable): the coefficient
     // rows kept at a joining layer until the pass reaches the variable the branch starts from, one buffer per slot.
-    struct OpenSkip { float *buf; int src; };
+    struct OpenSkip { float *buf; int src; float *max; };
     std::vector<OpenSkip> open_skips;
     auto stash_slot = [&](size_t slot) -> float * {
         const std::string name = slot == 0 ? std::string("skip_coeff") : "skip_coeff_" + std::to_string(slot);
         return (float *)ws_get(e, name.c_str(), (size_t)M * p.lda * 4);
+    };
+    auto free_slot = [&]() {   // the first buffer no open branch is using
+        size_t slot = 0;
+        for (bool taken = true; taken; ) {
+            taken = false;
+            for (const OpenSkip &o : open_skips) if (o.buf == stash_slot(slot)) { taken = true; ++slot; break; }
+        }
+        return slot;
+    };
+    // Layers whose rows go through the relaxation straight into their convolution's operand (nyb200_winrelax.cu), 1: a window's
+    // pairs, 2: pixel-major rows of an im2col-space product: the tables are the interval pass's (slopes in [0, 1], multipliers
+    // the uploaded ones), nothing else reads the rows, and an identity branch is kept and joined in the same pixel order.
+    std::vector<char> image((size_t)L, 0);
+    if (tensor && !fused && !ckpt && !partial && p.beta_max && !b.external_tables && !p.alpha_up && D <= 65535) {   // (grid)
+        auto same_image = [&](int i, int j) { const ConvGeom &x = net.geom[i], &y = net.geom[j]; return net.is_conv(i) && net.is_conv(j) && x.oc == y.oc && x.oh == y.oh && x.ow == y.ow; };
+        for (int k = 0; k < L - 1; ++k) {
+            if (!net.is_conv(k) || net.geom[k].oc % 4 != 0 || net.geom[k].oc > 128) continue;
+            if (net.win_bwd[k].ok) image[k] = net.win_bwd[k].in_cp <= 128 ? 1 : 0;
+            else image[k] = net.skip_of(k) < 0 ? 2 : 0;
+        }
+        for (bool again = true; again; ) {
+            again = false;
+            std::vector<int> joins((size_t)L, 0);
+            for (int k = 0; k < L; ++k) if (net.skip_of(k) >= 0) ++joins[net.skip_of(k)];
+            for (int k = 0; k < L; ++k) {
+                const int j = net.skip_of(k);
+                if (j < 0 || (!image[k] && !image[j])) continue;
+                if (image[k] && image[j] && joins[j] == 1 && same_image(k, j)) continue;
+                image[k] = image[j] = 0;
+                again = true;
+            }
+        }
+    }
+    // can layer k's window convolution leave its result in the order layer k - 1's image wants?
+    auto pixel_result = [&](int k) {
+        if (k == 0 || !image[k - 1] || !net.is_conv(k) || !net.win_bwd[k].ok || !net.win_bwd[k].pixel_out) return false;
+        const ConvGeom &g = net.geom[k], &h = net.geom[k - 1];
+        return g.ic == h.oc && g.ih == h.oh && g.iw == h.ow;
     };
     if (!fused) {
         if (partial) launch_seed_identity(e, S, D, p.lda, cur);
@@ -910,27 +954,30 @@ int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float
         // the relaxation writes its result into the ping-pong buffer instead of over its input.
         float *dst = (ckpt && k > 0) ? ckpt[k - 1] : nxt;
         int ldd = (ckpt && k > 0) ? ld_ckpt : p.lda;
-        if (net.skip_of(k) >= 0) {
+        if (net.skip_of(k) >= 0 && !image[k]) {
             // residual block: these coefficients also multiply relu(pre_j) directly; keep them until the pass
             // reaches that variable (iteration j + 1 below)
-            size_t slot = 0;   // the first buffer no open branch is using
-            for (bool taken = true; taken; ) {
-                taken = false;
-                for (const OpenSkip &o : open_skips) if (o.buf == stash_slot(slot)) { taken = true; ++slot; break; }
-            }
-            float *stash = stash_slot(slot);
+            float *stash = stash_slot(free_slot());
             if (!stash) return NYB200_ERR_OOM;
             NYB_CUDA(e, cudaMemcpy2DAsync(stash, (size_t)p.lda * 4, cur, (size_t)p.lda * 4, (size_t)K * 4, (size_t)M,
                                           cudaMemcpyDeviceToDevice, e->stream));
-            open_skips.push_back({stash, net.skip_of(k)});
+            open_skips.push_back({stash, net.skip_of(k), nullptr});
         }
+        const bool pixel = pixel_result(k), report = k > 0 && image[k - 1] == 1 && net.is_conv(k) && tensor && net.win_bwd[k].ok;
         if (e->timing.per_kernel) cudaEventRecord(next_kev(e->timing), e->stream);
-        if (net.is_conv(k) && tensor && net.win_bwd[k].ok) {
+        if (image[k] == 1) {   // its operand is there already (below, one layer earlier)
+            void *hi, *lo;
+            float *row_inv;
+            unsigned *row_max;
+            NYB_TRY(win_operand(e, net.win_bwd[k], M, &hi, &lo, &row_inv, &row_max));
+            if (report) NYB_CUDA(e, cudaMemsetAsync(row_max, 0, (size_t)M * 4, e->stream));
+            NYB_TRY(launch_win(e, net.win_bwd[k], M, hi, lo, row_inv, dst, ldd, derr, pixel, report ? row_max : nullptr));
+        } else if (net.is_conv(k) && tensor && net.win_bwd[k].ok) {
             // window form: the row sum of the charge weights carries the share of fp16's exponent range
             NYB_WS(qsum, float *, e, "win_qsum", (size_t)D * 4);
             const bool one = q_ds(k) == 0;
             NYB_TRY(launch_sum_weights(e, one ? 1 : D, K, p.q + nv.pre_off[k], np, qsum));
-            NYB_TRY(conv_win(e, net.win_bwd[k], M, cur, p.lda, dst, ldd, p.rpen, qsum, one ? M : R, derr));
+            NYB_TRY(conv_win(e, net.win_bwd[k], M, cur, p.lda, dst, ldd, p.rpen, qsum, one ? M : R, derr, pixel, report));
         } else if (net.is_conv(k) && tensor) {
             // reshape (implicit: channel-strided operand) + GEMM with W_col on the tensor cores + col2im gather
             const ConvGeom &g = net.geom[k];
@@ -938,7 +985,8 @@ int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float
             if ((long)M * plane > 0x7fffffffL) return set_err(e, NYB200_ERR_UNSUPPORTED, "batch too large for the convolution's im2col space");
             float *cols = (float *)ws_get(e, "conv_cols", (size_t)M * plane * taps * 4);
             if (!cols) return NYB200_ERR_OOM;
-            NYB_TRY(launch_umma(e, net.umma[k], M * plane, cur, p.lda, cols, taps, derr, plane));
+            if (image[k]) NYB_TRY(launch_umma(e, net.umma[k], M * plane, cur, g.oc, cols, taps, derr, plane, nullptr, true));
+            else NYB_TRY(launch_umma(e, net.umma[k], M * plane, cur, p.lda, cols, taps, derr, plane));
             launch_col2im(e, g, M, cols, dst, ldd);
         } else if (net.is_conv(k)) {
             const ConvGeom &g = net.geom[k];
@@ -966,6 +1014,34 @@ int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float
             launch_gemm_f64(e, M, N, K, cur, p.lda, nv.W[k], N, dst, ldd, R, zin_lo, zin_hi, zin_ds, p.rpen);
         }
         if (e->timing.per_kernel) cudaEventRecord(next_kev(e->timing), e->stream);
+        if (k > 0 && image[k - 1]) {
+            const bool pairs = image[k - 1] == 1;
+            ImageBranch join{nullptr, nullptr}, keep{nullptr, nullptr};
+            for (size_t oi = 0; oi < open_skips.size(); ++oi)
+                if (open_skips[oi].src == k - 1) { join = {open_skips[oi].buf, open_skips[oi].max}; break; }
+            if (net.skip_of(k - 1) >= 0) {
+                const size_t slot = free_slot();
+                keep.rows = stash_slot(slot);
+                keep.max = (float *)ws_get(e, ("skip_max_" + std::to_string(slot)).c_str(), (size_t)M * 4);
+                if (!keep.rows || !keep.max) return NYB200_ERR_OOM;
+            }
+            void *hi = nullptr, *lo = nullptr;
+            float *row_inv = nullptr;
+            unsigned *row_max = nullptr;
+            if (pairs) {
+                NYB_TRY(win_operand(e, net.win_bwd[k - 1], M, &hi, &lo, &row_inv, &row_max));
+                if (!report) NYB_TRY(row_maxima(e, M, N, dst, ldd, row_max));
+            } else
+                keep.rows = cur;   // (its rows have been read)
+            NYB_TRY(launch_relax_image(e, net, k - 1, p, D, R, S, dst, pixel, row_max, q_ds(k - 1), eps_for(k - 1), join.rows ? &join : nullptr,
+                                       keep.rows ? &keep : nullptr, hi, lo, row_inv));
+            for (size_t oi = 0; oi < open_skips.size(); ++oi)
+                if (open_skips[oi].src == k - 1) { open_skips.erase(open_skips.begin() + (long)oi); break; }
+            if (!pairs) continue;   // the rows are in `cur`
+            if (keep.rows) open_skips.push_back({keep.rows, net.skip_of(k - 1), keep.max});
+            float *t = cur; cur = nxt; nxt = t;
+            continue;
+        }
         for (size_t oi = 0; oi < open_skips.size();) {  // dst holds the coefficients of relu(pre_{k-1}): add the identity branches
             if (open_skips[oi].src != k - 1) { ++oi; continue; }
             launch_skip_coeff(e, M, N, dst, ldd, open_skips[oi].buf, p.lda, R, p.zl, p.zu, np, nv.pre_off[k - 1], p.rpen);

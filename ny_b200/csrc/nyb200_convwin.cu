@@ -33,7 +33,7 @@ namespace win {
 
 constexpr int TX = 8, TY = 16;            // output pixels of a tile: 128 rows of the product
 constexpr int MAXS = 16, MAXT = 64;       // input sources, taps
-constexpr int EPI_GROUPS = 4;             // epilogue groups of four warps, sixteen columns each
+constexpr int EPI_GROUPS = 2;             // epilogue groups of four warps, up to 32 columns each
 constexpr int THREADS = 128 + EPI_GROUPS * 128;
 constexpr int SMEM_MOST = 226 * 1024;
 
@@ -51,6 +51,8 @@ struct Params {
     float w_inv;
     float *out;
     long ldo;
+    int pixel_major;                             // the channels of a result's pixel together, not its planes
+    unsigned *row_max;                           // largest magnitude of a result's row (bits), or null
     int *err;
 };
 
@@ -59,26 +61,24 @@ struct Params {
 using namespace umma;
 using namespace win;
 
-// Roles: warp 0 loads halo tiles, warps 1 and 3 issue the products, warp 2 owns the tensor memory, the other sixteen warps are
-// four epilogue groups of sixteen columns each: a tile of 64 columns is drained by all four at once (one tensor-memory
-// round trip per chain; a group that walked all columns took eight, and 10 of the 14 thousand cycles of a tile), narrower
-// tiles go to them in turn (a small layer's tile is a few dozen products; its way through the barriers and tensor memory
-// is longer than they take).
+// Roles: warp 0 loads halo tiles, warps 1 and 3 issue the products, warp 2 owns the tensor memory, the other eight warps are
+// two epilogue groups of up to 32 columns each: a tile of 64 columns is drained by both at once, narrower tiles go to them in
+// turn (a small layer's tile is a few dozen products; its way through the barriers and tensor memory is longer than they take).
 // Per tile: warp 3 adds Al*Wh and Ah*Wl over all taps into the tile's CROSS columns, warp 1 Ah*Wh in chains, each into MAIN
 // columns of its own.  Up to 32 channels the high and low parts share a pixel's row (one load); from 64 on they are two tiles,
 // and the low one is free for the next loads after its pass.
-// What bounds it: the issue of products and the drain.  A 128 x 64 x 16 product of operands in shared memory takes 48 cycles
-// of the tensor core (their bytes), so a tile of 64 columns, 9 taps and 64 channels 5.2 thousand.  From one warp, whose loop
-// the compiler took for divergent, with [Wh | Wl] as one product of 128 columns (4.0 thousand) it was 12.2 thousand; with
-// converged loops (mbar_wait_warp) 9.7; with two warps and 64-column products, which halve what the epilogue drains and
-// double its buffers, 8.5, of which 3.7 are the epilogue's stores.  1024 domains of a classifier of two strided 4x4
-// convolutions 3.08 -> 2.76 ms a call, 256 domains of a residual network 48.8 -> 45.3, its attack 50.3 -> 47.5.
+// What bounds it: shared memory, at three quarters of its rate.  A 128 x 64 x 16 product takes 48 cycles (its operands' bytes),
+// so a tile of 64 columns, 9 taps and 64 channels 5.2 thousand.  From one warp, whose loop the compiler took for divergent, with
+// [Wh | Wl] as one product of 128 columns (4.0 thousand), a tile took 12.2 thousand; with converged loops (mbar_wait_warp) 9.7;
+// from two warps with 64-column products, which halve what the epilogue drains and double its buffers, 8.5; with eight epilogue
+// warps instead of sixteen, results pixel-major where the next pass wants them so (the stores were 3.7 thousand of it) and the
+// warp's number shuffled, so that the compiler knows it uniform, 7.1.  All products from one warp: 9.5.
 template <int KS, int NB>
 __global__ void __launch_bounds__(win::THREADS, 1)
 k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo, const __grid_constant__ CUtensorMap tm_w,
            const __grid_constant__ Params P) {
     constexpr bool PACK = KS < 4;
-    constexpr int CS = NB / 16, TG = EPI_GROUPS / CS;                       // column groups, tile groups
+    constexpr int GC = NB >= 32 ? 32 : 16, CS = NB / GC, TG = EPI_GROUPS / CS;   // columns of a group, column groups, tile groups
     constexpr int MAIN_BUFS = NB == 64 ? 6 : NB == 32 ? 10 : 16, CROSS_BUFS = NB == 64 ? 2 : NB == 32 ? 6 : 8;
     static_assert((MAIN_BUFS + CROSS_BUFS) * NB <= 512, "tensor memory columns");
     static_assert(CROSS_BUFS % TG == 0, "a cross buffer and its tile-start barrier belong to one group");
@@ -92,7 +92,7 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
     unsigned *tmem_slot = (unsigned *)(b_w + 1);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
     int *col_off = (int *)(tmem_slot + 2);        // [NB] output offset of a column; parities of a column behind it
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (the same in a warp, as the compiler sees it too)
     const int n_block = blockIdx.x % P.n_blocks;
     pdl_trigger();
     if (threadIdx.x == 0) {
@@ -116,7 +116,7 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     pdl_wait();
-    const unsigned tmem_base = *tmem_slot;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     // this CTA's tiles t0, t0 + tstep, ...: fewer than 2^31 of them in all (launch_win)
     const int per_row = P.tiles_y * P.tiles_x, tiles = P.rows * per_row, t0 = blockIdx.x / P.n_blocks, tstep = gridDim.x / P.n_blocks;
 
@@ -175,11 +175,8 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                         // the pixels' parts in the slot (a) times the weights' part (w), tap by tap, into the cross accumulator
                         auto cross_pass = [&](unsigned a, unsigned w) {
                             for (int tap = 0, tx = 0; tap < nt; ++tap) {
-#pragma unroll
-                                for (int k = 0; k < KS; ++k) {
-                                    mma_f16_elect(d_cross, desc(a_hi, a + 2 * k), desc(w_hi, w + 2 * k), idesc, on);
-                                    on = 1;
-                                }
+                                mma_f16_group<KS>(d_cross, desc(a_hi, a), desc(w_hi, w), idesc, on);
+                                on = 1;
                                 w += w_tap;
                                 a += px;
                                 if (++tx == tw) { tx = 0; a += row_step; }
@@ -216,11 +213,8 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                                 const int end = min(nt, tap + P.tpc);
                                 on = 0;
                                 for (; tap < end; ++tap) {
-#pragma unroll
-                                    for (int k = 0; k < KS; ++k) {
-                                        mma_f16_elect(d_main, desc(a_hi, a + 2 * k), desc(w_hi, w + 2 * k), idesc, on);
-                                        on = 1;
-                                    }
+                                    mma_f16_group<KS>(d_main, desc(a_hi, a), desc(w_hi, w), idesc, on);
+                                    on = 1;
                                     w += w_tap;
                                     a += px;
                                     if (++tx == tw) { tx = 0; a += row_step; }
@@ -238,18 +232,33 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
             }
         }
     } else {
-        // ------------------------------------------------------------ epilogue: thread = one pixel, sixteen columns
-        const int q = warp & 3, group = (warp - 4) >> 2, tgroup = group / CS, col0 = (group % CS) * 16;
+        // ------------------------------------------------------------ epilogue: thread = one pixel, GC columns
+        const int q = warp & 3, group = (warp - 4) >> 2, tgroup = group / CS, col0 = (group % CS) * GC;
         const unsigned lane_base = tmem_base + ((unsigned)(q * 32) << 16);
-        const int pr = q * 32 + lane, n_here = min(16, P.N - n_block * NB - col0);
+        const int pr = q * 32 + lane, n_here = min(GC, P.N - n_block * NB - col0);
         unsigned mbuf = (unsigned)(tgroup * P.chains) % MAIN_BUFS, mph = ((unsigned)(tgroup * P.chains) / MAIN_BUFS) & 1;
         int cb = tgroup % CROSS_BUFS;
         unsigned cph = 0;
-        for (int t = t0 + tgroup * tstep; t < tiles; t += TG * tstep) {
-            float sum[16];
+        // pixel-major results: sixteen columns of this thread are channels from n_first on, of one row parity where there are two
+        int n_first[GC / 16], n_row[GC / 16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) sum[j] = 0.f;
-            bool ok = __all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_ts[cb]), cph));
+        for (int h = 0; h < GC / 16; ++h) {
+            const int n = n_block * NB + col0 + 16 * h;
+            n_first[h] = P.s == 1 ? n : (n / 2) % P.out_c; n_row[h] = P.s == 1 ? 0 : n / (2 * P.out_c);
+        }
+        auto load = [&](unsigned from, unsigned (&r)[GC]) {
+#pragma unroll
+            for (int h = 0; h < GC / 16; ++h) tmem_ld16(lane_base + from + 16 * h, *(unsigned (*)[16])&r[16 * h]);
+        };
+        for (int t = t0 + tgroup * tstep; t < tiles; t += TG * tstep) {
+            float sum[GC];
+#pragma unroll
+            for (int j = 0; j < GC; ++j) sum[j] = 0.f;
+            // where the tile's results go, and the row's scale, on its way from memory while the products run
+            const int row = t / per_row, rt = t - row * per_row, ty = rt / P.tiles_x, tx = rt - ty * P.tiles_x;
+            const int y = (ty * TY + (pr >> 3)) * P.s, x = (tx * TX + (pr & 7)) * P.s;
+            const float row_scale = P.row_inv ? __ldg(P.row_inv + row) : 1.f;
+            bool ok = mbar_wait_warp(smem_u32(&b_ts[cb]), cph);
             if (!ok) { if (lane == 0) { atomicExch(P.err, 29); *abort_flag = 1; } break; }
             // two chains at a time: their loads out of tensor memory overlap
             for (int i = 0; i < P.chains && ok; i += 2) {
@@ -258,40 +267,40 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                 const unsigned m1 = mbuf, ph1 = mph;
                 const bool two = i + 1 < P.chains;
                 if (two && ++mbuf == MAIN_BUFS) { mbuf = 0; mph ^= 1; }
-                ok = __all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_mf[m0]), ph0));
+                ok = mbar_wait_warp(smem_u32(&b_mf[m0]), ph0);
                 if (!ok) { if (lane == 0) { atomicExch(P.err, 27); *abort_flag = 1; } break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                unsigned r[16], r1[16];
-                tmem_ld16(lane_base + m0 * NB + col0, r);
+                unsigned r[GC], r1[GC];
+                load(m0 * NB + col0, r);
                 if (two) {
-                    ok = __all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_mf[m1]), ph1));
+                    ok = mbar_wait_warp(smem_u32(&b_mf[m1]), ph1);
                     if (!ok) { if (lane == 0) { atomicExch(P.err, 27); *abort_flag = 1; } break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    tmem_ld16(lane_base + m1 * NB + col0, r1);
+                    load(m1 * NB + col0, r1);
                 }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) { mbar_arrive(smem_u32(&b_me[m0])); if (two) mbar_arrive(smem_u32(&b_me[m1])); }
 #pragma unroll
-                for (int u = 0; u < 16; ++u) sum[u] += __uint_as_float(r[u]);
+                for (int u = 0; u < GC; ++u) sum[u] += __uint_as_float(r[u]);
                 if (two)
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) sum[u] += __uint_as_float(r1[u]);
+                    for (int u = 0; u < GC; ++u) sum[u] += __uint_as_float(r1[u]);
             }
             if (!ok) break;
-            ok = __all_sync(0xffffffffu, mbar_wait_soon(smem_u32(&b_cf[cb]), cph));
+            ok = mbar_wait_warp(smem_u32(&b_cf[cb]), cph);
             if (!ok) { if (lane == 0) { atomicExch(P.err, 28); *abort_flag = 1; } break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             {
-                unsigned c[16];
-                tmem_ld16(lane_base + (MAIN_BUFS + cb) * NB + col0, c);
+                unsigned c[GC];
+                load((MAIN_BUFS + cb) * NB + col0, c);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&b_ce[cb]));
 #pragma unroll
-                for (int u = 0; u < 16; ++u) sum[u] = fmaf(__uint_as_float(c[u]), 4.8828125e-4f /* 2^-11 */, sum[u]);
+                for (int u = 0; u < GC; ++u) sum[u] = fmaf(__uint_as_float(c[u]), 4.8828125e-4f /* 2^-11 */, sum[u]);
             }
             // the chains and the cross buffers of the other groups' tiles lie in between
             const unsigned skip = (unsigned)((TG - 1) * P.chains) + mbuf;
@@ -299,18 +308,65 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
             mbuf = skip % MAIN_BUFS;
             cb += TG;
             if (cb >= CROSS_BUFS) { cb -= CROSS_BUFS; cph ^= 1; }
-            const int row = t / per_row, rt = t - row * per_row, ty = rt / P.tiles_x, tx = rt - ty * P.tiles_x;
-            const int y = (ty * TY + (pr >> 3)) * P.s, x = (tx * TX + (pr & 7)) * P.s;
-            const float scale = (P.row_inv ? P.row_inv[row] : 1.f) * P.w_inv;
+            const float scale = row_scale * P.w_inv;
+            const bool inside = y < P.out_h && x < P.out_w;
+            if (P.row_max) {   // (columns past the last one are zero; so are, with even sides, the pixels past the image)
+                float m = 0.f;
+#pragma unroll
+                for (int u = 0; u < GC; ++u) m = fmaxf(m, fabsf(sum[u]));
+                // a NaN is none of its row's maxima: its products say so themselves
+                const unsigned w = __reduce_max_sync(0xffffffffu, inside ? __float_as_uint(m * scale) : 0u);
+                if (lane == 0 && w) atomicMax(P.row_max + row, w);
+            }
+            if (P.pixel_major) {
+                float *o = P.out + (long)row * P.ldo;
+                if (P.s == 1) {
+                    // Sixteen channels of a pixel are 64 bytes.  Four lanes exchange theirs so that a store is eight runs of 64
+                    // bytes and not 32 of 16 (the line looked up is what a store costs).
+#pragma unroll
+                    for (int h = 0; h < GC / 16; ++h) {
+                        float4 q4[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            q4[k] = make_float4(sum[16 * h + 4 * k] * scale, sum[16 * h + 4 * k + 1] * scale, sum[16 * h + 4 * k + 2] * scale, sum[16 * h + 4 * k + 3] * scale);
+                        auto swap4 = [&](float4 &lo4, float4 &hi4, int step) {   // this lane's part of a 2 x 2 transposition
+                            const bool up = lane & step;
+                            float4 v = up ? lo4 : hi4;
+                            v.x = __shfl_xor_sync(0xffffffffu, v.x, step); v.y = __shfl_xor_sync(0xffffffffu, v.y, step);
+                            v.z = __shfl_xor_sync(0xffffffffu, v.z, step); v.w = __shfl_xor_sync(0xffffffffu, v.w, step);
+                            if (up) lo4 = v; else hi4 = v;
+                        };
+                        swap4(q4[0], q4[1], 1); swap4(q4[2], q4[3], 1);
+                        swap4(q4[0], q4[2], 2); swap4(q4[1], q4[3], 2);
+                        const int c4 = (lane & 3) * 4, x0 = x - (lane & 3);   // four pixels of a row from x0 on, channels c4 .. c4 + 3
+                        float *o1 = o + (long)(y * P.out_w + x0) * P.out_c + n_first[h] + c4;
+                        if (y < P.out_h && 16 * h + c4 < n_here)
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                if (x0 + k < P.out_w) *(float4 *)(o1 + (long)k * P.out_c) = q4[k];
+                    }
+                } else if (inside)   // eight channels of two pixels
+#pragma unroll
+                    for (int h = 0; h < GC / 16; ++h) {
+                        if (16 * h >= n_here) break;
+                        float *o2 = o + (long)((y + n_row[h]) * P.out_w + x) * P.out_c + n_first[h];
+#pragma unroll
+                        for (int p = 0; p < 2; ++p)
+#pragma unroll
+                            for (int k = 16 * h; k < 16 * h + 16; k += 8)
+                                *(float4 *)(o2 + p * P.out_c + (k - 16 * h) / 2) = make_float4(sum[k + p] * scale, sum[k + 2 + p] * scale, sum[k + 4 + p] * scale, sum[k + 6 + p] * scale);
+                    }
+                continue;
+            }
             float *o = P.out + (long)row * P.ldo + y * P.out_w + x;
-            if (y < P.out_h && x < P.out_w) {
+            if (inside) {
                 if (P.pair) {
 #pragma unroll
-                    for (int j = 0; j < 16; j += 2)
+                    for (int j = 0; j < GC; j += 2)
                         if (j < n_here) *(float2 *)(o + col_off[col0 + j]) = make_float2(sum[j] * scale, sum[j + 1] * scale);
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
+                    for (int j = 0; j < GC; ++j)
                         if (j < n_here && (P.exact || (y + (col_off[NB + col0 + j] >> 4) < P.out_h && x + (col_off[NB + col0 + j] & 15) < P.out_w)))
                             o[col_off[col0 + j]] = sum[j] * scale;
                 }
@@ -538,6 +594,8 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
     const long space = (long)g.oh * g.ow * g.ic * g.kh * g.kw, steps = (long)P.taps * P.nchunk * ksteps;
     if (kind == 0 && space < 650 * steps * P.tiles_y * P.tiles_x) return NYB200_OK;
     P.pair = P.s == 2 && P.exact && P.out_w % 2 == 0;
+    // pixel-major: a thread's sixteen columns are whole groups of four channels of one pixel, or eight of two
+    out->pixel_out = kind == 0 && ((P.s == 1 && P.out_c % 4 == 0) || (P.s == 2 && P.exact && P.out_c % 8 == 0));
     P.slot_bytes = (P.bx * P.by * P.swa + 1023) / 1024 * 1024;
     // columns per CTA: as many as leave room for the weights and three halo buffers
     for (int nb : {64, 32, 16}) {
@@ -576,16 +634,20 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
     if (enc((CUtensorMap *)out->tm_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, block, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
             swizzle_of(P.sw), CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return set_err(e, NYB200_ERR_INTERNAL, "cuTensorMapEncodeTiled failed for a convolution operand");
-    out->in_h = kind == 0 ? g.oh : g.ih; out->in_w = kind == 0 ? g.ow : g.iw; out->in_c = Cin;
+    out->in_h = kind == 0 ? g.oh : g.ih; out->in_w = kind == 0 ? g.ow : g.iw; out->in_c = Cin; out->in_cp = P.Cp;
     memcpy(out->params, &P, sizeof(P));
     return NYB200_OK;
 }
 
 // The window products of `rows` split images hi / lo (scales row_inv) into out [rows x ldo] (channel planes).
-int launch_win(nyb200_engine *e, const WinOp &op, int rows, const void *hi, const void *lo, const float *row_inv, float *out, long ldo, int *err) {
+int launch_win(nyb200_engine *e, const WinOp &op, int rows, const void *hi, const void *lo, const float *row_inv, float *out, long ldo, int *err,
+               bool pixel_major, unsigned *row_max) {
     Params P;
     memcpy(&P, op.params, sizeof(P));
     P.rows = rows; P.row_inv = row_inv; P.out = out; P.ldo = ldo; P.err = err;
+    P.pixel_major = pixel_major ? 1 : 0; P.row_max = row_max;
+    if (pixel_major && (!op.pixel_out || (ldo & 3) || (reinterpret_cast<uintptr_t>(out) & 15)))
+        return set_err(e, NYB200_ERR_INTERNAL, "a convolution's result cannot be pixel-major");
     EncodeFn enc = encoder();
     alignas(64) CUtensorMap tm[2];
     const bool packed = P.Cp <= 32;
@@ -616,23 +678,41 @@ int launch_win(nyb200_engine *e, const WinOp &op, int rows, const void *hi, cons
     return NYB200_OK;
 }
 
-// A whole convolution of fp32 rows A [rows x lda] (channel planes) into out [rows x ldo]: row magnitudes, split, window
-// products.  rpen / q_sum / R: see k_split_image (null where nothing is certified).
-int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long lda, float *out, long ldo, double *rpen, const float *q_sum, int R, int *err) {
-    const Params &P = *(const Params *)op.params;
-    const int plane = op.in_h * op.in_w;
-    const size_t n = (size_t)rows * plane * P.Cp;
+// The operand's place in the workspace, with the words that go with it: row_inv read by the products, row_max written by them.
+int win_operand(nyb200_engine *e, const WinOp &op, int rows, void **hi, void **lo, float **row_inv, unsigned **row_max) {
+    const size_t n = (size_t)rows * op.in_h * op.in_w * op.in_cp;
     NYB_WS(buf, char *, e, "win_operand", n * 4 + 512);
     NYB_WS(words, unsigned *, e, "win_rows", (size_t)rows * 8);
-    __half *hi = (__half *)buf, *lo = hi + ((n + 127) & ~(size_t)127);
-    float *row_inv = (float *)(words + rows);
-    NYB_CUDA(e, cudaMemsetAsync(words, 0, (size_t)rows * 4, e->stream));
-    const int nr = op.in_c * plane;
-    NYB_CUDA(e, launch_pdl(k_row_absmax, dim3((unsigned)rows, (unsigned)((nr + 4095) / 4096)), dim3(256), 0, e, nr, A, lda, words));
+    *hi = buf;
+    *lo = (__half *)buf + ((n + 127) & ~(size_t)127);
+    *row_max = words;
+    *row_inv = (float *)(words + rows);
+    return NYB200_OK;
+}
+
+int row_maxima(nyb200_engine *e, int rows, int n, const float *A, long lda, unsigned *row_max) {
+    NYB_CUDA(e, cudaMemsetAsync(row_max, 0, (size_t)rows * 4, e->stream));
+    NYB_CUDA(e, launch_pdl(k_row_absmax, dim3((unsigned)rows, (unsigned)((n + 4095) / 4096)), dim3(256), 0, e, n, A, lda, row_max));
+    e->launches++;
+    return NYB200_OK;
+}
+
+// A whole convolution of fp32 rows A [rows x lda] (channel planes) into out [rows x ldo]: row magnitudes, split, window
+// products.  rpen / q_sum / R: see k_split_image (null where nothing is certified).
+int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long lda, float *out, long ldo, double *rpen, const float *q_sum, int R, int *err,
+             bool pixel_major, bool report) {
+    const Params &P = *(const Params *)op.params;
+    const int plane = op.in_h * op.in_w;
+    void *hi, *lo;
+    float *row_inv;
+    unsigned *row_max;
+    NYB_TRY(win_operand(e, op, rows, &hi, &lo, &row_inv, &row_max));
+    NYB_TRY(row_maxima(e, rows, op.in_c * plane, A, lda, row_max));
     NYB_CUDA(e, launch_pdl(k_split_image, dim3((unsigned)rows, (unsigned)((plane + 31) / 32)), dim3(256), (size_t)64 * (P.Cp / 2 + 1) * 4, e, op.in_c, plane,
-                           P.Cp, A, lda, (const unsigned *)words, hi, lo, row_inv, rpen, q_sum, R));
-    e->launches += 2;
-    return launch_win(e, op, rows, hi, lo, row_inv, out, ldo, err);
+                           P.Cp, A, lda, (const unsigned *)row_max, (__half *)hi, (__half *)lo, row_inv, rpen, q_sum, R));
+    e->launches++;
+    if (report) NYB_CUDA(e, cudaMemsetAsync(row_max, 0, (size_t)rows * 4, e->stream));
+    return launch_win(e, op, rows, hi, lo, row_inv, out, ldo, err, pixel_major, report ? row_max : nullptr);
 }
 
 int launch_sum_weights(nyb200_engine *e, int D, int n, const float *q, long stride, float *q_sum) {

@@ -73,7 +73,8 @@ struct UmmaLayer {
 // A convolution in window form (nyb200_convwin.cu): its fp16 weights, their tensor map and the kernel's parameters.
 struct WinOp {
     bool ok = false;
-    int in_h = 0, in_w = 0, in_c = 0;
+    int in_h = 0, in_w = 0, in_c = 0, in_cp = 0;     // input image; channels padded
+    bool pixel_out = false;                          // its result can be left pixel-major
     alignas(64) unsigned char tm_w[128];
     alignas(8) unsigned char params[1280];
 };
@@ -107,6 +108,7 @@ struct Net {
     std::vector<int> skip;        // per layer: index of the layer whose post-activation output is added, or -1
     bool is_conv(int k) const { return !kind.empty() && kind[k] == NYB200_LAYER_CONV2D; }
     int skip_of(int k) const { return skip.empty() ? -1 : skip[k]; }
+    bool has_conv() const { for (int v : kind) if (v == NYB200_LAYER_CONV2D) return true; return false; }
     bool has_skip() const { for (int j : skip) if (j >= 0) return true; return false; }
     // operand sets, each built by the first call that reads it
     std::vector<UmmaLayer> umma;        // backward products: a layer's own form (the fused chain builds and reads entry 0 alone)
@@ -275,7 +277,7 @@ int check_cuda(nyb200_engine *e, cudaError_t st, const char *what);
 
 // ---- kernel launchers (nyb200_kernels.cu) ----
 void launch_scatter_splits(nyb200_engine *e, const NetView &nv, const nyb200_split *sp, const int *ns, int max_splits,
-                           int D, signed char *code, float *sbeta, int *flags);
+                           int D, signed char *code, float *sbeta, int *flags, float *beta_max = nullptr);
 // Interval mat-vec of Linear_k for Deff boxes (binary64 accumulation, outward rounded).
 void launch_ibp_linear(nyb200_engine *e, const NetView &nv, int k, int Deff, const float *zl, const float *zu,
                        long in_dstride, float *raw_lo, float *raw_hi, float *q, long out_dstride);
@@ -332,6 +334,7 @@ struct BatchPtrs {
     float *a_final = nullptr;  // set by run_backward: the coefficients on the input box, [D*R x lda]
     bool keep_final = false;   // the caller reads a_final afterwards: the last contraction must store its rows
     float *cj = nullptr;       // charge weights of the fused chain, when the interval pass already wrote them
+    float *beta_max = nullptr; // [L x D] largest |multiplier| of a domain's splits in a layer, while the tables are the interval pass's
     float *alpha_up = nullptr; // dual alpha: the upper path's own lower slopes [D x nps], or null (shared with the lower path)
 };
 int batch_ptrs(nyb200_engine *e, const Net &net, const Batch &b, BatchPtrs &p);
@@ -439,15 +442,28 @@ void launch_conv_plain(nyb200_engine *e, const ConvGeom &g, int rows, const floa
 constexpr double kWinFloor = 8.8817841970012523e-16;   // 2^-50: error of a vanishing element, of its row's largest magnitude
 double win_eps(const WinOp &op);
 int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g, int kind, WinOp *out, Carve &c);
-int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long lda, float *out, long ldo, double *rpen, const float *q_sum, int R, int *err);
+int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long lda, float *out, long ldo, double *rpen, const float *q_sum, int R, int *err,
+             bool pixel_major = false, bool report = false);
+// The same in parts: its operand's place (pairs of `rows` images) and the products alone.  pixel_major: the result's channels
+// of a pixel lie together (op.pixel_out); row_max: receives every row's largest magnitude (bits, cleared by the caller), or null.
+int win_operand(nyb200_engine *e, const WinOp &op, int rows, void **hi, void **lo, float **row_inv, unsigned **row_max);
+int row_maxima(nyb200_engine *e, int rows, int n, const float *A, long lda, unsigned *row_max);
+int launch_win(nyb200_engine *e, const WinOp &op, int rows, const void *hi, const void *lo, const float *row_inv, float *out, long ldo, int *err,
+               bool pixel_major = false, unsigned *row_max = nullptr);
+// Relaxation between two of them (nyb200_winrelax.cu).  Rows kept for, or joining from, an identity branch: pixel-major, with
+// their largest magnitudes.
+struct ImageBranch { float *rows; float *max; };
+int launch_relax_image(nyb200_engine *e, const Net &net, int lin, const BatchPtrs &p, int D, int R, int S, const float *A, bool pixel_major, const unsigned *row_max,
+                       long q_ds, double eps, const ImageBranch *join, const ImageBranch *keep, void *hi, void *lo, float *row_inv);
 int launch_sum_weights(nyb200_engine *e, int D, int n, const float *q, long stride, float *q_sum);
 
 // ---- tcgen05 contraction (nyb200_umma.cu) ----
 int umma_prepare_layer(nyb200_engine *e, const WeightSource &src, int K, int N, UmmaLayer *out, Carve &c);
 // a_plane > 0 selects the transposed-convolution form: GEMM row r = (m, p) with p < a_plane, operand element
-// k at A[m * lda + k * a_plane + p], result column n at C[(m * N + n) * a_plane + p] (ldc unused).
+// k at A[m * lda + k * a_plane + p], result column n at C[(m * N + n) * a_plane + p] (ldc unused).  pixel_major: the operand's
+// GEMM rows lie lda apart, their elements together, as without a_plane.
 int launch_umma(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err,
-                int a_plane = 0, const ConcFuse *cf = nullptr);
+                int a_plane = 0, const ConcFuse *cf = nullptr, bool pixel_major = false);
 // The same on fp16 operand pairs (nyb200_umma16.cu).
 int umma_prepare_f16(nyb200_engine *e, const WeightSource &src, int K, int N, float wmax, UmmaLayer *out, Carve &c);
 int launch_umma_f16(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err, const ConcFuse *cf = nullptr);

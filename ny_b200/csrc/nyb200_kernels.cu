@@ -42,7 +42,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 // ---------------------------------------------------------------- split scatter
 __global__ void k_scatter_splits(NetView nv, const nyb200_split *__restrict__ sp, const int *__restrict__ ns,
                                  int max_splits, int D, signed char *__restrict__ code, float *__restrict__ sbeta,
-                                 int *__restrict__ flags) {
+                                 int *__restrict__ flags, float *__restrict__ beta_max) {
     pdl_trigger();
     pdl_wait();
     long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -59,6 +59,7 @@ __global__ void k_scatter_splits(NetView nv, const nyb200_split *__restrict__ sp
     code[o] = (signed char)c.sign;
     // A non-finite multiplier is skipped, as relu_backward.rs:156-173 does.
     sbeta[o] = isfinite(c.beta) ? c.beta * (float)c.sign : 0.0f;
+    if (beta_max && isfinite(c.beta)) atomicMax((int *)beta_max + (long)c.relu * D + d, __float_as_int(fabsf(c.beta)));
 }
 
 // ---------------------------------------------------------------- interval mat-vec (Linear IBP)
@@ -876,10 +877,10 @@ k_skip_coeff_v4(int M, int n, float *__restrict__ A, int lda, const float *__res
 #define NYB_COUNT(e) ((e)->launches++)
 
 void launch_scatter_splits(nyb200_engine *e, const NetView &nv, const nyb200_split *sp, const int *ns, int max_splits,
-                           int D, signed char *code, float *sbeta, int *flags) {
+                           int D, signed char *code, float *sbeta, int *flags, float *beta_max) {
     long total = (long)D * max_splits;
     if (total == 0) return;
-    k_scatter_splits<<<(unsigned)((total + 255) / 256), 256, 0, e->stream>>>(nv, sp, ns, max_splits, D, code, sbeta, flags);
+    k_scatter_splits<<<(unsigned)((total + 255) / 256), 256, 0, e->stream>>>(nv, sp, ns, max_splits, D, code, sbeta, flags, beta_max);
     NYB_COUNT(e);
 }
 

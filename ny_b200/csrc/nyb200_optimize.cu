@@ -427,6 +427,7 @@ int optimize_batch(nyb200_engine *e, const nyb200_opt_config &cfg, float *grad_h
     bool clear = b.external_tables;
     if (!b.external_tables && direct) NYB_TRY(run_forward_direct(e, *net, b, p, b.mode, nullptr, D));
     else if (!b.external_tables) NYB_TRY(run_forward(e, *net, b, p, b.mode));
+    p.beta_max = nullptr;   // the multipliers change from here on
     if (dual) {
         long na = (long)D * np;
         k_init_alpha_up<<<(unsigned)((na + 255) / 256), 256, 0, e->stream>>>(na, p.tab, p.alpha_up);

@@ -70,10 +70,13 @@ __device__ __forceinline__ bool mbar_wait_soon(unsigned bar, unsigned parity) {
 // shared memory, that lets lanes leave one by one, they are vector values that each product first moves over: 130 SM cycles a
 // product where the tensor core takes 48 (128 x 64 x 16, operands in shared memory) to 64 (128 columns); from a single-lane
 // branch 95 to 105, and 169 instead of 128 for 256 columns.
+template <bool HINT = false>
 __device__ __forceinline__ bool mbar_wait_warp(unsigned bar, unsigned parity) {
     long long t0 = 0;
     for (;;) {
         unsigned ok;
+        if (HINT) ok = mbar_probe(bar, parity, WAIT_HINT_NS);
+        else
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -171,6 +174,32 @@ __device__ __forceinline__ void mma_f16_elect(unsigned d_tmem, unsigned long lon
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+// KS products along K (each 32 bytes further in both operands) of one elected lane; the first one adds to what the accumulator
+// holds or starts it.  One election and no descriptor arithmetic between them: the issuing warp shares its scheduler.
+template <int KS>
+__device__ __forceinline__ void mma_f16_group(unsigned d, unsigned long long a, unsigned long long b, unsigned idesc, unsigned accumulate) {
+    if constexpr (KS == 4)
+        asm volatile(
+            "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+            "add.s64 a1, %1, 2;\n\tadd.s64 a2, %1, 4;\n\tadd.s64 a3, %1, 6;\n\tadd.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+            "elect.sync _|q, 0xffffffff;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, t;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, t;\n\t}"
+            ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+    else if constexpr (KS == 2)
+        asm volatile(
+            "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a1, b1;\n\t"
+            "add.s64 a1, %1, 2;\n\tadd.s64 b1, %2, 2;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+            "elect.sync _|q, 0xffffffff;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n\t}"
+            ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+    else mma_f16_elect(d, a, b, idesc, accumulate);
 }
 __device__ __forceinline__ void mma_commit_elect(unsigned bar) {
     asm volatile(

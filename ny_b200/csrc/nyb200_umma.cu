@@ -480,7 +480,7 @@ int umma_prepare_layer(nyb200_engine *e, const WeightSource &src, int K, int N, 
 }
 
 int launch_umma(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int lda, float *C, int ldc, int *err,
-                int a_plane, const ConcFuse *cf) {
+                int a_plane, const ConcFuse *cf, bool pixel_major) {
     if (L.f16 && a_plane == 0) return launch_umma_f16(e, L, M, A, lda, C, ldc, err, cf);
     // the attribute is a per-device property of the function: set it once on every device that launches it
     static std::mutex attr_mu;
@@ -501,9 +501,11 @@ int launch_umma(nyb200_engine *e, const UmmaLayer &L, int M, const float *A, int
     // stride multiples of 16 bytes.  Columns past K and rows past M read as zero, like the direct loads.
     alignas(64) CUtensorMap tm_a;
     int a_tma = 0;
-    if (a_plane == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0 && lda >= L.K) {
+    if ((a_plane == 0 || pixel_major) && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0 && lda >= L.K) {
         if (make_tmap(&tm_a, A, M, L.K, lda, BM)) return set_err(e, NYB200_ERR_INTERNAL, "cuTensorMapEncodeTiled failed for the A operand");
         a_tma = 1;
+    } else if (pixel_major) {
+        return set_err(e, NYB200_ERR_INTERNAL, "a pixel-major operand of this shape cannot be loaded");
     } else {
         tm_a = *(const CUtensorMap *)L.tm_hi;  // unused by the kernel in this form; any valid map
     }

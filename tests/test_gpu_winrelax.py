@@ -1,0 +1,105 @@
+"""Relaxation between convolutions straight into the next one's operand: the whole bound on the tensor path, with the
+re-evaluation off, against binary64 contractions, whose pass goes layer by layer, over the forms the layers' rule
+accepts and refuses: channel counts at the edges of a warp's share and of the padding, odd images, strides, pixel-major
+and planar sources, identity branches that join and that are kept, more rows than a block holds, large multipliers.
+
+Slopes are given, so no tie decides a line; the bounds then differ by the tensor products' roundings, which both sides
+charge.  A window layer's rate is at most 2.5e-6 of a row's sum of magnitudes (win_eps), an im2col one's 3e-6, and up to
+six layers charge it: 1.8e-5 of that sum on either end.  A row's sum is at most a few times its domain's largest bound, so
+the bounds agree to 1e-4 of their value, or of a tenth of that largest one for rows that cancel."""
+import numpy as np
+import pytest
+
+from ny_b200 import SPLIT_DTYPE
+from ny_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def eng():
+    from ny_b200 import B200Engine
+
+    e = B200Engine(0)
+    yield e
+    e.close()
+
+
+def _conv(g, ci, co, k, s, p, hw):
+    from ny_b200 import Conv2d
+
+    return Conv2d((g.standard_normal((co, ci, k, k)) * np.sqrt(2.0 / (ci * k * k))).astype(np.float32),
+                  (g.standard_normal(co) * 0.1).astype(np.float32), (s, s), (p, p), hw)
+
+
+def _net(chw, convs, skips, n_out, seed):
+    from ny_b200 import Network
+
+    g = np.random.default_rng(seed)
+    c, h, w = chw
+    layers = []
+    for co, k, s, p in convs:
+        layers.append(_conv(g, c, co, k, s, p, (h, w)))
+        c, h, w = co, layers[-1].oh, layers[-1].ow
+    n = c * h * w
+    fc = (g.standard_normal((n_out, n)) * np.sqrt(2.0 / n)).astype(np.float32)
+    return Network(layers + [fc], [None] * len(layers) + [(g.standard_normal(n_out) * 0.1).astype(np.float32)], skips)
+
+
+K3 = (3, 1, 1)   # kernel, stride, padding
+CASES = [
+    # image, convolutions, identity branches, specification rows, domains, multipliers
+    ((3, 12, 10), [(12, *K3), (20, 4, 2, 1)], {}, 1, 70, 1.0),
+    ((2, 9, 7), [(16, *K3), (33, *K3), (36, *K3)], {}, 3, 70, 1.0),          # 33 channels: no image of that layer
+    ((3, 7, 9), [(64, *K3), (96, *K3), (64, *K3)], {}, 4, 66, 1.0),          # 96 channels: padded to 128
+    ((3, 8, 8), [(160, *K3), (32, *K3), (128, *K3)], {}, 2, 64, 1.0),        # 160: too many for a block
+    ((3, 8, 8), [(16, *K3)] * 5, {2: 0, 4: 2}, 9, 70, 1.0),                  # stem by im2col, branches kept and joined
+    ((3, 16, 16), [(64, *K3)] * 5, {2: 0, 4: 2}, 5, 64, 1.0),
+    ((3, 8, 8), [(16, *K3)] * 5, {2: 0, 4: 0}, 2, 70, 1.0),                  # two branches join one layer: not in one pass
+    ((3, 8, 8), [(16, *K3)] * 5, {3: 0, 4: 1}, 2, 70, 1.0),                  # overlapping branches
+    ((3, 13, 11), [(16, 4, 2, 1), (32, 4, 2, 1)], {}, 40, 20, 1.0),          # 80 rows a domain; few domains
+    ((3, 16, 12), [(8, 4, 2, 1), (16, 4, 2, 1), (24, 3, 3, 0)], {}, 6, 66, 80.0),
+]
+
+
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_rows_through_images_agree_with_binary64(eng, case):
+    from ny_b200 import engine
+
+    chw, convs, skips, S, D, scale = CASES[case]
+    net = _net(chw, convs, skips, S + 1, 90 + case)
+    g = np.random.default_rng(190 + case)
+    n0 = int(net.dims[0])
+    x = g.uniform(0, 1, n0).astype(np.float32)
+    lo, hi = (x - 0.02).astype(np.float32), (x + 0.02).astype(np.float32)
+    spec = W.margin_spec(S + 1, 0)[:S]
+    nid = eng.register_network(net)
+    pl, pu = eng.ibp_forward_gpu(nid, lo, hi)
+    rl, ru = pl[0], pu[0]
+    offs = np.concatenate([[0], np.cumsum(net.dims[1:-1])])
+    unstable = np.flatnonzero((rl[:offs[-1]] < 0) & (ru[:offs[-1]] > 0))
+    n = 6
+    edges = np.linspace(0, len(unstable), n + 1).astype(np.int64)
+    pick = unstable[edges[:-1] + (g.random((D, n)) * (edges[1:] - edges[:-1])).astype(np.int64)]
+    relu = np.searchsorted(offs, pick, side="right") - 1
+    sp = np.zeros((D, n), SPLIT_DTYPE)
+    sp["relu"], sp["neuron"] = relu, pick - offs[relu]
+    sp["sign"] = np.where(g.random((D, n)) < 0.5, 1, -1)
+    sp["beta"] = scale * g.random((D, n), dtype=np.float32)
+    ns = np.full(D, n, np.int32)
+    alpha = g.random((D, net.n_pre), dtype=np.float32)
+    out = {}
+    eng.set_refine_tolerance(0.0)
+    for path in (engine.PATH_TF32X3, engine.PATH_F64):
+        eng.set_path(path)
+        out[path] = eng.bab_bound_batch(nid, spec, lo, hi, rl, ru, sp, ns, 1, alpha)
+    eng.set_refine_tolerance(5e-5)
+    eng.set_path(engine.PATH_AUTO)
+    eng.release_network(nid)
+    (l, u, inf), (fl, fu, finf) = out[engine.PATH_TF32X3], out[engine.PATH_F64]
+    assert np.array_equal(inf, finf)
+    fin = np.isfinite(fl) & np.isfinite(fu)          # large multipliers empty a row: repaired to infinities
+    assert np.array_equal(np.isfinite(l) & np.isfinite(u), fin) and fin.mean() > 0.9
+    size = np.where(fin, np.maximum(np.abs(fl), np.abs(fu)), 0.0).max(axis=1, keepdims=True)
+    for got, want in ((l, fl), (u, fu)):
+        assert (np.abs(got - want) <= 1e-4 * np.maximum(np.abs(want), 0.1 * size))[fin].all()
