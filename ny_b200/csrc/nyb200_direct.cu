@@ -52,6 +52,13 @@ __device__ __forceinline__ float step_up(float x) {
     return (b & 0x80000000u) ? __uint_as_float(b - 1) : __uint_as_float(b + 1);
 }
 
+// Brings a line into L1: a load whose result nothing waits for (prefetch.global.L1 left the lines in L2: a table entry was
+// another 700 cycles away, for each of a warp's tiles in turn).
+__device__ __forceinline__ void touch(const void *p) {
+    unsigned v;
+    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+}
+
 __device__ __forceinline__ double eps64(int K) { return (double)(K + 2) * 1.1102230246251565e-16 * 1.000001; }
 
 // W [K x N] row-major -> float4 groups [n-tile][k-group of 16][lane]: component c of lane l is
@@ -159,6 +166,12 @@ __device__ __forceinline__ void centre(float pl, float pu, double &c, double &r)
 // Rounding rate of the interval sums: n products and their additions, the centre, the radius and the closing additions.
 __device__ __forceinline__ double gam_sweep(int n) { return eps64(n + 4); }
 
+// Weights that fit in L1 on their way there ahead of their use; a layer's reads are a chain of L2 latencies otherwise.
+__device__ __forceinline__ void warm_weights(const float *W, int n) {
+    if (n > 16384) return;
+    for (int i = threadIdx.x * 32; i < n; i += blockDim.x * 32) touch(W + i);
+}
+
 struct NoEarly { __device__ int operator()(int) const { return 0; } };
 
 // Outward rounding of an interval product and its bias: slack for the binary64 sums, directed casts.
@@ -175,6 +188,7 @@ k_crown_ibp(NetView nv, int zdim, const float *__restrict__ in_lo, const float *
             float *__restrict__ q, float *__restrict__ zl, float *__restrict__ zu, float *__restrict__ ibp_lo, float *__restrict__ ibp_hi,
             const signed char *__restrict__ code, int *__restrict__ flags) {
     pdl_trigger();
+    warm_weights(nv.W[0], nv.dims[0] * nv.dims[1]);
     pdl_wait();
     extern __shared__ double s_z[];   // two buffers of zl, zu
     const int d = blockIdx.x;
@@ -186,10 +200,11 @@ k_crown_ibp(NetView nv, int zdim, const float *__restrict__ in_lo, const float *
     for (int k = 0; k < nv.L; ++k) {
         const long o = row + nv.pre_off[k];
         const double gam = gam_sweep(nv.dims[k]);
+        if (k + 1 < nv.L) warm_weights(nv.W[k + 1], nv.dims[k + 1] * nv.dims[k + 2]);
         interval_sweep<2>(nv.W[k], nv.dims[k], 0, nv.dims[k + 1], zc, zc + zdim, k > 0, NoEarly(), [&](int j, double lo, double hi, double qq, int) {
             float l, u, qf;
             outward(lo, hi, qq, gam, nv.b[k], j, l, u, qf);
-            raw_lo[o + j] = l; raw_hi[o + j] = u; q[o + j] = qf;
+            if (k == 0) { raw_lo[o + j] = l; raw_hi[o + j] = u; q[o + j] = qf; }   // (k_crown_layer has its own image of the others)
             const int sc = (code && k < nv.L - 1) ? code[o + j] : 0;
             if (sc > 0) l = fmaxf(l, 0.f);
             else if (sc < 0) u = fminf(u, 0.f);
@@ -257,6 +272,7 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
     extern __shared__ double s_coef[];
     __shared__ double s_red[64][4];
     __shared__ int s_bad[64];
+    constexpr int KA = NT == 1 ? 4 : NT == 2 ? 2 : 1;
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const NetView &nv = pn.nv;
@@ -264,22 +280,31 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
     const int nw1 = NW / C;   // this CTA's share of the NW warps of a group
     const int mi = warp / nw1, ni = rank * nw1 + warp - mi * nw1;
     float4 *ring = (float4 *)(s_coef + bufs * MT * 8 * pitch) + warp * (kRing * NT * 32) + lane;
-    struct { int lay, nb, g, slot; } ahead = {top - 1, 0, 0, 0};   // next group to fetch
+    // Next group to fetch.  Where it lies is worked out once a layer: looking the layer up for every group, in parameters
+    // indexed by it, took longer than the group's products.
+    struct { int lay, nb, g, slot, kg, nt; const float4 *src; } ahead = {top, 0, 0, 0, 0, 0, nullptr};
+    auto next_layer = [&]() {
+        if (--ahead.lay < 0) return;
+        ahead.nb = 0;
+        ahead.kg = (nv.dims[ahead.lay + 1] + 15) >> 4; ahead.nt = (nv.dims[ahead.lay] + 7) >> 3;
+        ahead.src = pn.w[ahead.lay] + (long)ni * ahead.kg * 32 + lane;
+    };
+    if (RING) next_layer();
     auto fetch_group = [&]() {
         if (!RING) return;
         if (ahead.lay >= 0) {
-            const int kga = (nv.dims[ahead.lay + 1] + 15) >> 4, nta = (nv.dims[ahead.lay] + 7) >> 3;
-            const float4 *src = pn.w[ahead.lay] + (long)(ahead.nb + ni) * kga * 32 + ahead.g * 32 + lane;
             const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + ahead.slot * (NT * 32));
 #pragma unroll
             for (int t = 0; t < NT; ++t)
-                if (ahead.nb + ni + t * NW < nta)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + t * 512), "l"(src + (long)t * NW * kga * 32) : "memory");
+                if (ahead.nb + ni + t * NW < ahead.nt)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + t * 512), "l"(ahead.src + (long)t * NW * ahead.kg * 32) : "memory");
             ahead.slot = ahead.slot + 1 == kRing ? 0 : ahead.slot + 1;
-            if (++ahead.g == kga) {
+            ahead.src += 32;
+            if (++ahead.g == ahead.kg) {
                 ahead.g = 0;
                 ahead.nb += NW * NT;
-                if (ahead.nb >= nta) { ahead.nb = 0; --ahead.lay; }
+                if (ahead.nb >= ahead.nt) next_layer();
+                else ahead.src += (long)(NW * NT - 1) * ahead.kg * 32;   // (from the end of this tile's groups)
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -289,14 +314,16 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
 #pragma unroll 1
         for (int i = 0; i < kRing - 1; ++i) fetch_group();
     }
-    pdl_wait();
     // rows of all boxes one behind the other: a group of eight may span two boxes
     const int gr = ((int)(blockIdx.x / C) * MT + mi) * 8 + lr;
     const bool live = gr < boxes * 2 * n_rows;
     const int box = live ? gr / (2 * n_rows) : 0, r = live ? gr - box * 2 * n_rows : 0;
-    const int d = idx ? idx[box] : box;
     const bool upper = r >= n_rows;
     const int rr = upper ? r - n_rows : r;
+    if (NW > 1)   // a small launch: the rows it starts from (weights, or uploaded before the call's first kernel) into L1
+        for (int j = lq * 32; j < nv.dims[top]; j += 128) touch(seed + (long)rr * nv.dims[top] + j);
+    pdl_wait();
+    const int d = idx ? idx[box] : box;
     const PassEntry *dom = ptab + (long)d * nv.nps;
     double *cur = s_coef + (mi * 8 + lr) * pitch, *nxt = cur + (bufs > 1 ? MT * 8 * pitch : 0);
     int slot = 0;
@@ -335,18 +362,25 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
         const PassEntry *t4 = lay > 0 ? dom + nv.pre_off[lay - 1] : nullptr;
         const float *xl = in_lo + (long)d * box_ds, *xu = in_hi + (long)d * box_ds;
         for (int nb = 0; nb < nt; nb += NW * NT) {
-            double acc[NT][2];
+            // a narrow warp's products would be one dependent chain: it is cut into KA, added at the end
+            double acc[KA][NT][2];
 #pragma unroll
-            for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = 0.0;
+            for (int c = 0; c < KA; ++c)
+#pragma unroll
+                for (int t = 0; t < NT; ++t) acc[c][t][0] = acc[c][t][1] = 0.0;
             const double *arow = cur + lq;
             if (lay > 0) {   // the epilogue's table entries into L1 while the products run
 #pragma unroll
                 for (int t = 0; t < NT; ++t) {
-                    const int j = (nb + ni + t * NW) * 8 + (lane & 7);
-                    if (j < N) asm volatile("prefetch.global.L1 [%0];" ::"l"(t4 + j));
+                    const int j = (nb + ni + t * NW) * 8;
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {   // eight entries: twelve sectors, shared by the row's four lanes
+                        const char *at = (const char *)(t4 + j) + (lq + 4 * i) * 32;
+                        if (at < (const char *)(t4 + N)) touch(at);
+                    }
                 }
             }
-            const int have = (nt - nb - ni + NW - 1) / NW;   // live tiles of this warp in this sweep
+            const int have = (nt - nb - ni + NW - 1) >> (31 - __clz(NW));   // live tiles of this warp in this sweep (NW: a power of two)
             const float4 *wt = w + (long)(nb + ni) * kg * 32;
             const long ws = (long)NW * kg * 32;
             if (RING) {
@@ -361,22 +395,22 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
                         for (int t = 0; t < NT; ++t) b[t] = mine[t * 32];
                         fetch_group();
 #pragma unroll
-                        for (int t = 0; t < NT; ++t) dmma(acc[t][0], acc[t][1], a0, (double)b[t].x);
+                        for (int t = 0; t < NT; ++t) dmma(acc[0 % KA][t][0], acc[0 % KA][t][1], a0, (double)b[t].x);
 #pragma unroll
-                        for (int t = 0; t < NT; ++t) dmma(acc[t][0], acc[t][1], a1, (double)b[t].y);
+                        for (int t = 0; t < NT; ++t) dmma(acc[1 % KA][t][0], acc[1 % KA][t][1], a1, (double)b[t].y);
 #pragma unroll
-                        for (int t = 0; t < NT; ++t) dmma(acc[t][0], acc[t][1], a2, (double)b[t].z);
+                        for (int t = 0; t < NT; ++t) dmma(acc[2 % KA][t][0], acc[2 % KA][t][1], a2, (double)b[t].z);
 #pragma unroll
-                        for (int t = 0; t < NT; ++t) dmma(acc[t][0], acc[t][1], a3, (double)b[t].w);
+                        for (int t = 0; t < NT; ++t) dmma(acc[3 % KA][t][0], acc[3 % KA][t][1], a3, (double)b[t].w);
                     } else {
 #pragma unroll
                         for (int t = 0; t < NT; ++t) {
                             if (t >= have) break;
                             const float4 b = mine[t * 32];
-                            dmma(acc[t][0], acc[t][1], a0, (double)b.x);
-                            dmma(acc[t][0], acc[t][1], a1, (double)b.y);
-                            dmma(acc[t][0], acc[t][1], a2, (double)b.z);
-                            dmma(acc[t][0], acc[t][1], a3, (double)b.w);
+                            dmma(acc[0 % KA][t][0], acc[0 % KA][t][1], a0, (double)b.x);
+                            dmma(acc[1 % KA][t][0], acc[1 % KA][t][1], a1, (double)b.y);
+                            dmma(acc[2 % KA][t][0], acc[2 % KA][t][1], a2, (double)b.z);
+                            dmma(acc[3 % KA][t][0], acc[3 % KA][t][1], a3, (double)b.w);
                         }
                         fetch_group();
                     }
@@ -389,16 +423,16 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
                     const double a0 = arow[g * 16], a1 = arow[g * 16 + 4], a2 = arow[g * 16 + 8], a3 = arow[g * 16 + 12];
                     const int steps = g + 1 < kg ? 4 : tail;
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) dmma(acc[t][0], acc[t][1], a0, (double)b[t].x);
+                    for (int t = 0; t < NT; ++t) dmma(acc[0 % KA][t][0], acc[0 % KA][t][1], a0, (double)b[t].x);
                     if (steps < 2) break;
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) dmma(acc[t][0], acc[t][1], a1, (double)b[t].y);
+                    for (int t = 0; t < NT; ++t) dmma(acc[1 % KA][t][0], acc[1 % KA][t][1], a1, (double)b[t].y);
                     if (steps < 3) break;
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) dmma(acc[t][0], acc[t][1], a2, (double)b[t].z);
+                    for (int t = 0; t < NT; ++t) dmma(acc[2 % KA][t][0], acc[2 % KA][t][1], a2, (double)b[t].z);
                     if (steps < 4) break;
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) dmma(acc[t][0], acc[t][1], a3, (double)b[t].w);
+                    for (int t = 0; t < NT; ++t) dmma(acc[3 % KA][t][0], acc[3 % KA][t][1], a3, (double)b[t].w);
                 }
             } else {   // fewer tiles than the kernel is built for (a narrow layer, the last sweep)
                 for (int g = 0; g < kg; ++g) {
@@ -407,14 +441,37 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
                     for (int t = 0; t < NT; ++t) {
                         if (t >= have) break;
                         const float4 b = __ldg(wt + t * ws + g * 32);
-                        dmma(acc[t][0], acc[t][1], a0, (double)b.x);
-                        dmma(acc[t][0], acc[t][1], a1, (double)b.y);
-                        dmma(acc[t][0], acc[t][1], a2, (double)b.z);
-                        dmma(acc[t][0], acc[t][1], a3, (double)b.w);
+                        dmma(acc[0 % KA][t][0], acc[0 % KA][t][1], a0, (double)b.x);
+                        dmma(acc[1 % KA][t][0], acc[1 % KA][t][1], a1, (double)b.y);
+                        dmma(acc[2 % KA][t][0], acc[2 % KA][t][1], a2, (double)b.z);
+                        dmma(acc[3 % KA][t][0], acc[3 % KA][t][1], a3, (double)b.w);
                     }
                 }
             }
+#pragma unroll
+            for (int c = KA / 2; c > 0; c /= 2)
+#pragma unroll
+                for (int u = 0; u < c; ++u)
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) { acc[u][t][0] += acc[u + c][t][0]; acc[u][t][1] += acc[u + c][t][1]; }
             if (bufs == 1 && lay > 0) meet_rows();   // the rows are written in place
+            // The usual case without a branch, so that the coefficients' chains of conversions and table reads overlap (a row past
+            // the last one has zero coefficients and a valid table; its sums are not read): 5 of a layer's 18 thousand cycles
+            // at 256 columns, four tiles a warp, with a branch at every coefficient; 37 domains 249 -> 235 us a call.
+            if (lay > 0 && !ckpt && have >= NT && (nb + ni + (NT - 1) * NW) * 8 + 8 <= N) {
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    const int j0 = (nb + ni + t * NW) * 8 + lq * 2;
+                    const float4 *e0 = (const float4 *)(t4 + j0), *e1 = (const float4 *)(t4 + j0 + 1);
+                    const float4 f0 = e0[0], g0 = e0[1], i0 = e0[2], f1 = e1[0], g1 = e1[1], i1 = e1[2];
+                    const float c0 = cast_coeff(acc[0][t][0], upper, f0, g0.x, gp), c1 = cast_coeff(acc[0][t][1], upper, f1, g1.x, gp);
+                    double2 v;
+                    v.x = relax_step(c0, upper, f0, g0.y, __hiloint2double(__float_as_int(g0.w), __float_as_int(g0.z)), i0, rb, rp, gp);
+                    v.y = relax_step(c1, upper, f1, g1.y, __hiloint2double(__float_as_int(g1.w), __float_as_int(g1.z)), i1, rb, rp, gp);
+                    put2(nxt + j0, v);
+                }
+                continue;
+            }
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 if (t >= have) break;
@@ -425,7 +482,7 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
                         const PassEntry *te = t4 + j0;
                         const float4 f = *(const float4 *)&te->ls, g2 = *(const float4 *)&te->zlo;
                         const double cj = __hiloint2double(__float_as_int(g2.w), __float_as_int(g2.z));
-                        const float c = cast_coeff(acc[t][0], upper, f, g2.x, gp);
+                        const float c = cast_coeff(acc[0][t][0], upper, f, g2.x, gp);
                         if (ckpt) ckpt[(lay - 1) * ckpt_stride + ((long)d * 2 * n_rows + r) * lda + j0] = c;
                         v.x = relax_step(c, upper, f, g2.y, cj, *(const float4 *)&te->ui, rb, rp, gp);
                     }
@@ -433,7 +490,7 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
                         const PassEntry *te = t4 + j0 + 1;
                         const float4 f = *(const float4 *)&te->ls, g2 = *(const float4 *)&te->zlo;
                         const double cj = __hiloint2double(__float_as_int(g2.w), __float_as_int(g2.z));
-                        const float c = cast_coeff(acc[t][1], upper, f, g2.x, gp);
+                        const float c = cast_coeff(acc[0][t][1], upper, f, g2.x, gp);
                         if (ckpt) ckpt[(lay - 1) * ckpt_stride + ((long)d * 2 * n_rows + r) * lda + j0 + 1] = c;
                         v.y = relax_step(c, upper, f, g2.y, cj, *(const float4 *)&te->ui, rb, rp, gp);
                     }
@@ -443,8 +500,8 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
                     for (int h = 0; h < 2; ++h) {
                         const int j = j0 + h;
                         if (!live || j >= N) continue;
-                        const float c = (float)acc[t][h];
-                        const double e = acc[t][h] - (double)c, l = xl[j], u = xu[j];
+                        const float c = (float)acc[0][t][h];
+                        const double e = acc[0][t][h] - (double)c, l = xl[j], u = xu[j];
                         const double el = e * l, eu = e * u;   // the box may have any sign: k_gemm_f64's charge as it stands
                         rp += (upper ? fmax(el, eu) : fmax(-el, -eu)) + 2.9e-14 * fabs(e) * fmax(fabs(l), fabs(u));
                         if (!(fabsf(c) < 1e10f)) bad = true;   // is_crown_coeff_safe, crates/ny-core/src/gemm.rs:127
@@ -470,26 +527,25 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
         for (int i = 0; i < 4; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
         anybad |= __shfl_xor_sync(0xffffffffu, anybad, o);
     }
-    if (NW > 1) {
-        for (int w2 = 0; w2 < nw1; ++w2) {
-            if (ni - rank * nw1 == w2 && lq == 0) {
+    if (NW > 1) {   // the warps' sums in their order, by the row's lane of the group's first warp
+        if (lq == 0) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) s_red[mi * 8 + lr][i] = (w2 ? s_red[mi * 8 + lr][i] : 0.0) + v[i];
-                s_bad[mi * 8 + lr] = (w2 ? s_bad[mi * 8 + lr] : 0) | anybad;
-            }
-            __syncthreads();
+            for (int i = 0; i < 4; ++i) s_red[warp * 8 + lr][i] = v[i];
+            s_bad[warp * 8 + lr] = anybad;
         }
-        if (C > 1) cl.sync();
+        if (C > 1) cl.sync(); else __syncthreads();
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] = 0.0;
         anybad = 0;
-        if (ni == 0)
-            for (int p = 0; p < C; ++p) {
-                const double *o = cl.map_shared_rank(&s_red[mi * 8 + lr][0], p);
+        if (ni == 0 && lq == 0)
+            for (int p = 0; p < C; ++p)
+                for (int w2 = 0; w2 < nw1; ++w2) {
+                    const int at = (mi * nw1 + w2) * 8 + lr;
+                    const double *o = C > 1 ? cl.map_shared_rank(&s_red[at][0], p) : &s_red[at][0];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) v[i] += o[i];
-                anybad |= *cl.map_shared_rank(&s_bad[mi * 8 + lr], p);
-            }
+                    for (int i = 0; i < 4; ++i) v[i] += o[i];
+                    anybad |= C > 1 ? *cl.map_shared_rank(&s_bad[at], p) : s_bad[at];
+                }
     }
     if (ni == 0 && lq == 0 && live) {
         // 2^-40 >> (number of binary64 additions) * 2^-53, as k_concretize; the last term encloses underflowed products
@@ -516,32 +572,41 @@ __device__ __forceinline__ void repair(int f, float &l, float &u) {
 // (nyb200_crown.cu) and the pass table, one CTA per box.  c_lo null: no CROWN bounds for this layer (the first layer,
 // where the pass would repeat the interval image, and the last one, which takes the forward shortcut).
 __global__ void __launch_bounds__(512)
-k_crown_layer(NetView nv, int k, int zdim, const float *__restrict__ ibp_lo, const float *__restrict__ ibp_hi, float *raw_lo, float *raw_hi,
-              float *q, const float *__restrict__ c_lo, const float *__restrict__ c_hi, float *__restrict__ t_lo,
+k_crown_layer(NetView nv, int k, int zdim, const float *__restrict__ ibp_lo, const float *__restrict__ ibp_hi, const float *__restrict__ raw_lo, const float *__restrict__ raw_hi,
+              const float *__restrict__ q, const float *__restrict__ c_lo, const float *__restrict__ c_hi, float *__restrict__ t_lo,
               float *__restrict__ t_hi, float *zl, float *zu, PassEntry *__restrict__ ptab, const signed char *__restrict__ code,
               int *__restrict__ dflags, float *__restrict__ inter_lo, float *__restrict__ inter_hi) {
+    // The box's values in shared memory: what earlier kernels left, on its way while the image is summed, and the image.
+    extern __shared__ double s_z[];
+    float *s_ibl = (float *)(s_z + 2 * zdim), *s_ibu = s_ibl + zdim, *s_rl = s_ibu + zdim, *s_ru = s_rl + zdim, *s_q = s_ru + zdim, *s_cl = s_q + zdim,
+          *s_cu = s_cl + zdim;
     pdl_trigger();
-    pdl_wait();
     const int d = blockIdx.x, n = nv.dims[k + 1];
+    if (k > 0) warm_weights(nv.W[k], nv.dims[k] * n);
+    pdl_wait();
     const bool relu = k < nv.L - 1;
     const long o = (long)d * nv.nps + nv.pre_off[k];
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+        s_ibl[j] = ibp_lo[o + j]; s_ibu[j] = ibp_hi[o + j];
+        if (c_lo) { s_cl[j] = c_lo[(long)d * n + j]; s_cu[j] = c_hi[(long)d * n + j]; }
+        if (k == 0) { s_rl[j] = raw_lo[o + j]; s_ru[j] = raw_hi[o + j]; s_q[j] = q[o + j]; }
+    }
+    const int dfl = dflags[d];
     if (k > 0) {
-        extern __shared__ double s_z[];
         const long in = (long)d * nv.nps + nv.pre_off[k - 1];
         const int n_in = nv.dims[k];
         for (int i = threadIdx.x; i < n_in; i += blockDim.x) centre(zl[in + i], zu[in + i], s_z[i], s_z[zdim + i]);
         __syncthreads();
         const double gam = gam_sweep(n_in);
         interval_sweep<2>(nv.W[k], n_in, 0, n, s_z, s_z + zdim, true, NoEarly(), [&](int j, double lo, double hi, double qq, int) {
-            outward(lo, hi, qq, gam, nv.b[k], j, raw_lo[o + j], raw_hi[o + j], q[o + j]);
+            outward(lo, hi, qq, gam, nv.b[k], j, s_rl[j], s_ru[j], s_q[j]);
         });
-        __syncthreads();
     }
-    const int dfl = dflags[d];
+    __syncthreads();
     int unstable = 0, n_unst = 0;
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        if (!(ibp_lo[o + j] >= 0.f || ibp_hi[o + j] <= 0.f)) unstable = 1;
-        if (raw_lo[o + j] < 0.f && raw_hi[o + j] > 0.f) ++n_unst;
+        if (!(s_ibl[j] >= 0.f || s_ibu[j] <= 0.f)) unstable = 1;
+        if (s_rl[j] < 0.f && s_ru[j] > 0.f) ++n_unst;
     }
     __shared__ int s_cnt;
     if (threadIdx.x == 0) s_cnt = 0;
@@ -550,22 +615,22 @@ k_crown_layer(NetView nv, int k, int zdim, const float *__restrict__ ibp_lo, con
     __syncthreads();
     const bool sparse = s_cnt > 0 && !(1.0f - (float)s_cnt / (float)n < 0.9f);
     auto second = [&](int j, float &cl, float &cu) {
-        const float l = raw_lo[o + j], u = raw_hi[o + j];
+        const float l = s_rl[j], u = s_ru[j];
         if (c_lo == nullptr || (sparse && !(l < 0.f && u > 0.f))) { cl = l; cu = u; return; }
-        cl = c_lo[(long)d * n + j]; cu = c_hi[(long)d * n + j];
+        cl = s_cl[j]; cu = s_cu[j];
         repair(dfl, cl, cu);
     };
     int nan = 0;
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
         float cl, cu;
         second(j, cl, cu);
-        if (isnan(ibp_lo[o + j]) || isnan(ibp_hi[o + j]) || isnan(cl) || isnan(cu)) nan = 1;
+        if (isnan(s_ibl[j]) || isnan(s_ibu[j]) || isnan(cl) || isnan(cu)) nan = 1;
     }
     const bool any_nan = __syncthreads_or(nan);
     int found = 0;
     const double eps = eps64(n);
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const float il = ibp_lo[o + j], iu = ibp_hi[o + j];
+        const float il = s_ibl[j], iu = s_ibu[j];
         float l = il, u = iu;
         if (!(relu && all_stable) && !any_nan) {
             float cl, cu;
@@ -580,7 +645,7 @@ k_crown_layer(NetView nv, int k, int zdim, const float *__restrict__ ibp_lo, con
         t_lo[o + j] = l; t_hi[o + j] = u;
         const long io = (long)d * nv.n_pre + nv.pre_off[k] + j;
         inter_lo[io] = l; inter_hi[io] = u;
-        const double bias = nv.b[k] ? (double)nv.b[k][j] : 0.0, qv = q[o + j];
+        const double bias = nv.b[k] ? (double)nv.b[k][j] : 0.0, qv = s_q[j];
         PassEntry pe;
         pe.bias = bias; pe.sbeta = pe.zg = pe.zhi = pe.zlo = 0.f; pe.ui = 0.f; pe.lsu = 1.f;
         if (!relu) {   // the specification rows pass through unchanged
@@ -886,8 +951,9 @@ int launch_pass(nyb200_engine *e, const PackedNet &pn, int top, int n_rows, int 
     const size_t coef = (size_t)bufs * MT * 8 * pitch * 8;
     const int NTq = per > 8 ? 8 : per;
     const size_t ringb = (size_t)(NW / C) * MT * kRing * NTq * 512;
-    // weights that L1 keeps (shared memory takes its share of it) need no ring
-    const bool ring = NTq <= 4 && weights > 96 * 1024 && coef + ringb <= kPassMaxSmem;
+    // weights that L1 keeps (shared memory takes its share of it) need no ring, unless every CTA of the launch is the first on
+    // its SM and meets an empty L1 (one box of 5 -> 6x50 -> 5: 173 -> 162 us a call)
+    const bool ring = NTq <= 4 && (weights > 96 * 1024 || (groups + MT - 1) / MT * C <= sms) && coef + ringb <= kPassMaxSmem;
     const size_t smem = coef + (ring ? ringb : 0);
     dim3 grid((unsigned)((groups + MT - 1) / MT * C)), block((unsigned)(MT * (NW / C) * 32));
 #define NYB_PASS_AS(NT, RING)                                                                                                 \
@@ -972,10 +1038,10 @@ int crown_direct(nyb200_engine *e, int net_id, const float *spec, int S, const f
     // few boxes: a wide CTA shortens the serial chain over the layers; many: smaller ones share an SM
     const dim3 per_box((unsigned)D), box_threads(D < usable_sms(e) ? 512 : 256);
     int zdim = 0;
-    for (int k = 0; k < L; ++k) zdim = nv.dims[k] > zdim ? nv.dims[k] : zdim;
+    for (int k = 0; k <= L; ++k) zdim = nv.dims[k] > zdim ? nv.dims[k] : zdim;
     zdim = (zdim + 1) & ~1;
     NYB_TRY(allow_smem(e, (const void *)k_crown_ibp, (size_t)zdim * 32));
-    NYB_TRY(allow_smem(e, (const void *)k_crown_layer, (size_t)zdim * 16));
+    NYB_TRY(allow_smem(e, (const void *)k_crown_layer, (size_t)zdim * 44));
     NYB_CUDA(e, launch_pdl(k_crown_ibp, per_box, box_threads, (size_t)zdim * 32, e, nv, zdim, (const float *)p.in_lo, (const float *)p.in_hi, (long)box_stride,
                            p.raw_lo, p.raw_hi, p.q, p.zl, p.zu, ibp_lo, ibp_hi, code, p.flags));
     e->launches++;
@@ -983,8 +1049,8 @@ int crown_direct(nyb200_engine *e, int net_id, const float *spec, int S, const f
         NYB_DEADLINE(e, "plain CROWN");
         const bool pass = k > 0 && k < L - 1;
         if (pass) NYB_TRY(launch_pass(e, pn, k, nv.dims[k + 1], D, nullptr, nv.W[k], nv.b[k], p, box_stride, ptab, c_lo, c_hi, nullptr));
-        NYB_CUDA(e, launch_pdl(k_crown_layer, per_box, box_threads, (size_t)zdim * 16, e, nv, k, zdim, (const float *)ibp_lo, (const float *)ibp_hi, p.raw_lo,
-                               p.raw_hi, p.q, (const float *)(pass ? c_lo : nullptr), (const float *)(pass ? c_hi : nullptr), p.pre_lo,
+        NYB_CUDA(e, launch_pdl(k_crown_layer, per_box, box_threads, (size_t)zdim * 44, e, nv, k, zdim, (const float *)ibp_lo, (const float *)ibp_hi, (const float *)p.raw_lo,
+                               (const float *)p.raw_hi, (const float *)p.q, (const float *)(pass ? c_lo : nullptr), (const float *)(pass ? c_hi : nullptr), p.pre_lo,
                                p.pre_hi, p.zl, p.zu, ptab, code, p.flags, r_il, r_iu));
         e->launches++;
     }
