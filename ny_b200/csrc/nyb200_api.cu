@@ -293,11 +293,14 @@ int create_net(nyb200_engine *e, int32_t n_layers, const nyb200_layer_desc *ld, 
             const size_t nw = weights_of(k);
             NYB_CUDA(e, cudaMemcpyAsync(const_cast<float *>(net.v.W[k]), wflat + wo, nw * 4, cudaMemcpyHostToDevice, e->stream));
             wo += nw;
+            net.bmax.push_back(0.f);
             if (!l.has_bias) continue;
             if (!bflat) return set_err(e, NYB200_ERR_INVALID, "has_bias set but bflat is null");
             const size_t nb = conv ? (size_t)l.out_channels : (size_t)l.out_features;
-            for (size_t i = 0; i < nb; ++i)
+            for (size_t i = 0; i < nb; ++i) {
                 if (!std::isfinite(bflat[bo + i])) return set_err(e, NYB200_ERR_NUMERICAL, "non-finite bias");
+                net.bmax.back() = std::max(net.bmax.back(), std::fabs(bflat[bo + i]));
+            }
             const float *src = bflat + bo;
             if (conv) { expand_bias(bflat + bo, l.out_channels, l.out_h * l.out_w, expanded); src = expanded.data(); }
             NYB_CUDA(e, cudaMemcpyAsync(bias[k], src, (size_t)l.out_features * 4, cudaMemcpyHostToDevice, e->stream));

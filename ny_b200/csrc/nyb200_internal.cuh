@@ -118,6 +118,7 @@ struct Net {
     std::vector<UmmaLayer> umma_adj;    // forward products of the adjoint pass and the attack
     bool umma_whole = false;            // every entry of umma / win_bwd is there
     std::vector<float> wmax;          // per layer: largest |weight|; negative when some weight is too small beside it for fp16 pairs
+    std::vector<float> bmax;          // per layer: largest |bias|
     std::vector<WinOp> win_bwd, win_fwd;   // window forms of the convolution layers, with umma and umma_adj
     std::vector<float *> frag;        // weights in binary64-fragment order (nyb200_direct.cu)
 };
@@ -442,8 +443,17 @@ void launch_conv_plain(nyb200_engine *e, const ConvGeom &g, int rows, const floa
 constexpr double kWinFloor = 8.8817841970012523e-16;   // 2^-50: error of a vanishing element, of its row's largest magnitude
 double win_eps(const WinOp &op);
 int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g, int kind, WinOp *out, Carve &c);
+// What is done to the rows on their way into a window convolution: bias and ReLU, the result kept (in place, or not), or a mask.
+struct WinWith {
+    const float *bias = nullptr;    // [channels x plane], or null: neither bias nor ReLU
+    float bias_max = 0.f;           // its largest magnitude
+    float *keep = nullptr;
+    const float *mask = nullptr;    // rows of what has to be positive, or null
+    long keep_ld = 0, mask_ld = 0;
+    bool has_max = false;           // the rows' maxima are where win_operand puts them (reported by the products that left the rows)
+};
 int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long lda, float *out, long ldo, double *rpen, const float *q_sum, int R, int *err,
-             bool pixel_major = false, bool report = false);
+             bool pixel_major = false, bool report = false, const WinWith *with = nullptr);
 // The same in parts: its operand's place (pairs of `rows` images) and the products alone.  pixel_major: the result's channels
 // of a pixel lie together (op.pixel_out); row_max: receives every row's largest magnitude (bits, cleared by the caller), or null.
 int win_operand(nyb200_engine *e, const WinOp &op, int rows, void **hi, void **lo, float **row_inv, unsigned **row_max);

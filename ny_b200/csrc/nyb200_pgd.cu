@@ -5,6 +5,8 @@
 // bound propagation (tcgen05 3xTF32, or binary64 when that path is selected); convolutions use the plain
 // forward convolution and the transposed-convolution path.  The attack only proposes points: the value
 // returned for each restart comes from a final evaluation of its best point with binary64 contractions.
+#include <cmath>
+
 #include "nyb200_internal.cuh"
 
 namespace nyb {
@@ -15,94 +17,132 @@ struct PgdStep {
     float step, beta1, beta2, epsilon, bc2;
 };
 
+// The element-wise kernels: one row a grid row, four columns a thread where the row allows it (VEC); an index division per
+// element and one column a thread held them to a third of the copy rate (bias and ReLU of 1024 x 4096: 15.4 -> 7 us).
+#define NYB_ROWS(rows, n) dim3((unsigned)(((n) + 1023) / 1024), (unsigned)(rows)), 256
+template <class F>
+__device__ __forceinline__ void over_row(int n, bool vec, F f) {   // f(column, columns from there: 4 or 1)
+    const int j0 = blockIdx.x * 1024;
+    if (vec) {
+        const int j = j0 + threadIdx.x * 4;
+        if (j < n) f(j, 4);
+    } else
+        for (int j = j0 + threadIdx.x; j < min(n, j0 + 1024); j += 256) f(j, 1);
+}
+static bool vec4(int n, long ld, const void *a, const void *b = nullptr, const void *c = nullptr, const void *d = nullptr) {
+    return n % 4 == 0 && ld % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d)) & 15) == 0;
+}
+
 // z += bias; optionally ReLU.  Post-activations are kept: z > 0 afterwards is exactly the gradient mask.
-__global__ void k_bias_act(long rows, int n, float *__restrict__ Z, int ld, const float *__restrict__ bias, int relu) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= rows * n) return;
-    long r = t / n;
-    int j = (int)(t - r * n);
-    float v = Z[r * ld + j] + (bias ? bias[j] : 0.f);
-    Z[r * ld + j] = relu ? fmaxf(v, 0.f) : v;
+__global__ void __launch_bounds__(256) k_bias_act(int n, float *__restrict__ Z, long ld, const float *__restrict__ bias, int relu, bool vec) {
+    float *z = Z + (long)blockIdx.y * ld;
+    auto one = [&](float x, float b) { const float v = x + b; return relu ? fmaxf(v, 0.f) : v; };
+    over_row(n, vec, [&](int j, int w) {
+        if (w == 4) {
+            float4 x = *(float4 *)(z + j);
+            const float4 b = bias ? *(const float4 *)(bias + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            *(float4 *)(z + j) = make_float4(one(x.x, b.x), one(x.y, b.y), one(x.z, b.z), one(x.w, b.w));
+        } else z[j] = one(z[j], bias ? bias[j] : 0.f);
+    });
 }
 
 // Per restart: margins spec[s] . y, the smallest one and its row.  `track`: the step's point competes for the
 // restart's best objective (improved[r] tells k_keep_best to copy the point).  `seed`: G[r] = spec[row].
-__global__ void k_pgd_objective(int K, int S, int nL, const float *__restrict__ Y, int ldy, const float *__restrict__ spec,
+__global__ void __launch_bounds__(256) k_pgd_objective(int K, int S, int nL, const float *__restrict__ Y, int ldy, const float *__restrict__ spec,
                                 float *__restrict__ best, int *__restrict__ improved, float *__restrict__ G, int ldg,
                                 float *__restrict__ value_out) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
+    // one warp per restart, a lane per specification row (one thread per restart was a chain of S * nL loads: 17.7 us for 1024)
+    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (r >= K) return;
     const float *y = Y + (long)r * ldy;
     float mv = INFINITY;
     int ms = 0;
     bool bad = false;
-    for (int s = 0; s < S; ++s) {
+    for (int s = lane; s < S; s += 32) {
         double acc = 0.0;
         for (int j = 0; j < nL; ++j) acc = fma((double)spec[s * nL + j], (double)y[j], acc);
         float m = (float)acc;
         if (isnan(m)) bad = true;
         if (m < mv) { mv = m; ms = s; }
     }
+    for (int o = 16; o > 0; o >>= 1) {   // the smallest margin, the first row that has it
+        const float om = __shfl_xor_sync(0xffffffffu, mv, o);
+        const int os = __shfl_xor_sync(0xffffffffu, ms, o);
+        if (om < mv || (om == mv && om < INFINITY && os < ms)) { mv = om; ms = os; }
+    }
+    ms = mv < INFINITY ? ms : 0;
+    bad = __any_sync(0xffffffffu, bad);
     if (bad) mv = NAN;
-    if (value_out) value_out[r] = mv;
-    if (best) {
-        int imp = (!bad && mv < best[r]) ? 1 : 0;
-        if (imp) best[r] = mv;
-        improved[r] = imp;
+    if (lane == 0) {
+        if (value_out) value_out[r] = mv;
+        if (best) {
+            int imp = (!bad && mv < best[r]) ? 1 : 0;
+            if (imp) best[r] = mv;
+            improved[r] = imp;
+        }
     }
     if (G)
-        for (int j = 0; j < nL; ++j) G[(long)r * ldg + j] = spec[ms * nL + j];
+        for (int j = lane; j < nL; j += 32) G[(long)r * ldg + j] = spec[ms * nL + j];
 }
 
-__global__ void k_keep_best(int K, int n0, const float *__restrict__ X, int ldx, const int *__restrict__ improved,
-                            float *__restrict__ best_x) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)K * n0) return;
-    int r = (int)(t / n0), j = (int)(t % n0);
-    if (improved[r]) best_x[(long)r * n0 + j] = X[(long)r * ldx + j];
+__global__ void __launch_bounds__(256) k_keep_best(int n0, const float *__restrict__ X, long ldx, const int *__restrict__ improved, float *__restrict__ best_x, bool vec) {
+    const int r = blockIdx.y;
+    if (!improved[r]) return;
+    const float *x = X + (long)r * ldx;
+    float *b = best_x + (long)r * n0;
+    over_row(n0, vec, [&](int j, int w) { if (w == 4) *(float4 *)(b + j) = *(const float4 *)(x + j); else b[j] = x[j]; });
 }
 
 // G *= [Zpost > 0]
-__global__ void k_relu_mask(long rows, int n, float *__restrict__ G, int ldg, const float *__restrict__ Z, int ldz) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= rows * n) return;
-    long r = t / n;
-    int j = (int)(t - r * n);
-    if (!(Z[r * ldz + j] > 0.f)) G[r * ldg + j] = 0.f;
+__global__ void __launch_bounds__(256) k_relu_mask(int n, float *__restrict__ G, long ld, const float *__restrict__ Z, bool vec) {
+    float *g = G + (long)blockIdx.y * ld;
+    const float *z = Z + (long)blockIdx.y * ld;
+    over_row(n, vec, [&](int j, int w) {
+        if (w == 4) {
+            float4 v = *(float4 *)(g + j);
+            const float4 m = *(const float4 *)(z + j);
+            *(float4 *)(g + j) = make_float4(m.x > 0.f ? v.x : 0.f, m.y > 0.f ? v.y : 0.f, m.z > 0.f ? v.z : 0.f, m.w > 0.f ? v.w : 0.f);
+        } else if (!(z[j] > 0.f)) g[j] = 0.f;
+    });
 }
 
 // AdamClipping step (pgd_attack/adam_state.rs:46-88), descending the objective.  A restart whose gradient
 // holds a NaN skips the step (attacker/batched.rs:93-104): rows flagged in nan_row are left alone.
-__global__ void k_pgd_step(int K, int n0, float *__restrict__ X, int ldx, const float *__restrict__ G, int ldg,
+__global__ void __launch_bounds__(256) k_pgd_step(int n0, float *__restrict__ X, long ld, const float *__restrict__ G,
                            float *__restrict__ mom, float *__restrict__ var, const float *__restrict__ lo,
-                           const float *__restrict__ hi, const int *__restrict__ nan_row, PgdStep h) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)K * n0) return;
-    int r = (int)(t / n0), j = (int)(t % n0);
+                           const float *__restrict__ hi, const int *__restrict__ nan_row, PgdStep h, bool vec) {
+    const int r = blockIdx.y;
     if (nan_row[r]) return;
-    float g = G[(long)r * ldg + j];
-    float m = h.beta1 * mom[t] + (1.f - h.beta1) * g;
-    float v = h.beta2 * var[t] + (1.f - h.beta2) * g * g;
-    mom[t] = m; var[t] = v;
-    float denom = sqrtf(v / h.bc2) + h.epsilon;
-    float dir = 0.f;
-    if (isfinite(denom) && isfinite(m)) {
-        float q = m / denom;
-        dir = isnan(q) ? 0.f : copysignf(1.f, q);  // sign(+0) = +1, sign(-0) = -1
-    }
-    float x = X[(long)r * ldx + j] - dir * h.step;
-    float l = lo[j], u = hi[j];
-    x = isnan(x) ? l : fminf(fmaxf(x, l), u);
-    X[(long)r * ldx + j] = x;
+    float *x_row = X + (long)r * ld, *m_row = mom + (long)r * n0, *v_row = var + (long)r * n0;
+    const float *g_row = G + (long)r * ld;
+    auto one = [&](float g, float &m, float &v, float &x, float l, float u) {
+        m = h.beta1 * m + (1.f - h.beta1) * g;
+        v = h.beta2 * v + (1.f - h.beta2) * g * g;
+        float denom = sqrtf(v / h.bc2) + h.epsilon;
+        float dir = 0.f;
+        if (isfinite(denom) && isfinite(m)) {
+            float q = m / denom;
+            dir = isnan(q) ? 0.f : copysignf(1.f, q);  // sign(+0) = +1, sign(-0) = -1
+        }
+        x = x - dir * h.step;
+        x = isnan(x) ? l : fminf(fmaxf(x, l), u);
+    };
+    over_row(n0, vec, [&](int j, int w) {
+        if (w == 4) {
+            const float4 g = *(const float4 *)(g_row + j), l = *(const float4 *)(lo + j), u = *(const float4 *)(hi + j);
+            float4 m = *(float4 *)(m_row + j), v = *(float4 *)(v_row + j), x = *(float4 *)(x_row + j);
+            one(g.x, m.x, v.x, x.x, l.x, u.x); one(g.y, m.y, v.y, x.y, l.y, u.y); one(g.z, m.z, v.z, x.z, l.z, u.z); one(g.w, m.w, v.w, x.w, l.w, u.w);
+            *(float4 *)(m_row + j) = m; *(float4 *)(v_row + j) = v; *(float4 *)(x_row + j) = x;
+        } else one(g_row[j], m_row[j], v_row[j], x_row[j], lo[j], hi[j]);
+    });
 }
 
-__global__ void k_nan_rows(int K, int n0, const float *__restrict__ G, int ldg, int *__restrict__ nan_row) {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= K) return;
+__global__ void __launch_bounds__(256) k_nan_rows(int n0, const float *__restrict__ G, long ld, int *__restrict__ nan_row) {
+    const float *g = G + (long)blockIdx.x * ld;
     int bad = 0;
-    for (int j = lane; j < n0; j += 32) bad |= isnan(G[(long)warp * ldg + j]) ? 1 : 0;
-    bad = __any_sync(0xffffffffu, bad);
-    if (lane == 0) nan_row[warp] = bad;
+    for (int j = threadIdx.x; j < n0; j += 256) bad |= isnan(g[j]) ? 1 : 0;
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x == 0) nan_row[blockIdx.x] = bad;
 }
 
 // Y[r, j] += X[r, j]
@@ -125,6 +165,11 @@ __global__ void k_row_dot(int rows, int n, const float *__restrict__ X, int ldx,
     if (lane == 0) out[warp] = (float)acc;
 }
 
+__global__ void k_at_least(float *p, int n, float v) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) p[t] = fmaxf(p[t], v);
+}
+
 __global__ void k_fill_f32(float *p, long n, float v) {
     long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) p[t] = v;
@@ -135,23 +180,44 @@ __global__ void k_fill_f32(float *p, long n, float v) {
 // Concrete forward pass of `rows` points X [rows x ldx] through the network; act[k] receives layer k's
 // post-activation output (row stride ld), act[L-1] the network output.
 static int pgd_forward(nyb200_engine *e, Net &net, bool tensor, int rows, const float *X, int ldx, float *const *act, int ld,
-                       int *derr) {
+                       int *derr, const unsigned *x_rows = nullptr) {
     const NetView &nv = net.v;
     const float *cur = X;
     int ldc = ldx;
+    bool pending = false;   // cur is a convolution's result without its bias and ReLU: the next one's split adds them
     for (int k = 0; k < nv.L; ++k) {
         int K = nv.dims[k], N = nv.dims[k + 1];
-        if (net.is_conv(k) && tensor) NYB_TRY(conv_forward_tensor(e, net, k, rows, cur, ldc, act[k], ld, derr));
+        // (a layer that is alone between two window convolutions: its row maxima come with the products)
+        const bool defer = tensor && k + 1 < nv.L && net.is_conv(k) && net.win_fwd[k].ok && net.skip_of(k) < 0 && net.is_conv(k + 1) && net.win_fwd[k + 1].ok && nv.b[k];
+        if (net.is_conv(k) && tensor && net.win_fwd[k].ok) {
+            WinWith with;
+            if (pending) {
+                with.bias = nv.b[k - 1]; with.bias_max = net.bmax[k - 1]; with.keep = act[k - 1]; with.keep_ld = ld;
+                with.has_max = true;
+            } else if (k == 0 && x_rows) {   // points that stay in a box: their maxima are known
+                void *hi, *lo;
+                float *row_inv;
+                unsigned *row_max;
+                NYB_TRY(win_operand(e, net.win_fwd[0], rows, &hi, &lo, &row_inv, &row_max));
+                NYB_CUDA(e, cudaMemcpyAsync(row_max, x_rows, (size_t)rows * 4, cudaMemcpyDeviceToDevice, e->stream));
+                with.has_max = true;
+            }
+            NYB_TRY(conv_win(e, net.win_fwd[k], rows, cur, ldc, act[k], ld, nullptr, nullptr, 1, derr, false, defer, &with));
+        } else if (net.is_conv(k) && tensor) NYB_TRY(conv_forward_tensor(e, net, k, rows, cur, ldc, act[k], ld, derr));
         else if (net.is_conv(k)) launch_conv_plain(e, net.geom[k], rows, cur, ldc, nv.W[k], act[k], ld);
         else if (tensor) NYB_TRY(launch_umma(e, net.umma_adj[k], rows, cur, ldc, act[k], ld, derr));
         else launch_gemm_f64(e, rows, N, K, cur, ldc, net.wt[k], N, act[k], ld, 1, nullptr, nullptr, 0, nullptr);
-        long tot = (long)rows * N;
+        pending = defer;
         if (net.skip_of(k) >= 0) {  // residual: the block's input joins before the bias and the ReLU
+            long tot = (long)rows * N;
             k_add_rows<<<(unsigned)((tot + 255) / 256), 256, 0, e->stream>>>(rows, N, act[k], ld, act[net.skip_of(k)], ld);
             e->launches++;
         }
-        k_bias_act<<<(unsigned)((tot + 255) / 256), 256, 0, e->stream>>>(rows, N, act[k], ld, nv.b[k], k < nv.L - 1 ? 1 : 0);
-        e->launches++;
+        if (!pending)
+            for (int r0 = 0; r0 < rows; r0 += 65535) {   // (grid)
+                k_bias_act<<<NYB_ROWS(std::min(rows - r0, 65535), N), 0, e->stream>>>(N, act[k] + (size_t)r0 * ld, ld, nv.b[k], k < nv.L - 1 ? 1 : 0, vec4(N, ld, act[k], nv.b[k]));
+                e->launches++;
+            }
         cur = act[k];
         ldc = ld;
     }
@@ -168,6 +234,7 @@ static int pgd_backward(nyb200_engine *e, Net &net, bool tensor, int K, float *G
     cudaStream_t st = e->stream;
     double *cols64 = nullptr;
     float *g = G0, *gn = G1;
+    bool reported = false;   // the rows' maxima came with the products that left g
     struct OpenGrad { float *buf; int src; };   // gradients kept for identity branches (blocks may nest)
     std::vector<OpenGrad> open_grad;
     auto grad_slot = [&](size_t slot) -> float * {
@@ -183,11 +250,13 @@ static int pgd_backward(nyb200_engine *e, Net &net, bool tensor, int K, float *G
             e->launches++;
             open_grad.erase(open_grad.begin() + (long)oi);
         }
-        if (k < L - 1) {
-            long tot = (long)K * Kd;
-            k_relu_mask<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(K, Kd, g, ld, act[k], ld);
-            e->launches++;
-        }
+        // a window convolution's split masks its rows itself where nothing else reads them
+        const bool window = net.is_conv(k) && tensor && net.win_bwd[k].ok, masks = k < L - 1 && window && net.skip_of(k) < 0;
+        if (k < L - 1 && !masks)
+            for (int r0 = 0; r0 < K; r0 += 65535) {   // (grid)
+                k_relu_mask<<<NYB_ROWS(std::min(K - r0, 65535), Kd), 0, st>>>(Kd, g + (size_t)r0 * ld, ld, act[k] + (size_t)r0 * ld, vec4(Kd, ld, g, act[k]));
+                e->launches++;
+            }
         if (net.skip_of(k) >= 0) {  // the gradient of pre_k also reaches relu(pre_j) directly
             size_t slot = 0;
             for (bool taken = true; taken; ) {
@@ -199,8 +268,14 @@ static int pgd_backward(nyb200_engine *e, Net &net, bool tensor, int K, float *G
             NYB_CUDA(e, cudaMemcpyAsync(gstash, g, (size_t)K * ld * 4, cudaMemcpyDeviceToDevice, st));
             open_grad.push_back({gstash, net.skip_of(k)});
         }
-        if (net.is_conv(k) && tensor && net.win_bwd[k].ok) {
-            NYB_TRY(conv_win(e, net.win_bwd[k], K, g, ld, gn, ld, nullptr, nullptr, 1, derr));
+        if (window) {
+            WinWith with;
+            if (masks) { with.mask = act[k]; with.mask_ld = ld; }
+            with.has_max = reported;
+            // does the next layer's split want this result's maxima?  (an identity branch that joins in between changes them)
+            reported = k > 0 && net.is_conv(k - 1) && net.win_bwd[k - 1].ok;
+            for (const OpenGrad &o : open_grad) if (o.src == k - 1) reported = false;
+            NYB_TRY(conv_win(e, net.win_bwd[k], K, g, ld, gn, ld, nullptr, nullptr, 1, derr, false, reported, &with));
         } else if (net.is_conv(k) && tensor) {
             const ConvGeom &cg = net.geom[k];
             const int plane = cg.oh * cg.ow, taps = cg.ic * cg.kh * cg.kw;
@@ -218,6 +293,7 @@ static int pgd_backward(nyb200_engine *e, Net &net, bool tensor, int K, float *G
         } else {
             launch_gemm_f64(e, K, N, Kd, g, ld, nv.W[k], N, gn, ld, 1, nullptr, nullptr, 0, nullptr);
         }
+        if (!window) reported = false;
         float *tmp = g; g = gn; gn = tmp;
     }
     *result = g;
@@ -271,33 +347,46 @@ int pgd_attack(nyb200_engine *e, int net_id, const float *spec, int S, const flo
     NYB_CUDA(e, cudaMemsetAsync(var, 0, (size_t)K * n0 * 4, st));
     k_fill_f32<<<(K + 255) / 256, 256, 0, st>>>(dbest, K, INFINITY);
     e->launches++;
-    const unsigned gk = (unsigned)((K + 255) / 256);
-    const long nx = (long)K * n0;
-    const unsigned gx = (unsigned)((nx + 255) / 256);
+    const unsigned gw = (unsigned)(((long)K * 32 + 255) / 256);
+    float x_max = 0.f;   // of the box the points stay in
+    for (int j = 0; j < n0; ++j) x_max = std::max(x_max, std::max(std::fabs(in_lo[j]), std::fabs(in_hi[j])));
+    // A point's largest magnitude: the box's, or its first one's (the caller's, in the box or not; a restart whose gradient is
+    // not a number stays there).
+    unsigned *x_rows = nullptr;
+    if (tensor && net->is_conv(0) && net->win_fwd[0].ok && std::isfinite(x_max)) {
+        x_rows = (unsigned *)ws_get(e, "pgd_xmax", (size_t)K * 4);
+        if (!x_rows) return NYB200_ERR_OOM;
+        NYB_TRY(row_maxima(e, K, n0, X, ld, x_rows));
+        k_at_least<<<(unsigned)((K + 255) / 256), 256, 0, st>>>((float *)x_rows, K, x_max);
+        e->launches++;
+    }
 
     for (int t = 1; t <= cfg.steps + 1; ++t) {
         NYB_DEADLINE(e, "attack");
-        NYB_TRY(pgd_forward(e, *net, tensor, K, X, ld, act.data(), ld, derr));
+        NYB_TRY(pgd_forward(e, *net, tensor, K, X, ld, act.data(), ld, derr, x_rows));
         const bool last = t == cfg.steps + 1;
-        k_pgd_objective<<<gk, 256, 0, st>>>(K, S, nL, act[L - 1], ld, dspec, dbest, dimp, last ? nullptr : G0, ld, nullptr);
-        k_keep_best<<<gx, 256, 0, st>>>(K, n0, X, ld, dimp, dbx);
+        k_pgd_objective<<<gw, 256, 0, st>>>(K, S, nL, act[L - 1], ld, dspec, dbest, dimp, last ? nullptr : G0, ld, nullptr);
+        for (int r0 = 0; r0 < K; r0 += 65535)   // (grid)
+            k_keep_best<<<NYB_ROWS(std::min(K - r0, 65535), n0), 0, st>>>(n0, X + (size_t)r0 * ld, ld, dimp + r0, dbx + (size_t)r0 * n0, vec4(n0, ld, X, dbx));
         e->launches += 2;
         if (last) break;
         float *g = nullptr;
         NYB_TRY(pgd_backward(e, *net, tensor, K, G0, G1, act.data(), ld, derr, &g));
-        k_nan_rows<<<(unsigned)(((long)K * 32 + 255) / 256), 256, 0, st>>>(K, n0, g, ld, dnan);
+        k_nan_rows<<<(unsigned)K, 256, 0, st>>>(n0, g, ld, dnan);
         PgdStep h;
         float bc1 = 1.f - powf(b1, (float)t);
         h.bc2 = 1.f - powf(b2, (float)t);
         h.step = cfg.step_size * powf(decay, (float)(t - 1)) / bc1;
         h.beta1 = b1; h.beta2 = b2; h.epsilon = eps;
-        k_pgd_step<<<gx, 256, 0, st>>>(K, n0, X, ld, g, ld, mom, var, dlo, dhi, dnan, h);
+        for (int r0 = 0; r0 < K; r0 += 65535)
+            k_pgd_step<<<NYB_ROWS(std::min(K - r0, 65535), n0), 0, st>>>(n0, X + (size_t)r0 * ld, ld, g + (size_t)r0 * ld, mom + (size_t)r0 * n0, var + (size_t)r0 * n0, dlo, dhi,
+                                                                          dnan + r0, h, vec4(n0, ld, X, g, mom, var) && vec4(n0, ld, dlo, dhi));
         e->launches += 2;
     }
     // independent evaluation of every restart's best point with binary64 contractions
     NYB_TRY(prepare_transposed(e, *net, false));
     NYB_TRY(pgd_forward(e, *net, false, K, dbx, n0, act.data(), ld, derr));
-    k_pgd_objective<<<gk, 256, 0, st>>>(K, S, nL, act[L - 1], ld, dspec, nullptr, nullptr, nullptr, 0, dbest);
+    k_pgd_objective<<<gw, 256, 0, st>>>(K, S, nL, act[L - 1], ld, dspec, nullptr, nullptr, nullptr, 0, dbest);
     e->launches++;
     NYB_CUDA(e, cudaGetLastError());
     NYB_CUDA(e, cudaMemcpyAsync(best_margin, dbest, (size_t)K * 4, cudaMemcpyDeviceToHost, st));
