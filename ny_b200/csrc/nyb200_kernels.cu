@@ -421,70 +421,57 @@ k_relax_v4(int n, int off, int M, int R, int S, long nps, float *A, int lda, con
 // L1 against 8 for the coefficient itself).  Here a warp owns 128 columns of one domain (parts 1), or of its lower or its
 // upper rows (parts 2: where there are too few warps otherwise): every lane keeps the tables of its 4 columns in registers
 // and walks the rows, so the tables are read once or twice.
-template <bool UPPER, bool RELAX, bool BIAS>
-__device__ __forceinline__ void relax_dom_rows(int r0, int r1, long m0, int j, float *A, int lda, const float *Asrc, int lds,
-                                               const float4 &t0, const float4 &t1, const float4 &t2, const float4 &t3,
-                                               const float4 &za, const float4 &qv, const float4 &bk, const float4 &au,
-                                               float eps, int lane, bool live, double *__restrict__ rb, double *__restrict__ rabs,
-                                               double *__restrict__ rpen) {
-    // Rows are taken RB at a time: all their loads are issued before the first is used, so a lane has RB
-    // independent 16-byte requests in flight (a warp that walks one row after the other is latency bound), and their sums
-    // are reduced together: each step halves the rows a lane holds, six shuffles for up to four rows instead of twenty.
-    // (Three at a time are as fast for nine rows and lose where four would be one batch: 4096 domains, 512 columns, 4 rows
-    // 1380 -> 1333 us a call, 7 rows 1840 -> 1779; the residual network's 100 domains, 4 rows, 13.8 -> 13.4 ms.)
-    constexpr int RB = 4;
-    for (int rbase = r0; rbase < r1; rbase += RB) {
-        float4 a[RB];
+//
+// A warp's columns stay in registers as relax_prepared wants them, and its rows are taken kDomRows at a time, the next ones on
+// their way while these are worked on: a warp that walks one row after the other is latency bound.  (Rows loaded when their
+// turn came, four at a time, and relax_coeff's sums: 55 us for 36864 rows of 512, now 35; their bytes take 27.)
+constexpr int kDomRows = 3;   // nine specification rows are three whole batches
+struct DomColumns { float4 t[4], zg, cj, bias; float au[4], under; };
+
+template <bool UPPER, bool BIAS>
+__device__ __forceinline__ void relax_dom_batch(const float4 (&a)[kDomRows], int n, long m0, float *out, long lda, const DomColumns &c, int lane, bool live,
+                                                double *__restrict__ rb, double *__restrict__ rpen) {
+    double sb[kDomRows];
+    float sp[kDomRows];
 #pragma unroll
-        for (int u = 0; u < RB; ++u) {
-            const long m = m0 + rbase + u;
-            // lanes past the row's end take part in the reductions with zeros (their tables are zero too)
-            a[u] = (live && rbase + u < r1) ? *(const float4 *)(Asrc + m * lds + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        double sb[4] = {0.0, 0.0, 0.0, 0.0};
-        float sp[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int u = 0; u < kDomRows; ++u) {
+        sb[u] = 0.0; sp[u] = c.under;
+        if (u >= n) continue;   // uniform in the warp
+        float4 o;
+        auto one = [&](float x, int i, float zg, float cj, float bias) {
+            const float4 t = make_float4(UPPER ? c.au[i] : c.t[i].x, c.t[i].y, c.t[i].z, c.t[i].w);
+            return relax_prepared<UPPER, BIAS>(x, t, zg, cj, bias, sb[u], sp[u]);
+        };
+        o.x = one(a[u].x, 0, c.zg.x, c.cj.x, c.bias.x); o.y = one(a[u].y, 1, c.zg.y, c.cj.y, c.bias.y);
+        o.z = one(a[u].z, 2, c.zg.z, c.cj.z, c.bias.z); o.w = one(a[u].w, 3, c.zg.w, c.cj.w, c.bias.w);
+        if (live) __stcs((float4 *)(out + u * lda), o);   // streamed: the next reader is another kernel
+    }
+    // the rows' sums reduced together: each step halves the rows a lane holds
+    const bool hi16 = lane & 16, hi8 = lane & 8;
+    double b0 = (hi16 ? sb[2] : sb[0]) + __shfl_xor_sync(0xffffffffu, hi16 ? sb[0] : sb[2], 16);
+    double b1 = (hi16 ? 0.0 : sb[1]) + __shfl_xor_sync(0xffffffffu, hi16 ? sb[1] : 0.0, 16);
+    float p0 = __fadd_ru(hi16 ? sp[2] : sp[0], __shfl_xor_sync(0xffffffffu, hi16 ? sp[0] : sp[2], 16));
+    float p1 = __fadd_ru(hi16 ? 0.f : sp[1], __shfl_xor_sync(0xffffffffu, hi16 ? sp[1] : 0.f, 16));
+    b0 = (hi8 ? b1 : b0) + __shfl_xor_sync(0xffffffffu, hi8 ? b0 : b1, 8);
+    p0 = __fadd_ru(hi8 ? p1 : p0, __shfl_xor_sync(0xffffffffu, hi8 ? p0 : p1, 8));
 #pragma unroll
-        for (int u = 0; u < RB; ++u) {
-            if (rbase + u >= r1) break;  // uniform in the warp
-            const long m = m0 + rbase + u;
-            float sa = 0.f;
-            float4 o;
-            o.x = relax_one<UPPER, RELAX, BIAS>(a[u].x, t0, au.x, za.x, qv.x, bk.x, eps, sb[u], sa, sp[u]);
-            o.y = relax_one<UPPER, RELAX, BIAS>(a[u].y, t1, au.y, za.y, qv.y, bk.y, eps, sb[u], sa, sp[u]);
-            o.z = relax_one<UPPER, RELAX, BIAS>(a[u].z, t2, au.z, za.z, qv.z, bk.z, eps, sb[u], sa, sp[u]);
-            o.w = relax_one<UPPER, RELAX, BIAS>(a[u].w, t3, au.w, za.w, qv.w, bk.w, eps, sb[u], sa, sp[u]);
-            if (RELAX && live) __stcs((float4 *)(A + m * lda + j), o);  // streamed: the next reader is another kernel
-            // The magnitude sum only ever enters the bound as 2^-40 * rabs (the slack for the binary64 bias
-            // sums), so it is folded into the penalty here instead of being reduced on its own; the penalty
-            // is reduced in fp32 and inflated for the roundings of that reduction.
-            sp[u] = __fmaf_ru(sa, 9.1e-13f, sp[u]);
-        }
-        const bool hi16 = lane & 16, hi8 = lane & 8;
-        double b0 = (hi16 ? sb[2] : sb[0]) + __shfl_xor_sync(0xffffffffu, hi16 ? sb[0] : sb[2], 16);
-        double b1 = (hi16 ? sb[3] : sb[1]) + __shfl_xor_sync(0xffffffffu, hi16 ? sb[1] : sb[3], 16);
-        float p0 = __fadd_ru(hi16 ? sp[2] : sp[0], __shfl_xor_sync(0xffffffffu, hi16 ? sp[0] : sp[2], 16));
-        float p1 = __fadd_ru(hi16 ? sp[3] : sp[1], __shfl_xor_sync(0xffffffffu, hi16 ? sp[1] : sp[3], 16));
-        b0 = (hi8 ? b1 : b0) + __shfl_xor_sync(0xffffffffu, hi8 ? b0 : b1, 8);
-        p0 = __fadd_ru(hi8 ? p1 : p0, __shfl_xor_sync(0xffffffffu, hi8 ? p0 : p1, 8));
-#pragma unroll
-        for (int o2 = 4; o2 > 0; o2 >>= 1) {
-            b0 += __shfl_xor_sync(0xffffffffu, b0, o2);
-            p0 = __fadd_ru(p0, __shfl_xor_sync(0xffffffffu, p0, o2));
-        }
-        const int u = lane >> 3;   // the row whose sums this lane holds
-        if ((lane & 7) == 0 && u < RB && rbase + u < r1) {
-            atomicAdd(&rb[m0 + rbase + u], b0);
-            atomicAdd(&rpen[m0 + rbase + u], (double)p0 * 1.000002);
-        }
+    for (int o2 = 4; o2 > 0; o2 >>= 1) {
+        b0 += __shfl_xor_sync(0xffffffffu, b0, o2);
+        p0 = __fadd_ru(p0, __shfl_xor_sync(0xffffffffu, p0, o2));
+    }
+    const int u = lane >> 3;   // the row whose sums this lane holds
+    if ((lane & 7) == 0 && u < n) {
+        atomicAdd(&rb[m0 + u], b0);
+        atomicAdd(&rpen[m0 + u], (double)p0 * 1.000002);
     }
 }
 
-template <bool RELAX, bool BIAS>
-__global__ void __launch_bounds__(256)
-k_relax_dom(int n, int off, int D, int R, int S, int parts, long nps, float *A, int lda, const float *Asrc, int lds,
+template <bool BIAS>
+__global__ void __launch_bounds__(256, 2)
+k_relax_dom(int n, int off, int D, int R, int S, int parts, long nps, float *A, long lda, const float *Asrc, long lds,
             const float4 *__restrict__ tab, const float *__restrict__ zabs, const float *__restrict__ q, long q_ds,
             const float *__restrict__ bias_k, const float *__restrict__ aup, float eps, double *__restrict__ rb,
-            double *__restrict__ rabs, double *__restrict__ rpen) {
+            double *__restrict__ rpen) {
     const int slabs = (n + 127) >> 7;
     const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -492,22 +479,49 @@ k_relax_dom(int n, int off, int D, int R, int S, int parts, long nps, float *A, 
     const int d = (int)(warp / (slabs * parts)), rest = (int)(warp - (long)d * slabs * parts), slab = rest / parts, part = rest - slab * parts;
     const int j = slab * 128 + lane * 4;
     const bool live = j < n;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 t0 = zero, t1 = zero, t2 = zero, t3 = zero, za = zero, qv = zero, bk = zero;
+    const int r_first = parts == 2 && part == 1 ? S : 0, r_end = parts == 2 && part == 0 ? S : R;
+    const long m0 = (long)d * R;
+    auto batch_of = [&](int r) { return min(kDomRows, (r < S ? S : R) - r); };   // lower rows, then upper ones
+    const float *src = Asrc + (m0 + r_first) * lds + j;
+    float *out = A + (m0 + r_first) * lda + j;
+    float4 ahead[kDomRows];
+    auto fetch = [&](int k) {   // lanes past the row's end take part in the reductions with zeros (their tables are zero too)
+#pragma unroll
+        for (int u = 0; u < kDomRows; ++u) ahead[u] = live && u < k ? *(const float4 *)(src + u * lds) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    fetch(batch_of(r_first));
+    DomColumns c;
+    c.zg = c.cj = c.bias = make_float4(0.f, 0.f, 0.f, 0.f);
+    float zs = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { c.t[i] = make_float4(0.f, 0.f, 0.f, 0.f); c.au[i] = 0.f; }
     if (live) {
         const long tb = (long)d * nps + off + j;
-        qv = *(const float4 *)(q + (long)d * q_ds + off + j);
-        if (BIAS) bk = *(const float4 *)(bias_k + j);
-        if (RELAX) {
-            t0 = tab[tb]; t1 = tab[tb + 1]; t2 = tab[tb + 2]; t3 = tab[tb + 3];
-            za = *(const float4 *)(zabs + tb);
+        const float4 qv = *(const float4 *)(q + (long)d * q_ds + off + j), za = *(const float4 *)(zabs + tb);
+        if (BIAS) c.bias = *(const float4 *)(bias_k + j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            c.t[i] = tab[tb + i];
+            c.au[i] = aup ? aup[tb + i] : c.t[i].x;
+            const float z = (&za.x)[i];
+            (&c.cj.x)[i] = __fmaf_ru(9.1e-13f, __fadd_ru(z, fabsf((&c.bias.x)[i])), __fmul_ru(eps, (&qv.x)[i]));
+            (&c.zg.x)[i] = (c.t[i].y == 1.f && c.t[i].z == 0.f) ? 0.f : z;
+            zs = __fadd_ru(zs, z);
         }
     }
-    float4 au = make_float4(t0.x, t1.x, t2.x, t3.x);
-    if (RELAX && live && aup) au = *(const float4 *)(aup + (long)d * nps + off + j);
-    const long m0 = (long)d * R;
-    if (part == 0) relax_dom_rows<false, RELAX, BIAS>(0, S, m0, j, A, lda, Asrc, lds, t0, t1, t2, t3, za, qv, bk, au, eps, lane, live, rb, rabs, rpen);
-    if (part == parts - 1) relax_dom_rows<true, RELAX, BIAS>(S, R, m0, j, A, lda, Asrc, lds, t0, t1, t2, t3, za, qv, bk, au, eps, lane, live, rb, rabs, rpen);
+    c.under = __fmul_ru((float)kUnderflow, zs);
+    for (int r = r_first; r < r_end; ) {
+        const int k = batch_of(r), next = r + k;
+        float4 now[kDomRows];
+#pragma unroll
+        for (int u = 0; u < kDomRows; ++u) now[u] = ahead[u];
+        src += k * lds;
+        if (next < r_end) fetch(batch_of(next));   // while these are worked on
+        if (r < S) relax_dom_batch<false, BIAS>(now, k, m0 + r, out, lda, c, lane, live, rb, rpen);
+        else relax_dom_batch<true, BIAS>(now, k, m0 + r, out, lda, c, lane, live, rb, rpen);
+        out += k * lda;
+        r = next;
+    }
 }
 
 // ---------------------------------------------------------------- binary64-accumulated contraction
@@ -978,18 +992,14 @@ void launch_relax(nyb200_engine *e, const NetView &nv, int r, int lin_k, int M, 
         const int parts = slab_warps < (long)usable_sms(e) * 16 ? 2 : 1;
         const long dwarps = slab_warps * parts;
         const unsigned dgrid = (unsigned)((dwarps * 32 + 255) / 256);
-#define NYB_RELAX_DOM(RELAX, BIAS) \
-    k_relax_dom<RELAX, BIAS><<<dgrid, 256, 0, e->stream>>>(n, off, D, R, S, parts, (long)nv.nps, A, lda, Asrc, lds, tab, zabs, q, q_dstride, bk, aup, epsf, rb, rabs, rpen)
         // domain-major when a domain's rows amortise the table loads and there are enough warps to fill the GPU
-        const bool dom = R >= 4 && dwarps >= 2048;
-        if (dom) {
-            if (r >= 0) { if (bk) NYB_RELAX_DOM(true, true); else NYB_RELAX_DOM(true, false); }
-            else { if (bk) NYB_RELAX_DOM(false, true); else NYB_RELAX_DOM(false, false); }
+        if (r >= 0 && R >= 4 && dwarps >= 2048) {
+            if (bk) k_relax_dom<true><<<dgrid, 256, 0, e->stream>>>(n, off, D, R, S, parts, (long)nv.nps, A, lda, Asrc, lds, tab, zabs, q, q_dstride, bk, aup, epsf, rb, rpen);
+            else k_relax_dom<false><<<dgrid, 256, 0, e->stream>>>(n, off, D, R, S, parts, (long)nv.nps, A, lda, Asrc, lds, tab, zabs, q, q_dstride, bk, aup, epsf, rb, rpen);
         } else {
             if (r >= 0) { if (bk) NYB_RELAX_LAUNCH(true, true); else NYB_RELAX_LAUNCH(true, false); }
             else { if (bk) NYB_RELAX_LAUNCH(false, true); else NYB_RELAX_LAUNCH(false, false); }
         }
-#undef NYB_RELAX_DOM
 #undef NYB_RELAX_LAUNCH
     } else
         k_relax<<<grid, 256, 0, e->stream>>>(n, off, M, R, S, nv.nps, r < 0 ? 1 : 0, A, lda, Asrc, lds, tab, zabs, q, q_dstride,

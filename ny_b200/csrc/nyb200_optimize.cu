@@ -18,6 +18,8 @@
 // bound that is ever reported comes from step 1.
 #include <string.h>
 
+#include <algorithm>
+
 #include "nyb200_internal.cuh"
 
 namespace nyb {
@@ -55,23 +57,45 @@ __global__ void k_transpose(const float *__restrict__ W, int n_out, int n_in, fl
 
 // Z[d*Zr + s][j] = the box corner row (d, s) concretises on: lower rows (s < S) take x_lo where the coefficient
 // is >= 0, upper rows (S <= s < Zr, present with the dual alpha: Zr = 2S) take x_hi there.
-__global__ void k_adjoint_seed(int D, int S, int R, int Zr, int n0, const float *__restrict__ A, int lda,
-                               const float *__restrict__ in_lo, const float *__restrict__ in_hi, long box_ds,
-                               float *__restrict__ Z, int ldz) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)D * Zr * n0) return;
-    int j = (int)(t % n0);
-    long ds = t / n0;
-    int d = (int)(ds / Zr), s = (int)(ds % Zr);
-    float a = A[((long)d * R + s) * lda + j];
-    bool take_lo = (a >= 0.f) == (s < S);
-    Z[ds * ldz + j] = take_lo ? in_lo[(long)d * box_ds + j] : in_hi[(long)d * box_ds + j];
+// A row is a grid row, four columns a thread where it allows that (VEC); with two 64-bit divisions an element 78 us for 18432 rows
+// of 784, so 27.
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+k_adjoint_seed(long rows, int S, int R, int Zr, int n0, const float *__restrict__ A, int lda, const float *__restrict__ in_lo, const float *__restrict__ in_hi,
+               long box_ds, float *__restrict__ Z, int ldz) {
+    const int j = (blockIdx.x * 256 + threadIdx.x) * (VEC ? 4 : 1);
+    if (j >= n0) return;
+    for (long ds = blockIdx.y; ds < rows; ds += gridDim.y) {
+        const int d = (int)(ds / Zr), s = (int)(ds - (long)d * Zr);
+        const float *a = A + ((long)d * R + s) * lda + j, *l = in_lo + (long)d * box_ds + j, *u = in_hi + (long)d * box_ds + j;
+        auto one = [&](float x, float lo, float hi) { return (x >= 0.f) == (s < S) ? lo : hi; };
+        if constexpr (VEC) {
+            const float4 x = *(const float4 *)a, lo = *(const float4 *)l, hi = *(const float4 *)u;
+            *(float4 *)(Z + ds * ldz + j) = make_float4(one(x.x, lo.x, hi.x), one(x.y, lo.y, hi.y), one(x.z, lo.z, hi.z), one(x.w, lo.w, hi.w));
+        } else Z[ds * ldz + j] = one(*a, *l, *u);
+    }
 }
 
-// One thread per (domain, neuron) of ReLU `k`: adds the bias, harvests the parameter gradient over the
-// domain's S lower rows, maps Zpre to the post-activation adjoint in place, then takes the Adam step of the
-// parameter this neuron owns (alpha if unstable and unsplit, beta if split, none otherwise) and writes it
+// One thread per domain and V neurons of ReLU `k` (V 2 where rows and tables lie on even places): adds the bias, harvests the
+// parameter gradient over the domain's S lower rows, maps Zpre to the post-activation adjoint in place, then takes the Adam
+// step of the parameter a neuron owns (alpha if unstable and unsplit, beta if split, none otherwise) and writes it
 // into the relaxation table the next backward pass reads.
+// What bounds it: the latency of its loads.  What the step reads is fetched ahead of the rows, and nothing is divided: with
+// one neuron a thread, two 64-bit divisions each, and the step's reads behind the rows, 53 us a layer for 2048 domains of 9 rows
+// of 512 neurons, more than twice its bytes' time; so 40.
+template <int V>
+struct Vals { float v[V]; };
+template <int V>
+__device__ __forceinline__ Vals<V> load_vals(const float *p) {
+    Vals<V> r;
+    if constexpr (V == 2) { const float2 x = *(const float2 *)p; r.v[0] = x.x; r.v[1] = x.y; } else r.v[0] = *p;
+    return r;
+}
+template <int V>
+__device__ __forceinline__ void store_vals(float *p, const Vals<V> &r) {
+    if constexpr (V == 2) *(float2 *)p = make_float2(r.v[0], r.v[1]); else *p = r.v[0];
+}
+template <int V>
 __global__ void __launch_bounds__(256)
 k_adjoint_relu(int n, int off, int D, int S, int R, int Zr, long nps, float *__restrict__ Z, int ldz,
                const float *__restrict__ bias, const float *__restrict__ Apre, int ldc, float4 *__restrict__ tab,
@@ -80,99 +104,117 @@ k_adjoint_relu(int n, int off, int D, int S, int R, int Zr, long nps, float *__r
                const int *__restrict__ only_row, float *__restrict__ aup, float *__restrict__ mom_up,
                float *__restrict__ var_up, float *__restrict__ grad_out, AdamStep h, const int *__restrict__ stopped,
                unsigned *__restrict__ maxg, float *__restrict__ vmax, float *__restrict__ vmax_up) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)D * n) return;
-    int d = (int)(t / n), i = (int)(t % n);
+    const int i = (blockIdx.y * blockDim.x + threadIdx.x) * V, d = blockIdx.x * blockDim.y + threadIdx.y;
+    if (i >= n || d >= D) return;
     const bool frozen = stopped && stopped[d] != 0;  // a stopped domain keeps its parameters
-    long o = (long)d * nps + off + i;
-    float4 tb = tab[o];
-    float bk = bias ? bias[i] : 0.f;
-    float g_alpha = 0.f, g_sum = 0.f;
+    const long o = (long)d * nps + off + i;
+    float4 tb[V];
+    int c[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) { tb[e] = tab[o + e]; c[e] = code[o + e]; }
+    const Vals<V> l = load_vals<V>(pre_lo + o), u = load_vals<V>(pre_hi + o);
+    Vals<V> bk, m0, v0;
+#pragma unroll
+    for (int e = 0; e < V; ++e) bk.v[e] = m0.v[e] = v0.v[e] = 0.f;
+    if (bias) bk = load_vals<V>(bias + i);
+    if (h.rule != 1 && mom) { m0 = load_vals<V>(mom + o); v0 = load_vals<V>(var + o); }
+    float g_alpha[V] = {}, g_sum[V] = {};
     const int pick = only_row ? only_row[d] : -1;  // objective: one row of the domain, or the sum over its rows
     // Rows are taken RB at a time, all their loads before the first store: Z is updated in place, and row by row every
     // load waited for the store before it (2048 domains of 9 rows, 512 neurons: 61 us a layer, three times its traffic).
     constexpr int RB = 5;
+    float *zrow = Z + (long)d * Zr * ldz + i;
+    const float *arow = Apre + (long)d * R * ldc + i;
     for (int s0 = 0; s0 < S; s0 += RB) {
-        float zv[RB], av[RB];
+        Vals<V> zv[RB], av[RB];
 #pragma unroll
         for (int r = 0; r < RB; ++r) {
             const int s = min(s0 + r, S - 1);
-            zv[r] = Z[((long)d * Zr + s) * ldz + i];
-            av[r] = Apre[((long)d * R + s) * ldc + i];
+            zv[r] = load_vals<V>(zrow + (long)s * ldz);
+            av[r] = load_vals<V>(arow + (long)s * ldc);
         }
 #pragma unroll
         for (int r = 0; r < RB; ++r) {
             const int s = s0 + r;
             if (s >= S) break;
-            const float g = zv[r] + bk, ap = av[r];
-            if (pick < 0 || s == pick) {
-                g_alpha = fmaf(g, fmaxf(ap, 0.f), g_alpha);
-                g_sum += g;
+            Vals<V> out;
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                const float g = zv[r].v[e] + bk.v[e], ap = av[r].v[e];
+                if (pick < 0 || s == pick) {
+                    g_alpha[e] = fmaf(g, fmaxf(ap, 0.f), g_alpha[e]);
+                    g_sum[e] += g;
+                }
+                const bool pos = ap >= 0.f;
+                out.v[e] = fmaf(g, pos ? tb[e].x : tb[e].y, pos ? 0.f : tb[e].z);
             }
-            const bool pos = ap >= 0.f;
-            Z[((long)d * Zr + s) * ldz + i] = fmaf(g, pos ? tb.x : tb.y, pos ? 0.f : tb.z);
+            store_vals<V>(zrow + (long)s * ldz, out);
         }
     }
-    int c = code[o];
-    float l = pre_lo[o], u = pre_hi[o];
     if (Zr > S) {
         // dual alpha: the upper rows' adjoint; a >= 0 takes the chord, a < 0 the upper path's own slope, whose
         // gradient is sum_s Zpre * min(Apre, 0); the sum of the upper bounds descends
-        float au = aup[o], g_up = 0.f;
-        for (int s = S; s < Zr; ++s) {
-            long zr = ((long)d * Zr + s) * ldz + i;
-            float g = Z[zr] + bk;
-            float ap = Apre[((long)d * R + s) * ldc + i];
-            g_up = fmaf(g, fminf(ap, 0.f), g_up);
-            bool pos = ap >= 0.f;
-            Z[zr] = fmaf(g, pos ? tb.y : au, pos ? tb.z : 0.f);
-        }
-        if ((c == 0) && (l < 0.f) && (u > 0.f) && h.lr_alpha > 0.f && !frozen) {
-            float a, m = 0.f, v = 0.f;
-            if (h.rule == 1) a = au - h.lr_alpha * g_up;
-            else {
-                m = h.beta1 * mom_up[o] + (1.f - h.beta1) * g_up;
-                v = h.beta2 * var_up[o] + (1.f - h.beta2) * g_up * g_up;
-                float vu = v;
-                if (h.rule == 2) { vu = nan_max(vmax_up[o], v); vmax_up[o] = vu; }
-                a = au - h.lr_alpha * (m / h.bc1) / (sqrtf(vu / h.bc2) + h.epsilon);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            float au = aup[o + e], g_up = 0.f;
+            for (int s = S; s < Zr; ++s) {
+                float *zr = zrow + (long)s * ldz + e;
+                float g = *zr + bk.v[e];
+                float ap = arow[(long)s * ldc + e];
+                g_up = fmaf(g, fminf(ap, 0.f), g_up);
+                bool pos = ap >= 0.f;
+                *zr = fmaf(g, pos ? tb[e].y : au, pos ? tb[e].z : 0.f);
             }
-            a = fminf(fmaxf(a, 0.f), 1.f);
-            if (isnan(a)) { a = 0.5f; m = 0.f; v = 0.f; if (h.rule == 2) vmax_up[o] = 0.f; }
-            aup[o] = a;
-            if (h.rule != 1) { mom_up[o] = m; var_up[o] = v; }
+            if ((c[e] == 0) && (l.v[e] < 0.f) && (u.v[e] > 0.f) && h.lr_alpha > 0.f && !frozen) {
+                float a, m = 0.f, v = 0.f;
+                if (h.rule == 1) a = au - h.lr_alpha * g_up;
+                else {
+                    m = h.beta1 * mom_up[o + e] + (1.f - h.beta1) * g_up;
+                    v = h.beta2 * var_up[o + e] + (1.f - h.beta2) * g_up * g_up;
+                    float vu = v;
+                    if (h.rule == 2) { vu = nan_max(vmax_up[o + e], v); vmax_up[o + e] = vu; }
+                    a = au - h.lr_alpha * (m / h.bc1) / (sqrtf(vu / h.bc2) + h.epsilon);
+                }
+                a = fminf(fmaxf(a, 0.f), 1.f);
+                if (isnan(a)) { a = 0.5f; m = 0.f; v = 0.f; if (h.rule == 2) vmax_up[o + e] = 0.f; }
+                aup[o + e] = a;
+                if (h.rule != 1) { mom_up[o + e] = m; var_up[o + e] = v; }
+            }
         }
     }
-    if (grad_out)  // export: the slope's gradient of an unstable unsplit neuron, the multiplier's of a split one
-        grad_out[o] = ((c == 0) && (l < 0.f) && (u > 0.f)) ? g_alpha : (c != 0 ? (c > 0 ? -g_sum : g_sum) : 0.f);
-    bool is_alpha = (c == 0) && (l < 0.f) && (u > 0.f) && h.lr_alpha > 0.f;
-    bool is_beta = (c != 0) && h.lr_beta > 0.f;
-    if ((!is_alpha && !is_beta) || frozen) return;
-    float g = is_alpha ? g_alpha : (c > 0 ? -g_sum : g_sum);
-    if (is_beta && h.rule != 1 && h.clip_beta > 0.f) g = fminf(fmaxf(g, -h.clip_beta), h.clip_beta);
-    if (maxg) atomicMax(&maxg[d], __float_as_uint(fabsf(g)));  // the domain's convergence measure (NaN wins, as in the reference)
-    float m = 0.f, v = 0.f, step;
-    if (h.rule == 1) step = g;
-    else {
-        m = h.beta1 * mom[o] + (1.f - h.beta1) * g;
-        v = h.beta2 * var[o] + (1.f - h.beta2) * g * g;
-        float vu = v;
-        if (h.rule == 2) { vu = nan_max(vmax[o], v); vmax[o] = vu; }
-        step = (m / h.bc1) / (sqrtf(vu / h.bc2) + h.epsilon);
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+        const bool unstable = (c[e] == 0) && (l.v[e] < 0.f) && (u.v[e] > 0.f);
+        if (grad_out)  // export: the slope's gradient of an unstable unsplit neuron, the multiplier's of a split one
+            grad_out[o + e] = unstable ? g_alpha[e] : (c[e] != 0 ? (c[e] > 0 ? -g_sum[e] : g_sum[e]) : 0.f);
+        bool is_alpha = unstable && h.lr_alpha > 0.f;
+        bool is_beta = (c[e] != 0) && h.lr_beta > 0.f;
+        if ((!is_alpha && !is_beta) || frozen) continue;
+        float g = is_alpha ? g_alpha[e] : (c[e] > 0 ? -g_sum[e] : g_sum[e]);
+        if (is_beta && h.rule != 1 && h.clip_beta > 0.f) g = fminf(fmaxf(g, -h.clip_beta), h.clip_beta);
+        if (maxg) atomicMax(&maxg[d], __float_as_uint(fabsf(g)));  // the domain's convergence measure (NaN wins, as in the reference)
+        float m = 0.f, v = 0.f, step;
+        if (h.rule == 1) step = g;
+        else {
+            m = h.beta1 * m0.v[e] + (1.f - h.beta1) * g;
+            v = h.beta2 * v0.v[e] + (1.f - h.beta2) * g * g;
+            float vu = v;
+            if (h.rule == 2) { vu = nan_max(vmax[o + e], v); vmax[o + e] = vu; }
+            step = (m / h.bc1) / (sqrtf(vu / h.bc2) + h.epsilon);
+        }
+        if (is_alpha) {
+            float a = tb[e].x + h.lr_alpha * step;
+            a = fminf(fmaxf(a, 0.f), 1.f);
+            if (isnan(a)) { a = 0.5f; m = 0.f; v = 0.f; if (h.rule == 2) vmax[o + e] = 0.f; }
+            tab[o + e].x = a;
+        } else {
+            float sgn = c[e] > 0 ? 1.f : -1.f;
+            float b = fabsf(tb[e].w) + h.lr_beta * step;
+            if (isnan(b) || isinf(b)) { b = 0.f; m = 0.f; v = 0.f; if (h.rule == 2) vmax[o + e] = 0.f; }
+            tab[o + e].w = sgn * fmaxf(b, 0.f);
+        }
+        if (h.rule != 1) { mom[o + e] = m; var[o + e] = v; }
     }
-    if (is_alpha) {
-        float a = tb.x + h.lr_alpha * step;
-        a = fminf(fmaxf(a, 0.f), 1.f);
-        if (isnan(a)) { a = 0.5f; m = 0.f; v = 0.f; if (h.rule == 2) vmax[o] = 0.f; }
-        tb.x = a;
-    } else {
-        float sgn = c > 0 ? 1.f : -1.f;
-        float b = fabsf(tb.w) + h.lr_beta * step;
-        if (isnan(b) || isinf(b)) { b = 0.f; m = 0.f; v = 0.f; if (h.rule == 2) vmax[o] = 0.f; }
-        tb.w = sgn * fmaxf(b, 0.f);
-    }
-    if (h.rule != 1) { mom[o] = m; var[o] = v; }
-    tab[o] = tb;
 }
 
 // Y[r, j] += X[r, j]
@@ -459,9 +501,13 @@ int optimize_batch(nyb200_engine *e, const nyb200_opt_config &cfg, float *grad_h
         h.beta1 = b1; h.beta2 = b2; h.epsilon = eps; h.clip_beta = cfg.clip_beta; h.rule = cfg.rule;
         h.bc1 = fmaxf(1.f - powf(b1, (float)t), 1.1920929e-7f);
         h.bc2 = fmaxf(1.f - powf(b2, (float)t), 1.1920929e-7f);
-        long nseed = (long)D * Zr * nv.dims[0];
-        k_adjoint_seed<<<(unsigned)((nseed + 255) / 256), 256, 0, e->stream>>>(D, S, R, Zr, nv.dims[0], p.a_final, p.lda, p.in_lo,
-                                                                              p.in_hi, (long)b.box_stride, z0, ldz);
+        const long seeds = (long)D * Zr;
+        const int n0 = nv.dims[0];
+        const bool four = ((n0 | p.lda | ldz | b.box_stride) & 3) == 0 &&
+                          ((reinterpret_cast<uintptr_t>(p.a_final) | reinterpret_cast<uintptr_t>(p.in_lo) | reinterpret_cast<uintptr_t>(p.in_hi) | reinterpret_cast<uintptr_t>(z0)) & 15) == 0;
+        const dim3 seed_grid((unsigned)((n0 + (four ? 1023 : 255)) / (four ? 1024 : 256)), (unsigned)std::min<long>(seeds, 65535));
+        if (four) k_adjoint_seed<true><<<seed_grid, 256, 0, e->stream>>>(seeds, S, R, Zr, n0, p.a_final, p.lda, p.in_lo, p.in_hi, (long)b.box_stride, z0, ldz);
+        else k_adjoint_seed<false><<<seed_grid, 256, 0, e->stream>>>(seeds, S, R, Zr, n0, p.a_final, p.lda, p.in_lo, p.in_hi, (long)b.box_stride, z0, ldz);
         e->launches++;
         float *zc = z0, *zn = z1;
         // adjoints of relu(pre_k) that a later layer's identity branch still needs, one buffer per open source layer
@@ -490,11 +536,16 @@ int optimize_batch(nyb200_engine *e, const nyb200_opt_config &cfg, float *grad_h
                     break;
                 }
             }
-            long nt = (long)D * N;
-            k_adjoint_relu<<<(unsigned)((nt + 255) / 256), 256, 0, e->stream>>>(N, nv.pre_off[k], D, S, R, Zr, np, zn, ldz, nv.b[k],
-                                                                               ckpt[k], ldc, p.tab, p.code, p.pre_lo,
-                                                                               p.pre_hi, mom, var, only_row, p.alpha_up, mom_up, var_up, grad_dev, h,
-                                                                               rules ? ost.stopped : nullptr, rules ? ost.maxg : nullptr, vmax, vmax_up);
+            const bool two = ((N | nv.pre_off[k] | (int)np | ldz | ldc) & 1) == 0 &&
+                             ((reinterpret_cast<uintptr_t>(zn) | reinterpret_cast<uintptr_t>(ckpt[k]) | reinterpret_cast<uintptr_t>(nv.b[k])) & 7) == 0;
+            // a narrow layer's domains share a block
+            const int per = (N + (two ? 1 : 0)) / (two ? 2 : 1), tx = std::min(256, (per + 31) / 32 * 32), ty = 256 / tx;
+            const dim3 grid((unsigned)((D + ty - 1) / ty), (unsigned)((per + tx - 1) / tx)), block((unsigned)tx, (unsigned)ty);
+#define NYB_ADJOINT(V) k_adjoint_relu<V><<<grid, block, 0, e->stream>>>(N, nv.pre_off[k], D, S, R, Zr, np, zn, ldz, nv.b[k], ckpt[k], ldc, p.tab, p.code, p.pre_lo, \
+                                                                       p.pre_hi, mom, var, only_row, p.alpha_up, mom_up, var_up, grad_dev, h,                    \
+                                                                       rules ? ost.stopped : nullptr, rules ? ost.maxg : nullptr, vmax, vmax_up)
+            if (two) NYB_ADJOINT(2); else NYB_ADJOINT(1);
+#undef NYB_ADJOINT
             e->launches++;
             bool opens = false;  // is this layer's post-activation adjoint skipped forward to a later layer?
             for (int kk = k + 2; kk < L - 1; ++kk) opens |= net->skip_of(kk) == k;

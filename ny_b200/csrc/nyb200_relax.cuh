@@ -52,6 +52,27 @@ __device__ __forceinline__ float relax_coeff(const bool upper, float a, float4 t
     return nw;
 }
 
+// relax_coeff with its charges prepared per column: zg = max|z| where the outward step is charged (zero where z cannot be
+// negative), cj = eps q + 2^-40 (max|z| + |bias|), which bounds the contraction's rounding and, because an intercept only
+// applies on the upper line, where |a icp| <= |nw| max|z| (1 + 2^-21), that of the two binary64 sums.  A zero product stays zero;
+// one that underflowed (at most 2^-150) is covered by a charge of the caller's, kUnderflow times the sum of max|z|.
+constexpr double kUnderflow = 1e-45;
+template <bool UPPER, bool BIAS>
+__device__ __forceinline__ float relax_prepared(float a, const float4 &t, float zg, float cj, float bias, double &sb, float &sp) {
+    const bool pos = a > 0.f;
+    const float slope = (pos != UPPER) ? t.x : t.y;
+    const float prod = __fmul_rn(a, slope);
+    const int pb = __float_as_int(prod), away = (pb >> 31) | 1;   // a step on the bit pattern away from zero, signed
+    float nw = __int_as_float(UPPER ? pb + away : pb - away);     // one ulp up, or down
+    if (prod == 0.f) nw = 0.f;
+    sp = __fmaf_ru(fabsf(fmaf(a, slope, -nw)), zg, sp);
+    if (pos == UPPER) sb = fma((double)a, (double)t.z, sb);
+    nw = UPPER ? nw + t.w : nw - t.w;
+    if (BIAS) sb = fma((double)nw, (double)bias, sb);
+    sp = __fmaf_ru(fabsf(nw), cj, sp);
+    return nw;
+}
+
 // The same coefficient step for the fused backward chain, with the row sums arranged for issue rate: the coefficient
 // bits are those of relax_coeff (same product, same outward step, same beta addition); what differs is the
 // bookkeeping around them.

@@ -19,6 +19,7 @@
 #include <cuda_fp16.h>
 
 #include "nyb200_internal.cuh"
+#include "nyb200_relax.cuh"
 
 namespace nyb {
 
@@ -69,27 +70,6 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     return r;
 }
 
-// relax_coeff with its charges prepared per column: zg = max|z| where the outward step is charged (zero where z cannot be
-// negative), cj = eps q + 2^-40 (max|z| + |bias|), which bounds the contraction's rounding and, because an intercept only
-// applies on the upper line, where |a icp| <= |nw| max|z| (1 + 2^-21), that of the two binary64 sums.  A zero product stays zero;
-// one that underflowed (at most 2^-150) is covered by a charge of the block's (kUnderflow).
-constexpr double kUnderflow = 1e-45;
-template <bool UPPER>
-__device__ __forceinline__ float relax_prepared(float a, const float4 &t, float zg, float cj, float bias, double &sb, float &sp) {
-    const bool pos = a > 0.f;
-    const float slope = (pos != UPPER) ? t.x : t.y;
-    const float prod = __fmul_rn(a, slope);
-    const int pb = __float_as_int(prod), away = (pb >> 31) | 1;   // a step on the bit pattern away from zero, signed
-    float nw = __int_as_float(UPPER ? pb + away : pb - away);     // one ulp up, or down
-    if (prod == 0.f) nw = 0.f;
-    sp = __fmaf_ru(fabsf(fmaf(a, slope, -nw)), zg, sp);
-    if (pos == UPPER) sb = fma((double)a, (double)t.z, sb);
-    nw = UPPER ? nw + t.w : nw - t.w;
-    sb = fma((double)nw, (double)bias, sb);
-    sp = __fmaf_ru(fabsf(nw), cj, sp);
-    return nw;
-}
-
 // A thread's coefficients of a batch of rows, on their way from memory.
 template <bool JOIN>
 struct Batch3 { float4 a[kBatch], j[JOIN ? kBatch : 1]; };
@@ -131,10 +111,10 @@ __device__ __forceinline__ void image_batch(const ImageArgs &P, const Batch3<JOI
             add(a.x, in.j[u].x, c.zm.x); add(a.y, in.j[u].y, c.zm.y); add(a.z, in.j[u].z, c.zm.z); add(a.w, in.j[u].w, c.zm.w);
         }
         float4 o;
-        o.x = relax_prepared<UPPER>(a.x, c.t[0], c.zg.x, c.cj.x, c.bias.x, sb[u], sp[u]);
-        o.y = relax_prepared<UPPER>(a.y, c.t[1], c.zg.y, c.cj.y, c.bias.y, sb[u], sp[u]);
-        o.z = relax_prepared<UPPER>(a.z, c.t[2], c.zg.z, c.cj.z, c.bias.z, sb[u], sp[u]);
-        o.w = relax_prepared<UPPER>(a.w, c.t[3], c.zg.w, c.cj.w, c.bias.w, sb[u], sp[u]);
+        o.x = relax_prepared<UPPER, true>(a.x, c.t[0], c.zg.x, c.cj.x, c.bias.x, sb[u], sp[u]);
+        o.y = relax_prepared<UPPER, true>(a.y, c.t[1], c.zg.y, c.cj.y, c.bias.y, sb[u], sp[u]);
+        o.z = relax_prepared<UPPER, true>(a.z, c.t[2], c.zg.z, c.cj.z, c.bias.z, sb[u], sp[u]);
+        o.w = relax_prepared<UPPER, true>(a.w, c.t[3], c.zg.w, c.cj.w, c.bias.w, sb[u], sp[u]);
         if (P.stash && live) __stcs((float4 *)(keep + u * P.ldk), o);
         if (put) {   // (channels past the last one: zeros)
             const float s = scale[u], s2 = s * 2048.f;   // (a power of two)
