@@ -557,6 +557,158 @@ k_direct_pass(const __grid_constant__ PackedNet pn, int top, int boxes, const in
     if (C > 1) cl.sync();   // the sums have been read before their CTA leaves
 }
 
+// k_direct_pass for many rows of narrow layers (up to 64 columns): a warp alone takes two groups of eight rows, so that a weight is
+// loaded and converted once for both and twice the products are in flight.  What bounds the one-group form there is their
+// latency and the conversions, not the tensor instruction (1024 boxes of 5 -> 6x50 -> 5: 816 us of passes where the products take
+// 190).  A call on those boxes 1147 -> 1033 us, 512 of them 648 -> 600.
+template <int NT>
+__global__ void __launch_bounds__(128, 3)
+k_direct_rows(const __grid_constant__ PackedNet pn, int top, int boxes, const int *__restrict__ idx, int n_rows, int pitch, const float *__restrict__ seed,
+              const float *__restrict__ seed_bias, const float *__restrict__ in_lo, const float *__restrict__ in_hi, long box_ds,
+              const PassEntry *__restrict__ ptab, float *__restrict__ out_lo, float *__restrict__ out_hi, float *__restrict__ a_out, int lda) {
+    constexpr int MG = 2;
+    extern __shared__ double s_coef[];
+    const NetView &nv = pn.nv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lq = lane & 3;
+    pdl_trigger();
+    pdl_wait();
+    int d[MG], r[MG], rr[MG];
+    bool live[MG], upper[MG], bad[MG];
+    double rb[MG], rp[MG], cs[MG], ca[MG];
+    float gp[MG];
+    double *cur[MG];
+#pragma unroll
+    for (int m = 0; m < MG; ++m) {   // rows of all boxes one behind the other: a group may span boxes
+        const int gr = (((int)blockIdx.x * 4 + warp) * MG + m) * 8 + lr;
+        live[m] = gr < boxes * 2 * n_rows;
+        const int box = live[m] ? gr / (2 * n_rows) : 0;
+        r[m] = live[m] ? gr - box * 2 * n_rows : 0;
+        d[m] = idx ? idx[box] : box;
+        upper[m] = r[m] >= n_rows;
+        rr[m] = upper[m] ? r[m] - n_rows : r[m];
+        rb[m] = rp[m] = cs[m] = ca[m] = 0.0;
+        gp[m] = 0.f; bad[m] = false;
+        cur[m] = s_coef + ((warp * MG + m) * 8 + lr) * pitch;
+        const int n = nv.dims[top], np16 = (n + 15) & ~15;
+        const bool spec = top == nv.L;   // rows at the network's output: no ReLU in front of the first contraction
+        const PassEntry *t = ptab + (long)d[m] * nv.nps + nv.pre_off[top - 1];
+        for (int j = lq; j < np16; j += 4) {
+            double v = 0.0;
+            if (live[m] && j < n) {
+                const float a = seed[(long)rr[m] * n + j];
+                if (spec) { v = a; rb[m] += v * t[j].bias; rp[m] += fabs(v) * t[j].cj; }
+                else v = relax_step(a, upper[m], *(const float4 *)&t[j].ls, t[j].sbeta, t[j].cj, *(const float4 *)&t[j].ui, rb[m], rp[m], gp[m]);
+            }
+            cur[m][j] = v;
+        }
+        if (live[m] && seed_bias && lq == 0) { const double c = seed_bias[rr[m]]; rb[m] += c; rp[m] += 1.8189894035458565e-12 * fabs(c); }
+    }
+    __syncwarp();
+    for (int lay = top - 1; lay >= 0; --lay) {
+        const int K = nv.dims[lay + 1], N = nv.dims[lay], kg = (K + 15) >> 4, nt = (N + 7) >> 3;
+        const int tail = (K - (kg - 1) * 16 + 3) >> 2;   // m8n8k4 steps of the last group
+        const float4 *__restrict__ w = pn.w[lay] + lane;
+        for (int nb = 0; nb < nt; nb += NT) {   // (one sweep unless this is the input layer)
+            const int have = nt - nb;
+            double acc[MG][NT][2];
+#pragma unroll
+            for (int m = 0; m < MG; ++m)
+#pragma unroll
+                for (int t = 0; t < NT; ++t) acc[m][t][0] = acc[m][t][1] = 0.0;
+            const float4 *wt = w + (long)nb * kg * 32;
+            const long ws = (long)kg * 32;
+            for (int g = 0; g < kg; ++g) {
+                float4 b[NT];
+#pragma unroll
+                for (int t = 0; t < NT; ++t)
+                    if (t < have) b[t] = __ldg(wt + t * ws + g * 32);
+                const int steps = g + 1 < kg ? 4 : tail;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (c >= steps) break;
+                    double a[MG];
+#pragma unroll
+                    for (int m = 0; m < MG; ++m) a[m] = cur[m][g * 16 + c * 4 + lq];
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) {
+                        if (t >= have) break;
+                        const double bd = (double)(c == 0 ? b[t].x : c == 1 ? b[t].y : c == 2 ? b[t].z : b[t].w);
+#pragma unroll
+                        for (int m = 0; m < MG; ++m) dmma(acc[m][t][0], acc[m][t][1], a[m], bd);
+                    }
+                }
+            }
+            if (lay > 0) {
+                __syncwarp();   // the rows are written in place
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    if (t >= have) break;
+                    const int j0 = (nb + t) * 8 + lq * 2;
+                    const bool whole = (nb + t) * 8 + 8 <= N;
+#pragma unroll
+                    for (int m = 0; m < MG; ++m) {
+                        const PassEntry *te = ptab + (long)d[m] * nv.nps + nv.pre_off[lay - 1] + j0;
+                        double2 v = make_double2(0.0, 0.0);
+                        auto one = [&](const PassEntry *at, double sum) {
+                            const float4 f = *(const float4 *)&at->ls, g2 = *(const float4 *)&at->zlo, ib = *(const float4 *)&at->ui;
+                            const float c = cast_coeff(sum, upper[m], f, g2.x, gp[m]);
+                            return relax_step(c, upper[m], f, g2.y, __hiloint2double(__float_as_int(g2.w), __float_as_int(g2.z)), ib, rb[m], rp[m], gp[m]);
+                        };
+                        if (whole) { v.x = one(te, acc[m][t][0]); v.y = one(te + 1, acc[m][t][1]); }   // (dead rows: see k_direct_pass)
+                        else {
+                            if (j0 < N) v.x = one(te, acc[m][t][0]);
+                            if (j0 + 1 < N) v.y = one(te + 1, acc[m][t][1]);
+                        }
+                        *(double2 *)(cur[m] + j0) = v;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    if (t >= have) break;
+#pragma unroll
+                    for (int m = 0; m < MG; ++m)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int j = (nb + t) * 8 + lq * 2 + h;
+                            if (!live[m] || j >= N) continue;
+                            const float c = (float)acc[m][t][h];
+                            const double e = acc[m][t][h] - (double)c, l = in_lo[(long)d[m] * box_ds + j], u = in_hi[(long)d[m] * box_ds + j];
+                            const double el = e * l, eu = e * u;   // the box may have any sign: k_gemm_f64's charge as it stands
+                            rp[m] += (upper[m] ? fmax(el, eu) : fmax(-el, -eu)) + 2.9e-14 * fabs(e) * fmax(fabs(l), fabs(u));
+                            if (!(fabsf(c) < 1e10f)) bad[m] = true;   // is_crown_coeff_safe, crates/ny-core/src/gemm.rs:127
+                            const double x = ((c >= 0.f) != upper[m]) ? l : u;
+                            if (c != 0.f && x != 0.0) { const double p = (double)c * x; cs[m] += p; ca[m] += fabs(p); }
+                            if (a_out) a_out[((long)d[m] * 2 * n_rows + r[m]) * lda + j] = c;
+                        }
+                }
+            }
+        }
+        if (lay > 0) {
+            if (nt & 1)   // the groups of sixteen are read whole
+#pragma unroll
+                for (int m = 0; m < MG; ++m) *(double2 *)(cur[m] + nt * 8 + lq * 2) = make_double2(0.0, 0.0);
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < MG; ++m) {
+        double v[4] = {rb[m], rp[m] + (double)gp[m], cs[m], ca[m]};
+        int anybad = bad[m] ? 1 : 0;
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+            anybad |= __shfl_xor_sync(0xffffffffu, anybad, o);
+        }
+        if (lq == 0 && live[m]) {
+            const double slack = (v[3] + fabs(v[0])) * 9.094947017729282e-13 + 1e-200;   // as k_direct_pass
+            if (!upper[m]) { const double x = v[0] + v[2] - v[1] - slack; out_lo[(long)d[m] * n_rows + rr[m]] = (anybad || isnan(x)) ? -INFINITY : __double2float_rd(x); }
+            else { const double x = v[0] + v[2] + v[1] + slack; out_hi[(long)d[m] * n_rows + rr[m]] = (anybad || isnan(x)) ? INFINITY : __double2float_ru(x); }
+        }
+    }
+}
+
 __device__ __forceinline__ void meet(float &l, float &u, float bl, float bu) {
     const float tl = fmaxf(l, bl), tu = fminf(u, bu);
     if (tl <= tu) { l = tl; u = tu; }
@@ -942,6 +1094,20 @@ int launch_pass(nyb200_engine *e, const PackedNet &pn, int top, int n_rows, int 
     // a launch that leaves SMs idle all the same: clusters of two to eight CTAs of eight warps each
     int C = 1;
     while (NW >= 8 && C < 8 && groups * C * 2 <= sms && tiles >= NW * 2) { C *= 2; NW *= 2; }
+    // Warps alone with all columns of their rows: two groups of rows each (k_direct_rows) where that still fills the SMs' twelve
+    // places; fewer rows want the warps.
+    if (NW == 1 && C == 1 && !ckpt && groups >= sms * 24) {
+        const size_t rows_smem = (size_t)4 * 2 * 8 * pitch * 8;
+        const dim3 rows_grid((unsigned)((groups + 7) / 8));
+#define NYB_ROWS_PASS(NT) case NT:                                                                                              \
+        NYB_TRY(allow_smem(e, (const void *)k_direct_rows<NT>, rows_smem));                                                     \
+        NYB_CUDA(e, launch_pdl(k_direct_rows<NT>, rows_grid, dim3(128), rows_smem, e, pn, top, D, idx, n_rows, pitch, seed, seed_bias, \
+                               (const float *)p.in_lo, (const float *)p.in_hi, box_ds, ptab, c_lo, c_hi, a_out, p.lda)); break;
+        switch (tiles) { NYB_ROWS_PASS(1) NYB_ROWS_PASS(2) NYB_ROWS_PASS(3) NYB_ROWS_PASS(4) NYB_ROWS_PASS(5) NYB_ROWS_PASS(6) NYB_ROWS_PASS(7) NYB_ROWS_PASS(8) }
+#undef NYB_ROWS_PASS
+        e->launches++;
+        return NYB200_OK;
+    }
     const int per = (tiles + NW - 1) / NW;
     int MT = 8 / (NW / C);
     const int bufs = C > 1 || (written + 7) / 8 > NW * 8 ? 2 : 1;   // one sweep per layer: the rows are replaced in place
