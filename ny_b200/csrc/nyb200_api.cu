@@ -91,6 +91,8 @@ void nyb200_destroy(nyb200_engine *e) {
     if (e->frontier) nyb::frontier_free(e->frontier);
     if (e->frontier_spare) nyb::frontier_free(e->frontier_spare);
     if (e->own_stream) cudaStreamDestroy(e->own_stream);
+    if (e->side) cudaStreamDestroy(e->side);
+    for (cudaEvent_t ev : e->side_ev) if (ev) cudaEventDestroy(ev);
     for (int i = 0; i < 3; ++i) if (e->timing.ev[i]) cudaEventDestroy(e->timing.ev[i]);
     for (cudaEvent_t ev : e->timing.kev) cudaEventDestroy(ev);
     for (int i = 0; i < 2; ++i) if (e->timing.cev[i]) cudaEventDestroy(e->timing.cev[i]);
@@ -497,7 +499,7 @@ static void copy_past_caches(unsigned char *dst, const unsigned char *src, size_
 // they belong to, the device idle); here kLanes threads each copy blocks of rows into two pinned slots in turn, at the
 // device's pitch so that a block is one plain transfer, past the caches: 0.40 ms (0.85 with cached stores; 0.27 is the
 // bus).  More threads only share the same memory bandwidth; below one slot their start (60 us) costs what they save.
-int upload_rows(nyb200_engine *e, void *dst, size_t dst_pitch, const void *src, size_t width, size_t rows) {
+int upload_rows(nyb200_engine *e, void *dst, size_t dst_pitch, const void *src, size_t width, size_t rows, cudaStream_t stream) {
     const size_t per = std::min(kLaneSlot / dst_pitch, std::max<size_t>(1, (rows + 2 * kLanes - 1) / (2 * kLanes)));
     bool direct = per == 0 || rows * width < kLaneSlot || (dst_pitch & 15);
     if (!direct) {   // a pinned source needs no staging
@@ -511,8 +513,8 @@ int upload_rows(nyb200_engine *e, void *dst, size_t dst_pitch, const void *src, 
             if (!e->lane_done[i]) NYB_CUDA(e, cudaEventCreateWithFlags(&e->lane_done[i], cudaEventDisableTiming));
     }
     if (direct) {
-        if (dst_pitch == width) NYB_CUDA(e, cudaMemcpyAsync(dst, src, width * rows, cudaMemcpyHostToDevice, e->stream));
-        else NYB_CUDA(e, cudaMemcpy2DAsync(dst, dst_pitch, src, width, width, rows, cudaMemcpyHostToDevice, e->stream));
+        if (dst_pitch == width) NYB_CUDA(e, cudaMemcpyAsync(dst, src, width * rows, cudaMemcpyHostToDevice, stream));
+        else NYB_CUDA(e, cudaMemcpy2DAsync(dst, dst_pitch, src, width, width, rows, cudaMemcpyHostToDevice, stream));
         return NYB200_OK;
     }
     const size_t blocks = (rows + per - 1) / per;
@@ -529,8 +531,8 @@ int upload_rows(nyb200_engine *e, void *dst, size_t dst_pitch, const void *src, 
             if (dst_pitch == width) copy_past_caches(slot, from, n * width);
             else for (size_t r = 0; r < n; ++r) copy_past_caches(slot + r * dst_pitch, from + r * width, width);
             // (the last row without its padding: it may end the allocation)
-            st = cudaMemcpyAsync((char *)dst + r0 * dst_pitch, slot, (n - 1) * dst_pitch + width, cudaMemcpyHostToDevice, e->stream);
-            if (st == cudaSuccess) st = cudaEventRecord(e->lane_done[2 * t + i], e->stream);
+            st = cudaMemcpyAsync((char *)dst + r0 * dst_pitch, slot, (n - 1) * dst_pitch + width, cudaMemcpyHostToDevice, stream);
+            if (st == cudaSuccess) st = cudaEventRecord(e->lane_done[2 * t + i], stream);
         }
         if (st != cudaSuccess) failed = (int)st;
     };
@@ -555,7 +557,7 @@ int staged_upload(nyb200_engine *e, const UploadPiece *pc, int n) {
         const size_t row = 4096;
         for (int i = 0; i < n; ++i) {
             const size_t whole = pc[i].bytes / row * row;
-            if (whole) NYB_TRY(upload_rows(e, pc[i].dst, row, pc[i].src, row, whole / row));
+            if (whole) NYB_TRY(upload_rows(e, pc[i].dst, row, pc[i].src, row, whole / row, e->stream));
             if (pc[i].bytes > whole)
                 NYB_CUDA(e, cudaMemcpyAsync((char *)pc[i].dst + whole, (const char *)pc[i].src + whole, pc[i].bytes - whole, cudaMemcpyHostToDevice, e->stream));
         }
@@ -1072,7 +1074,7 @@ namespace {
 
 int upload_batch(nyb200_engine *e, int32_t net_id, const float *spec, int32_t S, const float *in_lo, const float *in_hi,
                  int32_t box_stride, const float *inh_lo, const float *inh_hi, const nyb200_split *splits,
-                 const int32_t *n_splits, int32_t max_splits, int32_t D, int32_t mode, const float *alpha) {
+                 const int32_t *n_splits, int32_t max_splits, int32_t D, int32_t mode, const float *alpha, bool alpha_later = false) {
     Net *net;
     NYB_TRY(find_net(e, net_id, &net));
     const NetView &nv = net->v;
@@ -1099,8 +1101,8 @@ int upload_batch(nyb200_engine *e, int32_t net_id, const float *spec, int32_t S,
                                {p.spec, spec, (size_t)S * nv.dims[nv.L] * 4}};
     NYB_TRY(staged_upload(e, up, 7));
     e->stage_out_valid = false;
-    if (alpha)
-        NYB_TRY(upload_rows(e, p.alpha, (size_t)nv.nps * 4, alpha, np * 4, (size_t)D));
+    if (alpha && !alpha_later)
+        NYB_TRY(upload_rows(e, p.alpha, (size_t)nv.nps * 4, alpha, np * 4, (size_t)D, e->stream));
     b.valid = true;
     e->batch = b;
     return NYB200_OK;
@@ -1123,7 +1125,9 @@ __global__ void k_publish_status(const int *__restrict__ derr, const int *__rest
     status[0] = seq;
 }
 
-int run_batch(nyb200_engine *e) {
+// late_alpha: the batch's slopes, still in the caller's array.  Bounds do not depend on them: they cross the bus beside the interval
+// pass, on a stream of their own, and are put into its tables when both are done (777 domains of 9 x 512, 14 MB: 1460 -> 1260 us a call).
+int run_batch(nyb200_engine *e, const float *late_alpha = nullptr) {
     if (!e->batch.valid) return set_err(e, NYB200_ERR_INVALID, "no batch uploaded");
     if (!e->status_host) {
         NYB_CUDA(e, cudaHostAlloc((void **)&e->status_host, 64, cudaHostAllocMapped));
@@ -1148,7 +1152,21 @@ int run_batch(nyb200_engine *e) {
     }
     cudaEventRecord(t.ev[0], e->stream);
     if (direct) NYB_TRY(run_forward_direct(e, *net, e->batch, p, e->batch.mode, nullptr, e->batch.D));
-    else NYB_TRY(run_forward(e, *net, e->batch, p, e->batch.mode));
+    else if (late_alpha) {
+        if (!e->side) {
+            NYB_CUDA(e, cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking));
+            for (cudaEvent_t &ev : e->side_ev) NYB_CUDA(e, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        }
+        NYB_CUDA(e, cudaEventRecord(e->side_ev[0], e->stream));   // the slopes' place may still be read by earlier work
+        NYB_CUDA(e, cudaStreamWaitEvent(e->side, e->side_ev[0], 0));
+        Batch plain = e->batch;
+        plain.has_alpha = false;
+        NYB_TRY(run_forward(e, *net, plain, p, e->batch.mode));
+        NYB_TRY(upload_rows(e, p.alpha, (size_t)net->v.nps * 4, late_alpha, (size_t)net->v.n_pre * 4, (size_t)e->batch.D, e->side));
+        NYB_CUDA(e, cudaEventRecord(e->side_ev[1], e->side));
+        NYB_CUDA(e, cudaStreamWaitEvent(e->stream, e->side_ev[1], 0));
+        launch_apply_alpha(e, net->v, e->batch.D, p.alpha, p.code, p.pre_lo, p.pre_hi, p.tab);
+    } else NYB_TRY(run_forward(e, *net, e->batch, p, e->batch.mode));
     cudaEventRecord(t.ev[1], e->stream);
     if (direct) NYB_TRY(run_backward_direct(e, *net, e->batch, p, nullptr, e->batch.D));
     else NYB_TRY(run_backward(e, *net, e->batch, p, nullptr, 0));
@@ -1403,8 +1421,8 @@ int32_t nyb200_batch_set_inherited(nyb200_engine *e, const float *inh_lo, const 
     const size_t w = (size_t)nv.n_pre * 4, pitch = (size_t)nv.nps * 4;
     NYB_CUDA(e, cudaMemsetAsync(p.inh_lo, 0, (size_t)e->batch.D * pitch, e->stream));
     NYB_CUDA(e, cudaMemsetAsync(p.inh_hi, 0, (size_t)e->batch.D * pitch, e->stream));
-    NYB_TRY(upload_rows(e, p.inh_lo, pitch, inh_lo, w, (size_t)e->batch.D));
-    NYB_TRY(upload_rows(e, p.inh_hi, pitch, inh_hi, w, (size_t)e->batch.D));
+    NYB_TRY(upload_rows(e, p.inh_lo, pitch, inh_lo, w, (size_t)e->batch.D, e->stream));
+    NYB_TRY(upload_rows(e, p.inh_hi, pitch, inh_hi, w, (size_t)e->batch.D, e->stream));
     NYB_CUDA(e, cudaStreamSynchronize(e->stream));
     e->batch.ran = false;
     e->batch.finished = false;
@@ -1431,9 +1449,19 @@ int32_t nyb200_bab_bound_batch(nyb200_engine *e, int32_t net_id, const float *sp
                                int32_t mode, const float *alpha, float *out_lo, float *out_hi, int32_t *infeasible) {
     if (!e || !out_lo || !out_hi) return NYB200_ERR_INVALID;
     std::lock_guard<std::mutex> g(e->mu);
+    // many slopes on the tensor path: after the interval pass (run_batch); fewer than a slot of the upload's lanes cost less than the
+    // second stream
+    Net *net;
+    NYB_TRY(find_net(e, net_id, &net));
+    const bool later = alpha && D > 0 && S > 0 && (size_t)D * net->v.n_pre * 4 >= kLaneSlot && e->path == NYB200_PATH_TF32X3 && !direct_pays(e, *net, S, D);
     NYB_TRY(upload_batch(e, net_id, spec, S, in_lo, in_hi, box_stride, inh_lo, inh_hi, splits, n_splits, max_splits, D, mode,
-                         alpha));
-    NYB_TRY(run_batch(e));
+                         alpha, later));
+    const int st = run_batch(e, later ? alpha : nullptr);
+    if (later && st != NYB200_OK) {   // the caller's array may go away, and the batch never had its slopes
+        if (e->side) cudaStreamSynchronize(e->side);
+        e->batch.valid = false;
+    }
+    NYB_TRY(st);
     return download_batch(e, out_lo, out_hi, infeasible);
 }
 

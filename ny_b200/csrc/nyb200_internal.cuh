@@ -178,6 +178,8 @@ struct nyb200_engine {
     int reserve_sms = 0;                          // see nyb200_set_reserved_sms
     bool launch_overlap = true;                   // see nyb200_set_launch_overlap
     cudaStream_t own_stream = nullptr;            // created by nyb200_use_own_stream, destroyed with the engine
+    cudaStream_t side = nullptr;                  // slopes on their way while the interval pass runs (nyb200_bab_bound_batch)
+    cudaEvent_t side_ev[2] = {nullptr, nullptr};
     int path = NYB200_PATH_TF32X3;                // _F64 or _TF32X3
     bool small_direct = true;                     // NYB200_PATH_AUTO: what binary64 does faster goes there
     float refine_tol = 5e-5f;  // see nyb200_set_refine_tolerance
@@ -313,6 +315,8 @@ void launch_gather_rows(nyb200_engine *e, void *dst, const void *src, const int 
 void launch_scatter_rows(nyb200_engine *e, void *dst, const void *src, const int *idx, int n_rows, long row_words);
 // min over feasible domains and rows of out_lo (the value the concretisation folds), recomputed from scratch
 void launch_min_lower(nyb200_engine *e, int D, int S, const float *out_lo, const int *flags, float *min_lower);
+// Slopes handed in by the caller into the tables of an interval pass that ran without them.
+void launch_apply_alpha(nyb200_engine *e, const NetView &nv, int D, const float *alpha, const signed char *code, const float *pre_lo, const float *pre_hi, float4 *tab);
 void launch_select_branch(nyb200_engine *e, const NetView &nv, int D, const float *pre_lo, const float *pre_hi,
                           const signed char *code, int *relu, int *neuron, float *width, int kind);
 void launch_fill_f64(nyb200_engine *e, double *p, size_t n, double v);
@@ -342,7 +346,7 @@ int batch_ptrs(nyb200_engine *e, const Net &net, const Batch &b, BatchPtrs &p);
 struct UploadPiece { void *dst; const void *src; size_t bytes; };
 struct FetchPiece { void *dst; size_t bytes; };
 int staged_upload(nyb200_engine *e, const UploadPiece *pieces, int n);
-int upload_rows(nyb200_engine *e, void *dst, size_t dst_pitch, const void *src, size_t width, size_t rows);
+int upload_rows(nyb200_engine *e, void *dst, size_t dst_pitch, const void *src, size_t width, size_t rows, cudaStream_t stream);
 int staged_fetch(nyb200_engine *e, const void *src, const FetchPiece *pieces, int n);
 int find_net(nyb200_engine *e, int net_id, Net **out);
 void free_net(Net &net);
