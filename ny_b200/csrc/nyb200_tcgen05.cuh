@@ -70,13 +70,10 @@ __device__ __forceinline__ bool mbar_wait_soon(unsigned bar, unsigned parity) {
 // shared memory, that lets lanes leave one by one, they are vector values that each product first moves over: 130 SM cycles a
 // product where the tensor core takes 48 (128 x 64 x 16, operands in shared memory) to 64 (128 columns); from a single-lane
 // branch 95 to 105, and 169 instead of 128 for 256 columns.
-template <bool HINT = false>
 __device__ __forceinline__ bool mbar_wait_warp(unsigned bar, unsigned parity) {
     long long t0 = 0;
     for (;;) {
         unsigned ok;
-        if (HINT) ok = mbar_probe(bar, parity, WAIT_HINT_NS);
-        else
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
