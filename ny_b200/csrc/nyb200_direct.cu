@@ -57,6 +57,7 @@ __device__ __forceinline__ float step_up(float x) {
 __device__ __forceinline__ void touch(const void *p) {
     unsigned v;
     asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    (void)v;
 }
 
 __device__ __forceinline__ double eps64(int K) { return (double)(K + 2) * 1.1102230246251565e-16 * 1.000001; }
