@@ -67,6 +67,12 @@ using namespace win;
 // Per tile: warp 3 adds Al*Wh and Ah*Wl over all taps into the tile's CROSS columns, warp 1 Ah*Wh in chains, each into MAIN
 // columns of its own.  Up to 32 channels the high and low parts share a pixel's row (one load); from 64 on they are two tiles,
 // and the low one is free for the next loads after its pass.
+// The ring: a wait on a barrier tells the phase it is for from the ones next to it, no more, so nobody may get two phases away from
+// a barrier it waits on.  A slot's b_full is completed by its load alone, and the next load waits for two arrivals at b_empty,
+// one of each issuing warp, each after that warp's own wait on this b_full: b_full's next phase begins behind both waits, and
+// b_empty's behind the loads' thread's.  That holds for low tiles too, which warp 1 does not read: were it to pass them by, a low
+// tile that is late (the slots' number may be odd: a slot then holds low and high tiles in turn) would leave b_full where the
+// high tile after it is waited for, and the low one, or half of it, would be multiplied in its place.
 // What bounds it: shared memory, at three quarters of its rate.  A 128 x 64 x 16 product takes 48 cycles (its operands' bytes),
 // so a tile of 64 columns, 9 taps and 64 channels 5.2 thousand.  From one warp, whose loop the compiler took for divergent, with
 // [Wh | Wl] as one product of 128 columns (4.0 thousand), a tile took 12.2 thousand; with converged loops (mbar_wait_warp) 9.7;
@@ -184,12 +190,16 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                         };
                         auto start_of_slot = [&]() { return (((smem_u32(ring) + (unsigned)(sl * P.slot_bytes)) & 0x3FFFF) >> 4) | (1u << 16); };
                         if (!PACK) {
-                            if (cross) {   // the low parts' tile is this warp's alone
-                                if (!mbar_wait_warp(smem_u32(&b_full[sl]), ph)) { fail(24); ok = false; break; }
-                                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            // The low parts' tile: the cross warp's data alone, but both warps wait for it and both release it (see
+                            // the ring, above)
+                            if (!mbar_wait_warp(smem_u32(&b_full[sl]), ph)) { fail(24); ok = false; break; }
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            if (cross) {
                                 cross_pass(start_of_slot(), w0);
                                 mma_commit_elect(smem_u32(&b_empty[sl]));
-                                mma_commit_elect(smem_u32(&b_empty[sl]));
+                            } else {
+                                if (lane == 0) mbar_arrive(smem_u32(&b_empty[sl]));
+                                __syncwarp();
                             }
                             next_slot();
                         }

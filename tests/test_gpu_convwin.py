@@ -3,6 +3,8 @@ pixel tile, one tile and many, kernels and strides in every parity, channel coun
 the 64-channel chunks, more columns than one block.  References: the binary64 path and the binary64 forward pass."""
 import numpy as np
 import pytest
+import torch
+import torch.nn.functional as F
 
 from ny_b200 import workloads as W
 
@@ -59,3 +61,48 @@ def test_window_convolutions_match_binary64(in_chw, convs):
     want = (W.forward(wl.net, x0) @ wl.spec.astype(np.float64).T).min(axis=1)
     assert np.allclose(tbest, want, rtol=1e-5, atol=2e-6 * np.abs(want).max())
     assert np.allclose(tstep, fstep, rtol=1e-4, atol=1e-4 * np.abs(want).max())
+
+
+# (input channels, output channels, kernel, stride, padding).  From 64 channels on a pixel's high and low parts are tiles of their own
+# in one ring, which holds low and high ones in turn where the number of slots is odd: 3 slots, forward and back, back on two chunks of
+# channels and on three (5), forward on four chunks, then 4 to 8 forward, and the union of a stride's parities back (3).
+RINGS = [(64, 64, (3, 3), 1, 1), (64, 128, (3, 3), 1, 1), (64, 192, (3, 3), 1, 1), (256, 16, (3, 3), 1, 1), (64, 16, (5, 5), 1, 2),
+         (64, 16, (4, 4), 1, 1), (64, 32, (3, 3), 1, 1), (64, 16, (4, 3), 1, 1), (64, 16, (3, 3), 1, 1), (64, 64, (4, 4), 2, 1)]
+
+
+@pytest.mark.parametrize("ring", RINGS)
+def test_a_ring_of_many_tiles(ring):
+    """Every tile of a long launch is multiplied from its own data: values and gradients of one layer over about seven tiles a
+    CTA, twice with the same bits, against binary64 with the products' rounding rate (at most 2.5e-6 of the sum of
+    magnitudes, win_eps).  A tile taken for another one is off by that sum's order itself."""
+    from ny_b200 import B200Engine, Conv2d, Network, engine
+
+    ic, oc, (kh, kw), s, pad = ring
+    g = np.random.default_rng(ic + oc + kh)
+    h, w = 48 * s, 24 * s
+    wt = g.standard_normal((oc, ic, kh, kw)).astype(np.float32)
+    layer = Conv2d(wt, np.zeros(oc, np.float32), (s, s), (pad, pad), (h, w))
+    rows = max(37, 5000 // (9 * max(4, (oc + 15) // 16)))
+    n1 = oc * layer.oh * layer.ow
+    x = g.standard_normal((rows, ic * h * w), dtype=np.float32)
+    spec = np.copysign(g.random((rows, n1), dtype=np.float32) + np.float32(0.5), g.random((rows, n1), dtype=np.float32) - np.float32(0.5))
+    eng = B200Engine(0)
+    eng.set_path(engine.PATH_TF32X3)
+    nid = eng.register_network(Network([layer], [None]))
+    grads, values = eng.point_vjp_batched(nid, spec, x=x)
+    for _ in range(3):
+        again = eng.point_vjp_batched(nid, spec, x=x)
+        assert np.array_equal(again[0], grads) and np.array_equal(again[1], values)
+    eng.close()
+    dev = "cuda:0"
+    t = torch.from_numpy(wt).to(dev).double()
+    extra = [(h + 2 * pad - kh) % s, (w + 2 * pad - kw) % s]
+    for r0 in range(0, rows, 16):
+        a = torch.from_numpy(spec[r0:r0 + 16]).to(dev).double().reshape(-1, oc, layer.oh, layer.ow)
+        xi = torch.from_numpy(x[r0:r0 + 16]).to(dev).double().reshape(-1, ic, h, w)
+        got = torch.from_numpy(grads[r0:r0 + 16]).to(dev).double().reshape(xi.shape)
+        err = (got - F.conv_transpose2d(a, t, None, s, pad, extra)).abs()
+        assert (err <= 3e-6 * F.conv_transpose2d(a.abs(), t.abs(), None, s, pad, extra)).all()
+        val = (a * F.conv2d(xi, t, None, s, pad)).flatten(1).sum(1).cpu().numpy()
+        mag = (a.abs() * F.conv2d(xi.abs(), t.abs(), None, s, pad)).flatten(1).sum(1).cpu().numpy()
+        assert np.all(np.abs(values[r0:r0 + 16] - val) <= 3e-6 * mag)
