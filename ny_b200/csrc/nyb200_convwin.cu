@@ -168,6 +168,7 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
             unsigned ph = 0, mph = 1, cph = 1;
             auto next_slot = [&]() { if (++sl == P.slots) { sl = 0; ph ^= 1; } };
             for (int t = t0; t < tiles && ok && !flag_warp(abort_flag); t += tstep) {
+                // (warp 1 too, for b_ts below)
                 if (!mbar_wait_warp(smem_u32(&b_ce[cb]), cph)) { fail(23); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned d_cross = tmem_base + (unsigned)((MAIN_BUFS + cb) * NB);
@@ -217,7 +218,8 @@ k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CU
                                 // groups', is over.  (A barrier's parity only tells one use from the next; a group that
                                 // waited two uses ahead would take the use before the last for its own.  The other buffers'
                                 // previous uses end before this chain does: the chains complete in order.)  One barrier per cross
-                                // buffer: the next tile that uses it waits for this one's groups.
+                                // buffer: its previous tile's groups have looked at it, since they have given that buffer back
+                                // (b_ce).  Chains alone do not tell: tiles of one or two fit the buffers many times.
                                 if (!begun) { if (lane == 0) mbar_arrive(smem_u32(&b_ts[cb])); __syncwarp(); begun = true; }
                                 const unsigned d_main = tmem_base + (unsigned)(mbuf * NB);
                                 const int end = min(nt, tap + P.tpc);

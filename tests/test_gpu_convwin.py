@@ -68,6 +68,9 @@ def test_window_convolutions_match_binary64(in_chw, convs):
 # channels and on three (5), forward on four chunks, then 4 to 8 forward, and the union of a stride's parities back (3).
 RINGS = [(64, 64, (3, 3), 1, 1), (64, 128, (3, 3), 1, 1), (64, 192, (3, 3), 1, 1), (256, 16, (3, 3), 1, 1), (64, 16, (5, 5), 1, 2),
          (64, 16, (4, 4), 1, 1), (64, 32, (3, 3), 1, 1), (64, 16, (4, 3), 1, 1), (64, 16, (3, 3), 1, 1), (64, 64, (4, 4), 2, 1)]
+# Tiles of one or two chains, of which the accumulators hold several: 64, 32 and 16 columns, one and two tiles in the ring.
+RINGS += [(16, 64, (1, 1), 1, 0), (16, 32, (2, 2), 1, 0), (16, 16, (1, 1), 1, 0), (32, 64, (2, 2), 1, 0), (64, 64, (1, 1), 1, 0), (64, 32, (1, 1), 1, 0),
+          (64, 16, (1, 2), 1, 0)]
 
 
 @pytest.mark.parametrize("ring", RINGS)
