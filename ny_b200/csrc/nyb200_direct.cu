@@ -1012,9 +1012,10 @@ k_direct_forward(NetView nv, int mode, int zdim, const int *__restrict__ idx, co
     if (rank == 0 && threadIdx.x == 0) flags[d] = s_flags;
 }
 
-// Pass table of a batch from its relaxation tables, intervals and charge weights.
+// Pass table of a batch from its relaxation tables, intervals and charge weights.  shared: all domains have one box, and the general
+// interval pass leaves the first layer's charge weights in the first domain's row alone.
 __global__ void __launch_bounds__(256)
-k_pass_table(NetView nv, int boxes, const int *__restrict__ idx, const float4 *__restrict__ tab, const float *__restrict__ zabs,
+k_pass_table(NetView nv, int boxes, bool shared, const int *__restrict__ idx, const float4 *__restrict__ tab, const float *__restrict__ zabs,
              const float *__restrict__ q, const float *__restrict__ zl, const float *__restrict__ zu, const float *__restrict__ alpha_up,
              PassEntry *__restrict__ ptab) {
     pdl_trigger();
@@ -1028,7 +1029,7 @@ k_pass_table(NetView nv, int boxes, const int *__restrict__ idx, const float4 *_
     const long o = (long)(idx ? idx[box] : box) * nv.nps + i;
     PassEntry pe;
     pe.bias = nv.b[k] ? (double)nv.b[k][j] : 0.0;
-    pe.cj = eps64(nv.dims[k + 1]) * (double)q[o] + 1.8189894035458565e-12 * fabs(pe.bias);   // 2^-39
+    pe.cj = eps64(nv.dims[k + 1]) * (double)q[shared && k == 0 ? i : o] + 1.8189894035458565e-12 * fabs(pe.bias);   // 2^-39
     if (k == nv.L - 1) {   // the specification rows pass through unchanged
         pe.ls = pe.us = pe.lsu = 1.f; pe.zg = pe.zhi = pe.zlo = pe.sbeta = pe.ui = 0.f;
     } else {
@@ -1302,7 +1303,7 @@ int run_backward_direct(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p
     NYB_TRY(prepare_fragments(e, net));
     NYB_WS(ptab, PassEntry *, e, "crown_ptab", (size_t)b.D * nv.nps * sizeof(PassEntry));
     const long tot = (long)n * nv.n_pre;
-    NYB_CUDA(e, launch_pdl(k_pass_table, dim3((unsigned)((tot + 255) / 256)), dim3(256), 0, e, nv, n, idx, (const float4 *)p.tab,
+    NYB_CUDA(e, launch_pdl(k_pass_table, dim3((unsigned)((tot + 255) / 256)), dim3(256), 0, e, nv, n, b.box_stride == 0, idx, (const float4 *)p.tab,
                            (const float *)p.zabs, (const float *)p.q, (const float *)(b.external_tables ? nullptr : p.zl),
                            (const float *)(b.external_tables ? nullptr : p.zu), (const float *)p.alpha_up, ptab));
     e->launches++;
