@@ -117,11 +117,12 @@ __device__ __forceinline__ void image_batch(const ImageArgs &P, const Batch3<JOI
         o.w = relax_prepared<UPPER, true>(a.w, c.t[3], c.zg.w, c.cj.w, c.bias.w, sb[u], sp[u]);
         if (P.stash && live) __stcs((float4 *)(keep + u * P.ldk), o);
         if (put) {   // (channels past the last one: zeros)
-            const float s = scale[u], s2 = s * 2048.f;   // (a power of two)
-            const float2 kn = make_float2(-2048.f, -2048.f);
-            const float2 o0 = make_float2(o.x, o.y), o1 = make_float2(o.z, o.w), v0 = mul2(o0, make_float2(s, s)), v1 = mul2(o1, make_float2(s, s));
+            // the low part from the scaled value: the scale alone may lie within 2^11 of fp32's end (rows below 2^-102)
+            const float s = scale[u];
+            const float2 k2 = make_float2(2048.f, 2048.f), kn = make_float2(-2048.f, -2048.f);
+            const float2 v0 = mul2(make_float2(o.x, o.y), make_float2(s, s)), v1 = mul2(make_float2(o.z, o.w), make_float2(s, s));
             const __half2 h0 = __floats2half2_rn(v0.x, v0.y), h1 = __floats2half2_rn(v1.x, v1.y);
-            const float2 w0 = fma2(__half22float2(h0), kn, mul2(o0, make_float2(s2, s2))), w1 = fma2(__half22float2(h1), kn, mul2(o1, make_float2(s2, s2)));   // exact
+            const float2 w0 = fma2(__half22float2(h0), kn, mul2(v0, k2)), w1 = fma2(__half22float2(h1), kn, mul2(v1, k2));   // exact
             const __half2 l0 = __floats2half2_rn(w0.x, w0.y), l1 = __floats2half2_rn(w1.x, w1.y);
             *(uint2 *)(hi + u * half_row) = make_uint2(*(const unsigned *)&h0, *(const unsigned *)&h1);
             *(uint2 *)(lo + u * half_row) = make_uint2(*(const unsigned *)&l0, *(const unsigned *)&l1);

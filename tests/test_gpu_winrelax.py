@@ -9,9 +9,12 @@ charge it: 2e-5 of that sum on either end.  The sum is taken as ten times the do
 cancel no further) and what its multipliers add: each times the largest magnitude of the neuron it stands at."""
 import numpy as np
 import pytest
+import torch
+import torch.nn.functional as F
 
 from ny_b200 import SPLIT_DTYPE
 from ny_b200 import workloads as W
+from test_gpu_rates import _f16_rate, _transposed_rate
 
 pytestmark = pytest.mark.gpu
 
@@ -106,3 +109,99 @@ def test_rows_through_images_agree_with_binary64(eng, case):
         off = np.abs(got - want)
         assert (off <= 2e-5 * total)[fin].all()
         assert np.median((off / size)[fin]) <= 1e-4
+
+
+def _exact(net, spec, lo, hi, rl, ru, sp, alpha):
+    """Bounds of the same lines in plain binary64, and per row what the layers' rounding rates charge: each layer's rate times the
+    sum of |coefficient| q, q its weights' magnitudes times its inputs'; and the sum of q alone."""
+    D, S, L = len(sp), len(spec), len(net.weights)
+    offs = np.concatenate([[0], np.cumsum(net.dims[1:])])
+    code, beta = np.zeros((D, offs[-1])), np.zeros((D, offs[-1]))
+    at = offs[sp["relu"]] + sp["neuron"]
+    np.put_along_axis(code, at, sp["sign"].astype(float), 1)
+    np.put_along_axis(beta, at, (sp["sign"] * sp["beta"]).astype(float), 1)
+    t = lambda x: torch.from_numpy(np.ascontiguousarray(x)).to("cuda:0").double()
+    code, beta, l, u, al = t(code), t(beta), t(rl).expand(D, -1), t(ru).expand(D, -1), t(alpha)
+    l, u = torch.where(code > 0, l.clamp(min=0), l), torch.where(code < 0, u.clamp(max=0), u)
+    on, off = (code > 0) | (l >= 0), (code < 0) | ((code <= 0) & (u <= 0))
+    us = torch.where(on, 1.0, torch.where(off, 0.0, u / (u - l).clamp(min=1e-8)))
+    ls, ui = torch.where(on, 1.0, torch.where(off, 0.0, al)), torch.where(on | off, 0.0, -us * l)
+
+    def forward(k, z):
+        w = net.weights[k]
+        if k == L - 1:
+            return z @ t(w).abs().T
+        return F.conv2d(z.reshape(-1, w.ic, w.ih, w.iw), t(w.weight).abs(), None, (w.sh, w.sw), (w.ph, w.pw)).flatten(1)
+
+    def back(k, a):
+        w = net.weights[k]
+        if k == L - 1:
+            return a @ t(w)
+        pad = [(n + 2 * p - kk) % s for n, p, kk, s in ((w.ih, w.ph, w.weight.shape[2], w.sh), (w.iw, w.pw, w.weight.shape[3], w.sw))]
+        return F.conv_transpose2d(a.reshape(-1, w.oc, w.oh, w.ow), t(w.weight), None, (w.sh, w.sw), (w.ph, w.pw), pad).flatten(1)
+
+    xl, xu = t(lo), t(hi)
+    z = [torch.maximum(xl.abs(), xu.abs()).expand(D, -1)] + [torch.where(code < 0, 0.0, u.clamp(min=0))[:, offs[k]:offs[k + 1]] for k in range(L - 1)]
+    a = t(np.concatenate([spec, spec])).repeat(D, 1)
+    upper = (torch.arange(2 * S, device=a.device) >= S).repeat(D)[:, None]
+    sign, rows = torch.where(upper, 1.0, -1.0), lambda x: x.repeat_interleave(2 * S, 0)
+    const, charge, floor, kept = torch.zeros(len(a), device=a.device).double(), 0.0, 0.0, {}
+    for k in range(L - 1, -1, -1):
+        b = net.biases[k] if k == L - 1 else np.repeat(net.weights[k].bias, net.weights[k].oh * net.weights[k].ow)
+        q = rows(forward(k, z[k]))
+        w = net.weights[k]
+        rate = _f16_rate(net.dims[L]) if k == L - 1 else _transposed_rate(w.ic, w.oc, w.weight.shape[2], w.sh, w.ph, w.oh, w.ow, w.ih, w.iw)[0]
+        const, charge, floor = const + a @ t(b), charge + rate * (a.abs() * q).sum(1), floor + q.sum(1)
+        if k in net.skips:
+            kept[net.skips[k]] = kept.get(net.skips[k], 0.0) + a
+        a = back(k, a)
+        if k:
+            j = slice(offs[k - 1], offs[k])
+            a = a + kept.get(k - 1, 0.0)
+            line = (a > 0) == upper        # the upper line, or the lower one
+            const = const + torch.where(line, a * rows(ui[:, j]), 0.0).sum(1)
+            a = torch.where(line, a * rows(us[:, j]), a * rows(ls[:, j])) + sign * rows(beta[:, j])
+    take = (a >= 0) == upper
+    bound = (const + torch.where(take, a * xu, a * xl).sum(1)).reshape(D, 2, S).cpu().numpy()
+    return bound[:, 0], bound[:, 1], charge.reshape(D, 2, S).cpu().numpy(), floor.reshape(D, 2, S).cpu().numpy()
+
+
+@pytest.mark.parametrize("scale", [1.0, 5e-32])
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_every_rounding_is_charged_outwards(eng, case, scale):
+    """A lower bound lies below the same lines' bound in plain binary64, an upper one above it, by what the layers charge, each at its
+    products' rate (window, im2col, fully connected): a twentieth is left for the actual roundings, which are a tenth of
+    their rates, and a quarter on top for the lines' own charges; rows of tiny coefficients, whose scale ends near fp32's,
+    add the share of the exponent range (1.1e-37 of the weights' and inputs' magnitudes).  A layer whose charge is lost, or
+    charged to the wrong side, falls short."""
+    from ny_b200 import engine
+
+    chw, convs, skips, S, D, mult = CASES[case]
+    net = _net(chw, convs, skips, S + 1, 90 + case)
+    g = np.random.default_rng(290 + case)
+    x = g.uniform(0, 1, int(net.dims[0])).astype(np.float32)
+    lo, hi = (x - 0.02).astype(np.float32), (x + 0.02).astype(np.float32)
+    spec = (W.margin_spec(S + 1, 0)[:S] * np.float32(scale)).astype(np.float32)
+    nid = eng.register_network(net)
+    pl, pu = eng.ibp_forward_gpu(nid, lo, hi)
+    offs = np.concatenate([[0], np.cumsum(net.dims[1:-1])])
+    unstable = np.flatnonzero((pl[0, :offs[-1]] < 0) & (pu[0, :offs[-1]] > 0))
+    edges = np.linspace(0, len(unstable), 5).astype(np.int64)
+    pick = unstable[edges[:-1] + (g.random((D, 4)) * (edges[1:] - edges[:-1])).astype(np.int64)]
+    relu = np.searchsorted(offs, pick, side="right") - 1
+    sp = np.zeros((D, 4), SPLIT_DTYPE)
+    sp["relu"], sp["neuron"] = relu, pick - offs[relu]
+    sp["sign"] = np.where(g.random((D, 4)) < 0.5, 1, -1)
+    sp["beta"] = np.float32(scale * min(mult, 2.0)) * g.random((D, 4), dtype=np.float32)
+    alpha = g.random((D, net.n_pre), dtype=np.float32)
+    eng.set_refine_tolerance(0.0)
+    eng.set_path(engine.PATH_TF32X3)
+    got_l, got_u, inf = eng.bab_bound_batch(nid, spec, lo, hi, pl[0], pu[0], sp, np.full(D, 4, np.int32), 0, alpha)   # the inherited intervals as they are
+    eng.set_refine_tolerance(5e-5)
+    eng.set_path(engine.PATH_AUTO)
+    eng.release_network(nid)
+    want_l, want_u, charge, floor = _exact(net, spec, lo, hi, pl[0], pu[0], sp, alpha)
+    assert not inf.any() and np.isfinite(got_l).all() and np.isfinite(got_u).all()
+    for short, c, f in ((want_l - got_l, charge[:, 0], floor[:, 0]), (got_u - want_u, charge[:, 1], floor[:, 1])):
+        assert (short >= 0.95 * c).all(), (short / c).min()
+        assert (short <= 1.25 * c + 1.1e-37 * f).all(), (short / c).max()
