@@ -301,7 +301,7 @@ int create_net(nyb200_engine *e, int32_t n_layers, const nyb200_layer_desc *ld, 
             const size_t nb = conv ? (size_t)l.out_channels : (size_t)l.out_features;
             for (size_t i = 0; i < nb; ++i) {
                 if (!std::isfinite(bflat[bo + i])) return set_err(e, NYB200_ERR_NUMERICAL, "non-finite bias");
-                net.bmax.back() = std::max(net.bmax.back(), std::fabs(bflat[bo + i]));
+                net.bmax.back() = std::max(net.bmax.back(), bflat[bo + i]);
             }
             const float *src = bflat + bo;
             if (conv) { expand_bias(bflat + bo, l.out_channels, l.out_h * l.out_w, expanded); src = expanded.data(); }

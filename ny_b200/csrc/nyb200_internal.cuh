@@ -118,7 +118,7 @@ struct Net {
     std::vector<UmmaLayer> umma_adj;    // forward products of the adjoint pass and the attack
     bool umma_whole = false;            // every entry of umma / win_bwd is there
     std::vector<float> wmax;          // per layer: largest |weight|; negative when some weight is too small beside it for fp16 pairs
-    std::vector<float> bmax;          // per layer: largest |bias|
+    std::vector<float> bmax;          // per layer: largest bias, at least zero: what it can add behind a ReLU
     std::vector<WinOp> win_bwd, win_fwd;   // window forms of the convolution layers, with umma and umma_adj
     std::vector<float *> frag;        // weights in binary64-fragment order (nyb200_direct.cu)
 };
@@ -450,7 +450,7 @@ int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g,
 // What is done to the rows on their way into a window convolution: bias and ReLU, the result kept (in place, or not), or a mask.
 struct WinWith {
     const float *bias = nullptr;    // [channels x plane], or null: neither bias nor ReLU
-    float bias_max = 0.f;           // its largest magnitude
+    float bias_max = 0.f;           // its largest value, at least zero (what it takes away is cut off)
     float *keep = nullptr;
     const float *mask = nullptr;    // rows of what has to be positive, or null
     long keep_ld = 0, mask_ld = 0;

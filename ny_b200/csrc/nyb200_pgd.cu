@@ -107,11 +107,13 @@ __global__ void __launch_bounds__(256) k_relu_mask(int n, float *__restrict__ G,
 }
 
 // AdamClipping step (pgd_attack/adam_state.rs:46-88), descending the objective.  A restart whose gradient
-// holds a NaN skips the step (attacker/batched.rs:93-104): rows flagged in nan_row are left alone.
+// holds a NaN skips the step (attacker/batched.rs:93-104): rows flagged in nan_row are left alone.  x_max (optional, cleared by
+// k_nan_rows): the stepped rows' largest magnitudes (bits), for the first convolution's split.
 __global__ void __launch_bounds__(256) k_pgd_step(int n0, float *__restrict__ X, long ld, const float *__restrict__ G,
                            float *__restrict__ mom, float *__restrict__ var, const float *__restrict__ lo,
-                           const float *__restrict__ hi, const int *__restrict__ nan_row, PgdStep h, bool vec) {
+                           const float *__restrict__ hi, const int *__restrict__ nan_row, unsigned *__restrict__ x_max, PgdStep h, bool vec) {
     const int r = blockIdx.y;
+    float most = 0.f;
     if (nan_row[r]) return;
     float *x_row = X + (long)r * ld, *m_row = mom + (long)r * n0, *v_row = var + (long)r * n0;
     const float *g_row = G + (long)r * ld;
@@ -126,6 +128,7 @@ __global__ void __launch_bounds__(256) k_pgd_step(int n0, float *__restrict__ X,
         }
         x = x - dir * h.step;
         x = isnan(x) ? l : fminf(fmaxf(x, l), u);
+        most = fmaxf(most, fabsf(x));
     };
     over_row(n0, vec, [&](int j, int w) {
         if (w == 4) {
@@ -135,14 +138,21 @@ __global__ void __launch_bounds__(256) k_pgd_step(int n0, float *__restrict__ X,
             *(float4 *)(m_row + j) = m; *(float4 *)(v_row + j) = v; *(float4 *)(x_row + j) = x;
         } else one(g_row[j], m_row[j], v_row[j], x_row[j], lo[j], hi[j]);
     });
+    if (x_max) {
+        const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(most));
+        if ((threadIdx.x & 31) == 0 && w) atomicMax(x_max + r, w);
+    }
 }
 
-__global__ void __launch_bounds__(256) k_nan_rows(int n0, const float *__restrict__ G, long ld, int *__restrict__ nan_row) {
+__global__ void __launch_bounds__(256) k_nan_rows(int n0, const float *__restrict__ G, long ld, int *__restrict__ nan_row, unsigned *__restrict__ x_max) {
     const float *g = G + (long)blockIdx.x * ld;
     int bad = 0;
     for (int j = threadIdx.x; j < n0; j += 256) bad |= isnan(g[j]) ? 1 : 0;
     bad = __syncthreads_or(bad);
-    if (threadIdx.x == 0) nan_row[blockIdx.x] = bad;
+    if (threadIdx.x == 0) {
+        nan_row[blockIdx.x] = bad;
+        if (x_max && !bad) x_max[blockIdx.x] = 0;   // (a row that is not stepped keeps its own)
+    }
 }
 
 // Y[r, j] += X[r, j]
@@ -163,11 +173,6 @@ __global__ void k_row_dot(int rows, int n, const float *__restrict__ X, int ldx,
     for (int j = lane; j < n; j += 32) acc = fma((double)X[(long)warp * ldx + j], (double)Y[(long)warp * ldy + j], acc);
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) out[warp] = (float)acc;
-}
-
-__global__ void k_at_least(float *p, int n, float v) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) p[t] = fmaxf(p[t], v);
 }
 
 __global__ void k_fill_f32(float *p, long n, float v) {
@@ -194,7 +199,7 @@ static int pgd_forward(nyb200_engine *e, Net &net, bool tensor, int rows, const 
             if (pending) {
                 with.bias = nv.b[k - 1]; with.bias_max = net.bmax[k - 1]; with.keep = act[k - 1]; with.keep_ld = ld;
                 with.has_max = true;
-            } else if (k == 0 && x_rows) {   // points that stay in a box: their maxima are known
+            } else if (k == 0 && x_rows) {   // the points' maxima are known
                 void *hi, *lo;
                 float *row_inv;
                 unsigned *row_max;
@@ -348,17 +353,12 @@ int pgd_attack(nyb200_engine *e, int net_id, const float *spec, int S, const flo
     k_fill_f32<<<(K + 255) / 256, 256, 0, st>>>(dbest, K, INFINITY);
     e->launches++;
     const unsigned gw = (unsigned)(((long)K * 32 + 255) / 256);
-    float x_max = 0.f;   // of the box the points stay in
-    for (int j = 0; j < n0; ++j) x_max = std::max(x_max, std::max(std::fabs(in_lo[j]), std::fabs(in_hi[j])));
-    // A point's largest magnitude: the box's, or its first one's (the caller's, in the box or not; a restart whose gradient is
-    // not a number stays there).
+    // The points' largest magnitudes, kept up to date by the steps.
     unsigned *x_rows = nullptr;
-    if (tensor && net->is_conv(0) && net->win_fwd[0].ok && std::isfinite(x_max)) {
+    if (tensor && net->is_conv(0) && net->win_fwd[0].ok) {
         x_rows = (unsigned *)ws_get(e, "pgd_xmax", (size_t)K * 4);
         if (!x_rows) return NYB200_ERR_OOM;
         NYB_TRY(row_maxima(e, K, n0, X, ld, x_rows));
-        k_at_least<<<(unsigned)((K + 255) / 256), 256, 0, st>>>((float *)x_rows, K, x_max);
-        e->launches++;
     }
 
     for (int t = 1; t <= cfg.steps + 1; ++t) {
@@ -372,7 +372,7 @@ int pgd_attack(nyb200_engine *e, int net_id, const float *spec, int S, const flo
         if (last) break;
         float *g = nullptr;
         NYB_TRY(pgd_backward(e, *net, tensor, K, G0, G1, act.data(), ld, derr, &g));
-        k_nan_rows<<<(unsigned)K, 256, 0, st>>>(n0, g, ld, dnan);
+        k_nan_rows<<<(unsigned)K, 256, 0, st>>>(n0, g, ld, dnan, x_rows);
         PgdStep h;
         float bc1 = 1.f - powf(b1, (float)t);
         h.bc2 = 1.f - powf(b2, (float)t);
@@ -380,7 +380,7 @@ int pgd_attack(nyb200_engine *e, int net_id, const float *spec, int S, const flo
         h.beta1 = b1; h.beta2 = b2; h.epsilon = eps;
         for (int r0 = 0; r0 < K; r0 += 65535)
             k_pgd_step<<<NYB_ROWS(std::min(K - r0, 65535), n0), 0, st>>>(n0, X + (size_t)r0 * ld, ld, g + (size_t)r0 * ld, mom + (size_t)r0 * n0, var + (size_t)r0 * n0, dlo, dhi,
-                                                                          dnan + r0, h, vec4(n0, ld, X, g, mom, var) && vec4(n0, ld, dlo, dhi));
+                                                                          dnan + r0, x_rows ? x_rows + r0 : nullptr, h, vec4(n0, ld, X, g, mom, var) && vec4(n0, ld, dlo, dhi));
         e->launches += 2;
     }
     // independent evaluation of every restart's best point with binary64 contractions
