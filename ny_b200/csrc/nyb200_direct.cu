@@ -1096,16 +1096,20 @@ int launch_pass(nyb200_engine *e, const PackedNet &pn, int top, int n_rows, int 
     // a launch that leaves SMs idle all the same: clusters of two to eight CTAs of eight warps each
     int C = 1;
     while (NW >= 8 && C < 8 && groups * C * 2 <= sms && tiles >= NW * 2) { C *= 2; NW *= 2; }
-    // Warps alone with all columns of their rows: two groups of rows each (k_direct_rows) where that still fills the SMs' twelve
-    // places; fewer rows want the warps.
-    if (NW == 1 && C == 1 && !ckpt && groups >= sms * 24) {
+    // Warps alone with all columns of their rows, six tiles of them and more: two groups of rows each (k_direct_rows), three CTAs of
+    // eight groups an SM where the one-group form has two.  It pays where that saves a wave of CTAs and costs where it does not:
+    // 5 -> 6x50 -> 5, us a call, one group / two, at n groups an SM: 16 311/347  20 429/357  24 442/406  26 458/505  32 484/525
+    // 34 580/532  48 676/627  56 833/789  72 991/883  96 1216/1110; 4x64: 24 263/238  32 278/316  36 329/331  48 367/362  72 538/522.
+    // Up to five tiles both have three CTAs: 4x20 and 5x33 within 2 % of each other from 8 to 96 groups an SM.
+    auto waves = [&](long per_sm) { return ((long)groups + per_sm * sms - 1) / (per_sm * sms); };
+    if (NW == 1 && C == 1 && !ckpt && tiles >= 6 && waves(24) < waves(16)) {
         const size_t rows_smem = (size_t)4 * 2 * 8 * pitch * 8;
         const dim3 rows_grid((unsigned)((groups + 7) / 8));
 #define NYB_ROWS_PASS(NT) case NT:                                                                                              \
         NYB_TRY(allow_smem(e, (const void *)k_direct_rows<NT>, rows_smem));                                                     \
         NYB_CUDA(e, launch_pdl(k_direct_rows<NT>, rows_grid, dim3(128), rows_smem, e, pn, top, D, idx, n_rows, pitch, seed, seed_bias, \
                                (const float *)p.in_lo, (const float *)p.in_hi, box_ds, ptab, c_lo, c_hi, a_out, p.lda)); break;
-        switch (tiles) { NYB_ROWS_PASS(1) NYB_ROWS_PASS(2) NYB_ROWS_PASS(3) NYB_ROWS_PASS(4) NYB_ROWS_PASS(5) NYB_ROWS_PASS(6) NYB_ROWS_PASS(7) NYB_ROWS_PASS(8) }
+        switch (tiles) { NYB_ROWS_PASS(6) NYB_ROWS_PASS(7) NYB_ROWS_PASS(8) }
 #undef NYB_ROWS_PASS
         e->launches++;
         return NYB200_OK;
