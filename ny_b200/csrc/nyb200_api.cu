@@ -885,14 +885,17 @@ int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float
     };
     // Layers whose rows go through the relaxation straight into their convolution's operand (nyb200_winrelax.cu), 1: a window's
     // pairs, 2: pixel-major rows of an im2col-space product: the tables are the interval pass's (slopes in [0, 1], multipliers
-    // the uploaded ones), nothing else reads the rows, and an identity branch is kept and joined in the same pixel order.
+    // the uploaded ones), nothing else reads the rows, and an identity branch is kept and joined in the same pixel order.  The second
+    // form is for layers that a branch starts from, whose partner wants that order (the stem of a residual network): elsewhere planar
+    // rows through k_relax_dom are as fast or faster (convolutional classifiers, 16 -> 32 channels, side 16: 512 domains 669 us a call
+    // in pixels, 649 in planes, 1024 1054 / 1011; 8 -> 16, side 28: 512 domains 2948 / 2900, 16 domains 522 / 525).
     std::vector<char> image((size_t)L, 0);
     if (tensor && !fused && !ckpt && !partial && p.beta_max && !b.external_tables && !p.alpha_up && D <= 65535) {   // (grid)
         auto same_image = [&](int i, int j) { const ConvGeom &x = net.geom[i], &y = net.geom[j]; return net.is_conv(i) && net.is_conv(j) && x.oc == y.oc && x.oh == y.oh && x.ow == y.ow; };
         for (int k = 0; k < L - 1; ++k) {
             if (!net.is_conv(k) || net.geom[k].oc % 4 != 0 || net.geom[k].oc > 128) continue;
             if (net.win_bwd[k].ok) image[k] = net.win_bwd[k].in_cp <= 128 ? 1 : 0;
-            else image[k] = net.skip_of(k) < 0 ? 2 : 0;
+            else image[k] = net.skip_of(k) < 0 && std::find(net.skip.begin(), net.skip.end(), k) != net.skip.end() ? 2 : 0;
         }
         for (bool again = true; again; ) {
             again = false;
