@@ -82,7 +82,8 @@ k_adjoint_seed(long rows, int S, int R, int Zr, int n0, const float *__restrict_
 // into the relaxation table the next backward pass reads.
 // What bounds it: the latency of its loads.  What the step reads is fetched ahead of the rows, and nothing is divided: with
 // one neuron a thread, two 64-bit divisions each, and the step's reads behind the rows, 53 us a layer for 2048 domains of 9 rows
-// of 512 neurons, more than twice its bytes' time; so 40.
+// of 512 neurons, more than twice its bytes' time; so 40.  One neuron a thread (odd widths) is held to 48 registers, five blocks an
+// SM: with 60 the threads of 500 domains of 301 neurons were one wave and a little (2.42 -> 2.36 ms for six iterations, seven rows).
 template <int V>
 struct Vals { float v[V]; };
 template <int V>
@@ -96,7 +97,7 @@ __device__ __forceinline__ void store_vals(float *p, const Vals<V> &r) {
     if constexpr (V == 2) *(float2 *)p = make_float2(r.v[0], r.v[1]); else *p = r.v[0];
 }
 template <int V>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, V == 1 ? 5 : 0)
 k_adjoint_relu(int n, int off, int D, int S, int R, int Zr, long nps, float *__restrict__ Z, int ldz,
                const float *__restrict__ bias, const float *__restrict__ Apre, int ldc, float4 *__restrict__ tab,
                const signed char *__restrict__ code, const float *__restrict__ pre_lo,
@@ -538,8 +539,9 @@ int optimize_batch(nyb200_engine *e, const nyb200_opt_config &cfg, float *grad_h
             }
             const bool two = ((N | nv.pre_off[k] | (int)np | ldz | ldc) & 1) == 0 &&
                              ((reinterpret_cast<uintptr_t>(zn) | reinterpret_cast<uintptr_t>(ckpt[k]) | reinterpret_cast<uintptr_t>(nv.b[k])) & 7) == 0;
-            // a narrow layer's domains share a block
-            const int per = (N + (two ? 1 : 0)) / (two ? 2 : 1), tx = std::min(256, (per + 31) / 32 * 32), ty = 256 / tx;
+            // a narrow layer's domains share a block; a wide one's neurons are spread evenly over its blocks (301 neurons, one a thread: two
+            // blocks of 160 and not of 256)
+            const int per = (N + (two ? 1 : 0)) / (two ? 2 : 1), blocks = (per + 255) / 256, tx = ((per + blocks - 1) / blocks + 31) / 32 * 32, ty = 256 / tx;
             const dim3 grid((unsigned)((D + ty - 1) / ty), (unsigned)((per + tx - 1) / tx)), block((unsigned)tx, (unsigned)ty);
 #define NYB_ADJOINT(V) k_adjoint_relu<V><<<grid, block, 0, e->stream>>>(N, nv.pre_off[k], D, S, R, Zr, np, zn, ldz, nv.b[k], ckpt[k], ldc, p.tab, p.code, p.pre_lo, \
                                                                        p.pre_hi, mom, var, only_row, p.alpha_up, mom_up, var_up, grad_dev, h,                    \
