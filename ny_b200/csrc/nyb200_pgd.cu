@@ -17,32 +17,38 @@ struct PgdStep {
     float step, beta1, beta2, epsilon, bc2;
 };
 
-// The element-wise kernels: one row a grid row, four columns a thread where the row allows it (VEC); an index division per
-// element and one column a thread held them to a third of the copy rate (bias and ReLU of 1024 x 4096: 15.4 -> 7 us).
-#define NYB_ROWS(rows, n) dim3((unsigned)(((n) + 1023) / 1024), (unsigned)(rows)), 256
+// The element-wise kernels.  Large launches: one row a grid row, four columns a thread where the row allows it (VEC); an index
+// division per element and one column a thread held them to a third of the copy rate (bias and ReLU of 1024 x 4096: 15.4 -> 7
+// us).  Small ones, a few hundred values an SM, take one value a thread and few blocks, rows one behind the other: 16 restarts x 40
+// steps on 30 -> 4x60 -> 10, some 25 launches a step, 3.88 ms by rows, 3.82 so; on 784 -> 4x256 -> 10 6.04 and 5.97; 64 restarts on the
+// convolutional classifier of side 28 4.76 and 4.70.
+#define NYB_ROWS(rows, n, vec) (vec) ? dim3((unsigned)(((n) + 1023) / 1024), (unsigned)(rows)) : dim3((unsigned)(((long)(rows) * (n) + 255) / 256)), 256
 template <class F>
-__device__ __forceinline__ void over_row(int n, bool vec, F f) {   // f(column, columns from there: 4 or 1)
-    const int j0 = blockIdx.x * 1024;
+__device__ __forceinline__ void over_rows(int rows, int n, bool vec, F f) {   // f(row, column, columns from there: 4 or 1)
     if (vec) {
-        const int j = j0 + threadIdx.x * 4;
-        if (j < n) f(j, 4);
-    } else
-        for (int j = j0 + threadIdx.x; j < min(n, j0 + 1024); j += 256) f(j, 1);
+        const int j = (blockIdx.x * 256 + threadIdx.x) * 4;
+        if (j < n) f((int)blockIdx.y, j, 4);
+    } else {
+        const unsigned t = blockIdx.x * 256 + threadIdx.x, r = t / (unsigned)n;
+        if (t < (unsigned)rows * (unsigned)n) f((int)r, (int)(t - r * n), 1);
+    }
 }
-static bool vec4(int n, long ld, const void *a, const void *b = nullptr, const void *c = nullptr, const void *d = nullptr) {
-    return n % 4 == 0 && ld % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d)) & 15) == 0;
+static int rows_most(int n) { return std::min(65535, 0x7fffffff / n); }   // of one launch: grid, 32-bit index
+static bool vec4(int rows, int n, long ld, const void *a, const void *b = nullptr, const void *c = nullptr, const void *d = nullptr) {
+    return (long)rows * n >= 65536 && n % 4 == 0 && ld % 4 == 0 &&
+           ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d)) & 15) == 0;
 }
 
 // z += bias; optionally ReLU.  Post-activations are kept: z > 0 afterwards is exactly the gradient mask.
-__global__ void __launch_bounds__(256) k_bias_act(int n, float *__restrict__ Z, long ld, const float *__restrict__ bias, int relu, bool vec) {
-    float *z = Z + (long)blockIdx.y * ld;
+__global__ void __launch_bounds__(256) k_bias_act(int rows, int n, float *__restrict__ Z, long ld, const float *__restrict__ bias, int relu, bool vec) {
     auto one = [&](float x, float b) { const float v = x + b; return relu ? fmaxf(v, 0.f) : v; };
-    over_row(n, vec, [&](int j, int w) {
+    over_rows(rows, n, vec, [&](int r, int j, int w) {
+        float *z = Z + (long)r * ld + j;
         if (w == 4) {
-            float4 x = *(float4 *)(z + j);
+            float4 x = *(float4 *)z;
             const float4 b = bias ? *(const float4 *)(bias + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-            *(float4 *)(z + j) = make_float4(one(x.x, b.x), one(x.y, b.y), one(x.z, b.z), one(x.w, b.w));
-        } else z[j] = one(z[j], bias ? bias[j] : 0.f);
+            *(float4 *)z = make_float4(one(x.x, b.x), one(x.y, b.y), one(x.z, b.z), one(x.w, b.w));
+        } else *z = one(*z, bias ? bias[j] : 0.f);
     });
 }
 
@@ -85,38 +91,36 @@ __global__ void __launch_bounds__(256) k_pgd_objective(int K, int S, int nL, con
         for (int j = lane; j < nL; j += 32) G[(long)r * ldg + j] = spec[ms * nL + j];
 }
 
-__global__ void __launch_bounds__(256) k_keep_best(int n0, const float *__restrict__ X, long ldx, const int *__restrict__ improved, float *__restrict__ best_x, bool vec) {
-    const int r = blockIdx.y;
-    if (!improved[r]) return;
-    const float *x = X + (long)r * ldx;
-    float *b = best_x + (long)r * n0;
-    over_row(n0, vec, [&](int j, int w) { if (w == 4) *(float4 *)(b + j) = *(const float4 *)(x + j); else b[j] = x[j]; });
+__global__ void __launch_bounds__(256) k_keep_best(int rows, int n0, const float *__restrict__ X, long ldx, const int *__restrict__ improved, float *__restrict__ best_x, bool vec) {
+    over_rows(rows, n0, vec, [&](int r, int j, int w) {
+        if (!improved[r]) return;
+        const float *x = X + (long)r * ldx + j;
+        float *b = best_x + (long)r * n0 + j;
+        if (w == 4) *(float4 *)b = *(const float4 *)x; else *b = *x;
+    });
 }
 
 // G *= [Zpost > 0]
-__global__ void __launch_bounds__(256) k_relu_mask(int n, float *__restrict__ G, long ld, const float *__restrict__ Z, bool vec) {
-    float *g = G + (long)blockIdx.y * ld;
-    const float *z = Z + (long)blockIdx.y * ld;
-    over_row(n, vec, [&](int j, int w) {
+__global__ void __launch_bounds__(256) k_relu_mask(int rows, int n, float *__restrict__ G, long ld, const float *__restrict__ Z, bool vec) {
+    over_rows(rows, n, vec, [&](int r, int j, int w) {
+        float *g = G + (long)r * ld + j;
+        const float *z = Z + (long)r * ld + j;
         if (w == 4) {
-            float4 v = *(float4 *)(g + j);
-            const float4 m = *(const float4 *)(z + j);
-            *(float4 *)(g + j) = make_float4(m.x > 0.f ? v.x : 0.f, m.y > 0.f ? v.y : 0.f, m.z > 0.f ? v.z : 0.f, m.w > 0.f ? v.w : 0.f);
-        } else if (!(z[j] > 0.f)) g[j] = 0.f;
+            float4 v = *(float4 *)g;
+            const float4 m = *(const float4 *)z;
+            *(float4 *)g = make_float4(m.x > 0.f ? v.x : 0.f, m.y > 0.f ? v.y : 0.f, m.z > 0.f ? v.z : 0.f, m.w > 0.f ? v.w : 0.f);
+        } else if (!(*z > 0.f)) *g = 0.f;
     });
 }
 
 // AdamClipping step (pgd_attack/adam_state.rs:46-88), descending the objective.  A restart whose gradient
 // holds a NaN skips the step (attacker/batched.rs:93-104): rows flagged in nan_row are left alone.  x_max (optional, cleared by
 // k_nan_rows): the stepped rows' largest magnitudes (bits), for the first convolution's split.
-__global__ void __launch_bounds__(256) k_pgd_step(int n0, float *__restrict__ X, long ld, const float *__restrict__ G,
+__global__ void __launch_bounds__(256) k_pgd_step(int rows, int n0, float *__restrict__ X, long ld, const float *__restrict__ G,
                            float *__restrict__ mom, float *__restrict__ var, const float *__restrict__ lo,
                            const float *__restrict__ hi, const int *__restrict__ nan_row, unsigned *__restrict__ x_max, PgdStep h, bool vec) {
-    const int r = blockIdx.y;
     float most = 0.f;
-    if (nan_row[r]) return;
-    float *x_row = X + (long)r * ld, *m_row = mom + (long)r * n0, *v_row = var + (long)r * n0;
-    const float *g_row = G + (long)r * ld;
+    int row = -1;
     auto one = [&](float g, float &m, float &v, float &x, float l, float u) {
         m = h.beta1 * m + (1.f - h.beta1) * g;
         v = h.beta2 * v + (1.f - h.beta2) * g * g;
@@ -130,17 +134,24 @@ __global__ void __launch_bounds__(256) k_pgd_step(int n0, float *__restrict__ X,
         x = isnan(x) ? l : fminf(fmaxf(x, l), u);
         most = fmaxf(most, fabsf(x));
     };
-    over_row(n0, vec, [&](int j, int w) {
+    over_rows(rows, n0, vec, [&](int r, int j, int w) {
+        if (nan_row[r]) return;
+        row = r;
+        float *x_at = X + (long)r * ld + j, *m_at = mom + (long)r * n0 + j, *v_at = var + (long)r * n0 + j;
+        const float *g_at = G + (long)r * ld + j;
         if (w == 4) {
-            const float4 g = *(const float4 *)(g_row + j), l = *(const float4 *)(lo + j), u = *(const float4 *)(hi + j);
-            float4 m = *(float4 *)(m_row + j), v = *(float4 *)(v_row + j), x = *(float4 *)(x_row + j);
+            const float4 g = *(const float4 *)g_at, l = *(const float4 *)(lo + j), u = *(const float4 *)(hi + j);
+            float4 m = *(float4 *)m_at, v = *(float4 *)v_at, x = *(float4 *)x_at;
             one(g.x, m.x, v.x, x.x, l.x, u.x); one(g.y, m.y, v.y, x.y, l.y, u.y); one(g.z, m.z, v.z, x.z, l.z, u.z); one(g.w, m.w, v.w, x.w, l.w, u.w);
-            *(float4 *)(m_row + j) = m; *(float4 *)(v_row + j) = v; *(float4 *)(x_row + j) = x;
-        } else one(g_row[j], m_row[j], v_row[j], x_row[j], lo[j], hi[j]);
+            *(float4 *)m_at = m; *(float4 *)v_at = v; *(float4 *)x_at = x;
+        } else one(*g_at, *m_at, *v_at, *x_at, lo[j], hi[j]);
     });
-    if (x_max) {
-        const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(most));
-        if ((threadIdx.x & 31) == 0 && w) atomicMax(x_max + r, w);
+    if (x_max) {   // (a warp may span rows, and lanes of it have none)
+        const int first = __shfl_sync(0xffffffffu, row, 0);
+        if (__all_sync(0xffffffffu, row == first)) {
+            const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(most));
+            if ((threadIdx.x & 31) == 0 && w) atomicMax(x_max + first, w);
+        } else if (most > 0.f) atomicMax(x_max + row, __float_as_uint(most));
     }
 }
 
@@ -219,8 +230,10 @@ static int pgd_forward(nyb200_engine *e, Net &net, bool tensor, int rows, const 
             e->launches++;
         }
         if (!pending)
-            for (int r0 = 0; r0 < rows; r0 += 65535) {   // (grid)
-                k_bias_act<<<NYB_ROWS(std::min(rows - r0, 65535), N), 0, e->stream>>>(N, act[k] + (size_t)r0 * ld, ld, nv.b[k], k < nv.L - 1 ? 1 : 0, vec4(N, ld, act[k], nv.b[k]));
+            for (int r0 = 0, most = rows_most(N); r0 < rows; r0 += most) {
+                const int n = std::min(rows - r0, most);
+                const bool vec = vec4(n, N, ld, act[k], nv.b[k]);
+                k_bias_act<<<NYB_ROWS(n, N, vec), 0, e->stream>>>(n, N, act[k] + (size_t)r0 * ld, ld, nv.b[k], k < nv.L - 1 ? 1 : 0, vec);
                 e->launches++;
             }
         cur = act[k];
@@ -258,8 +271,10 @@ static int pgd_backward(nyb200_engine *e, Net &net, bool tensor, int K, float *G
         // a window convolution's split masks its rows itself where nothing else reads them
         const bool window = net.is_conv(k) && tensor && net.win_bwd[k].ok, masks = k < L - 1 && window && net.skip_of(k) < 0;
         if (k < L - 1 && !masks)
-            for (int r0 = 0; r0 < K; r0 += 65535) {   // (grid)
-                k_relu_mask<<<NYB_ROWS(std::min(K - r0, 65535), Kd), 0, st>>>(Kd, g + (size_t)r0 * ld, ld, act[k] + (size_t)r0 * ld, vec4(Kd, ld, g, act[k]));
+            for (int r0 = 0, most = rows_most(Kd); r0 < K; r0 += most) {
+                const int n = std::min(K - r0, most);
+                const bool vec = vec4(n, Kd, ld, g, act[k]);
+                k_relu_mask<<<NYB_ROWS(n, Kd, vec), 0, st>>>(n, Kd, g + (size_t)r0 * ld, ld, act[k] + (size_t)r0 * ld, vec);
                 e->launches++;
             }
         if (net.skip_of(k) >= 0) {  // the gradient of pre_k also reaches relu(pre_j) directly
@@ -366,8 +381,11 @@ int pgd_attack(nyb200_engine *e, int net_id, const float *spec, int S, const flo
         NYB_TRY(pgd_forward(e, *net, tensor, K, X, ld, act.data(), ld, derr, x_rows));
         const bool last = t == cfg.steps + 1;
         k_pgd_objective<<<gw, 256, 0, st>>>(K, S, nL, act[L - 1], ld, dspec, dbest, dimp, last ? nullptr : G0, ld, nullptr);
-        for (int r0 = 0; r0 < K; r0 += 65535)   // (grid)
-            k_keep_best<<<NYB_ROWS(std::min(K - r0, 65535), n0), 0, st>>>(n0, X + (size_t)r0 * ld, ld, dimp + r0, dbx + (size_t)r0 * n0, vec4(n0, ld, X, dbx));
+        for (int r0 = 0, most = rows_most(n0); r0 < K; r0 += most) {
+            const int n = std::min(K - r0, most);
+            const bool vec = vec4(n, n0, ld, X, dbx);
+            k_keep_best<<<NYB_ROWS(n, n0, vec), 0, st>>>(n, n0, X + (size_t)r0 * ld, ld, dimp + r0, dbx + (size_t)r0 * n0, vec);
+        }
         e->launches += 2;
         if (last) break;
         float *g = nullptr;
@@ -378,9 +396,12 @@ int pgd_attack(nyb200_engine *e, int net_id, const float *spec, int S, const flo
         h.bc2 = 1.f - powf(b2, (float)t);
         h.step = cfg.step_size * powf(decay, (float)(t - 1)) / bc1;
         h.beta1 = b1; h.beta2 = b2; h.epsilon = eps;
-        for (int r0 = 0; r0 < K; r0 += 65535)
-            k_pgd_step<<<NYB_ROWS(std::min(K - r0, 65535), n0), 0, st>>>(n0, X + (size_t)r0 * ld, ld, g + (size_t)r0 * ld, mom + (size_t)r0 * n0, var + (size_t)r0 * n0, dlo, dhi,
-                                                                          dnan + r0, x_rows ? x_rows + r0 : nullptr, h, vec4(n0, ld, X, g, mom, var) && vec4(n0, ld, dlo, dhi));
+        for (int r0 = 0, most = rows_most(n0); r0 < K; r0 += most) {
+            const int n = std::min(K - r0, most);
+            const bool vec = vec4(n, n0, ld, X, g, mom, var) && vec4(n, n0, ld, dlo, dhi);
+            k_pgd_step<<<NYB_ROWS(n, n0, vec), 0, st>>>(n, n0, X + (size_t)r0 * ld, ld, g + (size_t)r0 * ld, mom + (size_t)r0 * n0, var + (size_t)r0 * n0, dlo, dhi,
+                                                        dnan + r0, x_rows ? x_rows + r0 : nullptr, h, vec);
+        }
         e->launches += 2;
     }
     // independent evaluation of every restart's best point with binary64 contractions
