@@ -997,7 +997,7 @@ k_direct_forward(NetView nv, int mode, int zdim, const int *__restrict__ idx, co
                 bad |= relax_neuron(s_code[off + j], alpha, o + j, l, u, t, pl, pu);
                 t.w = s_beta[off + j];
                 tab[o + j] = t;
-                zabs[o + j] = fmaxf(fabsf(l), fabsf(u));
+                zabs[o + j] = charge_magnitude(l, u);
                 zl[o + j] = pl; zu[o + j] = pu;
             }
             pre_lo[o + j] = l; pre_hi[o + j] = u;

@@ -274,7 +274,7 @@ __global__ void k_ibp_finish(NetView nv, int k, int D, int mode, int last, const
     pre_lo[o] = l; pre_hi[o] = u;
     t4.w = sbeta[o];
     tab[o] = t4;
-    const float za = fmaxf(fabsf(l), fabsf(u));
+    const float za = charge_magnitude(l, u);
     zabs[o] = za;
     if (cj) cj[o] = __fmaf_ru(1.9073487e-7f /* 1.6 * 2^-23 */ + cj_kappa * 1.001f, za, cw);
     zl[o] = pl; zu[o] = pu;

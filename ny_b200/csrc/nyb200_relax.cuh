@@ -4,6 +4,8 @@
 
 namespace nyb {
 
+constexpr float kMinWidth = 1e-8f;   // RELU_RELAX_MIN_WIDTH, relu/mod.rs:24
+
 // One coefficient `a` of a row (`upper`: the row bounds from above) through ReLU's relaxation
 // t = (lower slope, upper slope, upper intercept, signed beta), then the charges of the contraction that follows.
 // au: the upper path's own lower slope (dual alpha, activations/relu/mod.rs:570-1128); equals t.x otherwise.
@@ -52,10 +54,19 @@ __device__ __forceinline__ float relax_coeff(const bool upper, float a, float4 t
     return nw;
 }
 
+// What the charges take for a neuron's max|z|.  The intercepts' sums are charged through the coefficients behind them: an intercept
+// only applies on the upper line, where |nw| >= |a| slope, and intercept / slope is the chord's -l up to rounding, so that
+// |a icp| <= |nw| max|z| (1 + 2^-21).  Where relax_neuron holds the chord's width at 1e-8 the slope is u / 1e-8 and the intercept up to
+// u, whatever small value u has: there it is that width.  (The factor covers the roundings of both and of the constant.)
+__device__ __forceinline__ float charge_magnitude(float l, float u) {
+    const float m = fmaxf(fabsf(l), fabsf(u));
+    return l < 0.f && u > 0.f && u - l < kMinWidth ? fmaxf(m, kMinWidth * 1.0000005f) : m;
+}
+
 // relax_coeff with its charges prepared per column: zg = max|z| where the outward step is charged (zero where z cannot be
-// negative), cj = eps q + 2^-40 (max|z| + |bias|), which bounds the contraction's rounding and, because an intercept only
-// applies on the upper line, where |a icp| <= |nw| max|z| (1 + 2^-21), that of the two binary64 sums.  A zero product stays zero;
-// one that underflowed (at most 2^-150) is covered by a charge of the caller's, kUnderflow times the sum of max|z|.
+// negative), cj = eps q + 2^-40 (max|z| + |bias|), which bounds the contraction's rounding and (charge_magnitude) that of the
+// two binary64 sums.  A zero product stays zero; one that underflowed (at most 2^-150) is covered by a charge of the caller's, kUnderflow
+// times the sum of max|z|.
 constexpr double kUnderflow = 1e-45;
 template <bool UPPER, bool BIAS>
 __device__ __forceinline__ float relax_prepared(float a, const float4 &t, float zg, float cj, float bias, double &sb, float &sp) {
@@ -82,8 +93,7 @@ __device__ __forceinline__ float relax_prepared(float a, const float4 &t, float 
 //     for neurons that cannot be negative as well (at most 3% more than the contraction's own charge).  kappa covers
 //     the fp32 accumulation of the two dot products below: a run of n fused multiply-adds errs by at most
 //     n * 2^-24 times the run's magnitude sum, and that sum is bounded term by term: |nw bias| directly, and
-//     |a * intercept| <= |nw| * max|z| * (1 + 2^-21), because an intercept only applies on the upper line, where the
-//     outward step moves nw away from zero (|nw| >= |a| * slope) and intercept / slope = -l up to rounding.
+//     |a * intercept| <= |nw| * max|z| * (1 + 2^-21): see charge_magnitude.
 //     A product that underflows to zero stays zero; the floor of the charge encloses it.
 //   * The intercept and bias dot products are accumulated in fp32 (gi, gb: one fused multiply-add per term) over a
 //     short run of columns; the caller adds each run to the row's binary64 bias.
@@ -144,7 +154,7 @@ __device__ __forceinline__ int relax_neuron(int s, const float *alpha, long o, f
     } else if (l >= 0.f) { ls = 1.f; us = 1.f; ui = 0.f; }
     else if (u <= 0.f) { ls = 0.f; us = 0.f; ui = 0.f; }
     else {
-        float w = fmaxf(u - l, 1e-8f);  // RELU_RELAX_MIN_WIDTH, relu/mod.rs:24
+        float w = fmaxf(u - l, kMinWidth);
         us = __fdiv_rn(u, w);
         // The reference uses ui = -l*u/w in round-to-nearest.  The chord is only a valid upper line if
         // us*l + ui >= 0 and us*u + ui >= u, so the intercept is taken as the smallest fp32 that
