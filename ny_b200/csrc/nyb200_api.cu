@@ -1460,9 +1460,16 @@ int32_t nyb200_bab_bound_batch(nyb200_engine *e, int32_t net_id, const float *sp
     NYB_TRY(upload_batch(e, net_id, spec, S, in_lo, in_hi, box_stride, inh_lo, inh_hi, splits, n_splits, max_splits, D, mode,
                          alpha, later));
     const int st = run_batch(e, later ? alpha : nullptr);
-    if (later && st != NYB200_OK) {   // the caller's array may go away, and the batch never had its slopes
-        if (e->side) cudaStreamSynchronize(e->side);
-        e->batch.valid = false;
+    if (later && st != NYB200_OK) {
+        // A run that was given up (a deadline) leaves the batch resident, as where the slopes went ahead of it: they follow now, from
+        // an array that may go away behind this call.
+        const std::string why = e->err;
+        BatchPtrs p;
+        const bool there = (!e->side || cudaStreamSynchronize(e->side) == cudaSuccess) && batch_ptrs(e, *net, e->batch, p) == NYB200_OK &&
+                           upload_rows(e, p.alpha, (size_t)net->v.nps * 4, alpha, (size_t)net->v.n_pre * 4, (size_t)D, e->stream) == NYB200_OK &&
+                           cudaStreamSynchronize(e->stream) == cudaSuccess;
+        if (!there) e->batch.valid = false;
+        return set_err(e, st, why);
     }
     NYB_TRY(st);
     return download_batch(e, out_lo, out_hi, infeasible);

@@ -52,6 +52,33 @@ def test_late_slopes_are_the_uploaded_ones(case):
     eng.close()
 
 
+def test_a_given_up_call_leaves_its_batch_resident():
+    from ny_b200 import B200Engine, EngineError, engine
+
+    g = np.random.default_rng(23)
+    net, D = W.make_mlp([20, 300, 300, 300, 4], 3), 400
+    x = g.uniform(0, 1, 20).astype(np.float32)
+    lo, hi = x - np.float32(0.03), x + np.float32(0.03)
+    spec = W.margin_spec(4, 1)
+    eng = B200Engine(0)
+    nid = eng.register_network(net)
+    pl, pu = eng.ibp_forward_gpu(nid, lo, hi)
+    alpha = g.uniform(0, 1, (D, net.n_pre)).astype(np.float32)
+    assert alpha.nbytes >= 1 << 20
+    args = (nid, spec, lo, hi, pl[0], pu[0], np.zeros((D, 0), SPLIT_DTYPE), np.zeros(D, np.int32), 1, alpha)
+    want = eng.bab_bound_batch(*args)
+    eng.bab_bound_batch(*args[:-1], np.zeros_like(alpha))   # other slopes in the batch's place
+    eng.set_deadline(0.0)
+    with pytest.raises(EngineError) as ei:
+        eng.bab_bound_batch(*args)
+    assert ei.value.code == engine.DEADLINE and "deadline" in str(ei.value)
+    eng.set_deadline(None)
+    eng.batch_run()
+    for a, b in zip(eng.batch_download(), want):
+        assert np.array_equal(a, b)
+    eng.close()
+
+
 @pytest.mark.parametrize("widths", [(5, 6), (64, 66), (130, 127), (301, 3)])
 def test_branching_picks_the_first_widest(widths):
     from ny_b200 import B200Engine
