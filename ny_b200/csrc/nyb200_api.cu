@@ -844,7 +844,7 @@ int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float
     int D = b.D, S = b.S, R = b.R, L = partial ? top + 1 : nv.L;
     // Fused chain: seed, identity pass and the contractions L-1 .. 1 with their relaxations run as one kernel that
     // keeps the rows on the SM; what is left for the loop below is Linear_0's (wide) contraction.
-    const bool fused = tensor && e->fuse_chain && !ckpt && chain_eligible(net, L) && (nv.nps % 4 == 0) && (p.lda % 4 == 0);
+    const bool fused = tensor && e->fuse_chain && !ckpt && !b.steep && chain_eligible(net, L) && (nv.nps % 4 == 0) && (p.lda % 4 == 0);
     int *derr = nullptr;
     if (tensor) {
         NYB_TRY(prepare_backward_operands(e, net, fused));
@@ -1057,7 +1057,7 @@ int run_backward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, float
         }
         if (k > 0)
             launch_relax(e, nv, k - 1, k - 1, M, R, S, nxt, p.lda, p.tab, p.zabs, p.q, q_ds(k - 1), eps_for(k - 1), p.rb, p.rabs,
-                         p.rpen, dst == nxt ? nullptr : dst, ldd, p.alpha_up);
+                         p.rpen, dst == nxt ? nullptr : dst, ldd, p.alpha_up, b.steep);
         float *t = cur; cur = nxt; nxt = t;
     }
     p.a_final = cur;

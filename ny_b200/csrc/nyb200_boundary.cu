@@ -234,6 +234,7 @@ static int upload_domains(nyb200_engine *e, const nyb200_domain_ref *domains, in
                     return set_err(e, NYB200_ERR_NUMERICAL, "non-finite relaxation table or abs-max entry: the batch is refused as a whole");
                 tab[o] = t;
                 zabs[o] = na[j];
+                b.steep |= (double)std::fabs(t.z) > (double)std::fabs(t.y) * na[j] * (1.0 + 4.76837158203125e-07);   // 2^-21: see charge_magnitude
                 // the optimiser classifies neurons by their interval: any interval consistent with the baked line
                 const bool unstable = !(t.y == 1.f && t.z == 0.f) && !(t.y == 0.f && t.z == 0.f);
                 pre_lo[o] = unstable ? -na[j] : (t.y == 1.f ? 0.f : -na[j]);

@@ -143,6 +143,8 @@ struct Batch {
     int inh_stride = 0;     // 0: one inherited-bound vector for all domains; nps: one row per domain (nyb200_batch_set_inherited)
     bool external_tables = false;  // relaxation tables, abs-max tables and q were uploaded by a reference-shaped call:
                                    // nothing may re-derive them with an interval pass
+    bool steep = false;      // an uploaded intercept is larger than its slope times the magnitude: not for the kernels that charge
+                             // intercepts through the coefficients behind them (charge_magnitude)
     // Left behind by the last plain-CROWN call: the input-level coefficient rows of its final pass
     // ([crown_D * 2 * crown_S x crown_lda], per box S lower rows then S upper rows), until any call reuses the workspace.
     const float *crown_a = nullptr;
@@ -299,7 +301,7 @@ void launch_seed_identity(nyb200_engine *e, int n, int D, int lda, float *A);
 // With Asrc != nullptr the rows are read from Asrc (row stride lds) and the result written to A.
 void launch_relax(nyb200_engine *e, const NetView &nv, int r, int lin_k, int M, int R, int S, float *A, int lda,
                   const float4 *tab, const float *zabs, const float *q, long q_dstride, double eps_gemm, double *rb,
-                  double *rabs, double *rpen, const float *Asrc, int lds, const float *aup = nullptr);
+                  double *rabs, double *rpen, const float *Asrc, int lds, const float *aup = nullptr, bool steep = false);
 // C[M x N] = A[M x K] * W_k (binary64 accumulation), cast error charged to rpen.
 void launch_gemm_f64(nyb200_engine *e, int M, int N, int K, const float *A, int lda, const float *B, int ldb, float *C,
                      int ldc, int R, const float *zin_lo, const float *zin_hi, long zin_dstride, double *rpen);

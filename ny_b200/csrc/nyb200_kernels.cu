@@ -989,7 +989,7 @@ void launch_seed_identity(nyb200_engine *e, int n, int D, int lda, float *A) {
 
 void launch_relax(nyb200_engine *e, const NetView &nv, int r, int lin_k, int M, int R, int S, float *A, int lda,
                   const float4 *tab, const float *zabs, const float *q, long q_dstride, double eps_gemm, double *rb,
-                  double *rabs, double *rpen, const float *Asrc, int lds, const float *aup) {
+                  double *rabs, double *rpen, const float *Asrc, int lds, const float *aup, bool steep) {
     int n = nv.dims[lin_k + 1], off = nv.pre_off[lin_k];
     if (!Asrc) { Asrc = A; lds = lda; }
     long threads = (long)M * 32;
@@ -1011,8 +1011,9 @@ void launch_relax(nyb200_engine *e, const NetView &nv, int r, int lin_k, int M, 
         const int parts = slab_warps < (long)usable_sms(e) * 16 ? 2 : 1;
         const long dwarps = slab_warps * parts;
         const unsigned dgrid = (unsigned)((dwarps * 32 + 255) / 256);
-        // domain-major when a domain's rows amortise the table loads and there are enough warps to fill the GPU
-        if (r >= 0 && R >= 4 && dwarps >= 2048) {
+        // domain-major when a domain's rows amortise the table loads and there are enough warps to fill the GPU (steep: an uploaded
+        // intercept that only the other kernels charge)
+        if (r >= 0 && R >= 4 && dwarps >= 2048 && !steep) {
             if (bk) k_relax_dom<true><<<dgrid, 256, 0, e->stream>>>(n, off, D, R, S, parts, (long)nv.nps, A, lda, Asrc, lds, tab, zabs, q, q_dstride, bk, aup, epsf, rb, rpen);
             else k_relax_dom<false><<<dgrid, 256, 0, e->stream>>>(n, off, D, R, S, parts, (long)nv.nps, A, lda, Asrc, lds, tab, zabs, q, q_dstride, bk, aup, epsf, rb, rpen);
         } else {

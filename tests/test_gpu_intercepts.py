@@ -47,3 +47,34 @@ def test_intercepts_of_the_smallest_widths_are_charged():
     assert np.all(lo <= mine[0] - charge[0] + slack[0]) and np.all(hi >= mine[1] + charge[1] - slack[1])
     assert np.all(lo >= mine[0] - 4 * charge[0] - slack[0]) and np.all(hi <= mine[1] + 4 * charge[1] + slack[1])
     eng.close()
+
+
+@pytest.mark.parametrize("width,rows", [(64, 9), (260, 9), (260, 1)])
+def test_lines_of_the_caller_with_steep_intercepts_are_charged(width, rows):
+    """Constant upper lines (slope 0): nothing is left of the coefficients that the intercepts' sums could be charged through."""
+    from ny_b200 import B200Engine, engine
+
+    D = 700 if width > 256 else 70
+    net = _net(width, rows, width + rows)
+    zero, half = np.zeros(width, np.float32), np.full(width, 0.5, np.float32)
+    # a sum of 1 and seven terms of 2^-25: one behind the other in fp32 they are all lost
+    icp = np.full(width, 0.75, np.float32)
+    icp[:8] = [2.0, *[2.0 ** -24] * 7]
+    w = net.weights
+    w[-1][:, 8:] = 0
+    w[-1][:, :8] = np.where(np.arange(rows) % 2, 0.5, -0.5)[:, None]
+    layers = [("linear", w[2], net.biases[2]), ("act", zero, zero, None, icp), ("linear", w[1], net.biases[1]), ("act", zero, zero, None, half),
+              ("linear", w[0], net.biases[0])]
+    small = np.full(width, 1e-30, np.float32)
+    one = {"layers": layers, "lo": np.zeros(6, np.float32), "hi": np.ones(6, np.float32), "node_abs": [small, small], "beta_signed": [zero, zero]}
+    eng = B200Engine(0)
+    eng.set_path(engine.PATH_TF32X3)
+    eng.set_refine_tolerance(1e30)
+    lo, hi = eng.crown_resnet_beta_batched([one] * D, np.eye(rows, dtype=np.float32))
+    assert (lo == lo[0]).all() and (hi == hi[0]).all()
+    for s in range(rows):
+        terms = [Fraction(float(a)) * Fraction(float(i)) for a, i in zip(w[2][s], icp)]
+        below, above = sum(t for t in terms if t < 0), sum(t for t in terms if t > 0)
+        assert Fraction(float(lo[0, s])) <= below and Fraction(float(hi[0, s])) >= above
+        assert float(lo[0, s]) >= float(below) * (1 + 1e-6) - 1e-30 and float(hi[0, s]) <= float(above) * (1 + 1e-6) + 1e-30
+    eng.close()
