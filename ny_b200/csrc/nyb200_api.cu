@@ -646,7 +646,7 @@ int batch_ptrs(nyb200_engine *e, const Net &net, const Batch &b, BatchPtrs &p) {
     p.flags = (int *)(out_block + 256);
     p.out_lo = (float *)(out_block + 256 + b_ns); p.out_hi = p.out_lo + D * b.S;
     GET(code, signed char *, "code", D * np)
-    GET(sbeta, float *, "sbeta", D * np * 4)
+    GET(sbeta, float *, "sbeta", D * (np + (size_t)nv.L) * 4)   // and beta_max (run_forward) behind it: one fill clears both
     GET(raw_lo, float *, "raw_lo", D * np * 4)
     GET(raw_hi, float *, "raw_hi", D * np * 4)
     GET(q, float *, "q", D * np * 4)
@@ -741,13 +741,9 @@ int run_forward(nyb200_engine *e, Net &net, const Batch &b, BatchPtrs &p, int fw
     p.cj = cj;
     NYB_CUDA(e, cudaMemsetAsync(p.flags, 0, (size_t)D * 4, e->stream));
     NYB_CUDA(e, cudaMemsetAsync(p.code, 0, (size_t)D * np, e->stream));
-    NYB_CUDA(e, cudaMemsetAsync(p.sbeta, 0, (size_t)D * np * 4, e->stream));
-    p.beta_max = nullptr;
-    if (e->path == NYB200_PATH_TF32X3 && fwd_mode < 2 && net.has_conv()) {   // what k_relax_image bounds its rows with
-        p.beta_max = (float *)ws_get(e, "beta_max", (size_t)nv.L * D * 4);
-        if (!p.beta_max) return NYB200_ERR_OOM;
-        NYB_CUDA(e, cudaMemsetAsync(p.beta_max, 0, (size_t)nv.L * D * 4, e->stream));
-    }
+    const bool bounded = e->path == NYB200_PATH_TF32X3 && fwd_mode < 2 && net.has_conv();   // what k_relax_image bounds its rows with
+    NYB_CUDA(e, cudaMemsetAsync(p.sbeta, 0, ((size_t)D * np + (bounded ? (size_t)nv.L * D : 0)) * 4, e->stream));
+    p.beta_max = bounded ? p.sbeta + (size_t)D * np : nullptr;
     if (fwd_mode != 2 && b.max_splits > 0)
         launch_scatter_splits(e, nv, p.splits, p.nsplits, b.max_splits, D, p.code, p.sbeta, p.flags, p.beta_max);
     for (int k = 0; k < nv.L; ++k) {
