@@ -584,15 +584,17 @@ double win_eps(const WinOp &op) {
 // Window form of a convolution layer (kind: the `sel` of k_win_weights).  Leaves out->ok false where it does not apply:
 // strides over 4, weights that do not fit in shared memory next to three halo tiles, and transposed convolutions whose
 // im2col-space product is the faster form.  A tile costs its products whatever part of it lies inside the image, the product
-// space what is written there: the line lies at 650 elements of the space per product step of a tile.  Backward pass, 1024
+// space what is written there: the line lies at 650 elements of the space per product step of a tile.  A call of 1024
 // domains of a classifier of two strided 4x4 convolutions, 8 rows each, us in all; the second one as windows / as products:
-//   16 -> 16 channels, side 32 (1820 elements a step) 1460 / 1612   28 (1394) 1446 / 1654   16 (455) 727 / 686
-//   32 -> 16           side 32 ( 910)                 2017 / 2080   28 ( 697) 2081 / 2176   16 (228) 916 / 796
-//   32 ->  8           side 32 ( 455)                 1873 / 1818   28 ( 348) 1981 / 1929   16 (114) 871 / 706
-//   16 ->  8           side 32 ( 910)                 1334 / 1367   28 ( 697) 1363 / 1375   16 (228) 696 / 597
-// and the first one (3 input channels): side 32 (683) 1612 / 1687, 28 (523) 1651 / 1609, 16 (341) 686 / 627.  Residual blocks
-// lie far on the window's side (64 channels, side 8: 1024 a step, 878 / 1654), a stem of 64 channels on 3 x 32 x 32 on the
-// other (192; 256 domains 49.7 / 48.8 ms).  The forward form has no such cases.
+//   16 -> 16 channels, side 32 (1820 elements a step) 1130 / 1412   28 (1394) 1288 / 1565   16 (455) 593 / 601
+//   32 -> 16           side 32 ( 910)                 1661 / 1875   28 ( 697) 1892 / 2088   16 (228) 742 / 708
+//   32 ->  8           side 32 ( 455)                 1610 / 1671   28 ( 348) 1844 / 1866   16 (114) 711 / 622
+//   16 ->  8           side 32 ( 910)                 1100 / 1225   28 ( 697) 1242 / 1311   16 (228) 566 / 511
+// and the first one (3 input channels): side 32 (683) 1130 / 1333, 28 (523) 1168 / 1285, 16 (341) 601 / 601.  So windows win from
+// some 350 elements on; the line stands where products lost to a window kernel of one issuing warp, and shapes from 350 to 650 are
+// up to 10 % slower a call than they would be as windows.  Residual blocks lie far on the window's side (64 channels, side 8: 1024 a
+// step), and a stem of 64 channels on 3 x 32 x 32 (192) is as fast either way (128 domains of two blocks, 9 rows 10.4 / 10.4 ms).
+// The forward form has no such cases.
 int win_prepare(nyb200_engine *e, const float *W, float wmax, const ConvGeom &g, int kind, WinOp *out, Carve &c) {
     out->ok = false;
     static_assert(sizeof(Params) <= sizeof(out->params), "parameter storage");

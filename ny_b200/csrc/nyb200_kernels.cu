@@ -425,7 +425,10 @@ k_relax_v4(int n, int off, int M, int R, int S, long nps, float *A, int lda, con
 // A warp's columns stay in registers as relax_prepared wants them, and its rows are taken kDomRows at a time, the next ones on
 // their way while these are worked on: a warp that walks one row after the other is latency bound.  (Rows loaded when their
 // turn came, four at a time, and relax_coeff's sums: 55 us for 36864 rows of 512, now 35; their bytes take 27.)
-constexpr int kDomRows = 3;   // nine specification rows are three whole batches
+// Three a batch: nine specification rows are three whole ones.  Other numbers of rows gain less, none loses against rows four at
+// a time, loaded when their turn came: 3000 domains of 5 x 512, us a call, that form / this, 2 rows 796 / 769, 3 812 / 778, 4 921 / 894,
+// 5 1054 / 978, 6 1095 / 1007, 7 1205 / 1129, 8 1297 / 1209, 9 1384 / 1247; 1000 of 5 x 400: 4 453 / 447, 7 550 / 529, 8 559 / 533, 9 579 / 543.
+constexpr int kDomRows = 3;
 struct DomColumns { float4 t[4], zg, cj, bias; float au[4], under; };
 
 template <bool UPPER, bool BIAS>

@@ -26,7 +26,11 @@ namespace nyb {
 namespace {
 
 constexpr int kRows = 64;   // rows whose sums a block holds at a time
-constexpr int kBatch = 3;   // rows in flight together: nine specification rows are three whole batches
+// Rows in flight together: nine specification rows are three whole batches.  Other numbers of rows, us a call, passes of their own /
+// this: 1024 domains of the classifier 1 row 1364 / 1339, 2 1571 / 1438, 4 1978 / 1666, 5 2211 / 1766, 7 2616 / 1990, 8 2870 / 2088,
+// 9 3107 / 2190; 64 of a residual network with two blocks 1 row 6983 / 4335, 3 5424 / 4782, 4 5913 / 5081, 7 7423 / 5813, 8 7855 / 6049,
+// 9 8457 / 6271 (the window convolutions of both sides as they were with that form).
+constexpr int kBatch = 3;
 
 struct ImageArgs {
     int C, plane, Cp, R, S, vec;     // vec: rows are pixel-major, C channels a pixel; otherwise channel planes
@@ -128,7 +132,7 @@ __device__ __forceinline__ void image_batch(const ImageArgs &P, const Batch3<JOI
             *(uint2 *)(lo + u * half_row) = make_uint2(*(const unsigned *)&l0, *(const unsigned *)&l1);
         }
     }
-    // the rows' sums reduced together: each step halves the rows a lane holds (relax_dom_rows)
+    // the rows' sums reduced together: each step halves the rows a lane holds (as relax_dom_batch)
     const bool hi16 = lane & 16, hi8 = lane & 8;
     double b0 = (hi16 ? sb[2] : sb[0]) + __shfl_xor_sync(0xffffffffu, hi16 ? sb[0] : sb[2], 16);
     double b1 = (hi16 ? 0.0 : sb[1]) + __shfl_xor_sync(0xffffffffu, hi16 ? sb[1] : 0.0, 16);
