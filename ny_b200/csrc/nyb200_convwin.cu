@@ -78,7 +78,8 @@ using namespace win;
 // [Wh | Wl] as one product of 128 columns (4.0 thousand), a tile took 12.2 thousand; with converged loops (mbar_wait_warp) 9.7;
 // from two warps with 64-column products, which halve what the epilogue drains and double its buffers, 8.5; with eight epilogue
 // warps instead of sixteen, results pixel-major where the next pass wants them so (the stores were 3.7 thousand of it) and the
-// warp's number shuffled, so that the compiler knows it uniform, 7.1.  All products from one warp: 9.5.
+// warp's number shuffled, so that the compiler knows it uniform, 7.1 (7.3 since both issuing warps follow every slot of the ring).
+// All products from one warp: 9.5.
 template <int KS, int NB>
 __global__ void __launch_bounds__(win::THREADS, 1)
 k_conv_win(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo, const __grid_constant__ CUtensorMap tm_w,
