@@ -57,15 +57,15 @@ __global__ void k_transpose(const float *__restrict__ W, int n_out, int n_in, fl
 
 // Z[d*Zr + s][j] = the box corner row (d, s) concretises on: lower rows (s < S) take x_lo where the coefficient
 // is >= 0, upper rows (S <= s < Zr, present with the dual alpha: Zr = 2S) take x_hi there.
-// A row is a grid row, four columns a thread where it allows that (VEC); with two 64-bit divisions an element 78 us for 18432 rows
-// of 784, so 27.
+// A row is a block's row of threads, four columns a thread where it allows that (VEC); with two 64-bit divisions an element 78 us for
+// 18432 rows of 784, so 27.
 template <bool VEC>
 __global__ void __launch_bounds__(256)
 k_adjoint_seed(long rows, int S, int R, int Zr, int n0, const float *__restrict__ A, int lda, const float *__restrict__ in_lo, const float *__restrict__ in_hi,
                long box_ds, float *__restrict__ Z, int ldz) {
-    const int j = (blockIdx.x * 256 + threadIdx.x) * (VEC ? 4 : 1);
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) * (VEC ? 4 : 1);
     if (j >= n0) return;
-    for (long ds = blockIdx.y; ds < rows; ds += gridDim.y) {
+    for (long ds = (long)blockIdx.y * blockDim.y + threadIdx.y; ds < rows; ds += (long)gridDim.y * blockDim.y) {
         const int d = (int)(ds / Zr), s = (int)(ds - (long)d * Zr);
         const float *a = A + ((long)d * R + s) * lda + j, *l = in_lo + (long)d * box_ds + j, *u = in_hi + (long)d * box_ds + j;
         auto one = [&](float x, float lo, float hi) { return (x >= 0.f) == (s < S) ? lo : hi; };
@@ -506,9 +506,15 @@ int optimize_batch(nyb200_engine *e, const nyb200_opt_config &cfg, float *grad_h
         const int n0 = nv.dims[0];
         const bool four = ((n0 | p.lda | ldz | b.box_stride) & 3) == 0 &&
                           ((reinterpret_cast<uintptr_t>(p.a_final) | reinterpret_cast<uintptr_t>(p.in_lo) | reinterpret_cast<uintptr_t>(p.in_hi) | reinterpret_cast<uintptr_t>(z0)) & 15) == 0;
-        const dim3 seed_grid((unsigned)((n0 + (four ? 1023 : 255)) / (four ? 1024 : 256)), (unsigned)std::min<long>(seeds, 65535));
-        if (four) k_adjoint_seed<true><<<seed_grid, 256, 0, e->stream>>>(seeds, S, R, Zr, n0, p.a_final, p.lda, p.in_lo, p.in_hi, (long)b.box_stride, z0, ldz);
-        else k_adjoint_seed<false><<<seed_grid, 256, 0, e->stream>>>(seeds, S, R, Zr, n0, p.a_final, p.lda, p.in_lo, p.in_hi, (long)b.box_stride, z0, ldz);
+        // a narrow input's rows share a block
+        const int n_seed = four ? n0 / 4 : n0;
+        int sx = 1;
+        while (sx < n_seed && sx < 32) sx *= 2;
+        if (n_seed > 32) sx = std::min(256, (n_seed + 31) / 32 * 32);
+        const int sy = 256 / sx;
+        const dim3 seed_grid((unsigned)((n_seed + sx - 1) / sx), (unsigned)std::min<long>((seeds + sy - 1) / sy, 65535)), seed_block((unsigned)sx, (unsigned)sy);
+        if (four) k_adjoint_seed<true><<<seed_grid, seed_block, 0, e->stream>>>(seeds, S, R, Zr, n0, p.a_final, p.lda, p.in_lo, p.in_hi, (long)b.box_stride, z0, ldz);
+        else k_adjoint_seed<false><<<seed_grid, seed_block, 0, e->stream>>>(seeds, S, R, Zr, n0, p.a_final, p.lda, p.in_lo, p.in_hi, (long)b.box_stride, z0, ldz);
         e->launches++;
         float *zc = z0, *zn = z1;
         // adjoints of relu(pre_k) that a later layer's identity branch still needs, one buffer per open source layer
@@ -537,7 +543,10 @@ int optimize_batch(nyb200_engine *e, const nyb200_opt_config &cfg, float *grad_h
                     break;
                 }
             }
-            const bool two = ((N | nv.pre_off[k] | (int)np | ldz | ldc) & 1) == 0 &&
+            // Two neurons a thread where that leaves 400 threads an SM; with fewer the loads' latency shows.  Ten iterations, one a
+            // thread / two: 170 an SM (394 domains, 7 x 128) 2781 / 2856 us, 200 (300, 5 x 200) 2146 / 2188, 334 (988, 3 x 100) 1600 / 1617,
+            // 346 (200, 9 x 512) 5370 / 5428; 519 (400, 4 x 384) and 519 (600, 4 x 256) as fast either way, from 650 on two are faster.
+            const bool two = (long)D * (N / 2) >= 400L * usable_sms(e) && ((N | nv.pre_off[k] | (int)np | ldz | ldc) & 1) == 0 &&
                              ((reinterpret_cast<uintptr_t>(zn) | reinterpret_cast<uintptr_t>(ckpt[k]) | reinterpret_cast<uintptr_t>(nv.b[k])) & 7) == 0;
             // a narrow layer's domains share a block; a wide one's neurons are spread evenly over its blocks (301 neurons, one a thread: two
             // blocks of 160 and not of 256)

@@ -34,3 +34,9 @@ def test_optimised_bounds_at_odd_and_narrow_widths(width, rows, domains):
     got, want = out[engine.PATH_TF32X3], out[engine.PATH_F64]
     assert np.isfinite(want).all()
     assert (np.abs(got - want) <= 1e-3 * np.maximum(np.abs(want), 0.1 * np.abs(want).max(axis=1, keepdims=True))).all()
+
+
+# 400 threads an SM for pairs of neurons: on 148 of them 59200 threads are the line
+@pytest.mark.parametrize("width,rows,domains", [(64, 1, 1849), (64, 1, 1850), (258, 2, 460)])
+def test_optimised_bounds_on_both_sides_of_the_line_for_pairs(width, rows, domains):
+    test_optimised_bounds_at_odd_and_narrow_widths(width, rows, domains)
