@@ -440,14 +440,26 @@ struct SplitArgs {
     double *rpen;
     const float *q_sum;
 };
-__device__ __forceinline__ float split_value(const SplitArgs &P, int row, int c, int px, long at) {
-    float v = P.A[(long)row * P.lda + at];
-    if (P.bias) {
-        v = fmaxf(v + P.bias[at], 0.f);
-        P.keep[(long)row * P.keep_ld + at] = v;
+enum { SPLIT_PLAIN = 0, SPLIT_BIAS = 1, SPLIT_MASK = 2 };
+// N elements of a row, zero where there is none.  All loads before the first store and without a branch between them: one element
+// behind the other, with both cases looked at each time, they were a chain of that many latencies.  300 images of 64 x 32 x 32 55 us,
+// so 32; 210 of 64 x 16 x 16 13.6 and 8.4; one thread a pixel 210 of 16 x 8 x 8 12.6 and 4.1.
+template <int WITH, int N>
+__device__ __forceinline__ void split_values(const SplitArgs &P, int row, const long (&at)[N], const bool (&in)[N], float (&v)[N]) {
+    const float *a = P.A + (long)row * P.lda, *m = WITH == SPLIT_MASK ? P.mask + (long)row * P.mask_ld : P.bias;
+    float w[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = in[i] ? a[at[i]] : 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = WITH != SPLIT_PLAIN && in[i] ? m[at[i]] : 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        if (WITH == SPLIT_BIAS && in[i]) {
+            v[i] = fmaxf(v[i] + w[i], 0.f);
+            P.keep[(long)row * P.keep_ld + at[i]] = v[i];
+        }
+        if (WITH == SPLIT_MASK && !(w[i] > 0.f)) v[i] = 0.f;
     }
-    if (P.mask && !(P.mask[(long)row * P.mask_ld + at] > 0.f)) v = 0.f;
-    return v;
 }
 __device__ __forceinline__ void split_row(const SplitArgs &P, int row, bool first, float &s) {
     const float m = __uint_as_float(P.row_max[row]), bound = P.more_max > 0.f ? __fadd_ru(m, P.more_max) : m;
@@ -458,6 +470,7 @@ __device__ __forceinline__ void split_row(const SplitArgs &P, int row, bool firs
         if (P.rpen) P.rpen[row] += (3.5527137e-15 * (double)bound + 1e-37) * (double)P.q_sum[row / P.R];
     }
 }
+template <int WITH>
 __global__ void __launch_bounds__(256)
 k_split_image(const __grid_constant__ SplitArgs P) {
     extern __shared__ unsigned s_w[];   // [2][32][Cp / 2 + 1] channel pairs; the odd pitch keeps a warp's writes apart
@@ -467,16 +480,28 @@ k_split_image(const __grid_constant__ SplitArgs P) {
     float s;
     split_row(P, row, blockIdx.y == 0 && threadIdx.x == 0, s);
     const bool in = p0 + lane < plane;
-#pragma unroll 4
-    for (int c2 = warp; c2 < Cp / 2; c2 += 8) {
-        const int c = 2 * c2;
-        const long at = (long)c * plane + p0 + lane;
-        const float v0 = (in && c < C) ? split_value(P, row, c, p0 + lane, at) * s : 0.f, v1 = (in && c + 1 < C) ? split_value(P, row, c + 1, p0 + lane, at + plane) * s : 0.f;
-        const __half2 h = __floats2half2_rn(v0, v1);
-        const float2 hf = __half22float2(h);
-        const __half2 l = __floats2half2_rn((v0 - hf.x) * 2048.f, (v1 - hf.y) * 2048.f);
-        s_w[lane * pitch + c2] = *(const unsigned *)&h;
-        s_w[(32 + lane) * pitch + c2] = *(const unsigned *)&l;
+    for (int first = warp; first < Cp / 2; first += 32) {   // four pairs of channels a thread
+        long at[8];
+        bool has[8];
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int c = 2 * (first + 8 * (i / 2)) + i % 2;
+            at[i] = (long)c * plane + p0 + lane;
+            has[i] = in && c < C;
+        }
+        split_values<WITH>(P, row, at, has, v);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c2 = first + 8 * u;
+            if (c2 >= Cp / 2) break;
+            const float v0 = v[2 * u] * s, v1 = v[2 * u + 1] * s;
+            const __half2 h = __floats2half2_rn(v0, v1);
+            const float2 hf = __half22float2(h);
+            const __half2 l = __floats2half2_rn((v0 - hf.x) * 2048.f, (v1 - hf.y) * 2048.f);
+            s_w[lane * pitch + c2] = *(const unsigned *)&h;
+            s_w[(32 + lane) * pitch + c2] = *(const unsigned *)&l;
+        }
     }
     __syncthreads();
     const int n_px = min(32, plane - p0), vec = Cp / 8;   // 16-byte groups per pixel
@@ -496,21 +521,26 @@ k_split_image(const __grid_constant__ SplitArgs P) {
 }
 
 // The same up to sixteen channels, one thread a pixel: its pairs are 64 bytes, two whole sectors, and need no exchange (1024
-// images of 3 x 32 x 32: 54 -> 20 us, 16 x 16 x 16: 17 -> 9).
+// images of 3 x 32 x 32: 54 -> 22 us, 16 x 16 x 16: 17 -> 10, with bias and ReLU 13, with a mask 14).
+template <int WITH>
 __global__ void __launch_bounds__(256)
 k_split_pixels(const __grid_constant__ SplitArgs P) {
     pdl_trigger();
     pdl_wait();
-    const int row = blockIdx.x, px = blockIdx.y * 256 + threadIdx.x;
+    const int row = blockIdx.x, px = blockIdx.y * blockDim.x + threadIdx.x;
     float s;
     split_row(P, row, px == 0, s);
     if (px >= P.plane) return;
     unsigned h[8], l[8];
+    long from[16];
+    bool has[16];
+    float v[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) { from[c] = (long)c * P.plane + px; has[c] = c < P.C; }
+    split_values<WITH>(P, row, from, has, v);
 #pragma unroll
     for (int c2 = 0; c2 < 8; ++c2) {
-        const int c = 2 * c2;
-        const long at = (long)c * P.plane + px;
-        const float v0 = c < P.C ? split_value(P, row, c, px, at) * s : 0.f, v1 = c + 1 < P.C ? split_value(P, row, c + 1, px, at + P.plane) * s : 0.f;
+        const float v0 = v[2 * c2] * s, v1 = v[2 * c2 + 1] * s;
         const __half2 hh = __floats2half2_rn(v0, v1);
         const float2 hf = __half22float2(hh);
         const __half2 ll = __floats2half2_rn((v0 - hf.x) * 2048.f, (v1 - hf.y) * 2048.f);
@@ -784,10 +814,14 @@ int conv_win(nyb200_engine *e, const WinOp &op, int rows, const float *A, long l
         a.bias = with->bias; a.keep = with->keep; a.keep_ld = (int)with->keep_ld; a.more_max = with->bias ? with->bias_max : 0.f;
         a.mask = with->mask; a.mask_ld = (int)with->mask_ld;
     }
-    if (op.in_cp == 16)
-        NYB_CUDA(e, launch_pdl(k_split_pixels, dim3((unsigned)rows, (unsigned)((plane + 255) / 256)), dim3(256), 0, e, a));
-    else
-        NYB_CUDA(e, launch_pdl(k_split_image, dim3((unsigned)rows, (unsigned)((plane + 31) / 32)), dim3(256), (size_t)64 * (op.in_cp / 2 + 1) * 4, e, a));
+    const bool by_pixel = op.in_cp == 16;
+    const unsigned threads = by_pixel ? (unsigned)std::min(256, (plane + 31) / 32 * 32) : 256;   // (a small image's block is its size)
+    const dim3 grid((unsigned)rows, by_pixel ? (plane + threads - 1) / threads : (unsigned)((plane + 31) / 32));
+    const size_t smem = by_pixel ? 0 : (size_t)64 * (op.in_cp / 2 + 1) * 4;
+    auto split = [&](auto pixels, auto image) { return launch_pdl(by_pixel ? pixels : image, grid, dim3(threads), smem, e, a); };
+    if (a.bias && a.mask) return set_err(e, NYB200_ERR_INTERNAL, "a split with a bias and a mask");
+    NYB_CUDA(e, a.bias ? split(k_split_pixels<SPLIT_BIAS>, k_split_image<SPLIT_BIAS>) : a.mask ? split(k_split_pixels<SPLIT_MASK>, k_split_image<SPLIT_MASK>)
+                                                                                       : split(k_split_pixels<SPLIT_PLAIN>, k_split_image<SPLIT_PLAIN>));
     e->launches++;
     if (report) NYB_CUDA(e, cudaMemsetAsync(row_max, 0, (size_t)rows * 4, e->stream));
     return launch_win(e, op, rows, hi, lo, row_inv, out, ldo, err, pixel_major, report ? row_max : nullptr);
