@@ -115,3 +115,14 @@ def test_a_step_follows_the_gradient(form):
     assert sure.mean() > 0.5
     assert np.array_equal(points[clear & ~better], x[clear & ~better])
     assert np.allclose(points[better][sure[better]], moved[better][sure[better]], rtol=1e-6, atol=1e-5 * step)   # (the step's own rounding)
+
+
+# more than 64 channels: a thread of the split takes several groups of four pairs, the last one not whole
+WIDE = [((2, 10, 9), [(66, *K3), (96, *K3), (130, *K3), (4, *K3)], {}, True), ((3, 8, 8), [(48, *K3), (20, *K3), (100, *K3), (3, *K3)], {}, False)]
+CASES.extend(WIDE)
+
+
+@pytest.mark.parametrize("case", range(len(CASES) - len(WIDE), len(CASES)))
+@pytest.mark.parametrize("rows", [3, 130])
+def test_values_and_gradients_of_many_channels_agree_with_binary64(case, rows):
+    test_values_and_gradients_agree_with_binary64(case, rows)
