@@ -546,7 +546,9 @@ int optimize_batch(nyb200_engine *e, const nyb200_opt_config &cfg, float *grad_h
             // Two neurons a thread where that leaves 400 threads an SM; with fewer the loads' latency shows.  Ten iterations, one a
             // thread / two: 170 an SM (394 domains, 7 x 128) 2781 / 2856 us, 200 (300, 5 x 200) 2146 / 2188, 334 (988, 3 x 100) 1600 / 1617,
             // 346 (200, 9 x 512) 5370 / 5428; 519 (400, 4 x 384) and 519 (600, 4 x 256) as fast either way, from 650 on two are faster.
-            const bool two = (long)D * (N / 2) >= 400L * usable_sms(e) && ((N | nv.pre_off[k] | (int)np | ldz | ldc) & 1) == 0 &&
+            // With dual alpha the upper rows are a longer chain, and the line is twice that: eight iterations, 432 an SM (500, 4 x 256)
+            // 1753 / 1784, 519 (300, 3 x 512) 1417 / 1463, 605 (700, 6 x 256) 2512 / 2580, 865 (1000, 4 x 256) 2822 / 2685, 3459 (2000, 5 x 512) 10990 / 10680.
+            const bool two = (long)D * (N / 2) >= (Zr == S ? 400L : 800L) * usable_sms(e) && ((N | nv.pre_off[k] | (int)np | ldz | ldc) & 1) == 0 &&
                              ((reinterpret_cast<uintptr_t>(zn) | reinterpret_cast<uintptr_t>(ckpt[k]) | reinterpret_cast<uintptr_t>(nv.b[k])) & 7) == 0;
             // a narrow layer's domains share a block; a wide one's neurons are spread evenly over its blocks (301 neurons, one a thread: two
             // blocks of 160 and not of 256)
